@@ -1,0 +1,791 @@
+// Fused window correlation for the planar WIDIM pass (sm_100a).
+//
+// One CTA holds WPC interrogation windows in shared memory and runs, per
+// window, the whole of the reference's per-window chain
+//   load_windows!  (src/correlators.jl:188-263: column-major mean, apodize)
+//   FFT A, FFT B   (packed as one complex transform of A + iB)
+//   spectrum!      (src/correlators.jl:266-279: conj(FA) FB, or filtered phase)
+//   inverse FFT    (normalised by 1/N^2 like FFTW's inv(plan))
+//   fftshift_abs!, overlap gain (src/correlators.jl:282-289, 338-339)
+//   analyze_plane! (src/correlators.jl:459-468: regional-max or exclusion
+//                   peaks with the tie rules of src/localmax.jl:3-19,
+//                   gauss3/gauss9 in FP64, peak ratio, FP64 moment,
+//                   gauss3-refined alternatives)
+// writing the packed scalars of src/ka_backend.jl:497-506 straight into the
+// vector grid. Nothing but images in and scalars out touches HBM.
+//
+// Shared-memory plane layout: element (p, q) (row p, column q) of window w
+// lives at planes[w*N*LD + q*LD + p] with LD = N + 1, so a warp walking
+// either axis with one line per lane is bank-conflict free.
+//
+// The 2-D transform runs each axis as an in-register radix-N1 pass and, for
+// N > 32, a second radix-N2 pass (N = N1*N2). The forward transform leaves
+// frequency k at position N2*(k % N1) + k / N1 along each axis; the spectrum
+// step reads pairs (k, -k) from there and the inverse takes that order back
+// to natural order, so no bit-reversal pass exists anywhere.
+#pragma once
+#include "hh_corr_peaks.cuh"
+
+namespace hh {
+
+// ---------------------------------------------------------------------------
+// W is the extent of the data: the window, or with SRCH the frame-B search
+// area that holds the (runtime) frame-A window at its centre. VAR selects the
+// CTA shape (windows per CTA, threads per window) and register budget (CTAs
+// per SM the registers are sized for) and FFT split among the five the
+// autotuner times: 0 the default shape and budget, 1 the alternative shape,
+// 2 the default shape with one CTA per SM more in the budget (fewer
+// registers, more warps), 3 the default shape with one CTA less (more
+// registers, no spills) -- or, where the default budget is one CTA, the
+// alternative shape with one CTA more. Variants 0-3 compute the same
+// arithmetic on another thread mapping or register allocation, so their
+// results are identical. Variant 4 splits each axis's DFT differently
+// (AxisSplitAlt), so its planes differ from variant 0's by rounding.
+template <int N, int W, bool SRCH = false, int VAR = 0> struct CorrCfg {
+  // variant 4: the alternative FFT split (AxisSplitAlt) in the default shape and budget
+  static constexpr bool ALT = VAR == 4;
+  static constexpr int N1 = ALT ? AxisSplitAlt<N>::N1 : AxisSplit<N>::N1;
+  static constexpr int N2 = ALT ? AxisSplitAlt<N>::N2 : AxisSplit<N>::N2;
+  // budget of the default shape; shape of this variant (0 default, 1 alternative)
+  static constexpr int MINB0 = (N == 32 && W == 16) ? 3 : (N <= 48 ? 4 : (N <= 64 ? 3 : (N <= 96 ? 2 : 1)));
+  static constexpr int SH = (VAR == 1 || (VAR == 3 && MINB0 == 1)) ? 1 : 0;
+  // 16 x 16 windows padded to 32: every stage of the plane has at most 16
+  // lines (16 data columns, 16 canonical column items, 16 row pairs), so
+  // half a warp serves a window and each warp carries two
+  static constexpr bool HALF = SH == 0 && N == 32 && W == 16;
+  // alternatives: N <= 32 one window per warp in CTAs of 4 (half-warp
+  // windows) or 8 warps; N = 48 a 3-CTA register budget; N = 64 one window
+  // per 256-thread CTA; N = 96 512 threads and N = 128 256 threads per window
+  static constexpr int WPC = SH == 0 ? (HALF ? 8 : (N <= 32 ? 4 : (N <= 64 ? 2 : 1)))  // windows per CTA
+                                     : (N <= 32 ? (N == 32 && W == 16 ? 4 : 8) : (N <= 48 ? 2 : 1));
+  static constexpr int NT = SH == 0 ? (N <= 48 ? 128 : (N <= 96 ? 256 : 512))
+                                    : (N <= 32 ? (N == 32 && W == 16 ? 128 : 256)
+                                               : (N <= 48 ? 128 : (N <= 64 ? 256 : (N <= 96 ? 512 : 256))));
+  static constexpr int G = NT / WPC;  // threads per window
+  // CTAs per SM the register budget is sized for
+  static constexpr int MINB_SH = SH == 0 ? MINB0
+                                         : (N <= 32 ? (N == 32 && W == 16 ? 4 : 2) : (N <= 48 ? 3 : (N <= 64 ? 3 : 1)));
+  static constexpr int MINB = VAR == 2 ? MINB0 + 1
+                                       : (VAR == 3 ? (MINB0 > 1 ? MINB0 - 1 : MINB_SH + 1) : MINB_SH);
+  // the peak analysis inline (one window per CTA: its latency is the CTA's)
+  static constexpr bool INLINE_ANALYSIS = N >= 96;
+  // Canonical column c sits at storage column N2 (c % N1) + c / N1, and with
+  // LD = N + 1 a 64-bit element's bank pair is (column + row) mod 16, so with
+  // N2 = 8 consecutive canonical columns (8 storage columns apart) share two
+  // bank pairs. The first inverse pass then walks c = N1 u + v with u
+  // fastest (a model of the pass's addresses: 1088 wavefronts instead of
+  // 2112 for 520 ideal at N = 128, 624 instead of 912 for 296 at N = 96).
+  static constexpr bool SPREAD7 = N2 == 8;
+  // The spectrum is Hermitian, so the inverse transforms only the N/2 + 1
+  // canonical columns along p and then rows p and p + N/2 together along q
+  // (their outputs are real: one lands in the real part, one in the
+  // imaginary part). Every window is transformed on its own.
+  static constexpr int NC = N / 2 + 1;
+  static constexpr int IPT = ((N / 2) * N2 + G - 1) / G;  // final inverse items per thread
+  static constexpr int LD = N + 1;    // complex plane leading dimension (float2)
+  static constexpr int LDR = N + 1;   // real plane leading dimension (float), overlays the complex plane
+  static constexpr bool PADDED = (W * 2 == N);
+  static constexpr int NZ1 = PADDED ? (W / N2) : N1;  // nonzero inputs of a forward pass-A line
+
+  static constexpr int EPT = (W * W + G - 1) / G;             // window pixels per thread
+  static constexpr int NPART = SRCH ? 4 : 3;  // FP64 partial sums per warp: A, B, count (and count of B)
+  // plane stride in float2; the two windows of a half-warp pair start 16
+  // banks apart, so their 32-bit plane accesses (peak scan, real-plane
+  // writes) do not meet in one bank
+  static constexpr int PS = N * LD + (HALF ? 8 : 0);
+  static constexpr size_t PLANE_B = (size_t)PS * sizeof(float2);
+  static constexpr size_t BASE_B = WPC * PLANE_B + WPC * (G / 32) * NPART * sizeof(double) + N * sizeof(float2) +
+                                   WPC * (G / 32) * 2 * KMAX * sizeof(uint32_t) +
+                                   WPC * (KMAX * sizeof(float) + 2 * KMAX * sizeof(int)) + 3 * N * sizeof(int) + 64;
+  // CTAs per SM that shared memory allows (228 KB per SM, 1 KB of it
+  // reserved per CTA), capped by the register budget
+  static constexpr int occ(size_t b) {
+    return (int)((228 * 1024) / (b + 1024)) < MINB ? (int)((228 * 1024) / (b + 1024)) : MINB;
+  }
+  // The overlap gain table (N x N) is read by every window; from global
+  // memory its L1 lines are flushed by the window pixels (it took a third of
+  // the last inverse pass at 32 points, half of it at 128). It goes to shared
+  // memory where that costs no CTA per SM: every size but 64 points. (The
+  // apodization window in shared memory as well was no faster.)
+  // Where the full table would cost a CTA (64 points), its quarter does not:
+  // the gain of a symmetric apodization depends only on |lag| along each
+  // axis, and the table builder appends the quarter when that holds exactly.
+  static constexpr size_t GAIN_B = (size_t)N * N * sizeof(float);
+  static constexpr size_t GQ_B = (size_t)(N / 2 + 1) * (N / 2 + 1) * sizeof(float);
+  static constexpr bool GSM = occ(BASE_B + GAIN_B) >= occ(BASE_B);
+  static constexpr bool QSM = !GSM && occ(BASE_B + GQ_B) >= occ(BASE_B);
+  static constexpr size_t smem() { return BASE_B + (GSM ? GAIN_B : (QSM ? GQ_B : 0)); }
+  static_assert(W == N || 2 * W == N, "window must equal the FFT size or half of it");
+  static_assert((G >= 32 && G % 32 == 0) || G == 16, "a window group is whole warps or half a warp");
+  static_assert(N * LDR <= 2 * N * LD, "real plane must fit in the complex plane");
+};
+
+template <int N, int W, bool SRCH, int VAR>
+__global__ void __launch_bounds__(CorrCfg<N, W, SRCH, VAR>::NT, CorrCfg<N, W, SRCH, VAR>::MINB)
+    correlate_kernel(const CorrArgs a) {
+  using C = CorrCfg<N, W, SRCH, VAR>;
+  constexpr int WPC = C::WPC, NT = C::NT, LD = C::LD, LDR = C::LDR, N1 = C::N1, N2 = C::N2, IPT = C::IPT;
+  constexpr int G = C::G, EPT = C::EPT, NC = C::NC, H = N / 2;
+  constexpr int PS = C::PS;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  float2* planes = reinterpret_cast<float2*>(smem_raw);
+  double* s_part = reinterpret_cast<double*>(smem_raw + WPC * C::PLANE_B);  // NPART per warp
+  float2* tw = reinterpret_cast<float2*>(s_part + WPC * (G / 32) * C::NPART);
+  uint32_t* red = reinterpret_cast<uint32_t*>(tw + N);
+  float* s_vals = reinterpret_cast<float*>(red + WPC * (G / 32) * 2 * KMAX);
+  int* s_locs = reinterpret_cast<int*>(s_vals + WPC * KMAX);
+  // per-axis storage tables (N2 > 1): frequency of storage slot a, storage
+  // slot of the negated frequency, canonical storage columns kq = 0..N/2
+  int* s_freq = reinterpret_cast<int*>(s_locs + WPC * 2 * KMAX);
+  int* s_neg = s_freq + N;
+  int* s_canon = s_neg + N;
+  float* s_gain = reinterpret_cast<float*>(s_canon + N);  // N x N when C::GSM
+
+  const int tid = threadIdx.x;
+  const int K = a.npeaks > 2 ? a.npeaks : 2;
+  if (C::GSM && a.gain)
+    for (int m = tid; m < N * N; m += NT) s_gain[m] = a.gain[m];
+  // the quarter table (word N^2 of the gain buffer says whether it follows)
+  const bool gq = C::QSM && a.gain && a.gain[N * N] != 0.f;
+  if (gq)
+    for (int m = tid; m < (N / 2 + 1) * (N / 2 + 1); m += NT) s_gain[m] = a.gain[N * N + 1 + m];
+
+  if (N2 > 1) {
+    for (int m = tid; m < N; m += NT) {
+      double sn, cs;
+      sincospi(-2.0 * (double)m / (double)N, &sn, &cs);
+      tw[m] = make_float2((float)cs, (float)sn);  // W_N^m = exp(-2 pi i m / N)
+    }
+    for (int q = tid; q < N; q += NT) {
+      const int k = q / N2 + N1 * (q % N2);  // storage slot q holds frequency k
+      const int m = (N - k) % N;
+      s_freq[q] = k;
+      s_neg[q] = N2 * (m % N1) + m / N1;
+      if (q <= N / 2) s_canon[q] = N2 * (q % N1) + q / N1;
+    }
+  }
+  __syncthreads();  // the only CTA-wide barrier: from here on the window groups run independently
+
+  // Thread group w (G threads, named barrier w + 1) owns plane w and walks
+  // its own sequence of jobs; a group waits only for itself.
+  const int w = tid / G, gt = tid % G, lane = tid & 31, gw = gt >> 5;
+  const int bar = WPC == 1 ? 0 : w + 1;
+  float2* P = planes + w * PS;
+  float* Rw = reinterpret_cast<float*>(P);  // real plane, overlays the complex one after stage 8
+  double* part = s_part + w * (G / 32) * C::NPART;
+  const float scale = 1.0f / (float)(N * N);
+  // fftshifted rows / columns that can hold a nonzero correlation value (the
+  // support of the overlap gain; the whole plane without padding)
+  const int blo = a.box_hi > 0 ? a.box_lo : 0, bhi = a.box_hi > 0 ? a.box_hi : N - 1;
+  const ScanPlan sp = scan_plan(tid % G, G, blo, bhi, blo, bhi);
+  PeakOut po{a.du, a.dv, a.ratio, a.moment, a.alt_u, a.alt_v, a.nalt, a.G, a.packed, a.locs};
+
+  for (int64_t job = (int64_t)blockIdx.x * WPC + w; job < a.njobs; job += (int64_t)gridDim.x * WPC) {
+    // ---- the window's source (every thread of the group reads the same
+    //      descriptor words; they are broadcast from L1)
+    int rs, cs;
+    const float* A = a.A;
+    const float* B = a.B;
+    const uint8_t* M = a.mask;
+    int64_t ld = a.ld, gid;
+    PeakOut pw = po;
+    if (a.bp) {
+      const int p = a.jobs[4 * job];
+      const BPair& b = a.bp[p];
+      const int gij = a.jobs[4 * job + 1];
+      const int64_t cell = (int64_t)(gij & 0xFFFF) + (int64_t)(gij >> 16) * b.ny;
+      // pairs that converged or have no further sweep, and masked cells, are skipped
+      if (!bp_live(b, a.it, a.done, p) || (b.gmask && b.gmask[cell])) {
+        if (a.rec && a.finder == 0 && gt == 0) a.rec[job] = __int_as_float(-1);  // no record for the epilogue
+        continue;
+      }
+      rs = a.jobs[4 * job + 2];
+      cs = a.jobs[4 * job + 3];
+      const bool warped = a.it > 1 || b.has_pred0;
+      A = warped ? b.warpA : b.A;
+      B = warped ? b.warpB : b.B;
+      M = b.mask;
+      ld = b.nr;
+      gid = b.goff + cell;
+      pw.G = (int64_t)b.ny * b.nx;
+      pw.nalt = b.nalt;
+      pw.alt_u = a.alt_u ? a.alt_u + b.aoff - b.goff : nullptr;  // indexed by gid + m*G
+      pw.alt_v = a.alt_v ? a.alt_v + b.aoff - b.goff : nullptr;
+    } else {
+      rs = a.jobs[4 * job + 2];
+      cs = a.jobs[4 * job + 3];
+      gid = (int64_t)a.jobs[4 * job] + (int64_t)a.jobs[4 * job + 1] * a.ny;
+    }
+    // ---- stages 1-3: the group loads the window's pixels (coalesced down
+    //      the columns), reduces the window means in FP64, and stores
+    //      apod * (x - mean) into the plane; masked pixels enter as zero and
+    //      leave the mean (load_windows!, src/correlators.jl:188-263). The
+    //      mean is the exact sum over n rounded once, where the reference
+    //      folds in Float32 left to right; the two differ by a few ulp.
+    bool bad;
+    if constexpr (SRCH) {
+      // enlarged search area (load_windows!, src/correlators.jl:229-262):
+      // the W x W frame-B area starts (W - win) / 2 before the window on
+      // both axes; frame A enters only inside the centred window, apodized
+      // and less its own mean, frame B everywhere, less its mean, without
+      // apodization; a masked pixel is zero in both and leaves both means
+      const int wa = a.win, oa = (W - wa) / 2;
+      const int64_t r0 = rs - oa, c0 = cs - oa;
+      float2 z[EPT];
+      bool mk[EPT];
+      double sa = 0.0, sb = 0.0, na = 0.0, nb = 0.0;
+#pragma unroll
+      for (int i = 0; i < EPT; ++i) {
+        const int e = gt + i * G;
+        z[i] = make_float2(0.f, 0.f);
+        mk[i] = true;
+        if (e < W * W) {
+          const int p = e % W, q = e / W;
+          const bool ina = (unsigned)(p - oa) < (unsigned)wa && (unsigned)(q - oa) < (unsigned)wa;
+          const int64_t off = (r0 + p) + (c0 + q) * ld;
+          z[i] = make_float2(ina ? ld_stream(A + off) : 0.f, ld_stream(B + off));
+          mk[i] = M ? ld_stream(M + off) != 0 : false;
+          if (!mk[i]) {
+            sb += (double)z[i].y;
+            nb += 1.0;
+            if (ina) {
+              sa += (double)z[i].x;
+              na += 1.0;
+            }
+          }
+        }
+      }
+      const unsigned gm = grp_mask(G);
+#pragma unroll
+      for (int o = (G < 32 ? G : 32) / 2; o > 0; o >>= 1) {
+        sa += __shfl_xor_sync(gm, sa, o);
+        sb += __shfl_xor_sync(gm, sb, o);
+        na += __shfl_xor_sync(gm, na, o);
+        nb += __shfl_xor_sync(gm, nb, o);
+      }
+      double ta = sa, tb = sb, tna = na, tnb = nb;
+      if (G > 32) {
+        if (lane == 0) {
+          part[4 * gw] = sa;
+          part[4 * gw + 1] = sb;
+          part[4 * gw + 2] = na;
+          part[4 * gw + 3] = nb;
+        }
+        grp_sync(bar, G);
+        ta = tb = tna = tnb = 0.0;
+        for (int k = 0; k < G / 32; ++k) {
+          ta += part[4 * k];
+          tb += part[4 * k + 1];
+          tna += part[4 * k + 2];
+          tnb += part[4 * k + 3];
+        }
+      }
+      const float ma = tna > 0 ? (float)(ta / tna) : 0.f, mb = tnb > 0 ? (float)(tb / tnb) : 0.f;
+      bad = !(isfinite(ta) && isfinite(tb));
+#pragma unroll
+      for (int i = 0; i < EPT; ++i) {
+        const int e = gt + i * G;
+        if (e < W * W) {
+          const int p = e % W, q = e / W;
+          const bool ina = (unsigned)(p - oa) < (unsigned)wa && (unsigned)(q - oa) < (unsigned)wa;
+          float2 v = make_float2(0.f, 0.f);
+          if (!(mk[i] || bad)) {
+            v.y = z[i].y - mb;
+            if (ina) v.x = ld_keep(a.apod + (p - oa) + (q - oa) * wa) * (z[i].x - ma);
+          }
+          P[q * LD + p] = v;
+        }
+      }
+    } else {
+      float2 z[EPT];
+      bool mk[EPT];
+      double sa = 0.0, sb = 0.0, cnt = 0.0;
+#pragma unroll
+      for (int i = 0; i < EPT; ++i) {
+        const int e = gt + i * G;
+        z[i] = make_float2(0.f, 0.f);
+        mk[i] = true;
+        if (e < W * W) {
+          const int p = e % W, q = e / W;
+          const int64_t off = (int64_t)(rs + p) + (int64_t)(cs + q) * ld;
+          z[i] = make_float2(ld_stream(A + off), ld_stream(B + off));
+          mk[i] = M ? ld_stream(M + off) != 0 : false;
+          if (!mk[i]) {
+            sa += (double)z[i].x;
+            sb += (double)z[i].y;
+            cnt += 1.0;
+          }
+        }
+      }
+      const unsigned gm = grp_mask(G);
+#pragma unroll
+      for (int o = (G < 32 ? G : 32) / 2; o > 0; o >>= 1) {
+        sa += __shfl_xor_sync(gm, sa, o);
+        sb += __shfl_xor_sync(gm, sb, o);
+        cnt += __shfl_xor_sync(gm, cnt, o);
+      }
+      double ta = sa, tb = sb, tn = cnt;
+      if (G > 32) {
+        if (lane == 0) {
+          part[3 * gw] = sa;
+          part[3 * gw + 1] = sb;
+          part[3 * gw + 2] = cnt;
+        }
+        grp_sync(bar, G);
+        ta = tb = tn = 0.0;
+        for (int k = 0; k < G / 32; ++k) {
+          ta += part[3 * k];
+          tb += part[3 * k + 1];
+          tn += part[3 * k + 2];
+        }
+      }
+      const float ma = tn > 0 ? (float)(ta / tn) : 0.f, mb = tn > 0 ? (float)(tb / tn) : 0.f;
+      bad = !(isfinite(ta) && isfinite(tb));  // the window holds NaN or Inf
+#pragma unroll
+      for (int i = 0; i < EPT; ++i) {
+        const int e = gt + i * G;
+        if (e < W * W) {
+          const int p = e % W, q = e / W;
+          const float ap = ld_keep(a.apod + e);
+          P[q * LD + p] = (mk[i] || bad) ? make_float2(0.f, 0.f) : make_float2(ap * (z[i].x - ma), ap * (z[i].y - mb));
+        }
+      }
+    }
+    grp_sync(bar, G);
+
+    // ---- stage 4: forward transform along p (only the W data columns)
+    for (int it = gt; it < W * N2; it += G) {
+      const int q = it % W, n2 = it / W;
+      float2* L = P + q * LD;
+      float2 x[N1];
+#pragma unroll
+      for (int n1 = 0; n1 < N1; ++n1) x[n1] = n1 < C::NZ1 ? L[N2 * n1 + n2] : make_float2(0.f, 0.f);
+      RDFT<N1, false>::run(x, C::NZ1);
+      if (N2 > 1) {
+#pragma unroll
+        for (int k1 = 1; k1 < N1; ++k1) x[k1] = cmul(x[k1], tw[(n2 * k1) % N]);
+      }
+#pragma unroll
+      for (int k1 = 0; k1 < N1; ++k1) L[N2 * k1 + n2] = x[k1];
+    }
+    if (N2 > 1) {
+      grp_sync(bar, G);
+      for (int it = gt; it < W * N1; it += G) {
+        const int q = it % W, k1 = it / W;
+        float2* L = P + q * LD + N2 * k1;
+        float2 x[N2];
+#pragma unroll
+        for (int n2 = 0; n2 < N2; ++n2) x[n2] = L[n2];
+        RDFT<N2, false>::run(x, N2);
+#pragma unroll
+        for (int k2 = 0; k2 < N2; ++k2) L[k2] = x[k2];
+      }
+    }
+    grp_sync(bar, G);
+    // ---- stage 5: forward transform along q for every row p
+    for (int it = gt; it < N * N2; it += G) {
+      const int p = it % N, n2 = it / N;
+      float2* L = P + p;
+      float2 x[N1];
+#pragma unroll
+      for (int n1 = 0; n1 < N1; ++n1) x[n1] = n1 < C::NZ1 ? L[(N2 * n1 + n2) * LD] : make_float2(0.f, 0.f);
+      RDFT<N1, false>::run(x, C::NZ1);
+      if (N2 > 1) {
+#pragma unroll
+        for (int k1 = 1; k1 < N1; ++k1) x[k1] = cmul(x[k1], tw[(n2 * k1) % N]);
+      }
+#pragma unroll
+      for (int k1 = 0; k1 < N1; ++k1) L[(N2 * k1 + n2) * LD] = x[k1];
+    }
+    if (N2 > 1) {
+      grp_sync(bar, G);
+      for (int it = gt; it < N * N1; it += G) {
+        const int p = it % N, k1 = it / N;
+        float2* L = P + p + (N2 * k1) * LD;
+        float2 x[N2];
+#pragma unroll
+        for (int n2 = 0; n2 < N2; ++n2) x[n2] = L[n2 * LD];
+        RDFT<N2, false>::run(x, N2);
+#pragma unroll
+        for (int k2 = 0; k2 < N2; ++k2) L[k2 * LD] = x[k2];
+      }
+    }
+    grp_sync(bar, G);
+    // ---- stages 6-7: cross-power (or filtered phase) spectrum over Hermitian
+    //      pairs (k, -k) and the inverse along p, on the canonical columns
+    //      kq = 0..N/2 only (frequencies in storage order for N2 > 1, natural
+    //      order otherwise); the conjugate column -kq is then filled in as
+    //      conj of column kq. (i) The two self-paired columns (kq = 0, N/2)
+    //      pair rows within the column: their spectrum is formed first, in
+    //      place (for N <= 32 every canonical column is done here: folding
+    //      the spectrum into the single-pass inverse costs more registers
+    //      than the separate pass costs time).
+    if constexpr (N2 == 1 && G <= N && N % G == 0) {
+      // each thread owns rows ap = gt + j G (j < N / G) of every canonical
+      // column; the columns are unrolled, so every address is the row's base
+      // plus a constant, and CB columns' operands are loaded before any of
+      // their results is stored (no item reads a cell another item writes:
+      // column -c is read only, and a self-paired column's rows ap and -ap
+      // belong to one item)
+      constexpr int RPT = G <= N ? N / G : 1, CB = RPT >= 2 ? 2 : 4;
+      int ra[RPT], rb[RPT];
+#pragma unroll
+      for (int j = 0; j < RPT; ++j) {
+        ra[j] = gt + j * G;
+        rb[j] = (N - ra[j]) % N;
+      }
+#pragma unroll
+      for (int c0 = 0; c0 < NC; c0 += CB) {
+        float2 xa[CB][RPT], xb[CB][RPT];
+        float wk[CB][RPT];
+#pragma unroll
+        for (int u = 0; u < CB; ++u) {
+          const int c = c0 + u, cb = (N - c) % N;
+          if (c < NC) {
+#pragma unroll
+            for (int j = 0; j < RPT; ++j) {
+              if (c == cb && ra[j] > rb[j]) continue;  // a self pair is done by its upper row
+              xa[u][j] = P[c * LD + ra[j]];
+              xb[u][j] = P[cb * LD + rb[j]];
+              wk[u][j] = a.method == 1 ? ld_keep(a.phasew + c * N + ra[j]) : 1.f;
+            }
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < CB; ++u) {
+          const int c = c0 + u, cb = (N - c) % N;
+          if (c < NC) {
+#pragma unroll
+            for (int j = 0; j < RPT; ++j) {
+              if (c == cb && ra[j] > rb[j]) continue;
+              const float2 S = cross_spectrum(xa[u][j], xb[u][j], a.method, wk[u][j]);
+              P[c * LD + ra[j]] = S;
+              if (c == cb) P[c * LD + rb[j]] = make_float2(S.x, -S.y);
+            }
+          }
+        }
+      }
+    } else if constexpr (N2 == 1) {
+      // items (row ap, canonical column c) in batches of SB per thread: the
+      // batch's operands are loaded before any of its results is stored (no
+      // item reads a cell another item writes: column -c is read only, and a
+      // self-paired column's rows ap and -ap belong to one item)
+      constexpr int SB = 4, NIT = NC * N;  // (batches of 8 were slower: registers)
+#pragma unroll 1
+      for (int it0 = gt; it0 < NIT; it0 += SB * G) {
+        float2 xa[SB], xb[SB];
+        int ia[SB], ib[SB];
+        bool on[SB], self[SB];
+        float wk[SB];
+#pragma unroll
+        for (int u = 0; u < SB; ++u) {
+          const int it = it0 + u * G;
+          const int ap = it % N, c = it / N, bq = (N - c) % N, bp = (N - ap) % N;
+          self[u] = c == bq;
+          on[u] = it < NIT && !(self[u] && ap > bp);  // a self pair is done by its upper row
+          ia[u] = c * LD + ap;
+          ib[u] = bq * LD + bp;
+          wk[u] = on[u] && a.method == 1 ? ld_keep(a.phasew + c * N + ap) : 1.f;
+          if (on[u]) {
+            xa[u] = P[ia[u]];
+            xb[u] = P[ib[u]];
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < SB; ++u)
+          if (on[u]) {
+            const float2 S = cross_spectrum(xa[u], xb[u], a.method, wk[u]);
+            P[ia[u]] = S;
+            if (self[u]) P[ib[u]] = make_float2(S.x, -S.y);
+          }
+      }
+    } else {
+      // the two self-paired columns kq = 0 and N/2 (storage order)
+#pragma unroll 1
+      for (int it = gt; it < 2 * N; it += G) {
+        const int ap = it % N, c = (it / N) * H;
+        const int aq = s_canon[c], bp = s_neg[ap], kp = s_freq[ap];
+        if (ap > bp) continue;  // its partner row does this pair
+        const float wk = a.method == 1 ? ld_keep(a.phasew + c * N + kp) : 1.f;
+        const float2 S = cross_spectrum(P[aq * LD + ap], P[aq * LD + bp], a.method, wk);
+        P[aq * LD + ap] = S;
+        P[aq * LD + bp] = make_float2(S.x, -S.y);
+      }
+    }
+    grp_sync(bar, G);
+    //      (ii) for N > 32 every other canonical column forms its spectrum
+    //      while it is read for its first inverse pass; its partner column
+    //      -kq is read only by it, and written only after the pass.
+    if (N2 > 1) {
+#pragma unroll 1
+      for (int it = gt; it < NC * N1; it += G) {
+        int c, k1;
+        if (C::SPREAD7) {  // c = N1 u + v with u fastest, then v, then k1; c = N/2 last
+          if (it < H * N1) {
+            constexpr int U = N2 / 2 > 0 ? N2 / 2 : 1;
+            const int u = it % U, w = it / U;
+            c = N1 * u + w % N1;
+            k1 = w / N1;
+          } else {
+            c = H;
+            k1 = it - H * N1;
+          }
+        } else {
+          c = it % NC;
+          k1 = it / NC;
+        }
+        const int aq = s_canon[c], bq = s_neg[aq];
+        float2* L = P + aq * LD + N2 * k1;
+        const float2* Lb = P + bq * LD;
+        // slot N2 k1 + k2 holds frequency k1 + N1 k2; its negation sits at
+        // slot N2 (N1 - k1) + N2 - 1 - k2 (k1 > 0), or N2 - k2 (k1 = 0, k2 > 0),
+        // or 0: the row base is per item, the offsets constants
+        const int nb0 = k1 == 0 ? N2 : N2 * (N1 - k1) + N2 - 1;
+        float2 x[N2];
+#pragma unroll
+        for (int k2 = 0; k2 < N2; ++k2) {
+          x[k2] = L[k2];
+          if (aq != bq) {
+            const int neg = (k1 == 0 && k2 == 0) ? 0 : nb0 - k2;
+            const float wk = a.method == 1 ? ld_keep(a.phasew + c * N + k1 + N1 * k2) : 1.f;
+            x[k2] = cross_spectrum(x[k2], Lb[neg], a.method, wk);
+          }
+        }
+        RDFT<N2, true>::run(x, N2);
+#pragma unroll
+        for (int n2 = 1; n2 < N2; ++n2) {
+          const float2 t = tw[(n2 * k1) % N];
+          x[n2] = cmul(x[n2], make_float2(t.x, -t.y));
+        }
+#pragma unroll
+        for (int n2 = 0; n2 < N2; ++n2) L[n2] = x[n2];
+      }
+      grp_sync(bar, G);
+    }
+#pragma unroll 1
+    //      With N2 = 1 the two self-paired columns kq = 0 and N/2, whose
+    //      results are real, share one transform as col0 + i col(N/2) (real
+    //      part: column 0, imaginary part: column N/2): H items in all.
+    //      With N2 > 1 consecutive threads take consecutive n2 of one column
+    //      (the canonical columns sit N2 storage columns apart, which alias
+    //      to two banks; rows n2 of one column do not).
+    for (int it = gt; it < (N2 == 1 ? H : NC * N2); it += G) {
+      const bool pk = N2 == 1 && it == 0;
+      const int c = N2 == 1 ? it : it / N2, n2 = N2 == 1 ? 0 : it % N2;
+      const int aq = N2 == 1 ? c : s_canon[c];
+      const int bq = pk ? H : (N2 == 1 ? N - c : s_neg[aq]);
+      float2* L = P + aq * LD;
+      float2* Lb = P + bq * LD;
+      float2 x[N1];
+#pragma unroll
+      for (int k1 = 0; k1 < N1; ++k1) {
+        const float2 u = L[N2 * k1 + n2];
+        if (pk) {
+          const float2 v = Lb[k1];
+          x[k1] = make_float2(u.x - v.y, u.y + v.x);
+        } else {
+          x[k1] = u;
+        }
+      }
+      RDFT<N1, true>::run(x, N1);
+#pragma unroll
+      for (int n1 = 0; n1 < N1; ++n1) {
+        if (pk) {
+          L[n1] = make_float2(x[n1].x, 0.f);
+          Lb[n1] = make_float2(x[n1].y, 0.f);
+        } else {
+          L[N2 * n1 + n2] = x[n1];
+          if (bq != aq) Lb[N2 * n1 + n2] = make_float2(x[n1].x, -x[n1].y);
+        }
+      }
+    }
+    grp_sync(bar, G);
+    // ---- stage 8: inverse along q for the rows R needs: fftshifted rows
+    //      blo..bhi (the overlap gain is zero on every other row, so R is
+    //      exactly 0 there), taken in pairs (blo + t, blo + t + nh) packed as
+    //      T(p) + i T(p'). The normalised, gain-weighted magnitudes are held
+    //      in registers across a barrier, then written as the real plane R
+    //      over the complex one; the other rows are written as zeros.
+    const int nb = bhi - blo + 1, nh = (nb + 1) / 2;
+    if (N2 > 1) {
+#pragma unroll 1
+      for (int it = gt; it < H * N1; it += G) {  // items (t, k1) at it = t + H k1, t < nh used
+        const int t = it % H, k1 = it / H;
+        if (t >= nh) continue;
+        const bool hasb = t + nh < nb;
+        const int pa = (blo + t + H) % N, pb = hasb ? (blo + t + nh + H) % N : pa;
+        float2* La = P + pa + (N2 * k1) * LD;
+        const float2* Lb = P + pb + (N2 * k1) * LD;
+        float2 x[N2];
+#pragma unroll
+        for (int k2 = 0; k2 < N2; ++k2) {
+          const float2 u = La[k2 * LD];
+          const float2 v = hasb ? Lb[k2 * LD] : make_float2(0.f, 0.f);
+          x[k2] = make_float2(u.x - v.y, u.y + v.x);
+        }
+        RDFT<N2, true>::run(x, N2);
+#pragma unroll
+        for (int n2 = 1; n2 < N2; ++n2) {
+          const float2 tt = tw[(n2 * k1) % N];
+          x[n2] = cmul(x[n2], make_float2(tt.x, -tt.y));
+        }
+#pragma unroll
+        for (int n2 = 0; n2 < N2; ++n2) La[n2 * LD] = x[n2];
+      }
+      grp_sync(bar, G);
+    }
+    {
+      float rv[IPT][2][N1];
+#pragma unroll
+      for (int i = 0; i < IPT; ++i) {
+        const int it = gt + i * G;  // items (t, n2) at it = t + H n2, t < nh used
+        if (it < H * N2 && it % H < nh) {
+          const int t = it % H, n2 = it / H;
+          const bool hasb = t + nh < nb;
+          const int pa = (blo + t + H) % N, pb = hasb ? (blo + t + nh + H) % N : pa;
+          const float2* La = P + pa;
+          const float2* Lb = P + pb;
+          float2 x[N1];
+#pragma unroll
+          for (int k1 = 0; k1 < N1; ++k1) {
+            if (N2 == 1) {
+              const float2 u = La[k1 * LD];
+              const float2 v = hasb ? Lb[k1 * LD] : make_float2(0.f, 0.f);
+              x[k1] = make_float2(u.x - v.y, u.y + v.x);
+            } else {
+              x[k1] = La[(N2 * k1 + n2) * LD];
+            }
+          }
+          RDFT<N1, true>::run(x, N1);
+          const int ps0 = blo + t, ps1 = blo + t + nh;  // fftshifted rows of pa and pb
+#pragma unroll
+          for (int n1 = 0; n1 < N1; ++n1) {
+            const int qs = (N2 * n1 + n2 + H) % N;
+            float r0 = fabsf(x[n1].x) * scale, r1 = fabsf(x[n1].y) * scale;
+            if (a.gain) {
+              if (C::GSM) {
+                r0 *= s_gain[qs * N + ps0];
+                r1 *= hasb ? s_gain[qs * N + ps1] : 0.f;
+              } else if (gq) {
+                const int bq = abs(qs - H) * (H + 1);
+                r0 *= s_gain[abs(ps0 - H) + bq];
+                r1 *= hasb ? s_gain[abs(ps1 - H) + bq] : 0.f;
+              } else {
+                r0 *= ld_keep(a.gain + qs * N + ps0);
+                r1 *= hasb ? ld_keep(a.gain + qs * N + ps1) : 0.f;
+              }
+            }
+            if (SRCH && (qs < blo || qs > bhi)) r0 = r1 = 0.f;  // lags outside the search range
+            rv[i][0][n1] = r0;
+            rv[i][1][n1] = r1;
+          }
+        }
+      }
+      grp_sync(bar, G);
+#pragma unroll
+      for (int i = 0; i < IPT; ++i) {
+        const int it = gt + i * G;
+        if (it < H * N2 && it % H < nh) {
+          const int t = it % H, n2 = it / H;
+          const bool hasb = t + nh < nb;
+          const int ps0 = blo + t, ps1 = blo + t + nh;
+#pragma unroll
+          for (int n1 = 0; n1 < N1; ++n1) {
+            const int qs = (N2 * n1 + n2 + H) % N;
+            Rw[qs * LDR + ps0] = rv[i][0][n1];
+            if (hasb) Rw[qs * LDR + ps1] = rv[i][1][n1];
+          }
+        }
+      }
+      const int nz = N - nb;  // rows outside [blo, bhi]
+      for (int j = gt; j < nz; j += G) {
+        const int ps = j < blo ? j : j + nb;
+#pragma unroll 4
+        for (int qs = 0; qs < N; ++qs) Rw[qs * LDR + ps] = 0.f;
+      }
+    }
+    grp_sync(bar, G);
+    if (a.planes) {
+      float* dst = a.planes + job * (int64_t)(N * N);
+      for (int it = gt; it < N * N; it += G) {
+        const int p = it % N, q = it / N;
+        const float r = Rw[q * LDR + p];
+        // ensemble: per-pair planes summed in pair order; a window with
+        // non-finite data poisons its sum as the reference's NaN plane does
+        const float rr = bad ? __int_as_float(0x7fc00000) : r;
+        dst[q * N + p] = a.accumulate ? dst[q * N + p] + rr : rr;
+      }
+      if (a.accumulate) {  // ensemble planes are analysed once, after the last pair
+        grp_sync(bar, G);
+        continue;
+      }
+    }
+    // ---- stage 9: peak analysis by the group (the output pointers are
+    //      needed only when the outputs are formed here, not from a record)
+    const bool defer = a.rec && a.finder == 0;
+    uint32_t* gred = red + w * (G / 32) * 2 * KMAX;
+    if (C::INLINE_ANALYSIS && K <= 4)
+      analyze_body<4, false>(Rw, N, N, LDR, K, a.npeaks, a.finder, a.subpixel, gt, G, gred, true, s_vals + w * KMAX,
+                      s_locs + w * 2 * KMAX, gid, job, defer ? nullptr : &pw, bad, bar, sp, a.rec, a.njobs);
+    else if (C::INLINE_ANALYSIS)
+      analyze_body<KMAX, false>(Rw, N, N, LDR, K, a.npeaks, a.finder, a.subpixel, gt, G, gred, true, s_vals + w * KMAX,
+                         s_locs + w * 2 * KMAX, gid, job, defer ? nullptr : &pw, bad, bar, sp, a.rec, a.njobs);
+    else
+      analyze_group<C::HALF>(Rw, N, N, LDR, K, a.npeaks, a.finder, a.subpixel, gt, G, gred, true, s_vals + w * KMAX,
+                    s_locs + w * 2 * KMAX, gid, job, defer ? nullptr : &pw, bad, bar, sp, a.rec, a.njobs);
+    grp_sync(bar, G);  // the plane is reused by the group's next window
+  }
+}
+
+// ---------------------------------------------------------------------------
+template <int N, int W, bool SRCH, int VAR>
+static cudaError_t launch_nw(const CorrArgs& a, cudaStream_t s, int num_sms) {
+  using C = CorrCfg<N, W, SRCH, VAR>;
+  const size_t sm = C::smem();
+  static bool attr_set = false;
+  if (!attr_set) {
+    cudaError_t e = cudaFuncSetAttribute(correlate_kernel<N, W, SRCH, VAR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    if (e != cudaSuccess) return e;
+    // the planes live in shared memory: ask for the largest carveout so the
+    // register budget, not the L1 split, sets the CTAs per SM
+    e = cudaFuncSetAttribute(correlate_kernel<N, W, SRCH, VAR>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                             (int)cudaSharedmemCarveoutMaxShared);
+    if (e != cudaSuccess) return e;
+    attr_set = true;
+  }
+  int per_sm = 0;
+  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, correlate_kernel<N, W, SRCH, VAR>, C::NT, sm);
+  if (e != cudaSuccess) return e;
+  if (per_sm < 1) per_sm = 1;
+  const int64_t units = (a.njobs + C::WPC - 1) / C::WPC;
+  int64_t grid = (int64_t)per_sm * num_sms;
+  if (grid > units) grid = units;
+  if (grid < 1) grid = 1;
+  correlate_kernel<N, W, SRCH, VAR><<<(unsigned)grid, C::NT, sm, s>>>(a);
+  e = cudaGetLastError();
+  if (e == cudaSuccess && a.rec && a.finder == 0 && !a.accumulate) e = launch_peak_epilogue(a, N, s, num_sms);
+  return e;
+}
+
+// The variant of (N, W) that `a` asks for.
+template <int N, int W> static cudaError_t launch_corr_nw(const CorrArgs& a, cudaStream_t s, int num_sms) {
+  if (a.win > 0 && a.win < W) return launch_nw<N, W, true, 0>(a, s, num_sms);
+  switch (a.variant) {
+    case 1: return launch_nw<N, W, false, 1>(a, s, num_sms);
+    case 2: return launch_nw<N, W, false, 2>(a, s, num_sms);
+    case 3: return launch_nw<N, W, false, 3>(a, s, num_sms);
+    case 4: return launch_nw<N, W, false, 4>(a, s, num_sms);
+    default: return launch_nw<N, W, false, 0>(a, s, num_sms);
+  }
+}
+
+// The launch of one FFT size: each size is a translation unit of its own
+// (k_corr_<N>.cu), because the five variants of all sizes together take
+// minutes to compile.
+#define HH_CORR_SIZE(N)                                                                                       \
+  cudaError_t launch_corr_##N(const CorrArgs& a, int W, cudaStream_t s, int num_sms) {                       \
+    return W == N ? launch_corr_nw<N, N>(a, s, num_sms) : launch_corr_nw<N, N / 2>(a, s, num_sms);            \
+  }                                                                                                           \
+  size_t corr_smem_##N(int W) { return W == N ? CorrCfg<N, N>::smem() : CorrCfg<N, N / 2>::smem(); }
+
+}  // namespace hh

@@ -87,6 +87,8 @@ struct CorrArgs {
 // Launch the correlation kernel for FFT size N (square) and window W (the
 // search area when a.win is set).
 cudaError_t launch_correlate(const CorrArgs& a, int N, int W, cudaStream_t s, int num_sms);
+// outputs from the peak records of a fused correlation launch of FFT size N
+cudaError_t launch_peak_epilogue(const CorrArgs& a, int N, cudaStream_t s, int num_sms);
 bool correlate_supported(int N, int W);
 // The general-shape correlation (any FFT lengths, rectangular windows and
 // search areas): a.wr .. a.gc_smem_lines set by the host (gcorr_prepare).

@@ -96,7 +96,8 @@ template <int N, int W, bool SRCH = false, int VAR = 0> struct CorrCfg {
   static constexpr size_t PLANE_B = (size_t)PS * sizeof(float2);
   static constexpr size_t BASE_B = WPC * PLANE_B + WPC * (G / 32) * NPART * sizeof(double) + N * sizeof(float2) +
                                    WPC * (G / 32) * 2 * KMAX * sizeof(uint32_t) +
-                                   WPC * (KMAX * sizeof(float) + 2 * KMAX * sizeof(int)) + 3 * N * sizeof(int) + 64;
+                                   WPC * (KMAX * sizeof(float) + 2 * KMAX * sizeof(int)) + 3 * N * sizeof(int) +
+                                   (W == N ? WPC * N * sizeof(uint32_t) : 0) + 64;
   // CTAs per SM that shared memory allows (228 KB per SM, 1 KB of it
   // reserved per CTA), capped by the register budget
   static constexpr int occ(size_t b) {
@@ -117,7 +118,7 @@ template <int N, int W, bool SRCH = false, int VAR = 0> struct CorrCfg {
   static constexpr size_t smem() { return BASE_B + (GSM ? GAIN_B : (QSM ? GQ_B : 0)); }
   static_assert(W == N || 2 * W == N, "window must equal the FFT size or half of it");
   static_assert((G >= 32 && G % 32 == 0) || G == 16, "a window group is whole warps or half a warp");
-  static_assert(N * LDR <= 2 * N * LD, "real plane must fit in the complex plane");
+  static_assert(N * LDR * 4 + (W == N ? (G + 31) / 32 * 64 * 2 : 0) <= 2 * N * LD * 4, "real plane and scan lists fit in the complex plane");
 };
 
 template <int N, int W, bool SRCH, int VAR>
@@ -139,7 +140,8 @@ __global__ void __launch_bounds__(CorrCfg<N, W, SRCH, VAR>::NT, CorrCfg<N, W, SR
   int* s_freq = reinterpret_cast<int*>(s_locs + WPC * 2 * KMAX);
   int* s_neg = s_freq + N;
   int* s_canon = s_neg + N;
-  float* s_gain = reinterpret_cast<float*>(s_canon + N);  // N x N when C::GSM
+  uint32_t* s_rmax = reinterpret_cast<uint32_t*>(s_canon + N);  // per window: its plane's row maxima
+  float* s_gain = reinterpret_cast<float*>(s_rmax + (W == N ? WPC * N : 0));  // N x N when C::GSM
 
   const int tid = threadIdx.x;
   const int K = a.npeaks > 2 ? a.npeaks : 2;
@@ -172,6 +174,20 @@ __global__ void __launch_bounds__(CorrCfg<N, W, SRCH, VAR>::NT, CorrCfg<N, W, SR
   const int bar = WPC == 1 ? 0 : w + 1;
   float2* P = planes + w * PS;
   float* Rw = reinterpret_cast<float*>(P);  // real plane, overlays the complex one after stage 8
+  uint32_t* rmax = s_rmax + w * N;
+  // Peak scan from the row maxima (scan_rows) where the box is the whole plane
+  // or the search lags: unpadded windows. A padded window's box is at most
+  // half the plane (its overlap weight halves by then) and 13 x 13 of 32 x 32
+  // with the Gaussian apodization, where walking the column strips costs no
+  // more (16.5 / 16.9 ns at 48 points, 28.0 / 27.6 at 64, 124 / 126 at 128)
+  // and half-warp groups lose (5.6 / 10.1 ns at 32 points: the halves' loops
+  // run one after the other). Unpadded, strips / row maxima: 16.2 / 12.4 ns
+  // at 32 points, 38.2 / 31.2 at 48, 57.8 / 51.9 at 64, 168 / 121 at 96,
+  // 264 / 220 at 128.
+  constexpr bool ROWSCAN = W == N;
+  constexpr int FN = ROWSCAN ? N : 0;
+  // the peak scan's list, in the half of the plane that the real plane leaves
+  uint16_t* list = reinterpret_cast<uint16_t*>(Rw + N * LDR);
   double* part = s_part + w * (G / 32) * C::NPART;
   const float scale = 1.0f / (float)(N * N);
   // fftshifted rows / columns that can hold a nonzero correlation value (the
@@ -223,6 +239,8 @@ __global__ void __launch_bounds__(CorrCfg<N, W, SRCH, VAR>::NT, CorrCfg<N, W, SR
     //      mean is the exact sum over n rounded once, where the reference
     //      folds in Float32 left to right; the two differ by a few ulp.
     bool bad;
+    if (ROWSCAN && N2 > 1)
+      for (int r = gt; r < N; r += G) rmax[r] = 0u;  // raised by the last inverse pass, barriers later
     if constexpr (SRCH) {
       // enlarged search area (load_windows!, src/correlators.jl:229-262):
       // the W x W frame-B area starts (W - win) / 2 before the window on
@@ -658,6 +676,7 @@ __global__ void __launch_bounds__(CorrCfg<N, W, SRCH, VAR>::NT, CorrCfg<N, W, SR
           }
           RDFT<N1, true>::run(x, N1);
           const int ps0 = blo + t, ps1 = blo + t + nh;  // fftshifted rows of pa and pb
+          float m0 = 0.f, m1 = 0.f;  // maxima of the two rows over this item's columns (a NaN drops out)
 #pragma unroll
           for (int n1 = 0; n1 < N1; ++n1) {
             const int qs = (N2 * n1 + n2 + H) % N;
@@ -678,6 +697,16 @@ __global__ void __launch_bounds__(CorrCfg<N, W, SRCH, VAR>::NT, CorrCfg<N, W, SR
             if (SRCH && (qs < blo || qs > bhi)) r0 = r1 = 0.f;  // lags outside the search range
             rv[i][0][n1] = r0;
             rv[i][1][n1] = r1;
+            m0 = fmaxf(m0, r0);
+            m1 = fmaxf(m1, r1);
+          }
+          if (!ROWSCAN) {
+          } else if (N2 == 1) {
+            rmax[ps0] = __float_as_uint(m0);
+            if (hasb) rmax[ps1] = __float_as_uint(m1);
+          } else {
+            atomicMax(rmax + ps0, __float_as_uint(m0));
+            if (hasb) atomicMax(rmax + ps1, __float_as_uint(m1));
           }
         }
       }
@@ -725,14 +754,17 @@ __global__ void __launch_bounds__(CorrCfg<N, W, SRCH, VAR>::NT, CorrCfg<N, W, SR
     const bool defer = a.rec && a.finder == 0;
     uint32_t* gred = red + w * (G / 32) * 2 * KMAX;
     if (C::INLINE_ANALYSIS && K <= 4)
-      analyze_body<4, false>(Rw, N, N, LDR, K, a.npeaks, a.finder, a.subpixel, gt, G, gred, true, s_vals + w * KMAX,
-                      s_locs + w * 2 * KMAX, gid, job, defer ? nullptr : &pw, bad, bar, sp, a.rec, a.njobs);
+      analyze_body<4, FN, C::HALF>(Rw, N, N, LDR, K, a.npeaks, a.finder, a.subpixel, gt, G, gred, true, s_vals + w * KMAX,
+                            s_locs + w * 2 * KMAX, gid, job, defer ? nullptr : &pw, bad, bar, sp, a.rec, a.njobs, rmax,
+                          list);
     else if (C::INLINE_ANALYSIS)
-      analyze_body<KMAX, false>(Rw, N, N, LDR, K, a.npeaks, a.finder, a.subpixel, gt, G, gred, true, s_vals + w * KMAX,
-                         s_locs + w * 2 * KMAX, gid, job, defer ? nullptr : &pw, bad, bar, sp, a.rec, a.njobs);
+      analyze_body<KMAX, FN, C::HALF>(Rw, N, N, LDR, K, a.npeaks, a.finder, a.subpixel, gt, G, gred, true, s_vals + w * KMAX,
+                               s_locs + w * 2 * KMAX, gid, job, defer ? nullptr : &pw, bad, bar, sp, a.rec, a.njobs,
+                               rmax, list);
     else
-      analyze_group<C::HALF>(Rw, N, N, LDR, K, a.npeaks, a.finder, a.subpixel, gt, G, gred, true, s_vals + w * KMAX,
-                    s_locs + w * 2 * KMAX, gid, job, defer ? nullptr : &pw, bad, bar, sp, a.rec, a.njobs);
+      analyze_group<FN, C::HALF>(Rw, N, N, LDR, K, a.npeaks, a.finder, a.subpixel, gt, G, gred, true, s_vals + w * KMAX,
+                          s_locs + w * 2 * KMAX, gid, job, defer ? nullptr : &pw, bad, bar, sp, a.rec, a.njobs, rmax,
+                          list);
     grp_sync(bar, G);  // the plane is reused by the group's next window
   }
 }

@@ -490,12 +490,113 @@ struct StripScan {
   }
 };
 
-template <int KC, bool PAIRS>
+// The regional maxima of an N x N plane of values >= 0 from its row maxima,
+// for the fused kernels, whose last inverse pass holds whole rows (or N1
+// columns of one) in registers: rmax[r] is the largest value of row r (as
+// its bits, 0 for a row without one). A row maximum above those of both
+// neighbouring rows belongs to a regional maximum (the last of its equals in
+// the row), so the K-th largest of these is a lower bound of the K-th peak,
+// and only pixels at or above it need the neighbour test. Few rows hold such
+// pixels (the flanks of the strongest peaks: 5-8 of 31 at 32 points): they
+// are read a row at a time, the pixels found are listed, and the lanes then
+// test one each. With fewer than K such rows the bound is 0 and every pixel
+// of the box is tested. A NaN neither blocks a neighbour nor is a peak, as
+// in is_local_max; -0 does not occur. The lanes of a warp (or its half) take
+// the rows lo + lane + j LANES; with several warps per plane each forms the
+// bound by itself and reads every nwarps-th of the rows. list: room for
+// 2 LANES entries per warp.
+template <int N, int LANES, class TK>
+__device__ __forceinline__ void scan_rows(TK& tk, const float* R, int ldr, int K, int lo, int hi, const uint32_t* rmax,
+                                          uint16_t* list, int gtid, int nwarps) {
+  constexpr int J = (N + LANES - 1) / LANES;
+  const int lane = gtid & (LANES - 1), gwarp = gtid / LANES;
+  const unsigned gm = grp_mask(LANES);
+  const int sh = LANES < 32 ? (threadIdx.x & 31) & ~(LANES - 1) : 0;  // the group's first lane
+  constexpr unsigned ALL = LANES < 32 ? (1u << (LANES & 31)) - 1u : 0xffffffffu;
+  uint32_t M[J], cand[J];
+#pragma unroll
+  for (int j = 0; j < J; ++j) {
+    const int r = lo + lane + j * LANES;
+    M[j] = cand[j] = 0u;
+    if (r <= hi) {
+      M[j] = rmax[r];
+      // rows outside the box are zero; a row outside the plane counts as one
+      const uint32_t up = r > lo ? rmax[r - 1] : 0u, dn = r < hi ? rmax[r + 1] : 0u;
+      cand[j] = M[j] > up && M[j] > dn ? M[j] : 0u;
+    }
+  }
+  uint32_t thr = 0u;
+  for (int k = 0; k < K; ++k) {  // equal candidates count once: the bound only gets lower
+    uint32_t h = 0u;
+#pragma unroll
+    for (int j = 0; j < J; ++j) h = max(h, cand[j]);
+    thr = __reduce_max_sync(gm, h);
+    if (thr == 0u) break;
+#pragma unroll
+    for (int j = 0; j < J; ++j) cand[j] = cand[j] == thr ? 0u : cand[j];
+  }
+  // pixel e = r + c N of the list: a peak unless a neighbour blocks it
+  // (neighbours outside the plane never do: NaN compares false)
+  auto test = [&](int e) {
+    const int r = e % N, c = e / N;
+    const float* p = R + c * ldr + r;
+    const float x = __int_as_float(0x7fc00000), v = *p;
+    const bool hu = r > 0, hd = r < N - 1, hl = c > 0, hr = c < N - 1;
+    const float ul = hu && hl ? p[-ldr - 1] : x, l = hl ? p[-ldr] : x, dl = hd && hl ? p[-ldr + 1] : x;
+    const float u = hu ? p[-1] : x, d = hd ? p[1] : x;
+    const float ur = hu && hr ? p[ldr - 1] : x, rt = hr ? p[ldr] : x, dr = hd && hr ? p[ldr + 1] : x;
+    const float b = fmaxf(fmaxf(ul, l), fmaxf(dl, u)), t = fmaxf(fmaxf(ur, rt), fmaxf(dr, d));
+    if (!isnan(v) && !(b > v) && !(t >= v)) tk.insert(fkey(v), ~(uint32_t)e, K);
+  };
+  list += gwarp * 2 * LANES;
+  int cnt = 0, turn = 0;
+#pragma unroll
+  for (int j = 0; j < J; ++j) {
+    const int base = lo + j * LANES;
+    unsigned bits = (__ballot_sync(gm, base + lane <= hi && M[j] >= thr) >> sh) & ALL;
+    while (bits) {
+      const int r = base + __ffs(bits) - 1;
+      bits &= bits - 1;
+      if (nwarps > 1 && (turn++ % nwarps) != gwarp) continue;
+      uint32_t v[J];
+#pragma unroll
+      for (int i = 0; i < J; ++i) {
+        const int c = lo + lane + i * LANES;
+        v[i] = c <= hi ? __float_as_uint(R[c * ldr + r]) : 0u;
+      }
+#pragma unroll
+      for (int i = 0; i < J; ++i) {
+        const int c = lo + lane + i * LANES;
+        const bool in = c <= hi && v[i] >= thr;
+        const unsigned b = (__ballot_sync(gm, in) >> sh) & ALL;
+        if (in) list[cnt + __popc(b & ((1u << lane) - 1u))] = (uint16_t)(r + c * N);
+        cnt += __popc(b);
+        if (cnt >= LANES) {  // a full round of tests; the rest moves down
+          __syncwarp(gm);
+          test(list[lane]);
+          const uint16_t q = list[LANES + lane];
+          __syncwarp(gm);
+          list[lane] = q;
+          cnt -= LANES;
+        }
+      }
+    }
+  }
+  __syncwarp(gm);
+  if (lane < cnt) test(list[lane]);
+}
+
+// FN > 0: an FN x FN plane of a fused kernel with its row maxima (scan_rows);
+// FN = 0: any plane, by column strips. PAIRS: walk two strips per thread at a
+// time, for groups that can have more strips than threads (half-warp groups);
+// elsewhere the second strip's registers would only add spills.
+template <int KC, int FN, bool PAIRS>
 __device__ __forceinline__ void analyze_body(const float* R, int nr, int nc, int ldr, int K, int npeaks, int finder,
                                              int subpixel, int gtid, int gsize, uint32_t* red, bool active,
                                              float* s_vals, int* s_locs, int64_t grid_id, int64_t job,
                                              const PeakOut* o, bool poison, int bar, const ScanPlan sp,
-                                             float* rec, int64_t rec_stride) {
+                                             float* rec, int64_t rec_stride, const uint32_t* rmax = nullptr,
+                                             uint16_t* list = nullptr) {
   const int rlo = sp.rlo, rhi = sp.rhi, clo = sp.clo, chi = sp.chi;
   // a poisoned plane (non-finite window data: the reference's plane is all
   // NaN there) yields no peak, so every output is NaN
@@ -508,7 +609,9 @@ __device__ __forceinline__ void analyze_body(const float* R, int nr, int nc, int
     // of the box top to bottom (StripScan), keeping its K best in registers
     TopK<KC> tk;
     tk.init();
-    if (scan) {
+    if constexpr (FN > 0) {
+      if (scan) scan_rows<FN, 32>(tk, R, ldr, K, rlo, rhi, rmax, list, gtid, nwarps);
+    } else if (scan) {
       const int bw = sp.bw, S = sp.S, rps = sp.rps, ns = bw * S;
       // blocks of SU rows: the next SU rows of the three columns are loaded
       // together, so the loads of a block overlap instead of each row
@@ -569,10 +672,10 @@ __device__ __forceinline__ void analyze_body(const float* R, int nr, int nc, int
           }
         }
       }
-      if (gtid == 0 && (rhi < nr - 1 || chi < nc - 1)) {  // the last pixel, outside the box
-        const int r = nr - 1, c = nc - 1;
-        if (is_local_max(R, nr, nc, ldr, r, c, R[c * ldr + r])) tk.insert(fkey(R[c * ldr + r]), ~(uint32_t)(r + c * nr), K);
-      }
+    }
+    if (scan && gtid == 0 && (rhi < nr - 1 || chi < nc - 1)) {  // the last pixel, outside the box
+      const int r = nr - 1, c = nc - 1;
+      if (is_local_max(R, nr, nc, ldr, r, c, R[c * ldr + r])) tk.insert(fkey(R[c * ldr + r]), ~(uint32_t)(r + c * nr), K);
     }
     // Merge: each warp takes its K best from its threads' lists by shuffle
     // rounds (lane m keeps the m-th); with several warps the warps' lists
@@ -689,21 +792,19 @@ __device__ __forceinline__ void analyze_body(const float* R, int nr, int nc, int
 
 // The analysis as a call: small planes keep it out of line (the kernel's
 // transform stages then keep their registers); large planes inline it.
-// PAIRS: walk two column strips per thread at a time, for groups with more
-// strips than threads (half-warp groups of 32-point planes); elsewhere the
-// second strip's registers would only add spills.
-template <bool PAIRS = false>
+template <int FN = 0, bool PAIRS = false>
 __device__ __noinline__ void analyze_group(const float* R, int nr, int nc, int ldr, int K, int npeaks, int finder,
                                            int subpixel, int gtid, int gsize, uint32_t* red, bool active,
                                            float* s_vals, int* s_locs, int64_t grid_id, int64_t job,
                                            const PeakOut* o, bool poison, int bar, const ScanPlan sp,
-                                           float* rec, int64_t rec_stride) {
+                                           float* rec, int64_t rec_stride, const uint32_t* rmax = nullptr,
+                                           uint16_t* list = nullptr) {
   if (K <= 4)
-    analyze_body<4, PAIRS>(R, nr, nc, ldr, K, npeaks, finder, subpixel, gtid, gsize, red, active, s_vals, s_locs, grid_id, job,
-                    o, poison, bar, sp, rec, rec_stride);
+    analyze_body<4, FN, PAIRS>(R, nr, nc, ldr, K, npeaks, finder, subpixel, gtid, gsize, red, active, s_vals, s_locs,
+                               grid_id, job, o, poison, bar, sp, rec, rec_stride, rmax, list);
   else
-    analyze_body<KMAX, PAIRS>(R, nr, nc, ldr, K, npeaks, finder, subpixel, gtid, gsize, red, active, s_vals, s_locs, grid_id,
-                       job, o, poison, bar, sp, rec, rec_stride);
+    analyze_body<KMAX, FN, PAIRS>(R, nr, nc, ldr, K, npeaks, finder, subpixel, gtid, gsize, red, active, s_vals, s_locs,
+                                  grid_id, job, o, poison, bar, sp, rec, rec_stride, rmax, list);
 }
 
 // S(k) = conj(FA(k)) FB(k) of the packed transform Z = F(a + i b), from

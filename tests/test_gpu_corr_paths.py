@@ -1,0 +1,55 @@
+"""The peak paths of the fused correlation kernels against the plane analysis.
+
+process_windows ranks the peaks inside the correlation kernel (from the row
+maxima of an unpadded plane, by column strips of the box of a padded one);
+correlation_planes + analyze_planes ranks them from the whole plane, pixel by
+pixel. Both see the same plane, so peaks and refined values are the same bit
+for bit, at every FFT size, for ties (quantised and constant images), planes
+with fewer regional maxima than peaks asked for, and windows holding NaN."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _image(kind, n, rng):
+    if kind == "noise":
+        return rng.random((n, n)), rng.random((n, n))
+    if kind == "steps":  # few grey levels: equal values all over the plane
+        a = rng.integers(0, 2, (n, n)).astype(float)
+        return a, np.roll(a, (2, 3), (0, 1))
+    if kind == "stripes":  # rows of the plane repeat: no row maximum stands out
+        a = np.tile((np.arange(n) % 4 == 0).astype(float), (n, 1))
+        return a, a
+    a = np.zeros((n, n))  # flat except for one speck, and a NaN and an Inf pixel
+    b = a.copy()
+    a[n // 3, n // 3] = b[n // 3 + 1, n // 3 + 2] = 1.0
+    a[5, 5], b[n - 6, 7] = np.nan, np.inf
+    return a, b
+
+
+@pytest.mark.parametrize("padding", [False, True])
+@pytest.mark.parametrize("fft", [16, 24, 32, 48, 64, 96, 128])
+def test_peaks_equal_plane_analysis(fft, padding):
+    import hammerhead_b200 as hb
+    from hammerhead_b200 import hooks
+
+    w = fft // 2 if padding else fft
+    n = 3 * w + 5  # a ragged grid: several windows per CTA, a part-empty last one
+    rng = np.random.default_rng(fft + padding)
+    with hb.piv_workspace() as ws:
+        d = hooks.DeviceSession(ws)
+        for kind in ("noise", "steps", "stripes", "speck"):
+            A, B = _image(kind, n, rng)
+            d.stage_pair(A.astype(np.float32), B.astype(np.float32))
+            for n_peaks, finder, apod, search in ((3, "regionalmax", "gauss", w), (8, "regionalmax", "none", w),
+                                                  (4, "exclusion", "none", w), (3, "regionalmax", "none", w - 6)):
+                if search != w and padding:
+                    continue
+                p = hb.PIVParameters(window_size=search, search_area_size=w, overlap=search // 2, padding=padding,
+                                     apodization=apod, n_peaks=n_peaks, peak_finder=finder)
+                _, _, _, jobs = hb.pass_grid((n, n), p)
+                out, locs, _ = d.process_windows(p, jobs, want_locs=True)
+                ref, rlocs = hooks.analyze_planes(ws, d.correlation_planes(p, jobs), n_peaks, finder)
+                np.testing.assert_array_equal(locs, rlocs, err_msg=f"{kind} {n_peaks} {finder} {apod} {search}")
+                np.testing.assert_array_equal(out, ref, err_msg=f"{kind} {n_peaks} {finder} {apod} {search}")

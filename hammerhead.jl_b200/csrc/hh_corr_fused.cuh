@@ -81,10 +81,24 @@ template <int N, int W, bool SRCH = false, int VAR = 0> struct CorrCfg {
   // (their outputs are real: one lands in the real part, one in the
   // imaginary part). Every window is transformed on its own.
   static constexpr int NC = N / 2 + 1;
-  static constexpr int IPT = ((N / 2) * N2 + G - 1) / G;  // final inverse items per thread
   static constexpr int LD = N + 1;    // complex plane leading dimension (float2)
   static constexpr int LDR = N + 1;   // real plane leading dimension (float), overlays the complex plane
   static constexpr bool PADDED = (W * 2 == N);
+  // A padded window keeps only lags |lag| <= N/4 on either axis: the overlap
+  // gain is zero where the weight (the apodization window's autocorrelation)
+  // is below half its maximum, which for the triangle of the plain window
+  // starts past W/2 = N/4 and for the Gaussian earlier (6 of 32 points). So
+  // both inverse axes form only the outputs that hold such a lag: keep(n1)
+  // of the last pass (the others' butterflies fold away and nothing is
+  // stored for them), at most Q + 1 row pairs, and a real plane whose cells
+  // outside the box are never stored but read as the zeros they are. Half of
+  // the inverse's stores and a third of its arithmetic are for lags outside
+  // N/4. launch_nw checks that the table's box is inside it.
+  static constexpr bool BOXED = PADDED && !SRCH;
+  static constexpr int Q = N / 4;
+  static constexpr bool keep(int n1) { return !BOXED || N2 * n1 <= Q || N2 * n1 + N2 - 1 >= N - Q; }
+  static constexpr int NHMAX = BOXED ? Q + 1 : N / 2;  // row pairs of the last inverse axis
+  static constexpr int IPT = (NHMAX * N2 + G - 1) / G;  // final inverse items per thread
   static constexpr int NZ1 = PADDED ? (W / N2) : N1;  // nonzero inputs of a forward pass-A line
 
   static constexpr int EPT = (W * W + G - 1) / G;             // window pixels per thread
@@ -98,24 +112,15 @@ template <int N, int W, bool SRCH = false, int VAR = 0> struct CorrCfg {
                                    WPC * (G / 32) * 2 * KMAX * sizeof(uint32_t) +
                                    WPC * (KMAX * sizeof(float) + 2 * KMAX * sizeof(int)) + 3 * N * sizeof(int) +
                                    (W == N ? WPC * N * sizeof(uint32_t) : 0) + 64;
-  // CTAs per SM that shared memory allows (228 KB per SM, 1 KB of it
-  // reserved per CTA), capped by the register budget
-  static constexpr int occ(size_t b) {
-    return (int)((228 * 1024) / (b + 1024)) < MINB ? (int)((228 * 1024) / (b + 1024)) : MINB;
-  }
-  // The overlap gain table (N x N) is read by every window; from global
-  // memory its L1 lines are flushed by the window pixels (it took a third of
-  // the last inverse pass at 32 points, half of it at 128). It goes to shared
-  // memory where that costs no CTA per SM: every size but 64 points. (The
-  // apodization window in shared memory as well was no faster.)
-  // Where the full table would cost a CTA (64 points), its quarter does not:
-  // the gain of a symmetric apodization depends only on |lag| along each
-  // axis, and the table builder appends the quarter when that holds exactly.
-  static constexpr size_t GAIN_B = (size_t)N * N * sizeof(float);
-  static constexpr size_t GQ_B = (size_t)(N / 2 + 1) * (N / 2 + 1) * sizeof(float);
-  static constexpr bool GSM = occ(BASE_B + GAIN_B) >= occ(BASE_B);
-  static constexpr bool QSM = !GSM && occ(BASE_B + GQ_B) >= occ(BASE_B);
-  static constexpr size_t smem() { return BASE_B + (GSM ? GAIN_B : (QSM ? GQ_B : 0)); }
+  // The overlap gain is read by every window; from global memory its L1
+  // lines are flushed by the window pixels (it took a third of the last
+  // inverse pass at 32 points, half of it at 128). The gain of a symmetric
+  // apodization depends only on |lag| along each axis, so the (Q + 1)^2
+  // quarter of the kept lags goes to shared memory (the table builder appends
+  // the quarter when that holds exactly). (The apodization window in shared
+  // memory as well was no faster.)
+  static constexpr size_t GAIN_B = BOXED ? (size_t)(Q + 1) * (Q + 1) * sizeof(float) : 0;
+  static constexpr size_t smem() { return BASE_B + GAIN_B; }
   static_assert(W == N || 2 * W == N, "window must equal the FFT size or half of it");
   static_assert((G >= 32 && G % 32 == 0) || G == 16, "a window group is whole warps or half a warp");
   static_assert(N * LDR * 4 + (W == N ? (G + 31) / 32 * 64 * 2 : 0) <= 2 * N * LD * 4, "real plane and scan lists fit in the complex plane");
@@ -141,16 +146,15 @@ __global__ void __launch_bounds__(CorrCfg<N, W, SRCH, VAR>::NT, CorrCfg<N, W, SR
   int* s_neg = s_freq + N;
   int* s_canon = s_neg + N;
   uint32_t* s_rmax = reinterpret_cast<uint32_t*>(s_canon + N);  // per window: its plane's row maxima
-  float* s_gain = reinterpret_cast<float*>(s_rmax + (W == N ? WPC * N : 0));  // N x N when C::GSM
+  float* s_gain = reinterpret_cast<float*>(s_rmax + (W == N ? WPC * N : 0));  // (Q + 1)^2 when C::BOXED
 
   const int tid = threadIdx.x;
   const int K = a.npeaks > 2 ? a.npeaks : 2;
-  if (C::GSM && a.gain)
-    for (int m = tid; m < N * N; m += NT) s_gain[m] = a.gain[m];
   // the quarter table (word N^2 of the gain buffer says whether it follows)
-  const bool gq = C::QSM && a.gain && a.gain[N * N] != 0.f;
+  const bool gq = C::BOXED && a.gain[N * N] != 0.f;
   if (gq)
-    for (int m = tid; m < (N / 2 + 1) * (N / 2 + 1); m += NT) s_gain[m] = a.gain[N * N + 1 + m];
+    for (int m = tid; m < (C::Q + 1) * (C::Q + 1); m += NT)
+      s_gain[m] = a.gain[N * N + 1 + m % (C::Q + 1) + m / (C::Q + 1) * (H + 1)];
 
   if (N2 > 1) {
     for (int m = tid; m < N; m += NT) {
@@ -193,6 +197,9 @@ __global__ void __launch_bounds__(CorrCfg<N, W, SRCH, VAR>::NT, CorrCfg<N, W, SR
   // fftshifted rows / columns that can hold a nonzero correlation value (the
   // support of the overlap gain; the whole plane without padding)
   const int blo = a.box_hi > 0 ? a.box_lo : 0, bhi = a.box_hi > 0 ? a.box_hi : N - 1;
+  // row pairs of the last inverse axis; it / nh as a multiplication, exact for it < 1024
+  const int nb = bhi - blo + 1, nh = (nb + 1) / 2;
+  const uint32_t inv_nh = (65536u + nh - 1) / nh;
   const ScanPlan sp = scan_plan(tid % G, G, blo, bhi, blo, bhi);
   PeakOut po{a.du, a.dv, a.ratio, a.moment, a.alt_u, a.alt_v, a.nalt, a.G, a.packed, a.locs};
 
@@ -591,9 +598,8 @@ __global__ void __launch_bounds__(CorrCfg<N, W, SRCH, VAR>::NT, CorrCfg<N, W, SR
       const bool pk = N2 == 1 && it == 0;
       const int c = N2 == 1 ? it : it / N2, n2 = N2 == 1 ? 0 : it % N2;
       const int aq = N2 == 1 ? c : s_canon[c];
-      const int bq = pk ? H : (N2 == 1 ? N - c : s_neg[aq]);
       float2* L = P + aq * LD;
-      float2* Lb = P + bq * LD;
+      float2* Lb = P + H * LD;  // column N/2, for the packed item only
       float2 x[N1];
 #pragma unroll
       for (int k1 = 0; k1 < N1; ++k1) {
@@ -608,12 +614,12 @@ __global__ void __launch_bounds__(CorrCfg<N, W, SRCH, VAR>::NT, CorrCfg<N, W, SR
       RDFT<N1, true>::run(x, N1);
 #pragma unroll
       for (int n1 = 0; n1 < N1; ++n1) {
+        if (!C::keep(n1)) continue;
         if (pk) {
           L[n1] = make_float2(x[n1].x, 0.f);
           Lb[n1] = make_float2(x[n1].y, 0.f);
         } else {
           L[N2 * n1 + n2] = x[n1];
-          if (bq != aq) Lb[N2 * n1 + n2] = make_float2(x[n1].x, -x[n1].y);
         }
       }
     }
@@ -621,34 +627,62 @@ __global__ void __launch_bounds__(CorrCfg<N, W, SRCH, VAR>::NT, CorrCfg<N, W, SR
     // ---- stage 8: inverse along q for the rows R needs: fftshifted rows
     //      blo..bhi (the overlap gain is zero on every other row, so R is
     //      exactly 0 there), taken in pairs (blo + t, blo + t + nh) packed as
-    //      T(p) + i T(p'). The normalised, gain-weighted magnitudes are held
-    //      in registers across a barrier, then written as the real plane R
-    //      over the complex one; the other rows are written as zeros.
-    const int nb = bhi - blo + 1, nh = (nb + 1) / 2;
-    if (N2 > 1) {
+    //      T(p) + i T(p'). Column -kq of T is the conjugate of column kq, so
+    //      only the canonical columns were stored; each value read (u, v of
+    //      the two rows) gives u + i v for kq and conj(u) + i conj(v) for
+    //      -kq. The normalised, gain-weighted magnitudes are held in registers
+    //      across a barrier, then written as the real plane R over the
+    //      complex one.
+    if constexpr (N2 > 1) {
+      // The first pass takes the groups k1 = j and N1 - j (0 and N1/2 for
+      // j = 0) of a row pair together: slot k2 of group k1 (frequency
+      // k1 + N1 k2) is canonical for k2 < N2/2 (and N2/2 of group 0), and the
+      // other half of each group mirrors the first half of the other (of
+      // itself for j = 0), so the item reads what it overwrites and nothing
+      // that another item writes.
+      constexpr int h2 = N2 / 2, HN = N1 / 2;
 #pragma unroll 1
-      for (int it = gt; it < H * N1; it += G) {  // items (t, k1) at it = t + H k1, t < nh used
-        const int t = it % H, k1 = it / H;
-        if (t >= nh) continue;
-        const bool hasb = t + nh < nb;
+      for (int it = gt; it < nh * HN; it += G) {
+        const int j = (it * inv_nh) >> 16, t = it - j * nh;
+        const bool hasb = t + nh < nb, j0 = j == 0;
         const int pa = (blo + t + H) % N, pb = hasb ? (blo + t + nh + H) % N : pa;
-        float2* La = P + pa + (N2 * k1) * LD;
-        const float2* Lb = P + pb + (N2 * k1) * LD;
-        float2 x[N2];
+        const int ga = N2 * j, gb = N2 * (j0 ? HN : N1 - j);
+        float2* La = P + pa;
+        const float2* Lb = P + pb;
+        float2 x1[N2], x2[N2], ma[h2 + 1], mb[h2];
+        auto row_pair = [&](int slot, float2& direct, float2& mirror) {
+          const float2 u = La[slot * LD];
+          const float2 v = hasb ? Lb[slot * LD] : make_float2(0.f, 0.f);
+          direct = make_float2(u.x - v.y, u.y + v.x);
+          mirror = make_float2(u.x + v.y, v.x - u.y);
+        };
 #pragma unroll
-        for (int k2 = 0; k2 < N2; ++k2) {
-          const float2 u = La[k2 * LD];
-          const float2 v = hasb ? Lb[k2 * LD] : make_float2(0.f, 0.f);
-          x[k2] = make_float2(u.x - v.y, u.y + v.x);
+        for (int k2 = 0; k2 < h2; ++k2) {
+          row_pair(ga + k2, x1[k2], ma[k2]);
+          row_pair(gb + k2, x2[k2], mb[k2]);
         }
-        RDFT<N2, true>::run(x, N2);
+        float2 mid = make_float2(0.f, 0.f);
+        if (j0) row_pair(h2, mid, ma[h2]);
+#pragma unroll
+        for (int k2 = h2; k2 < N2; ++k2) {
+          const float2 own = k2 == h2 ? mid : ma[N2 - k2];
+          x1[k2] = j0 ? own : mb[N2 - 1 - k2];
+          x2[k2] = j0 ? mb[N2 - 1 - k2] : ma[N2 - 1 - k2];
+        }
+        RDFT<N2, true>::run(x1, N2);
+        RDFT<N2, true>::run(x2, N2);
+        const int kb = j0 ? HN : N1 - j;
 #pragma unroll
         for (int n2 = 1; n2 < N2; ++n2) {
-          const float2 tt = tw[(n2 * k1) % N];
-          x[n2] = cmul(x[n2], make_float2(tt.x, -tt.y));
+          const float2 ta = tw[(n2 * j) % N], tb = tw[(n2 * kb) % N];
+          x1[n2] = cmul(x1[n2], make_float2(ta.x, -ta.y));
+          x2[n2] = cmul(x2[n2], make_float2(tb.x, -tb.y));
         }
 #pragma unroll
-        for (int n2 = 0; n2 < N2; ++n2) La[n2 * LD] = x[n2];
+        for (int n2 = 0; n2 < N2; ++n2) {
+          La[(ga + n2) * LD] = x1[n2];
+          La[(gb + n2) * LD] = x2[n2];
+        }
       }
       grp_sync(bar, G);
     }
@@ -656,39 +690,44 @@ __global__ void __launch_bounds__(CorrCfg<N, W, SRCH, VAR>::NT, CorrCfg<N, W, SR
       float rv[IPT][2][N1];
 #pragma unroll
       for (int i = 0; i < IPT; ++i) {
-        const int it = gt + i * G;  // items (t, n2) at it = t + H n2, t < nh used
-        if (it < H * N2 && it % H < nh) {
-          const int t = it % H, n2 = it / H;
+        const int it = gt + i * G;  // items (t, n2) at it = t + nh n2
+        if (it < nh * N2) {
+          const int n2 = N2 == 1 ? 0 : (it * inv_nh) >> 16, t = it - n2 * nh;
           const bool hasb = t + nh < nb;
           const int pa = (blo + t + H) % N, pb = hasb ? (blo + t + nh + H) % N : pa;
           const float2* La = P + pa;
           const float2* Lb = P + pb;
           float2 x[N1];
+          if (N2 == 1) {
 #pragma unroll
-          for (int k1 = 0; k1 < N1; ++k1) {
-            if (N2 == 1) {
+            for (int k1 = 0; k1 <= H; ++k1) {
               const float2 u = La[k1 * LD];
               const float2 v = hasb ? Lb[k1 * LD] : make_float2(0.f, 0.f);
-              x[k1] = make_float2(u.x - v.y, u.y + v.x);
-            } else {
-              x[k1] = La[(N2 * k1 + n2) * LD];
+              x[k1 % N1] = make_float2(u.x - v.y, u.y + v.x);
+              if (k1 > 0 && k1 < H) x[(N - k1) % N1] = make_float2(u.x + v.y, v.x - u.y);
             }
+          } else {
+#pragma unroll
+            for (int k1 = 0; k1 < N1; ++k1) x[k1] = La[(N2 * k1 + n2) * LD];
           }
           RDFT<N1, true>::run(x, N1);
           const int ps0 = blo + t, ps1 = blo + t + nh;  // fftshifted rows of pa and pb
           float m0 = 0.f, m1 = 0.f;  // maxima of the two rows over this item's columns (a NaN drops out)
+          // |lag| of column N2 n1 + n2: itself in the first half, N - itself in the second
+          const float* g0 = s_gain + abs(ps0 - H);
+          const float* g1 = s_gain + (hasb ? abs(ps1 - H) : 0);
 #pragma unroll
           for (int n1 = 0; n1 < N1; ++n1) {
-            const int qs = (N2 * n1 + n2 + H) % N;
+            if (!C::keep(n1)) continue;
+            const int q = N2 * n1 + n2, qs = (q + H) % N;
             float r0 = fabsf(x[n1].x) * scale, r1 = fabsf(x[n1].y) * scale;
-            if (a.gain) {
-              if (C::GSM) {
-                r0 *= s_gain[qs * N + ps0];
-                r1 *= hasb ? s_gain[qs * N + ps1] : 0.f;
-              } else if (gq) {
-                const int bq = abs(qs - H) * (H + 1);
-                r0 *= s_gain[abs(ps0 - H) + bq];
-                r1 *= hasb ? s_gain[abs(ps1 - H) + bq] : 0.f;
+            if (C::BOXED) {
+              const int lag = 2 * n1 < N1 ? q : N - q;
+              if (gq) {
+                if (N2 == 1 || lag <= C::Q) {  // past Q only for columns no lag is kept of
+                  r0 *= g0[lag * (C::Q + 1)];
+                  r1 *= hasb ? g1[lag * (C::Q + 1)] : 0.f;
+                }
               } else {
                 r0 *= ld_keep(a.gain + qs * N + ps0);
                 r1 *= hasb ? ld_keep(a.gain + qs * N + ps1) : 0.f;
@@ -714,23 +753,26 @@ __global__ void __launch_bounds__(CorrCfg<N, W, SRCH, VAR>::NT, CorrCfg<N, W, SR
 #pragma unroll
       for (int i = 0; i < IPT; ++i) {
         const int it = gt + i * G;
-        if (it < H * N2 && it % H < nh) {
-          const int t = it % H, n2 = it / H;
+        if (it < nh * N2) {
+          const int n2 = N2 == 1 ? 0 : (it * inv_nh) >> 16, t = it - n2 * nh;
           const bool hasb = t + nh < nb;
           const int ps0 = blo + t, ps1 = blo + t + nh;
 #pragma unroll
           for (int n1 = 0; n1 < N1; ++n1) {
+            if (!C::keep(n1)) continue;
             const int qs = (N2 * n1 + n2 + H) % N;
             Rw[qs * LDR + ps0] = rv[i][0][n1];
             if (hasb) Rw[qs * LDR + ps1] = rv[i][1][n1];
           }
         }
       }
-      const int nz = N - nb;  // rows outside [blo, bhi]
-      for (int j = gt; j < nz; j += G) {
-        const int ps = j < blo ? j : j + nb;
+      if (!C::BOXED) {
+        const int nz = N - nb;  // rows outside [blo, bhi]
+        for (int j = gt; j < nz; j += G) {
+          const int ps = j < blo ? j : j + nb;
 #pragma unroll 4
-        for (int qs = 0; qs < N; ++qs) Rw[qs * LDR + ps] = 0.f;
+          for (int qs = 0; qs < N; ++qs) Rw[qs * LDR + ps] = 0.f;
+        }
       }
     }
     grp_sync(bar, G);
@@ -738,7 +780,8 @@ __global__ void __launch_bounds__(CorrCfg<N, W, SRCH, VAR>::NT, CorrCfg<N, W, SR
       float* dst = a.planes + job * (int64_t)(N * N);
       for (int it = gt; it < N * N; it += G) {
         const int p = it % N, q = it / N;
-        const float r = Rw[q * LDR + p];
+        const bool in = !C::BOXED || (p >= blo && p <= bhi && q >= blo && q <= bhi);
+        const float r = in ? Rw[q * LDR + p] : 0.f;
         // ensemble: per-pair planes summed in pair order; a window with
         // non-finite data poisons its sum as the reference's NaN plane does
         const float rr = bad ? __int_as_float(0x7fc00000) : r;
@@ -754,15 +797,15 @@ __global__ void __launch_bounds__(CorrCfg<N, W, SRCH, VAR>::NT, CorrCfg<N, W, SR
     const bool defer = a.rec && a.finder == 0;
     uint32_t* gred = red + w * (G / 32) * 2 * KMAX;
     if (C::INLINE_ANALYSIS && K <= 4)
-      analyze_body<4, FN, C::HALF>(Rw, N, N, LDR, K, a.npeaks, a.finder, a.subpixel, gt, G, gred, true, s_vals + w * KMAX,
+      analyze_body<4, FN, C::BOXED>(Rw, N, N, LDR, K, a.npeaks, a.finder, a.subpixel, gt, G, gred, true, s_vals + w * KMAX,
                             s_locs + w * 2 * KMAX, gid, job, defer ? nullptr : &pw, bad, bar, sp, a.rec, a.njobs, rmax,
                           list);
     else if (C::INLINE_ANALYSIS)
-      analyze_body<KMAX, FN, C::HALF>(Rw, N, N, LDR, K, a.npeaks, a.finder, a.subpixel, gt, G, gred, true, s_vals + w * KMAX,
+      analyze_body<KMAX, FN, C::BOXED>(Rw, N, N, LDR, K, a.npeaks, a.finder, a.subpixel, gt, G, gred, true, s_vals + w * KMAX,
                                s_locs + w * 2 * KMAX, gid, job, defer ? nullptr : &pw, bad, bar, sp, a.rec, a.njobs,
                                rmax, list);
     else
-      analyze_group<FN, C::HALF>(Rw, N, N, LDR, K, a.npeaks, a.finder, a.subpixel, gt, G, gred, true, s_vals + w * KMAX,
+      analyze_group<FN, C::BOXED>(Rw, N, N, LDR, K, a.npeaks, a.finder, a.subpixel, gt, G, gred, true, s_vals + w * KMAX,
                           s_locs + w * 2 * KMAX, gid, job, defer ? nullptr : &pw, bad, bar, sp, a.rec, a.njobs, rmax,
                           list);
     grp_sync(bar, G);  // the plane is reused by the group's next window
@@ -774,6 +817,8 @@ template <int N, int W, bool SRCH, int VAR>
 static cudaError_t launch_nw(const CorrArgs& a, cudaStream_t s, int num_sms) {
   using C = CorrCfg<N, W, SRCH, VAR>;
   const size_t sm = C::smem();
+  if (C::BOXED && !(a.gain && a.box_hi > 0 && a.box_lo >= N / 2 - C::Q && a.box_hi <= N / 2 + C::Q))
+    return cudaErrorInvalidValue;
   static bool attr_set = false;
   if (!attr_set) {
     cudaError_t e = cudaFuncSetAttribute(correlate_kernel<N, W, SRCH, VAR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);

@@ -195,6 +195,14 @@ struct PlaneAcc {
   int ld;
   __device__ __forceinline__ float operator()(int i, int j) const { return p[j * ld + i]; }
 };
+// a plane that is zero, and not stored, outside rows and columns [lo, hi]
+struct BoxAcc {
+  const float* p;
+  int ld, lo, hi;
+  __device__ __forceinline__ float operator()(int i, int j) const {
+    return i >= lo && i <= hi && j >= lo && j <= hi ? p[j * ld + i] : 0.f;
+  }
+};
 struct RecAcc {
   const float* p;
   int64_t stride;
@@ -310,6 +318,10 @@ struct PlaneSrc {
   const float* R;
   int ld;
   __device__ __forceinline__ PlaneAcc at(int, int, int) const { return PlaneAcc{R, ld}; }
+};
+struct BoxSrc {
+  BoxAcc acc;
+  __device__ __forceinline__ BoxAcc at(int, int, int) const { return acc; }
 };
 // ... or the patches of a peak record
 struct RecSrc {
@@ -429,24 +441,27 @@ __device__ __forceinline__ ScanPlan scan_plan(int gtid, int gsize, int rlo, int 
 // must not exceed the value, later ones (the right column and the pixel
 // below) must stay below it; fmaxf drops NaN neighbours, which never block
 // in the reference either.
-struct StripScan {
+template <bool BOXED> struct StripScan {
   const float* Cl;
   const float* Cc;
   const float* Cr;
   bool hl, hr;
   int c, r1;
   float lt, ct, rt, lm, cm, rm;
-  __device__ __forceinline__ void init(const float* R, int ldr, int nc, int c_, int r0, int r1_) {
-    const float NaNf = __int_as_float(0x7fc00000);
+  // clo, chi, rlo: the box (BOXED: its outside is zero and not stored)
+  static __device__ __forceinline__ float none() { return BOXED ? 0.f : __int_as_float(0x7fc00000); }
+  __device__ __forceinline__ void init(const float* R, int ldr, int nc, int c_, int r0, int r1_, int clo, int chi,
+                                       int rlo) {
+    const float NaNf = none();
     c = c_;
     r1 = r1_;
-    hl = c > 0;
-    hr = c < nc - 1;
+    hl = c > (BOXED ? clo : 0);
+    hr = c < (BOXED ? chi : nc - 1);
     Cc = R + c * ldr;
     Cl = hl ? Cc - ldr : Cc;
     Cr = hr ? Cc + ldr : Cc;
     lt = ct = rt = NaNf;
-    if (r0 > 0) {
+    if (r0 > (BOXED ? rlo : 0)) {
       lt = hl ? Cl[r0 - 1] : NaNf;
       ct = Cc[r0 - 1];
       rt = hr ? Cr[r0 - 1] : NaNf;
@@ -456,26 +471,27 @@ struct StripScan {
     rm = hr ? Cr[r0] : NaNf;
   }
   // rows rb0 + 1 .. rb0 + SU of the three columns (NaN past the plane)
-  template <int SU> __device__ __forceinline__ void load(int rb0, int nr, float* l, float* m, float* r) const {
-    const float NaNf = __int_as_float(0x7fc00000);
+  // (past row rend: the box's or the plane's end)
+  template <int SU> __device__ __forceinline__ void load(int rb0, int rend, float* l, float* m, float* r) const {
+    const float NaNf = none();
 #pragma unroll
     for (int u = 0; u < SU; ++u) {
       const int rr = rb0 + 1 + u;
-      const bool ok = rr < nr;
+      const bool ok = rr < rend;
       l[u] = ok && hl ? Cl[rr] : NaNf;
       m[u] = ok ? Cc[rr] : NaNf;
       r[u] = ok && hr ? Cr[rr] : NaNf;
     }
   }
-  // tests row r (the centre value cm) and rolls down one row. Without TIES a
-  // full list rejects a key equal to its K-th: the strips of a thread reach
-  // the list in index order, so a later index cannot win the tie.
-  template <bool TIES, class TK>
+  // tests row r (the centre value cm) and rolls down one row. A full list
+  // rejects a key equal to its K-th: the strips of a thread reach the list in
+  // index order, so a later index cannot win the tie.
+  template <class TK>
   __device__ __forceinline__ void step(int r, float lb, float cb, float rbv, int nr, TK& tk, int K) {
     const float v = cm;
     if (r < r1 && !isnan(v)) {
       const uint32_t h = fkey(v);
-      if (TIES ? h >= tk.thr : h > tk.thr) {
+      if (h > tk.thr) {
         const float e = fmaxf(fmaxf(lt, lm), fmaxf(lb, ct));
         const float l = fmaxf(fmaxf(rt, rm), fmaxf(rbv, cb));
         if (!(e > v) && !(l >= v)) tk.insert(h, ~(uint32_t)(r + c * nr), K);
@@ -587,10 +603,10 @@ __device__ __forceinline__ void scan_rows(TK& tk, const float* R, int ldr, int K
 }
 
 // FN > 0: an FN x FN plane of a fused kernel with its row maxima (scan_rows);
-// FN = 0: any plane, by column strips. PAIRS: walk two strips per thread at a
-// time, for groups that can have more strips than threads (half-warp groups);
-// elsewhere the second strip's registers would only add spills.
-template <int KC, int FN, bool PAIRS>
+// FN = 0: any plane, by column strips. BOXED: the plane is zero, and not
+// stored, outside the box [rlo, rhi] x [clo, chi] (square, and away from the
+// plane's edges).
+template <int KC, int FN, bool BOXED>
 __device__ __forceinline__ void analyze_body(const float* R, int nr, int nc, int ldr, int K, int npeaks, int finder,
                                              int subpixel, int gtid, int gsize, uint32_t* red, bool active,
                                              float* s_vals, int* s_locs, int64_t grid_id, int64_t job,
@@ -603,6 +619,8 @@ __device__ __forceinline__ void analyze_body(const float* R, int nr, int nc, int
   const bool scan = active && !poison;
   const int gwarp = gtid >> 5, nwarps = gsize >> 5;
   const int P = nr * nc;
+  const BoxAcc box{R, ldr, rlo, rhi};
+  auto at = [&](int i, int j) { return BOXED ? box(i, j) : R[j * ldr + i]; };
   int nfound = 0;
   if (finder == 0) {
     // regional maxima (src/localmax.jl:3-19): each thread walks column strips
@@ -633,49 +651,25 @@ __device__ __forceinline__ void analyze_body(const float* R, int nr, int nc, int
           r0 = r1 = rlo;
         }
       };
-      if (PAIRS && ns > gsize) {
-        // Two strips per thread at a time, their rows interleaved, so the
-        // two strips' loads and tests are independent chains. Their pixels
-        // then reach the list out of index order, so a key equal to the
-        // list's K-th goes to the insert's full (key, index) comparison.
-        for (int sa = gtid; sa < ns; sa += 2 * gsize) {
-          int ca, ra0, ra1, cb0, rb0, rb1;
-          strip_at(sa, ca, ra0, ra1);
-          strip_at(sa + gsize, cb0, rb0, rb1);
-          StripScan A, B;
-          A.init(R, ldr, nc, ca, ra0, ra1);
-          B.init(R, ldr, nc, cb0, rb0, rb1);
-          const int nrow = max(ra1 - ra0, rb1 - rb0);
-          for (int rb = 0; rb < nrow; rb += SU) {
-            float al[SU], ac[SU], ar[SU], bl[SU], bc[SU], br[SU];  // rows + 1 .. + SU
-            A.load<SU>(ra0 + rb, nr, al, ac, ar);
-            B.load<SU>(rb0 + rb, nr, bl, bc, br);
+      for (int strip = gtid; strip < ns; strip += gsize) {
+        int c, r0, r1;
+        strip_at(strip, c, r0, r1);
+        if (r0 >= r1) continue;
+        StripScan<BOXED> A;
+        A.init(R, ldr, nc, c, r0, r1, clo, chi, rlo);
+        for (int rb0 = r0; rb0 < r1; rb0 += SU) {
+          float lb[SU], cb[SU], rbv[SU];  // rows rb0 + 1 .. rb0 + SU
+          A.template load<SU>(rb0, BOXED ? rhi + 1 : nr, lb, cb, rbv);
 #pragma unroll
-            for (int u = 0; u < SU; ++u) {
-              A.template step<true>(ra0 + rb + u, al[u], ac[u], ar[u], nr, tk, K);
-              B.template step<true>(rb0 + rb + u, bl[u], bc[u], br[u], nr, tk, K);
-            }
-          }
-        }
-      } else {
-        for (int strip = gtid; strip < ns; strip += gsize) {
-          int c, r0, r1;
-          strip_at(strip, c, r0, r1);
-          if (r0 >= r1) continue;
-          StripScan A;
-          A.init(R, ldr, nc, c, r0, r1);
-          for (int rb0 = r0; rb0 < r1; rb0 += SU) {
-            float lb[SU], cb[SU], rbv[SU];  // rows rb0 + 1 .. rb0 + SU
-            A.load<SU>(rb0, nr, lb, cb, rbv);
-#pragma unroll
-            for (int u = 0; u < SU; ++u) A.template step<false>(rb0 + u, lb[u], cb[u], rbv[u], nr, tk, K);
-          }
+          for (int u = 0; u < SU; ++u) A.step(rb0 + u, lb[u], cb[u], rbv[u], nr, tk, K);
         }
       }
     }
     if (scan && gtid == 0 && (rhi < nr - 1 || chi < nc - 1)) {  // the last pixel, outside the box
       const int r = nr - 1, c = nc - 1;
-      if (is_local_max(R, nr, nc, ldr, r, c, R[c * ldr + r])) tk.insert(fkey(R[c * ldr + r]), ~(uint32_t)(r + c * nr), K);
+      if (BOXED) tk.insert(fkey(0.f), ~(uint32_t)(r + c * nr), K);  // a zero among zeros
+      else if (is_local_max(R, nr, nc, ldr, r, c, R[c * ldr + r]))
+        tk.insert(fkey(R[c * ldr + r]), ~(uint32_t)(r + c * nr), K);
     }
     // Merge: each warp takes its K best from its threads' lists by shuffle
     // rounds (lane m keeps the m-th); with several warps the warps' lists
@@ -704,7 +698,7 @@ __device__ __forceinline__ void analyze_body(const float* R, int nr, int nc, int
       nfound = nw;
       if (lane < nw) {
         const int lin = (int)(~ml);
-        s_vals[lane] = R[(lin / nr) * ldr + (lin % nr)];
+        s_vals[lane] = at(lin % nr, lin / nr);
         s_locs[2 * lane] = lin % nr;
         s_locs[2 * lane + 1] = lin / nr;
       }
@@ -727,7 +721,7 @@ __device__ __forceinline__ void analyze_body(const float* R, int nr, int nc, int
             for (int q = 0; q < nfound; ++q)
               if (abs(r - s_locs[2 * q]) <= 2 && abs(c - s_locs[2 * q + 1]) <= 2) { ex = true; break; }
             if (ex) continue;
-            const float v = R[c * ldr + r];
+            const float v = at(r, c);
             if (!(v > -INFINITY)) continue;  // NaN and -Inf never beat the initial -Inf
             const uint32_t h = fkey(v), l = ~(uint32_t)(r + c * nr);
             if (h > bh || (h == bh && l > bl)) { bh = h; bl = l; }
@@ -738,7 +732,7 @@ __device__ __forceinline__ void analyze_body(const float* R, int nr, int nc, int
       }
       if (!done && whi != 0u) {
         const int lin = (int)(~wlo);
-        const float best = R[(lin / nr) * ldr + (lin % nr)];
+        const float best = at(lin % nr, lin / nr);
         if (nfound > 0 && !(best > 0.f)) {
           done = true;  // secondary peaks must be positive
         } else {
@@ -780,19 +774,24 @@ __device__ __forceinline__ void analyze_body(const float* R, int nr, int nc, int
         const int h = m == 0 ? 2 : 1, w = 2 * h + 1;
         if (m < nfound) {
           const int i = s_locs[2 * m] + cell % w - h, j = s_locs[2 * m + 1] + cell / w - h;
-          val = (i >= 0 && i < nr && j >= 0 && j < nc) ? R[j * ldr + i] : 0.f;
+          val = (i >= 0 && i < nr && j >= 0 && j < nc) ? at(i, j) : 0.f;
         }
       }
       rec[(int64_t)wd * rec_stride + job] = val;
     }
     return;
   }
-  if (gtid == 0) peak_outputs(PlaneSrc{R, ldr}, nr, nc, K, npeaks, subpixel, nfound, s_vals, s_locs, grid_id, job, *o);
+  if (gtid == 0) {
+    if constexpr (BOXED)
+      peak_outputs(BoxSrc{{R, ldr, rlo, rhi}}, nr, nc, K, npeaks, subpixel, nfound, s_vals, s_locs, grid_id, job, *o);
+    else
+      peak_outputs(PlaneSrc{R, ldr}, nr, nc, K, npeaks, subpixel, nfound, s_vals, s_locs, grid_id, job, *o);
+  }
 }
 
 // The analysis as a call: small planes keep it out of line (the kernel's
 // transform stages then keep their registers); large planes inline it.
-template <int FN = 0, bool PAIRS = false>
+template <int FN = 0, bool BOXED = false>
 __device__ __noinline__ void analyze_group(const float* R, int nr, int nc, int ldr, int K, int npeaks, int finder,
                                            int subpixel, int gtid, int gsize, uint32_t* red, bool active,
                                            float* s_vals, int* s_locs, int64_t grid_id, int64_t job,
@@ -800,10 +799,10 @@ __device__ __noinline__ void analyze_group(const float* R, int nr, int nc, int l
                                            float* rec, int64_t rec_stride, const uint32_t* rmax = nullptr,
                                            uint16_t* list = nullptr) {
   if (K <= 4)
-    analyze_body<4, FN, PAIRS>(R, nr, nc, ldr, K, npeaks, finder, subpixel, gtid, gsize, red, active, s_vals, s_locs,
+    analyze_body<4, FN, BOXED>(R, nr, nc, ldr, K, npeaks, finder, subpixel, gtid, gsize, red, active, s_vals, s_locs,
                                grid_id, job, o, poison, bar, sp, rec, rec_stride, rmax, list);
   else
-    analyze_body<KMAX, FN, PAIRS>(R, nr, nc, ldr, K, npeaks, finder, subpixel, gtid, gsize, red, active, s_vals, s_locs,
+    analyze_body<KMAX, FN, BOXED>(R, nr, nc, ldr, K, npeaks, finder, subpixel, gtid, gsize, red, active, s_vals, s_locs,
                                   grid_id, job, o, poison, bar, sp, rec, rec_stride, rmax, list);
 }
 

@@ -25,6 +25,7 @@
 // to natural order, so no bit-reversal pass exists anywhere.
 #pragma once
 #include "hh_corr_peaks.cuh"
+#include "hh_corr_seg.cuh"
 
 namespace hh {
 
@@ -847,6 +848,13 @@ static cudaError_t launch_nw(const CorrArgs& a, cudaStream_t s, int num_sms) {
 // The variant of (N, W) that `a` asks for.
 template <int N, int W> static cudaError_t launch_corr_nw(const CorrArgs& a, cudaStream_t s, int num_sms) {
   if (a.win > 0 && a.win < W) return launch_nw<N, W, true, 0>(a, s, num_sms);
+  // 16 and 32 points: several windows per warp (hh_corr_seg.cuh) for the
+  // regional-maximum finder and the ensemble sums; the exclusion finder, which
+  // ranks its peaks in place, keeps this file's kernel. ns per window on one
+  // 2048^2 pair, this kernel / that one: 8 px padded 2.8 / 1.0, 16 px padded
+  // 5.0 / 3.5, 16 px 4.0 / 2.3, 32 px 11.7 / 7.3.
+  if constexpr (N == 16 || N == 32)
+    if (a.variant == 0 && seg_serves(a)) return launch_seg<N, W>(a, s, num_sms);
   switch (a.variant) {
     case 1: return launch_nw<N, W, false, 1>(a, s, num_sms);
     case 2: return launch_nw<N, W, false, 2>(a, s, num_sms);

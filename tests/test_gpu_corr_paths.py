@@ -53,3 +53,37 @@ def test_peaks_equal_plane_analysis(fft, padding):
                 ref, rlocs = hooks.analyze_planes(ws, d.correlation_planes(p, jobs), n_peaks, finder)
                 np.testing.assert_array_equal(locs, rlocs, err_msg=f"{kind} {n_peaks} {finder} {apod} {search}")
                 np.testing.assert_array_equal(out, ref, err_msg=f"{kind} {n_peaks} {finder} {apod} {search}")
+
+
+@pytest.mark.parametrize("method", ["cross", "phase"])
+@pytest.mark.parametrize("padding", [False, True])
+@pytest.mark.parametrize("fft", [16, 32, 48, 64])
+def test_default_equals_alternative_shape(fft, padding, method):
+    """The default kernel of a class against its alternative CTA shape
+    (variant 1, the same arithmetic on another thread mapping), with an image
+    mask, partly and fully masked windows, and a part-empty last unit: planes,
+    peaks and packed scalars bit for bit."""
+    import hammerhead_b200 as hb
+    from hammerhead_b200 import hooks
+
+    w = fft // 2 if padding else fft
+    n, m = 5 * w + 3, 4 * w + 1
+    rng = np.random.default_rng(fft)
+    A, B = rng.random((2, n, m)).astype(np.float32)
+    mask = np.zeros((n, m), np.uint8)
+    mask[: w + w // 2, : 2 * w] = 1
+    mask[rng.integers(0, n, 40), rng.integers(0, m, 40)] = 1
+    p = hb.PIVParameters(window_size=w, overlap=w // 4, padding=padding, correlation_method=method, apodization="gauss")
+    _, _, _, jobs = hb.pass_grid((n, m), p)
+    got = []
+    with hb.piv_workspace() as ws:
+        d = hooks.DeviceSession(ws)
+        d.stage_pair(A, B)
+        for use in (None, mask):
+            d.stage_mask(use)
+            for v in (0, 1):
+                hb.tuning.set_variant(ws, fft, w, v)
+                got.append(d.process_windows(p, jobs[:-1], want_locs=True)[:2] + (d.correlation_planes(p, jobs[:-1]),))
+    for k in (0, 2):
+        for x, y in zip(got[k], got[k + 1]):
+            np.testing.assert_array_equal(x, y)

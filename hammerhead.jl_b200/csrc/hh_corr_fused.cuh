@@ -103,6 +103,7 @@ template <int N, int W, bool SRCH = false, int VAR = 0> struct CorrCfg {
   static constexpr int NZ1 = PADDED ? (W / N2) : N1;  // nonzero inputs of a forward pass-A line
 
   static constexpr int EPT = (W * W + G - 1) / G;             // window pixels per thread
+  static constexpr bool VIA = !SRCH && EPT > 16;  // pixels wait in the plane for their mean, not in registers
   static constexpr int NPART = SRCH ? 4 : 3;  // FP64 partial sums per warp: A, B, count (and count of B)
   // plane stride in float2; the two windows of a half-warp pair start 16
   // banks apart, so their 32-bit plane accesses (peak scan, real-plane
@@ -115,19 +116,19 @@ template <int N, int W, bool SRCH = false, int VAR = 0> struct CorrCfg {
                                    (W == N ? WPC * N * sizeof(uint32_t) : 0) + 64;
   // The overlap gain is read by every window; from global memory its L1
   // lines are flushed by the window pixels (it took a third of the last
-  // inverse pass at 32 points, half of it at 128). The gain of a symmetric
-  // apodization depends only on |lag| along each axis, so the (Q + 1)^2
-  // quarter of the kept lags goes to shared memory (the table builder appends
-  // the quarter when that holds exactly). (The apodization window in shared
+  // inverse pass at 32 points, half of it at 128), so the kept lags' part of
+  // the table goes to shared memory. (The apodization window in shared
   // memory as well was no faster.)
-  static constexpr size_t GAIN_B = BOXED ? (size_t)(Q + 1) * (Q + 1) * sizeof(float) : 0;
+  static constexpr size_t GAIN_B = BOXED ? (size_t)(2 * Q + 1) * (2 * Q + 1) * sizeof(float) : 0;
   static constexpr size_t smem() { return BASE_B + GAIN_B; }
   static_assert(W == N || 2 * W == N, "window must equal the FFT size or half of it");
   static_assert((G >= 32 && G % 32 == 0) || G == 16, "a window group is whole warps or half a warp");
   static_assert(N * LDR * 4 + (W == N ? (G + 31) / 32 * 64 * 2 : 0) <= 2 * N * LD * 4, "real plane and scan lists fit in the complex plane");
 };
 
-template <int N, int W, bool SRCH, int VAR>
+// ANY: the correlation method is read at run time (else cross correlation,
+// without a branch per spectrum value).
+template <int N, int W, bool SRCH, int VAR, bool ANY>
 __global__ void __launch_bounds__(CorrCfg<N, W, SRCH, VAR>::NT, CorrCfg<N, W, SRCH, VAR>::MINB)
     correlate_kernel(const CorrArgs a) {
   using C = CorrCfg<N, W, SRCH, VAR>;
@@ -147,15 +148,14 @@ __global__ void __launch_bounds__(CorrCfg<N, W, SRCH, VAR>::NT, CorrCfg<N, W, SR
   int* s_neg = s_freq + N;
   int* s_canon = s_neg + N;
   uint32_t* s_rmax = reinterpret_cast<uint32_t*>(s_canon + N);  // per window: its plane's row maxima
-  float* s_gain = reinterpret_cast<float*>(s_rmax + (W == N ? WPC * N : 0));  // (Q + 1)^2 when C::BOXED
+  float* s_gain = reinterpret_cast<float*>(s_rmax + (W == N ? WPC * N : 0));  // (2Q + 1)^2 when C::BOXED
 
   const int tid = threadIdx.x;
+  const int method = ANY ? a.method : 0;
   const int K = a.npeaks > 2 ? a.npeaks : 2;
-  // the quarter table (word N^2 of the gain buffer says whether it follows)
-  const bool gq = C::BOXED && a.gain[N * N] != 0.f;
-  if (gq)
-    for (int m = tid; m < (C::Q + 1) * (C::Q + 1); m += NT)
-      s_gain[m] = a.gain[N * N + 1 + m % (C::Q + 1) + m / (C::Q + 1) * (H + 1)];
+  constexpr int GB = 2 * C::Q + 1;
+  if (C::BOXED)
+    for (int m = tid; m < GB * GB; m += NT) s_gain[m] = a.gain[H - C::Q + m % GB + (H - C::Q + m / GB) * N];
 
   if (N2 > 1) {
     for (int m = tid; m < N; m += NT) {
@@ -259,27 +259,24 @@ __global__ void __launch_bounds__(CorrCfg<N, W, SRCH, VAR>::NT, CorrCfg<N, W, SR
       const int64_t r0 = rs - oa, c0 = cs - oa;
       float2 z[EPT];
       bool mk[EPT];
+#pragma unroll
+      for (int i = 0; i < EPT; ++i) {
+        const int e = gt + i * G, p = e % W, q = e / W;
+        const bool in = W * W % G == 0 || e < W * W;
+        const bool ina = (unsigned)(p - oa) < (unsigned)wa && (unsigned)(q - oa) < (unsigned)wa;
+        const int64_t off = (r0 + p) + (c0 + q) * ld;
+        z[i] = make_float2(ld_stream_if(A + off, in && ina), ld_stream_if(B + off, in));
+        mk[i] = !in || ld_stream_if(M + off, in && M) != 0;
+      }
       double sa = 0.0, sb = 0.0, na = 0.0, nb = 0.0;
 #pragma unroll
       for (int i = 0; i < EPT; ++i) {
-        const int e = gt + i * G;
-        z[i] = make_float2(0.f, 0.f);
-        mk[i] = true;
-        if (e < W * W) {
-          const int p = e % W, q = e / W;
-          const bool ina = (unsigned)(p - oa) < (unsigned)wa && (unsigned)(q - oa) < (unsigned)wa;
-          const int64_t off = (r0 + p) + (c0 + q) * ld;
-          z[i] = make_float2(ina ? ld_stream(A + off) : 0.f, ld_stream(B + off));
-          mk[i] = M ? ld_stream(M + off) != 0 : false;
-          if (!mk[i]) {
-            sb += (double)z[i].y;
-            nb += 1.0;
-            if (ina) {
-              sa += (double)z[i].x;
-              na += 1.0;
-            }
-          }
-        }
+        const int e = gt + i * G, p = e % W, q = e / W;
+        const bool ina = (unsigned)(p - oa) < (unsigned)wa && (unsigned)(q - oa) < (unsigned)wa;
+        sb += (double)(mk[i] ? 0.f : z[i].y);
+        sa += (double)(mk[i] ? 0.f : z[i].x);  // 0 outside the window
+        nb += mk[i] ? 0.0 : 1.0;
+        na += mk[i] || !ina ? 0.0 : 1.0;
       }
       const unsigned gm = grp_mask(G);
 #pragma unroll
@@ -323,25 +320,43 @@ __global__ void __launch_bounds__(CorrCfg<N, W, SRCH, VAR>::NT, CorrCfg<N, W, SR
         }
       }
     } else {
-      float2 z[EPT];
-      bool mk[EPT];
+      // in batches of LB pixel pairs, a batch's loads in flight together
+      constexpr int LB = C::VIA ? 8 : EPT;
+      float2 z[LB];
+      uint32_t mk[(EPT + 31) / 32] = {};  // masked, or past the window
       double sa = 0.0, sb = 0.0, cnt = 0.0;
+      auto load = [&](int i0) {
+        const int64_t w0 = (int64_t)rs + (int64_t)cs * ld;
+        uint32_t m = 0u;
 #pragma unroll
-      for (int i = 0; i < EPT; ++i) {
-        const int e = gt + i * G;
-        z[i] = make_float2(0.f, 0.f);
-        mk[i] = true;
-        if (e < W * W) {
-          const int p = e % W, q = e / W;
-          const int64_t off = (int64_t)(rs + p) + (int64_t)(cs + q) * ld;
-          z[i] = make_float2(ld_stream(A + off), ld_stream(B + off));
-          mk[i] = M ? ld_stream(M + off) != 0 : false;
-          if (!mk[i]) {
-            sa += (double)z[i].x;
-            sb += (double)z[i].y;
-            cnt += 1.0;
+        for (int i = 0; i < LB; ++i) {
+          const int e = gt + (i0 + i) * G;
+          const bool in = W * W % (G * LB) == 0 || e < W * W;
+          const int64_t off = w0 + e % W + (int64_t)(e / W) * ld;
+          z[i] = make_float2(ld_stream_if(A + off, in), ld_stream_if(B + off, in));
+          m |= (uint32_t)(!in || ld_stream_if(M + off, in && M) != 0) << i;
+        }
+#pragma unroll
+        for (int i = 0; i < LB; ++i) {
+          const bool k = m >> i & 1u;
+          sa += (double)(k ? 0.f : z[i].x);
+          sb += (double)(k ? 0.f : z[i].y);
+          cnt += k ? 0.0 : 1.0;
+        }
+        return m;
+      };
+      if constexpr (C::VIA) {
+#pragma unroll
+        for (int i0 = 0; i0 < EPT; i0 += LB) {
+          mk[i0 / 32] |= load(i0) << (i0 % 32);
+#pragma unroll
+          for (int i = 0; i < LB; ++i) {
+            const int e = gt + (i0 + i) * G;
+            if (W * W % (G * LB) == 0 || e < W * W) P[e / W * LD + e % W] = z[i];
           }
         }
+      } else {
+        mk[0] = load(0);
       }
       const unsigned gm = grp_mask(G);
 #pragma unroll
@@ -370,10 +385,11 @@ __global__ void __launch_bounds__(CorrCfg<N, W, SRCH, VAR>::NT, CorrCfg<N, W, SR
 #pragma unroll
       for (int i = 0; i < EPT; ++i) {
         const int e = gt + i * G;
-        if (e < W * W) {
-          const int p = e % W, q = e / W;
+        if (W * W % G == 0 || e < W * W) {
+          float2* c = P + e / W * LD + e % W;
           const float ap = ld_keep(a.apod + e);
-          P[q * LD + p] = (mk[i] || bad) ? make_float2(0.f, 0.f) : make_float2(ap * (z[i].x - ma), ap * (z[i].y - mb));
+          const float2 v = C::VIA ? *c : z[i % LB];
+          *c = (mk[i / 32] >> (i % 32) & 1u) || bad ? make_float2(0.f, 0.f) : make_float2(ap * (v.x - ma), ap * (v.y - mb));
         }
       }
     }
@@ -389,7 +405,7 @@ __global__ void __launch_bounds__(CorrCfg<N, W, SRCH, VAR>::NT, CorrCfg<N, W, SR
       RDFT<N1, false>::run(x, C::NZ1);
       if (N2 > 1) {
 #pragma unroll
-        for (int k1 = 1; k1 < N1; ++k1) x[k1] = cmul(x[k1], tw[(n2 * k1) % N]);
+        for (int k1 = 1; k1 < N1; ++k1) x[k1] = cmul(x[k1], tw[n2 * k1]);
       }
 #pragma unroll
       for (int k1 = 0; k1 < N1; ++k1) L[N2 * k1 + n2] = x[k1];
@@ -418,7 +434,7 @@ __global__ void __launch_bounds__(CorrCfg<N, W, SRCH, VAR>::NT, CorrCfg<N, W, SR
       RDFT<N1, false>::run(x, C::NZ1);
       if (N2 > 1) {
 #pragma unroll
-        for (int k1 = 1; k1 < N1; ++k1) x[k1] = cmul(x[k1], tw[(n2 * k1) % N]);
+        for (int k1 = 1; k1 < N1; ++k1) x[k1] = cmul(x[k1], tw[n2 * k1]);
       }
 #pragma unroll
       for (int k1 = 0; k1 < N1; ++k1) L[(N2 * k1 + n2) * LD] = x[k1];
@@ -473,7 +489,7 @@ __global__ void __launch_bounds__(CorrCfg<N, W, SRCH, VAR>::NT, CorrCfg<N, W, SR
               if (c == cb && ra[j] > rb[j]) continue;  // a self pair is done by its upper row
               xa[u][j] = P[c * LD + ra[j]];
               xb[u][j] = P[cb * LD + rb[j]];
-              wk[u][j] = a.method == 1 ? ld_keep(a.phasew + c * N + ra[j]) : 1.f;
+              wk[u][j] = method == 1 ? ld_keep(a.phasew + c * N + ra[j]) : 1.f;
             }
           }
         }
@@ -484,7 +500,7 @@ __global__ void __launch_bounds__(CorrCfg<N, W, SRCH, VAR>::NT, CorrCfg<N, W, SR
 #pragma unroll
             for (int j = 0; j < RPT; ++j) {
               if (c == cb && ra[j] > rb[j]) continue;
-              const float2 S = cross_spectrum(xa[u][j], xb[u][j], a.method, wk[u][j]);
+              const float2 S = cross_spectrum(xa[u][j], xb[u][j], method, wk[u][j]);
               P[c * LD + ra[j]] = S;
               if (c == cb) P[c * LD + rb[j]] = make_float2(S.x, -S.y);
             }
@@ -511,7 +527,7 @@ __global__ void __launch_bounds__(CorrCfg<N, W, SRCH, VAR>::NT, CorrCfg<N, W, SR
           on[u] = it < NIT && !(self[u] && ap > bp);  // a self pair is done by its upper row
           ia[u] = c * LD + ap;
           ib[u] = bq * LD + bp;
-          wk[u] = on[u] && a.method == 1 ? ld_keep(a.phasew + c * N + ap) : 1.f;
+          wk[u] = on[u] && method == 1 ? ld_keep(a.phasew + c * N + ap) : 1.f;
           if (on[u]) {
             xa[u] = P[ia[u]];
             xb[u] = P[ib[u]];
@@ -520,7 +536,7 @@ __global__ void __launch_bounds__(CorrCfg<N, W, SRCH, VAR>::NT, CorrCfg<N, W, SR
 #pragma unroll
         for (int u = 0; u < SB; ++u)
           if (on[u]) {
-            const float2 S = cross_spectrum(xa[u], xb[u], a.method, wk[u]);
+            const float2 S = cross_spectrum(xa[u], xb[u], method, wk[u]);
             P[ia[u]] = S;
             if (self[u]) P[ib[u]] = make_float2(S.x, -S.y);
           }
@@ -532,8 +548,8 @@ __global__ void __launch_bounds__(CorrCfg<N, W, SRCH, VAR>::NT, CorrCfg<N, W, SR
         const int ap = it % N, c = (it / N) * H;
         const int aq = s_canon[c], bp = s_neg[ap], kp = s_freq[ap];
         if (ap > bp) continue;  // its partner row does this pair
-        const float wk = a.method == 1 ? ld_keep(a.phasew + c * N + kp) : 1.f;
-        const float2 S = cross_spectrum(P[aq * LD + ap], P[aq * LD + bp], a.method, wk);
+        const float wk = method == 1 ? ld_keep(a.phasew + c * N + kp) : 1.f;
+        const float2 S = cross_spectrum(P[aq * LD + ap], P[aq * LD + bp], method, wk);
         P[aq * LD + ap] = S;
         P[aq * LD + bp] = make_float2(S.x, -S.y);
       }
@@ -573,14 +589,14 @@ __global__ void __launch_bounds__(CorrCfg<N, W, SRCH, VAR>::NT, CorrCfg<N, W, SR
           x[k2] = L[k2];
           if (aq != bq) {
             const int neg = (k1 == 0 && k2 == 0) ? 0 : nb0 - k2;
-            const float wk = a.method == 1 ? ld_keep(a.phasew + c * N + k1 + N1 * k2) : 1.f;
-            x[k2] = cross_spectrum(x[k2], Lb[neg], a.method, wk);
+            const float wk = method == 1 ? ld_keep(a.phasew + c * N + k1 + N1 * k2) : 1.f;
+            x[k2] = cross_spectrum(x[k2], Lb[neg], method, wk);
           }
         }
         RDFT<N2, true>::run(x, N2);
 #pragma unroll
         for (int n2 = 1; n2 < N2; ++n2) {
-          const float2 t = tw[(n2 * k1) % N];
+          const float2 t = tw[n2 * k1];
           x[n2] = cmul(x[n2], make_float2(t.x, -t.y));
         }
 #pragma unroll
@@ -675,7 +691,7 @@ __global__ void __launch_bounds__(CorrCfg<N, W, SRCH, VAR>::NT, CorrCfg<N, W, SR
         const int kb = j0 ? HN : N1 - j;
 #pragma unroll
         for (int n2 = 1; n2 < N2; ++n2) {
-          const float2 ta = tw[(n2 * j) % N], tb = tw[(n2 * kb) % N];
+          const float2 ta = tw[n2 * j], tb = tw[n2 * kb];
           x1[n2] = cmul(x1[n2], make_float2(ta.x, -ta.y));
           x2[n2] = cmul(x2[n2], make_float2(tb.x, -tb.y));
         }
@@ -714,24 +730,19 @@ __global__ void __launch_bounds__(CorrCfg<N, W, SRCH, VAR>::NT, CorrCfg<N, W, SR
           RDFT<N1, true>::run(x, N1);
           const int ps0 = blo + t, ps1 = blo + t + nh;  // fftshifted rows of pa and pb
           float m0 = 0.f, m1 = 0.f;  // maxima of the two rows over this item's columns (a NaN drops out)
-          // |lag| of column N2 n1 + n2: itself in the first half, N - itself in the second
-          const float* g0 = s_gain + abs(ps0 - H);
-          const float* g1 = s_gain + (hasb ? abs(ps1 - H) : 0);
+          const float* g0 = s_gain + (ps0 - (H - C::Q));  // row lag + Q of the gain table
+          const float* g1 = s_gain + (hasb ? ps1 - (H - C::Q) : 0);
 #pragma unroll
           for (int n1 = 0; n1 < N1; ++n1) {
             if (!C::keep(n1)) continue;
             const int q = N2 * n1 + n2, qs = (q + H) % N;
             float r0 = fabsf(x[n1].x) * scale, r1 = fabsf(x[n1].y) * scale;
             if (C::BOXED) {
-              const int lag = 2 * n1 < N1 ? q : N - q;
-              if (gq) {
-                if (N2 == 1 || lag <= C::Q) {  // past Q only for columns no lag is kept of
-                  r0 *= g0[lag * (C::Q + 1)];
-                  r1 *= hasb ? g1[lag * (C::Q + 1)] : 0.f;
-                }
-              } else {
-                r0 *= ld_keep(a.gain + qs * N + ps0);
-                r1 *= hasb ? ld_keep(a.gain + qs * N + ps1) : 0.f;
+              // columns past Q, which no lag is kept of, appear for N2 > 1 only
+              const int gc = 2 * n1 < N1 ? q + C::Q : q + C::Q - N;
+              if (N2 == 1 || (gc >= 0 && gc < GB)) {
+                r0 *= g0[gc * GB];
+                r1 *= g1[gc * GB];
               }
             }
             if (SRCH && (qs < blo || qs > bhi)) r0 = r1 = 0.f;  // lags outside the search range
@@ -814,7 +825,7 @@ __global__ void __launch_bounds__(CorrCfg<N, W, SRCH, VAR>::NT, CorrCfg<N, W, SR
 }
 
 // ---------------------------------------------------------------------------
-template <int N, int W, bool SRCH, int VAR>
+template <int N, int W, bool SRCH, int VAR, bool ANY = true>
 static cudaError_t launch_nw(const CorrArgs& a, cudaStream_t s, int num_sms) {
   using C = CorrCfg<N, W, SRCH, VAR>;
   const size_t sm = C::smem();
@@ -822,24 +833,24 @@ static cudaError_t launch_nw(const CorrArgs& a, cudaStream_t s, int num_sms) {
     return cudaErrorInvalidValue;
   static bool attr_set = false;
   if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(correlate_kernel<N, W, SRCH, VAR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    cudaError_t e = cudaFuncSetAttribute(correlate_kernel<N, W, SRCH, VAR, ANY>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (e != cudaSuccess) return e;
     // the planes live in shared memory: ask for the largest carveout so the
     // register budget, not the L1 split, sets the CTAs per SM
-    e = cudaFuncSetAttribute(correlate_kernel<N, W, SRCH, VAR>, cudaFuncAttributePreferredSharedMemoryCarveout,
+    e = cudaFuncSetAttribute(correlate_kernel<N, W, SRCH, VAR, ANY>, cudaFuncAttributePreferredSharedMemoryCarveout,
                              (int)cudaSharedmemCarveoutMaxShared);
     if (e != cudaSuccess) return e;
     attr_set = true;
   }
   int per_sm = 0;
-  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, correlate_kernel<N, W, SRCH, VAR>, C::NT, sm);
+  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, correlate_kernel<N, W, SRCH, VAR, ANY>, C::NT, sm);
   if (e != cudaSuccess) return e;
   if (per_sm < 1) per_sm = 1;
   const int64_t units = (a.njobs + C::WPC - 1) / C::WPC;
   int64_t grid = (int64_t)per_sm * num_sms;
   if (grid > units) grid = units;
   if (grid < 1) grid = 1;
-  correlate_kernel<N, W, SRCH, VAR><<<(unsigned)grid, C::NT, sm, s>>>(a);
+  correlate_kernel<N, W, SRCH, VAR, ANY><<<(unsigned)grid, C::NT, sm, s>>>(a);
   e = cudaGetLastError();
   if (e == cudaSuccess && a.rec && a.finder == 0 && !a.accumulate) e = launch_peak_epilogue(a, N, s, num_sms);
   return e;
@@ -860,7 +871,8 @@ template <int N, int W> static cudaError_t launch_corr_nw(const CorrArgs& a, cud
     case 2: return launch_nw<N, W, false, 2>(a, s, num_sms);
     case 3: return launch_nw<N, W, false, 3>(a, s, num_sms);
     case 4: return launch_nw<N, W, false, 4>(a, s, num_sms);
-    default: return launch_nw<N, W, false, 0>(a, s, num_sms);
+    default:
+      return a.method == 1 ? launch_nw<N, W, false, 0>(a, s, num_sms) : launch_nw<N, W, false, 0, false>(a, s, num_sms);
   }
 }
 

@@ -27,6 +27,22 @@ __device__ __forceinline__ uint8_t ld_stream(const uint8_t* p) {
   asm("ld.global.nc.L1::no_allocate.u8 %0, [%1];" : "=h"(v) : "l"(p));
   return (uint8_t)v;
 }
+// the same where `on`, else 0, as one predicated load: a branch per pixel
+// would send the loads of a window out one by one
+__device__ __forceinline__ float ld_stream_if(const float* p, bool on) {
+  float v;
+  asm("{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %2, 0;\n\tmov.f32 %0, 0f00000000;\n\t"
+      "@p ld.global.nc.L1::no_allocate.f32 %0, [%1];\n\t}"
+      : "=f"(v) : "l"(p), "r"((int)on));
+  return v;
+}
+__device__ __forceinline__ uint8_t ld_stream_if(const uint8_t* p, bool on) {
+  unsigned short v;
+  asm("{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %2, 0;\n\tmov.u16 %0, 0;\n\t"
+      "@p ld.global.nc.L1::no_allocate.u8 %0, [%1];\n\t}"
+      : "=h"(v) : "l"(p), "r"((int)on));
+  return (uint8_t)v;
+}
 __device__ __forceinline__ float ld_keep(const float* p) {
   float v;
   asm("ld.global.nc.L1::evict_last.f32 %0, [%1];" : "=f"(v) : "l"(p));

@@ -9,6 +9,7 @@ loads it. Objects go to _build/ (not committed). Usage:
 import argparse
 import concurrent.futures as cf
 import os
+import re
 import shutil
 import subprocess
 import sys
@@ -31,6 +32,18 @@ def nvcc():
     return path
 
 
+def _includes(path, seen):
+    """The project headers that `path` includes, directly or through others."""
+    with open(path) as f:
+        for name in re.findall(r'^\s*#include "([^"]+)"', f.read(), re.M):
+            for d in (CSRC, os.path.join(ROOT, "include")):
+                p = os.path.join(d, name)
+                if os.path.exists(p) and p not in seen:
+                    seen.add(p)
+                    _includes(p, seen)
+    return seen
+
+
 def _stale(src, obj, deps):
     if not os.path.exists(obj):
         return True
@@ -41,8 +54,6 @@ def _stale(src, obj, deps):
 def build(force=False, verbose=False, jobs=None):
     os.makedirs(BUILD, exist_ok=True)
     sources = sorted(f for f in os.listdir(CSRC) if f.endswith(".cu"))
-    headers = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cuh", ".h"))]
-    headers.append(os.path.join(ROOT, "include", "hammerhead_b200.h"))
     cc = nvcc()
     todo = []
     objs = []
@@ -50,7 +61,7 @@ def build(force=False, verbose=False, jobs=None):
         src = os.path.join(CSRC, s)
         obj = os.path.join(BUILD, s.replace(".cu", ".o"))
         objs.append(obj)
-        if force or _stale(src, obj, headers):
+        if force or _stale(src, obj, list(_includes(src, set()))):
             todo.append((src, obj))
 
     def compile_one(item):

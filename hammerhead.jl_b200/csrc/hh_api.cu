@@ -551,11 +551,12 @@ hh_status hh_ncc_loss_grad(hh_ctx* ctx, const float* P, int32_t gny, int32_t gnx
     HH_CK(cudaMemcpyAsync(dP, P, G2 * sizeof(float), cudaMemcpyHostToDevice, s));
     a.P = dP;
   }
-  HH_TRY(buf(ctx, "ncc_wstat", (size_t)6 * a.wy * a.wx, &a.wstat));
+  HH_TRY(buf(ctx, "ncc_wstat", (size_t)hh::ncc_wstat_words(a.wy, a.wx), &a.wstat));
   HH_TRY(buf(ctx, "ncc_loss", 1, &a.loss));
   float* dG = nullptr;
   if (dLdP) {
     HH_TRY(buf(ctx, "ncc_gpix", (size_t)2 * Px, &a.gpix));
+    HH_TRY(buf(ctx, "ncc_cells", (size_t)2 * (ctx->nr + ctx->nc), &a.cells));
     if (device_ptrs) {
       a.grad = dLdP;
     } else {

@@ -213,11 +213,13 @@ struct NccArgs {
   float y0, ysp, x0, xsp;
   int32_t W, step;  // windows: W x W at origins (jr * step, jc * step)
   int32_t wy, wx;   // window grid
-  double* wstat;    // 6 per window (scratch)
+  double* wstat;    // ncc_wstat_words (scratch): 6 per window, then a sum per tile of windows
   float* gpix;      // 2 x nr x nc pixel gradient (scratch), when grad
+  int32_t* cells;   // predictor cell and fraction bits per row, then per column (scratch), when grad
   float* grad;      // 2 x gny x gnx dL/dP, or nullptr (loss only)
   double* loss;     // device scalar
 };
+int64_t ncc_wstat_words(int32_t wy, int32_t wx);
 cudaError_t launch_ncc_loss_grad(const NccArgs& a, cudaStream_t s);
 
 }  // namespace hh

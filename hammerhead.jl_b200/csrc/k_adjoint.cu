@@ -7,18 +7,27 @@
 // WIDIM sweep deforms it (bilinear predictor with flat extrapolation, cubic
 // B-spline samples at -+ (u, v)/2; deform_columns!, src/pipeline.jl:957-965).
 //
-// Three launches, no atomics, no stored deformed image:
-//   1. per window (one CTA): recompute the deformed window, FP64 moments,
-//      and the window constants of the gradient;
+// Three launches (and the loss), no atomics, no stored deformed image:
+//   1. per tile of neighbouring windows (one CTA): the tile's pixels deformed
+//      once into shared memory, then FP64 moments and the window constants of
+//      the gradient, a warp per window;
 //   2. per pixel: recompute the deformed samples and their B-spline
 //      derivatives, sum dL/da, dL/db over the windows holding the pixel,
 //      chain through -+ 1/2 to the pixel displacement gradient (gu, gv);
 //   3. per node: the transpose of the bilinear predictor interpolation,
-//      gathered over the node's support in FP64.
+//      gathered over the node's support in FP64, axis by axis.
+// Bound by issue. Windows at 50 % overlap share each pixel four times; a CTA
+// per window deformed it each time and spent as long on its ten block-wide
+// barriers. The predictor's cell and fraction along an axis (two divisions)
+// depend on the row or the column alone, so they are formed once per row and
+// column of a tile, and the B-spline weights divide by 6 without a division.
+// 1024^2, 16 px windows at 50 %, P 127 x 127, loss and gradient: 295 us a
+// call in the earlier form, 113 us now.
 #include <math.h>
 #include <stdint.h>
 
 #include "hh_internal.h"
+#include "hh_spline.cuh"
 
 namespace hh {
 
@@ -26,10 +35,10 @@ namespace {
 
 __device__ __forceinline__ void cubw_f(float d, float* w) {
   const float x3 = d * d * d, c = 1.f - d, c3 = c * c * c;
-  w[0] = c3 / 6.f;
+  w[0] = div6(c3);
   w[1] = 2.f / 3.f - d * d + x3 / 2.f;
   w[2] = 2.f / 3.f - c * c + c3 / 2.f;
-  w[3] = x3 / 6.f;
+  w[3] = div6(x3);
 }
 // d/dd of the cubic B-spline weights
 __device__ __forceinline__ void cubw_df(float d, float* w) {
@@ -93,26 +102,33 @@ __device__ __forceinline__ void lin_axis_f(float q, float q0, float step, int n,
   d = __fdiv_rn(__fsub_rn(q, k0), __fsub_rn(k1, k0));
 }
 
-__device__ __forceinline__ float bilin(const float* f, const NccArgs& a, float qy, float qx) {
-  int iy, ix;
-  float dy, dx;
-  lin_axis_f(qy, a.y0, a.ysp, a.gny, iy, dy);
-  lin_axis_f(qx, a.x0, a.xsp, a.gnx, ix, dx);
-  const int iy2 = a.gny == 1 ? iy : iy + 1, ix2 = a.gnx == 1 ? ix : ix + 1;
-  const float f00 = f[iy + ix * a.gny], f01 = f[iy + ix2 * a.gny], f10 = f[iy2 + ix * a.gny],
+// where a pixel row or column falls on the predictor's nodes
+struct Cell {
+  int i;    // cell
+  float d;  // fraction
+};
+__device__ __forceinline__ Cell cell_at(float q, float q0, float step, int n) {
+  Cell c;
+  lin_axis_f(q, q0, step, n, c.i, c.d);
+  return c;
+}
+
+__device__ __forceinline__ float bilin(const float* f, const NccArgs& a, Cell y, Cell x) {
+  const int iy2 = a.gny == 1 ? y.i : y.i + 1, ix2 = a.gnx == 1 ? x.i : x.i + 1;
+  const float f00 = f[y.i + x.i * a.gny], f01 = f[y.i + ix2 * a.gny], f10 = f[iy2 + x.i * a.gny],
               f11 = f[iy2 + ix2 * a.gny];
-  const float p = __fadd_rn(__fmul_rn(__fsub_rn(1.f, dx), f00), __fmul_rn(dx, f01));
-  const float q = __fadd_rn(__fmul_rn(__fsub_rn(1.f, dx), f10), __fmul_rn(dx, f11));
-  return __fadd_rn(__fmul_rn(__fsub_rn(1.f, dy), p), __fmul_rn(dy, q));
+  const float p = __fadd_rn(__fmul_rn(__fsub_rn(1.f, x.d), f00), __fmul_rn(x.d, f01));
+  const float q = __fadd_rn(__fmul_rn(__fsub_rn(1.f, x.d), f10), __fmul_rn(x.d, f11));
+  return __fadd_rn(__fmul_rn(__fsub_rn(1.f, y.d), p), __fmul_rn(y.d, q));
 }
 
 // deformed samples of pixel (r, c) (0-based) of both frames
 template <bool GRAD>
-__device__ __forceinline__ void deformed(const NccArgs& a, int64_t r, int64_t c, float& va, float& vb, float& ay,
-                                         float& ax, float& by, float& bx) {
+__device__ __forceinline__ void deformed(const NccArgs& a, int64_t r, int64_t c, Cell y, Cell x, float& va, float& vb,
+                                         float& ay, float& ax, float& by, float& bx) {
   const float R = (float)(r + 1), Cc = (float)(c + 1);
-  const float u2 = __fdiv_rn(bilin(a.P, a, R, Cc), 2.f);
-  const float v2 = __fdiv_rn(bilin(a.P + (int64_t)a.gny * a.gnx, a, R, Cc), 2.f);
+  const float u2 = __fmul_rn(bilin(a.P, a, y, x), 0.5f);
+  const float v2 = __fmul_rn(bilin(a.P + (int64_t)a.gny * a.gnx, a, y, x), 0.5f);
   va = bs_sample<GRAD>(a.CA, a.nr, a.nc, __fsub_rn(R, v2), __fsub_rn(Cc, u2), ay, ax);
   vb = bs_sample<GRAD>(a.CB, a.nr, a.nc, __fadd_rn(R, v2), __fadd_rn(Cc, u2), by, bx);
 }
@@ -130,160 +146,256 @@ __device__ __forceinline__ double block_sum(double v, double* red) {
   return t;
 }
 
-// 1. window constants: ncc, abar, bbar, inv = 1/sqrt(Saa Sbb), ca = ncc/Saa, cb = ncc/Sbb
-template <int PPT>
-__global__ void __launch_bounds__(NCC_THREADS) ncc_window_kernel(const NccArgs a) {
-  __shared__ double red[NCC_THREADS / 32];
-  const int W = a.W, n = W * W;
-  const int64_t nwin = (int64_t)a.wy * a.wx;
-  for (int64_t j = blockIdx.x; j < nwin; j += gridDim.x) {
-    const int64_t rs = (j % a.wy) * a.step, cs = (j / a.wy) * a.step;
-    float va[PPT], vb[PPT];
+__device__ __forceinline__ double warp_sum_d(double v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// Windows of a tile along one axis: as many as fit the side. 64 px (a tile's
+// deformed pixels, float2, take 33 KB) leave 6 CTAs per SM and, at 1024^2 with
+// 16 px windows, more CTAs than SMs, while a pixel is deformed 1.3 times on
+// average; sides of 96 px deform 1.2 times but leave one CTA per SM there
+// (53 us against 40 us). Windows above 32 px need the larger side to share.
+__host__ __device__ __forceinline__ int tile_windows(int W, int step) { return 1 + ((W <= 32 ? 64 : 96) - W) / step; }
+__host__ __device__ __forceinline__ int tile_side(int W, int step) { return W + (tile_windows(W, step) - 1) * step; }
+constexpr int NCC_SIDE = 96;  // the largest
+static size_t tile_smem(int W, int step) {
+  const size_t n = tile_side(W, step);
+  return n * (n + 1) * sizeof(float2) + 2 * n * sizeof(Cell) + NCC_THREADS / 32 * sizeof(double);
+}
+
+// 1. window constants: ncc, abar, bbar, inv = 1/sqrt(Saa Sbb), ca = ncc/Saa, cb = ncc/Sbb;
+//    and per CTA the sum of its ncc (after the constants of all windows)
+__global__ void __launch_bounds__(NCC_THREADS) ncc_tile_kernel(const NccArgs a) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int W = a.W, n = W * W, TW = tile_windows(W, a.step), side = tile_side(W, a.step), ld = side + 1;
+  float2* T = reinterpret_cast<float2*>(smem_raw);  // column c of the tile at c * ld
+  Cell* ry = reinterpret_cast<Cell*>(T + side * ld);
+  Cell* cx = ry + side;
+  double* part = reinterpret_cast<double*>(cx + side);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int jr0 = blockIdx.x * TW, jc0 = blockIdx.y * TW;
+  const int ty = min(TW, a.wy - jr0), tx = min(TW, a.wx - jc0);           // windows of this tile
+  const int rt = W + (ty - 1) * a.step, ct = W + (tx - 1) * a.step;       // its pixels
+  const int64_t r0 = (int64_t)jr0 * a.step, c0 = (int64_t)jc0 * a.step;
+  for (int k = tid; k < rt + ct; k += NCC_THREADS) {
+    if (k < rt) ry[k] = cell_at((float)(r0 + k + 1), a.y0, a.ysp, a.gny);
+    else cx[k - rt] = cell_at((float)(c0 + k - rt + 1), a.x0, a.xsp, a.gnx);
+  }
+  __syncthreads();
+  // k / rt as a multiplication, exact for k rt < 2^22 (k < 96^2)
+  const uint32_t inv_rt = (1u << 22) / rt + 1;
+  for (int k = tid; k < rt * ct; k += NCC_THREADS) {
+    const int c = (int)(((uint32_t)k * inv_rt) >> 22), r = k - c * rt;
+    float2 v;
+    float d0, d1, d2, d3;
+    deformed<false>(a, r0 + r, c0 + c, ry[r], cx[c], v.x, v.y, d0, d1, d2, d3);
+    T[c * ld + r] = v;
+  }
+  __syncthreads();
+  const uint32_t inv_w = (1u << 20) / W + 1;  // k / W, exact for k W < 2^20 (k < 64^2)
+  double loss = 0.0;
+  for (int w = warp; w < ty * tx; w += NCC_THREADS / 32) {
+    const int wr = w % ty, wc = w / ty;
+    const float2* B = T + wc * a.step * ld + wr * a.step;
     double sa = 0.0, sb = 0.0;
-#pragma unroll
-    for (int i = 0; i < PPT; ++i) {
-      const int k = threadIdx.x + i * NCC_THREADS;
-      va[i] = vb[i] = 0.f;
-      if (k < n) {
-        float d0, d1, d2, d3;
-        deformed<false>(a, rs + k % W, cs + k / W, va[i], vb[i], d0, d1, d2, d3);
-        sa += (double)va[i];
-        sb += (double)vb[i];
-      }
+#pragma unroll 4
+    for (int k = lane; k < n; k += 32) {
+      const int q = (int)(((uint32_t)k * inv_w) >> 20);
+      const float2 v = B[q * ld + k - q * W];
+      sa += (double)v.x;
+      sb += (double)v.y;
     }
-    const double ma = block_sum(sa, red) / n, mb = block_sum(sb, red) / n;
+    const double ma = warp_sum_d(sa) / n, mb = warp_sum_d(sb) / n;
     double saa = 0.0, sbb = 0.0, sab = 0.0;
-#pragma unroll
-    for (int i = 0; i < PPT; ++i) {
-      const int k = threadIdx.x + i * NCC_THREADS;
-      if (k < n) {
-        const double da = (double)va[i] - ma, db = (double)vb[i] - mb;
-        saa += da * da;
-        sbb += db * db;
-        sab += da * db;
-      }
+#pragma unroll 4
+    for (int k = lane; k < n; k += 32) {
+      const int q = (int)(((uint32_t)k * inv_w) >> 20);
+      const float2 v = B[q * ld + k - q * W];
+      const double da = (double)v.x - ma, db = (double)v.y - mb;
+      saa += da * da;
+      sbb += db * db;
+      sab += da * db;
     }
-    saa = block_sum(saa, red);
-    sbb = block_sum(sbb, red);
-    sab = block_sum(sab, red);
-    if (threadIdx.x == 0) {
-      double* o = a.wstat + 6 * j;
-      if (saa > 0 && sbb > 0) {
-        const double inv = 1.0 / sqrt(saa * sbb), ncc = sab * inv;
-        o[0] = ncc;
-        o[1] = ma;
-        o[2] = mb;
-        o[3] = inv;
-        o[4] = ncc / saa;
-        o[5] = ncc / sbb;
-      } else {  // a flat window contributes nothing
-        o[0] = o[1] = o[2] = o[3] = o[4] = o[5] = 0.0;
-      }
+    saa = warp_sum_d(saa);
+    sbb = warp_sum_d(sbb);
+    sab = warp_sum_d(sab);
+    const bool flat = !(saa > 0 && sbb > 0);  // a flat window contributes nothing
+    const double inv = flat ? 0.0 : 1.0 / sqrt(saa * sbb), ncc = flat ? 0.0 : sab * inv;
+    loss += ncc;
+    if (lane == 0) {
+      double* o = a.wstat + 6 * ((int64_t)(jr0 + wr) + (int64_t)(jc0 + wc) * a.wy);
+      o[0] = ncc;
+      o[1] = flat ? 0.0 : ma;
+      o[2] = flat ? 0.0 : mb;
+      o[3] = inv;
+      o[4] = flat ? 0.0 : ncc / saa;
+      o[5] = flat ? 0.0 : ncc / sbb;
     }
+  }
+  if (lane == 0) part[warp] = loss;
+  __syncthreads();
+  if (tid == 0) {
+    double t = 0.0;
+    for (int k = 0; k < NCC_THREADS / 32; ++k) t += part[k];
+    a.wstat[6 * (int64_t)a.wy * a.wx + blockIdx.x + (int64_t)blockIdx.y * gridDim.x] = t;
   }
 }
 
-// 2. pixel displacement gradient (gu, gv) = dL/d(u, v) at every pixel
-__global__ void __launch_bounds__(256) ncc_pixel_kernel(const NccArgs a) {
-  const int64_t P = a.nr * a.nc;
-  for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < P; k += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t r = k % a.nr, c = k / a.nr;
-    // windows j = (jr, jc) with jr*step <= r < jr*step + W
-    const int64_t jr0 = r - a.W + 1 <= 0 ? 0 : (r - a.W + 1 + a.step - 1) / a.step;
-    const int64_t jr1 = min((int64_t)a.wy - 1, r / a.step);
-    const int64_t jc0 = c - a.W + 1 <= 0 ? 0 : (c - a.W + 1 + a.step - 1) / a.step;
-    const int64_t jc1 = min((int64_t)a.wx - 1, c / a.step);
-    float gu = 0.f, gv = 0.f;
-    if (jr0 <= jr1 && jc0 <= jc1) {
-      float va, vb, ay, ax, by, bx;
-      deformed<true>(a, r, c, va, vb, ay, ax, by, bx);
-      double ga = 0.0, gb = 0.0;
-      for (int64_t jc = jc0; jc <= jc1; ++jc)
-        for (int64_t jr = jr0; jr <= jr1; ++jr) {
-          const double* s = a.wstat + 6 * (jr + jc * a.wy);
-          const double da = (double)va - s[1], db = (double)vb - s[2];
-          ga += -db * s[3] + s[4] * da;
-          gb += -da * s[3] + s[5] * db;
+// 2. pixel displacement gradient (gu, gv) = dL/d(u, v) at every pixel: a
+//    thread keeps its row and walks NCC_PC columns, so what belongs to a row
+//    (predictor cell, windows that hold it) or to a column is formed once
+constexpr int NCC_PR = 128, NCC_PC = 8;
+struct Span {
+  int j0, j1;  // windows j0..j1 hold the row or column
+};
+__device__ __forceinline__ Span span_at(int64_t p, int W, int step, int nw) {
+  return Span{p < W ? 0 : (int)((p - W) / step + 1), min(nw - 1, (int)(p / step))};
+}
+__global__ void __launch_bounds__(NCC_PR) ncc_pixel_kernel(const NccArgs a) {
+  __shared__ Cell cx[NCC_PC];
+  __shared__ Span cw[NCC_PC];
+  const int64_t P = a.nr * a.nc, r = (int64_t)blockIdx.x * NCC_PR + threadIdx.x, c0 = (int64_t)blockIdx.y * NCC_PC;
+  const int nc = (int)min((int64_t)NCC_PC, a.nc - c0);
+  if (threadIdx.x < nc) {
+    cx[threadIdx.x] = cell_at((float)(c0 + threadIdx.x + 1), a.x0, a.xsp, a.gnx);
+    cw[threadIdx.x] = span_at(c0 + threadIdx.x, a.W, a.step, a.wx);
+  }
+  __syncthreads();
+  if (r >= a.nr) return;
+  const Cell y = cell_at((float)(r + 1), a.y0, a.ysp, a.gny);
+  // the rows' and columns' cells, for the node kernel
+  if (blockIdx.y == 0) {
+    a.cells[2 * r] = y.i;
+    a.cells[2 * r + 1] = __float_as_int(y.d);
+  }
+  if (blockIdx.x == 0 && threadIdx.x < nc) {
+    a.cells[2 * (a.nr + c0 + threadIdx.x)] = cx[threadIdx.x].i;
+    a.cells[2 * (a.nr + c0 + threadIdx.x) + 1] = __float_as_int(cx[threadIdx.x].d);
+  }
+  const Span rw = span_at(r, a.W, a.step, a.wy);
+  // dL/da = sum_j -(b - bbar_j) inv_j + ca_j (a - abar_j) over the windows j
+  // that hold the pixel, dL/db likewise: the sums of the constants change only
+  // with the set of windows, every `step` columns
+  double si = 0.0, sca = 0.0, scb = 0.0, ka = 0.0, kb = 0.0;
+  for (int k = 0; k < nc; ++k) {
+    const int64_t c = c0 + k;
+    if (k == 0 || cw[k].j0 != cw[k - 1].j0 || cw[k].j1 != cw[k - 1].j1) {
+      si = sca = scb = ka = kb = 0.0;
+      for (int jc = cw[k].j0; jc <= cw[k].j1; ++jc)
+        for (int jr = rw.j0; jr <= rw.j1; ++jr) {
+          const double* s = a.wstat + 6 * ((int64_t)jr + (int64_t)jc * a.wy);
+          si += s[3];
+          sca += s[4];
+          scb += s[5];
+          ka += s[2] * s[3] - s[4] * s[1];
+          kb += s[1] * s[3] - s[5] * s[2];
         }
+    }
+    float gu = 0.f, gv = 0.f;
+    if (rw.j0 <= rw.j1 && cw[k].j0 <= cw[k].j1) {
+      float va, vb, ay, ax, by, bx;
+      deformed<true>(a, r, c, y, cx[k], va, vb, ay, ax, by, bx);
+      const double ga = sca * (double)va - si * (double)vb + ka, gb = scb * (double)vb - si * (double)va + kb;
       const float fa = (float)ga, fb = (float)gb;
       gu = fa * (-0.5f * ax) + fb * (0.5f * bx);
       gv = fa * (-0.5f * ay) + fb * (0.5f * by);
     }
-    a.gpix[k] = gu;
-    a.gpix[P + k] = gv;
+    a.gpix[r + c * a.nr] = gu;
+    a.gpix[P + r + c * a.nr] = gv;
   }
 }
 
-// bilinear weight of node g for query q (flat outside)
-__device__ __forceinline__ float node_w(float q, float q0, float step, int n, int g) {
-  int i;
-  float d;
-  lin_axis_f(q, q0, step, n, i, d);
-  const int i2 = n == 1 ? i : i + 1;
-  return (i == g ? 1.f - d : 0.f) + (i2 == g ? d : 0.f);
+// 3. dL/dP at every node: the transpose of the bilinear interpolation, axis by
+//    axis. A CTA takes NODE_R x NODE_C nodes and walks the image columns of
+//    their support NODE_K at a time: first each (node row, column) sums its
+//    rows, then each node its columns. (A warp per node read every pixel of a
+//    node's support for itself, a third of its lanes idle, and formed the
+//    weights again for each node: 48 us at 1024^2 against 21 us.)
+constexpr int NODE_R = 16, NODE_C = 8, NODE_K = 32, NODE_THREADS = 256;
+struct Reach {
+  int64_t lo, hi;  // 1-based pixels whose stencil may reach the node
+};
+__device__ __forceinline__ Reach reach_of(int g, int n, float q0, float step, int64_t np) {
+  return Reach{g == 0 ? 1 : max((int64_t)1, (int64_t)floorf(q0 + (g - 1) * step)),
+               g == n - 1 ? np : min(np, (int64_t)ceilf(q0 + (g + 1) * step))};
 }
-
-// 3. dL/dP at every node: the transpose of the bilinear interpolation
-__global__ void __launch_bounds__(256) ncc_node_kernel(const NccArgs a) {
-  const int64_t G = (int64_t)a.gny * a.gnx;
-  for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < 2 * G; k += (int64_t)gridDim.x * blockDim.x) {
-    const int comp = (int)(k / G);
-    const int64_t node = k % G;
-    const int gy = (int)(node % a.gny), gx = (int)(node / a.gny);
-    // 1-based pixel rows / columns whose stencil may reach the node
-    const int64_t r_lo = gy == 0 ? 1 : max((int64_t)1, (int64_t)floorf(a.y0 + (gy - 1) * a.ysp));
-    const int64_t r_hi = gy == a.gny - 1 ? a.nr : min(a.nr, (int64_t)ceilf(a.y0 + (gy + 1) * a.ysp));
-    const int64_t c_lo = gx == 0 ? 1 : max((int64_t)1, (int64_t)floorf(a.x0 + (gx - 1) * a.xsp));
-    const int64_t c_hi = gx == a.gnx - 1 ? a.nc : min(a.nc, (int64_t)ceilf(a.x0 + (gx + 1) * a.xsp));
-    const float* g = a.gpix + comp * a.nr * a.nc;
-    double acc = 0.0;
-    for (int64_t C = c_lo; C <= c_hi; ++C) {
-      const float wx = node_w((float)C, a.x0, a.xsp, a.gnx, gx);
-      if (wx == 0.f) continue;
-      double col = 0.0;
-      for (int64_t R = r_lo; R <= r_hi; ++R) {
-        const float wy = node_w((float)R, a.y0, a.ysp, a.gny, gy);
-        if (wy != 0.f) col += (double)wy * (double)g[(R - 1) + (C - 1) * a.nr];
+// weight of node g in the cell of pixel p (0-based), which has n nodes
+__device__ __forceinline__ float cell_w(const int* cells, int64_t p, int g, int n) {
+  const int i = cells[2 * p];
+  const float d = __int_as_float(cells[2 * p + 1]);
+  return (i == g ? 1.f - d : 0.f) + ((n == 1 ? i : i + 1) == g ? d : 0.f);
+}
+__global__ void __launch_bounds__(NODE_THREADS) ncc_node_kernel(const NccArgs a) {
+  __shared__ double t[2][NODE_K][NODE_R + 1];
+  const int64_t G = (int64_t)a.gny * a.gnx, P = a.nr * a.nc;
+  const int gy0 = blockIdx.x * NODE_R, gx0 = blockIdx.y * NODE_C;
+  const int64_t c_lo = reach_of(gx0, a.gnx, a.x0, a.xsp, a.nc).lo;
+  const int64_t c_hi = reach_of(min(gx0 + NODE_C, a.gnx) - 1, a.gnx, a.x0, a.xsp, a.nc).hi;
+  // this thread's node and component in the second step
+  const int ny = threadIdx.x % NODE_R, nx = threadIdx.x / NODE_R % NODE_C, comp = threadIdx.x / (NODE_R * NODE_C);
+  const int gx = gx0 + nx;
+  const Reach cr = reach_of(min(gx, a.gnx - 1), a.gnx, a.x0, a.xsp, a.nc);
+  double acc = 0.0;
+  for (int64_t cb = c_lo; cb <= c_hi; cb += NODE_K) {
+    for (int e = threadIdx.x; e < NODE_R * NODE_K; e += NODE_THREADS) {
+      const int gy = gy0 + e % NODE_R, k = e / NODE_R;
+      double su = 0.0, sv = 0.0;
+      if (gy < a.gny && cb + k <= c_hi) {
+        const Reach rr = reach_of(gy, a.gny, a.y0, a.ysp, a.nr);
+        const float* g = a.gpix + (cb + k - 1) * a.nr - 1;
+#pragma unroll 6
+        for (int64_t R = rr.lo; R <= rr.hi; ++R) {
+          const float w = cell_w(a.cells, R - 1, gy, a.gny);
+          const bool on = w != 0.f;  // a pixel without weight does not count (it may hold NaN)
+          su += (double)w * (double)(on ? g[R] : 0.f);
+          sv += (double)w * (double)(on ? g[P + R] : 0.f);
+        }
       }
-      acc += (double)wx * col;
+      t[0][k][e % NODE_R] = su;
+      t[1][k][e % NODE_R] = sv;
     }
-    a.grad[k] = (float)acc;
+    __syncthreads();
+    const int k0 = (int)max((int64_t)0, cr.lo - cb), k1 = (int)min((int64_t)NODE_K - 1, cr.hi - cb);
+    for (int k = k0; k <= k1; ++k) {
+      const float w = cell_w(a.cells, a.nr + cb + k - 1, gx, a.gnx);
+      if (w != 0.f) acc += (double)w * t[comp][k][ny];
+    }
+    __syncthreads();
   }
+  if (gy0 + ny < a.gny && gx < a.gnx) a.grad[comp * G + (gy0 + ny) + (int64_t)gx * a.gny] = (float)acc;
 }
 
-// loss = -sum of the window correlations, in window order (one CTA)
-__global__ void __launch_bounds__(NCC_THREADS) ncc_loss_kernel(const NccArgs a) {
+// loss = -sum of the tiles' sums (one CTA)
+__global__ void __launch_bounds__(NCC_THREADS) ncc_loss_kernel(const NccArgs a, int64_t ntiles) {
   __shared__ double red[NCC_THREADS / 32];
-  const int64_t nwin = (int64_t)a.wy * a.wx;
+  const double* part = a.wstat + 6 * (int64_t)a.wy * a.wx;
   double s = 0.0;
-  for (int64_t j = threadIdx.x; j < nwin; j += NCC_THREADS) s += a.wstat[6 * j];
+  for (int64_t j = threadIdx.x; j < ntiles; j += NCC_THREADS) s += part[j];
   s = block_sum(s, red);
   if (threadIdx.x == 0) *a.loss = -s;
 }
 
-template <int PPT> static void launch_win(const NccArgs& a, int64_t nwin, cudaStream_t s) {
-  const int64_t grid = nwin < 148 * 8 ? nwin : 148 * 8;
-  ncc_window_kernel<PPT><<<(unsigned)grid, NCC_THREADS, 0, s>>>(a);
-}
-
 }  // namespace
 
+int64_t ncc_wstat_words(int32_t wy, int32_t wx) { return 7 * (int64_t)wy * wx; }  // at most a tile per window
+
 cudaError_t launch_ncc_loss_grad(const NccArgs& a, cudaStream_t s) {
-  const int64_t nwin = (int64_t)a.wy * a.wx;
-  if (nwin <= 0 || a.W < 2) return cudaErrorInvalidValue;
-  const int n = a.W * a.W;
-  if (n <= NCC_THREADS) launch_win<1>(a, nwin, s);
-  else if (n <= 4 * NCC_THREADS) launch_win<4>(a, nwin, s);
-  else if (n <= 16 * NCC_THREADS) launch_win<16>(a, nwin, s);
-  else return cudaErrorInvalidValue;
-  ncc_loss_kernel<<<1, NCC_THREADS, 0, s>>>(a);
+  if (a.wy < 1 || a.wx < 1 || a.W < 2 || a.W > 64 || a.step < 1) return cudaErrorInvalidValue;
+  const size_t sm = tile_smem(a.W, a.step);
+  cudaError_t e = cudaFuncSetAttribute(ncc_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)(NCC_SIDE * (NCC_SIDE + 1) * sizeof(float2) + 4096));
+  if (e != cudaSuccess) return e;
+  const int TW = tile_windows(a.W, a.step);
+  const dim3 tiles((a.wy + TW - 1) / TW, (a.wx + TW - 1) / TW);
+  ncc_tile_kernel<<<tiles, NCC_THREADS, sm, s>>>(a);
+  ncc_loss_kernel<<<1, NCC_THREADS, 0, s>>>(a, (int64_t)tiles.x * tiles.y);
   if (a.grad) {
-    const int64_t P = a.nr * a.nc, G2 = 2 * (int64_t)a.gny * a.gnx;
-    int64_t b1 = (P + 255) / 256, b2 = (G2 + 255) / 256;
-    if (b1 > 148 * 16) b1 = 148 * 16;
-    if (b2 > 148 * 16) b2 = 148 * 16;
-    ncc_pixel_kernel<<<(unsigned)b1, 256, 0, s>>>(a);
-    ncc_node_kernel<<<(unsigned)(b2 < 1 ? 1 : b2), 256, 0, s>>>(a);
+    const dim3 px((unsigned)((a.nr + NCC_PR - 1) / NCC_PR), (unsigned)((a.nc + NCC_PC - 1) / NCC_PC));
+    ncc_pixel_kernel<<<px, NCC_PR, 0, s>>>(a);
+    const dim3 nodes((a.gny + NODE_R - 1) / NODE_R, (a.gnx + NODE_C - 1) / NODE_C);
+    ncc_node_kernel<<<nodes, NODE_THREADS, 0, s>>>(a);
   }
   return cudaGetLastError();
 }

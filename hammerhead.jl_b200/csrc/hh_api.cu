@@ -11,8 +11,8 @@ namespace hhd {
 // The device-resident schedule: run_piv + piv_pass with every sweep, the
 // deformation, validation and uncertainty on the context stream.
 hh_status run_schedule(hh_ctx* ctx, const float* dA, const float* dB, int64_t nr, int64_t nc,
-                       const hh_pass_desc* passes, int np, const uint8_t* hmask, const uint8_t* dmask, double thr,
-                       bool smoothing, hh_result* out) {
+                       const hh_pass_desc* passes, int np, const uint8_t* dmask, double thr, bool smoothing,
+                       hh_result* out) {
   cudaStream_t s = ctx->stream;
   HH_TRY(check_passes(ctx, passes, np));
   if (nr < 1 || nc < 1) return fail(ctx, HH_ERR_ARG, "images must be non-empty");
@@ -26,28 +26,25 @@ hh_status run_schedule(hh_ctx* ctx, const float* dA, const float* dB, int64_t nr
     HH_TRY(buf(ctx, "warpA", (size_t)P, &warpA));
     HH_TRY(buf(ctx, "warpB", (size_t)P, &warpB));
   }
-  // grids of every pass (host) and the largest grid
-  std::vector<Grid> grids(np);
+  std::vector<Grid> grids;
+  HH_TRY(pass_grids(ctx, nr, nc, passes, np, dmask, thr, grids));
   int64_t Gmax = 1, Jmax = 1;
   int nalt_max = 0;
   for (int k = 0; k < np; ++k) {
-    HH_TRY(make_grid(ctx, nr, nc, passes[k], hmask, thr, grids[k]));
-    Gmax = std::max<int64_t>(Gmax, (int64_t)grids[k].ny * grids[k].nx);
-    Jmax = std::max<int64_t>(Jmax, (int64_t)grids[k].jobs.size() / 4);
+    Gmax = std::max<int64_t>(Gmax, grids[k].G());
+    Jmax = std::max<int64_t>(Jmax, grid_njobs(grids[k]));
     nalt_max = std::max(nalt_max, passes[k].n_peaks - 1);
   }
-  float *u, *v, *resu, *resv, *ratio, *moment, *uncu, *uncv, *altu = nullptr, *altv = nullptr;
-  float *predu, *predv, *predw_u, *predw_v, *prevu, *prevv, *measu, *measv, *dx, *dy, *fc, *fcout;
-  uint8_t *outl, *outl2, *gm;
+  ResultBlock rb;
+  HH_TRY(result_block(ctx, Gmax, rb));
+  float *u = rb.u, *v = rb.v, *ratio = rb.ratio, *moment = rb.moment, *uncu = rb.uncu, *uncv = rb.uncv;
+  uint8_t* outl = rb.outl;
+  float *resu, *resv, *altu = nullptr, *altv = nullptr;
+  float *predu, *predv, *predw_u, *predw_v, *prevu, *prevv, *measu, *measv, *fc, *fcout;
+  uint8_t *outl2, *gm;
   int32_t* djobs;
-  HH_TRY(buf(ctx, "u", Gmax, &u));
-  HH_TRY(buf(ctx, "v", Gmax, &v));
   HH_TRY(buf(ctx, "resu", Gmax, &resu));
   HH_TRY(buf(ctx, "resv", Gmax, &resv));
-  HH_TRY(buf(ctx, "ratio", Gmax, &ratio));
-  HH_TRY(buf(ctx, "moment", Gmax, &moment));
-  HH_TRY(buf(ctx, "uncu", Gmax, &uncu));
-  HH_TRY(buf(ctx, "uncv", Gmax, &uncv));
   if (nalt_max > 0) {
     HH_TRY(buf(ctx, "altu", Gmax * nalt_max, &altu));
     HH_TRY(buf(ctx, "altv", Gmax * nalt_max, &altv));
@@ -60,11 +57,8 @@ hh_status run_schedule(hh_ctx* ctx, const float* dA, const float* dB, int64_t nr
   HH_TRY(buf(ctx, "prevv", Gmax, &prevv));
   HH_TRY(buf(ctx, "measu", Gmax, &measu));
   HH_TRY(buf(ctx, "measv", Gmax, &measv));
-  HH_TRY(buf(ctx, "gx", Gmax, &dx));
-  HH_TRY(buf(ctx, "gy", Gmax, &dy));
   HH_TRY(buf(ctx, "fc", Gmax + 64, &fc));
   HH_TRY(buf(ctx, "fcout", 4, &fcout));
-  HH_TRY(buf(ctx, "outl", Gmax, &outl));
   HH_TRY(buf(ctx, "outl2", Gmax, &outl2));
   HH_TRY(buf(ctx, "gmask", Gmax, &gm));
   HH_TRY(buf(ctx, "jobs", 4 * Jmax, &djobs));
@@ -96,52 +90,29 @@ hh_status run_schedule(hh_ctx* ctx, const float* dA, const float* dB, int64_t nr
     const bool force_replace = k < np - 1;
     const int ny = g.ny, nx = g.nx;
     const int64_t G = (int64_t)ny * nx;
-    const int64_t njobs = (int64_t)g.jobs.size() / 4;
-    const int W = p.window[0], N = fft_size(p);
+    const int64_t njobs = grid_njobs(g);
+    const int W = p.window[0];
     const int nalt = p.n_peaks - 1;
     Tables tb;
     HH_TRY(get_tables(ctx, p, tb));
-    if (k > 0) {
-      // build_predictor (src/pipeline.jl:454-464) from the previous pass
-      const Grid& pgd = grids[k - 1];
-      const int64_t Gp = (int64_t)pgd.ny * pgd.nx;
-      HH_CK(cudaMemcpyAsync(predw_u, u, Gp * sizeof(float), cudaMemcpyDeviceToDevice, s));
-      HH_CK(cudaMemcpyAsync(predw_v, v, Gp * sizeof(float), cudaMemcpyDeviceToDevice, s));
-      if (pgd.any_mask) HH_K(HH_K_VECTOR, 1, 0, 10 * Gp, Gp, hh::launch_replace(predw_u, predw_v, nullptr, gm, pgd.ny, pgd.nx, 0, s));
-      if (smoothing) {
-        HH_K(HH_K_VECTOR, 1, 0, 8 * Gp, Gp, hh::launch_smooth(predw_u, pgd.ny, pgd.nx, predu, s));
-        HH_K(HH_K_VECTOR, 1, 0, 8 * Gp, Gp, hh::launch_smooth(predw_v, pgd.ny, pgd.nx, predv, s));
-        pred_src_u = predu;
-        pred_src_v = predv;
-      } else {
-        pred_src_u = predw_u;
-        pred_src_v = predw_v;
-      }
-      pg.gny = pgd.ny;
-      pg.gnx = pgd.nx;
-      pg.y0 = pgd.y[0];
-      pg.x0 = pgd.x[0];
-      pg.ysp = pgd.ny > 1 ? pgd.y[1] - pgd.y[0] : 1.f;
-      pg.xsp = pgd.nx > 1 ? pgd.x[1] - pgd.x[0] : 1.f;
+    // the predictor from the validated field of grid gf (build_predictor)
+    auto build_pred = [&](const Grid& gf, bool keep) -> hh_status {
+      HH_K(HH_K_VECTOR, 1, 0, 24 * gf.G(), gf.G(),
+           hh::launch_predictor(u, v, gf.any_mask ? gm : nullptr, gf.ny, gf.nx, smoothing, predw_u, predw_v, predu, predv,
+                                keep ? prevu : nullptr, keep ? prevv : nullptr, s));
+      pred_src_u = smoothing ? predu : predw_u;
+      pred_src_v = smoothing ? predv : predw_v;
+      pg = pred_grid(gf);
       have_pred = true;
-    }
-    // this pass's grid
-    HH_CK(cudaMemcpyAsync(djobs, g.jobs.data(), g.jobs.size() * sizeof(int32_t), cudaMemcpyHostToDevice, s));
-    HH_CK(cudaMemcpyAsync(gm, g.gmask.data(), G, cudaMemcpyHostToDevice, s));
-    HH_CK(cudaMemcpyAsync(dx, g.x.data(), nx * sizeof(float), cudaMemcpyHostToDevice, s));
-    HH_CK(cudaMemcpyAsync(dy, g.y.data(), ny * sizeof(float), cudaMemcpyHostToDevice, s));
-    HH_CK(cudaMemsetAsync(resu, 0, G * sizeof(float), s));
-    HH_CK(cudaMemsetAsync(resv, 0, G * sizeof(float), s));
-    HH_CK(cudaMemsetAsync(ratio, 0, G * sizeof(float), s));
-    HH_CK(cudaMemsetAsync(moment, 0, G * sizeof(float), s));
-    const float NaN = std::nanf("");
-    HH_K(HH_K_VECTOR, 1, 0, 4 * G, G, hh::launch_fill(uncu, NaN, G, s));
-    HH_K(HH_K_VECTOR, 1, 0, 4 * G, G, hh::launch_fill(uncv, NaN, G, s));
-    if (nalt > 0) {
-      HH_K(HH_K_VECTOR, 1, 0, 4 * G * nalt, G, hh::launch_fill(altu, NaN, G * nalt, s));
-      HH_K(HH_K_VECTOR, 1, 0, 4 * G * nalt, G, hh::launch_fill(altv, NaN, G * nalt, s));
-    }
+      return HH_OK;
+    };
+    if (k > 0) HH_TRY(build_pred(grids[k - 1], false));
+    HH_TRY(stage_grid(ctx, g, djobs, gm));
     const bool unc = p.uncertainty && !force_replace;
+    if (unc && g.any_mask) {  // a masked cell has no estimate
+      HH_K(HH_K_VECTOR, 1, 0, 4 * G, G, hh::launch_fill(uncu, std::nanf(""), G, s));
+      HH_K(HH_K_VECTOR, 1, 0, 4 * G, G, hh::launch_fill(uncv, std::nanf(""), G, s));
+    }
     const bool fused_unc = unc && p.max_iterations == 1;
     const bool keep_measured = p.max_iterations > 1 && !(force_replace || p.replace_outliers);
     bool have_prev = false;
@@ -151,13 +122,10 @@ hh_status run_schedule(hh_ctx* ctx, const float* dA, const float* dB, int64_t nr
     for (int it = 1; it <= p.max_iterations; ++it) {
       ++sweeps;
       if (have_pred) {
-        HH_K(HH_K_VECTOR, 1, 0, 8 * G, G, hh::launch_node_values(pred_src_u, pred_src_v, pg, dy, ny, dx, nx, u, v, s));
         HH_K(HH_K_DEFORM, 1, 120 * P, 16 * P, P, hh::launch_deform(coefA, coefB, nr, nc, pred_src_u, pred_src_v, pg, warpA, warpB, s));
         srcA = warpA;
         srcB = warpB;
       } else {
-        HH_CK(cudaMemsetAsync(u, 0, G * sizeof(float), s));
-        HH_CK(cudaMemsetAsync(v, 0, G * sizeof(float), s));
         srcA = dA;
         srcB = dB;
       }
@@ -197,9 +165,11 @@ hh_status run_schedule(hh_ctx* ctx, const float* dA, const float* dB, int64_t nr
         HH_K(HH_K_UQ, 1, uq_flops(p, njobs), 8.0 * p.window[0] * p.window[1] * njobs, njobs,
              hh::launch_uq(ua, s, ctx->num_sms));
       }
-      HH_K(HH_K_VECTOR, 1, 0, (28 + 8 * nalt) * G, G, hh::launch_combine(u, v, resu, resv, ratio, moment, nalt > 0 ? altu : nullptr, nalt > 0 ? altv : nullptr,
-                               nalt, g.any_mask ? gm : nullptr, G, keep_measured ? measu : nullptr,
-                               keep_measured ? measv : nullptr, s));
+      HH_K(HH_K_VECTOR, 1, 0, (28 + 8 * nalt) * G, G,
+           hh::launch_combine(u, v, resu, resv, ratio, moment, nalt > 0 ? altu : nullptr, nalt > 0 ? altv : nullptr, nalt,
+                              g.any_mask ? gm : nullptr, ny, nx,
+                              have_pred ? node_pred(pred_src_u, pred_src_v, pg, g) : hh::NodePred{},
+                              keep_measured ? measu : nullptr, keep_measured ? measv : nullptr, s));
       HH_TRY(validate_device(ctx, p, ny, nx, u, v, ratio, moment, outl, outl2, gm, g.any_mask,
                              nalt > 0 ? altu : nullptr, nalt > 0 ? altv : nullptr, nalt,
                              force_replace || p.max_iterations > 1));
@@ -213,29 +183,10 @@ hh_status run_schedule(hh_ctx* ctx, const float* dA, const float* dB, int64_t nr
           HH_TRY(read_scalar(ctx, fcout, &change));
           if ((double)change < p.convergence_tol) break;
         }
-        HH_CK(cudaMemcpyAsync(prevu, u, G * sizeof(float), cudaMemcpyDeviceToDevice, s));
-        HH_CK(cudaMemcpyAsync(prevv, v, G * sizeof(float), cudaMemcpyDeviceToDevice, s));
       }
-      // predictor for the next sweep from this sweep's validated field
-      HH_CK(cudaMemcpyAsync(predw_u, u, G * sizeof(float), cudaMemcpyDeviceToDevice, s));
-      HH_CK(cudaMemcpyAsync(predw_v, v, G * sizeof(float), cudaMemcpyDeviceToDevice, s));
-      if (g.any_mask) HH_K(HH_K_VECTOR, 1, 0, 10 * G, G, hh::launch_replace(predw_u, predw_v, nullptr, gm, ny, nx, 0, s));
-      if (smoothing) {
-        HH_K(HH_K_VECTOR, 1, 0, 8 * G, G, hh::launch_smooth(predw_u, ny, nx, predu, s));
-        HH_K(HH_K_VECTOR, 1, 0, 8 * G, G, hh::launch_smooth(predw_v, ny, nx, predv, s));
-        pred_src_u = predu;
-        pred_src_v = predv;
-      } else {
-        pred_src_u = predw_u;
-        pred_src_v = predw_v;
-      }
-      pg.gny = ny;
-      pg.gnx = nx;
-      pg.y0 = g.y[0];
-      pg.x0 = g.x[0];
-      pg.ysp = ny > 1 ? g.y[1] - g.y[0] : 1.f;
-      pg.xsp = nx > 1 ? g.x[1] - g.x[0] : 1.f;
-      have_pred = true;
+      // predictor for the next sweep from this sweep's validated field, which
+      // the convergence test of that sweep needs as well
+      HH_TRY(build_pred(g, p.convergence_tol > 0));
     }
     if (unc && !fused_unc) {
       hh::UQArgs ua{srcA, srcB, dmask, nr, djobs, njobs, ny, W, tb.apod, nullptr, uncu, uncv};
@@ -248,24 +199,8 @@ hh_status run_schedule(hh_ctx* ctx, const float* dA, const float* dB, int64_t nr
     HH_CK(cudaEventRecord(ctx->events[k + 1], s));
   }
   // final pass -> host
-  const Grid& g = grids[np - 1];
-  const int64_t G = (int64_t)g.ny * g.nx;
-  if (out) {
-    out->ny = g.ny;
-    out->nx = g.nx;
-    if (out->x) memcpy(out->x, g.x.data(), g.nx * sizeof(float));
-    if (out->y) memcpy(out->y, g.y.data(), g.ny * sizeof(float));
-    if (out->u) HH_CK(cudaMemcpyAsync(out->u, u, G * sizeof(float), cudaMemcpyDeviceToHost, s));
-    if (out->v) HH_CK(cudaMemcpyAsync(out->v, v, G * sizeof(float), cudaMemcpyDeviceToHost, s));
-    if (out->peak_ratio) HH_CK(cudaMemcpyAsync(out->peak_ratio, ratio, G * sizeof(float), cudaMemcpyDeviceToHost, s));
-    if (out->correlation_moment)
-      HH_CK(cudaMemcpyAsync(out->correlation_moment, moment, G * sizeof(float), cudaMemcpyDeviceToHost, s));
-    if (out->uncertainty_u) HH_CK(cudaMemcpyAsync(out->uncertainty_u, uncu, G * sizeof(float), cudaMemcpyDeviceToHost, s));
-    if (out->uncertainty_v) HH_CK(cudaMemcpyAsync(out->uncertainty_v, uncv, G * sizeof(float), cudaMemcpyDeviceToHost, s));
-    if (out->outliers) HH_CK(cudaMemcpyAsync(out->outliers, outl, G, cudaMemcpyDeviceToHost, s));
-    if (out->mask) memcpy(out->mask, g.gmask.data(), G);
-  }
-  HH_CK(cudaStreamSynchronize(s));
+  if (out) HH_TRY(read_results(ctx, grids[np - 1], rb, Gmax, passes[np - 1].uncertainty != 0, out));
+  else HH_CK(cudaStreamSynchronize(s));
   for (int k = 0; k < np; ++k) HH_CK(cudaEventElapsedTime(&ctx->pass_ms[k], ctx->events[k], ctx->events[k + 1]));
   return flush_profile(ctx);
 }
@@ -364,15 +299,19 @@ hh_status hh_pass_grid(int64_t nr, int64_t nc, const hh_pass_desc* p, const uint
   hh_ctx* ctx = nullptr;
   HH_TRY(hh_pass_validate(p));
   Grid g;
-  HH_TRY(make_grid(ctx, nr, nc, *p, mask, thr, g));
+  if (!mask && !jobs) HH_TRY(grid_axes(ctx, nr, nc, *p, g));
+  else HH_TRY(make_grid(ctx, nr, nc, *p, mask, thr, g));
   if (ny) *ny = g.ny;
   if (nx) *nx = g.nx;
   if (x) memcpy(x, g.x.data(), g.nx * sizeof(float));
   if (y) memcpy(y, g.y.data(), g.ny * sizeof(float));
-  if (grid_mask) memcpy(grid_mask, g.gmask.data(), g.gmask.size());
+  if (grid_mask) {
+    if (mask) memcpy(grid_mask, g.gmask.data(), g.gmask.size());
+    else memset(grid_mask, 0, (size_t)g.G());
+  }
   if (jobs)
     for (size_t k = 0; k < g.jobs.size(); ++k) jobs[k] = g.jobs[k] + 1;
-  if (njobs) *njobs = (int64_t)g.jobs.size() / 4;
+  if (njobs) *njobs = mask || jobs ? (int64_t)g.jobs.size() / 4 : g.G();
   return HH_OK;
 }
 
@@ -403,7 +342,7 @@ hh_status hh_ctx_create(int32_t device, hh_ctx** out) {
     }
   }
   if (cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking) != cudaSuccess ||
-      cudaMallocHost(&ctx->pinned, 64) != cudaSuccess) {
+      cudaMallocHost(&ctx->pinned, HH_PINNED_BYTES) != cudaSuccess) {
     g_err = "stream or pinned buffer creation failed";
     delete ctx;
     return HH_ERR_CUDA;
@@ -459,7 +398,7 @@ hh_status hh_run_piv(hh_ctx* ctx, const float* A, const float* B, int64_t nr, in
     HH_TRY(buf(ctx, "imgmask", (size_t)P, &dm));
     HH_CK(cudaMemcpyAsync(dm, mask, P, cudaMemcpyHostToDevice, ctx->stream));
   }
-  return run_schedule(ctx, dA, dB, nr, nc, passes, npasses, mask, dm, thr, smoothing != 0, out);
+  return run_schedule(ctx, dA, dB, nr, nc, passes, npasses, dm, thr, smoothing != 0, out);
 }
 
 hh_status hh_run_piv_device(hh_ctx* ctx, const float* dA, const float* dB, int64_t nr, int64_t nc,
@@ -468,14 +407,7 @@ hh_status hh_run_piv_device(hh_ctx* ctx, const float* dA, const float* dB, int64
   if (!ctx) return fail(nullptr, HH_ERR_ARG, "context is NULL");
   HH_TRY(set_device(ctx));
   if (!dA || !dB) return fail(ctx, HH_ERR_ARG, "image pointers must not be NULL");
-  std::vector<uint8_t> hmask;
-  if (dmask) {
-    hmask.resize((size_t)(nr * nc));
-    HH_CK(cudaMemcpyAsync(hmask.data(), dmask, hmask.size(), cudaMemcpyDeviceToHost, ctx->stream));
-    HH_CK(cudaStreamSynchronize(ctx->stream));
-  }
-  return run_schedule(ctx, dA, dB, nr, nc, passes, npasses, dmask ? hmask.data() : nullptr, dmask, thr, smoothing != 0,
-                      out);
+  return run_schedule(ctx, dA, dB, nr, nc, passes, npasses, dmask, thr, smoothing != 0, out);
 }
 
 hh_status hh_last_pass_times(const hh_ctx* ctx, int32_t npasses, float* ms, int32_t* sweeps) {

@@ -756,7 +756,7 @@ hh_status hh_batch_grid(const hh_batch_pair* pairs, int32_t npairs, const hh_pas
     const hh_batch_pair& q = pairs[p];
     Grid g;
     for (int k = schedule_offsets[q.schedule]; k < schedule_offsets[q.schedule + 1]; ++k)
-      HH_TRY(make_grid(ctx, q.nr, q.nc, passes[k], nullptr, 0.5, g));
+      HH_TRY(grid_axes(ctx, q.nr, q.nc, passes[k], g));
     if (ny) ny[p] = g.ny;
     if (nx) nx[p] = g.nx;
     if (offsets) offsets[p] = off;

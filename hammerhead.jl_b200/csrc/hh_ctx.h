@@ -54,7 +54,7 @@ struct hh_ctx {
   std::map<std::string, hhd::DevBuf> bufs;
   std::map<hhd::TableKey, hhd::Tables> tables;
   std::map<int64_t, std::pair<float*, float*>> bs_factors;  // line length -> (cp, inv)
-  float* pinned = nullptr;  // small pinned scratch for scalar reads
+  float* pinned = nullptr;  // page-locked block (HH_PINNED_BYTES) for scalars and small results
   // staged pair for the hook-level entry points
   int64_t nr = 0, nc = 0;
   const float* curA = nullptr;
@@ -95,6 +95,10 @@ struct hh_ctx {
 };
 
 namespace hhd {
+
+// Page-locked block of a context: a result of up to 40 k vectors comes back
+// through it in one copy instead of one pageable copy per field (8-10 us each).
+constexpr size_t HH_PINNED_BYTES = 1 << 20;
 
 inline hh_status fail(hh_ctx* ctx, hh_status code, const std::string& msg) {
   if (ctx) ctx->err = msg;
@@ -160,55 +164,67 @@ template <class T> hh_status buf(hh_ctx* ctx, const char* name, size_t count, T*
 // Host grid: pass_grid (src/pipeline.jl:529-555)
 struct Grid {
   int ny = 0, nx = 0;
+  hh::WinGrid win{};  // where its windows lie
   std::vector<float> x, y;
   std::vector<uint8_t> gmask;
   std::vector<int32_t> jobs;  // 0-based gi, gj, rs, cs
   bool any_mask = false;
+  int64_t G() const { return (int64_t)ny * nx; }
 };
 
-inline hh_status make_grid(hh_ctx* ctx, int64_t nr, int64_t nc, const hh_pass_desc& p, const uint8_t* mask, double thr,
-                    Grid& g) {
+// The grid without its mask and window list.
+inline hh_status grid_axes(hh_ctx* ctx, int64_t nr, int64_t nc, const hh_pass_desc& p, Grid& g) {
   const int wr = p.window[0], wc = p.window[1], sr = p.search[0], sc = p.search[1];
   const int mr = (sr - wr) / 2, mc = (sc - wc) / 2;
   if (sr > nr || sc > nc)
     return fail(ctx, HH_ERR_ARG, "search area " + tup(p.search) + " exceeds image size (" + std::to_string(nr) + ", " +
                                      std::to_string(nc) + ")");
-  std::vector<int64_t> rows, cols;
-  for (int64_t s = 1 + mr; s <= nr - wr - mr + 1; s += wr - p.overlap[0]) rows.push_back(s);
-  for (int64_t s = 1 + mc; s <= nc - wc - mc + 1; s += wc - p.overlap[1]) cols.push_back(s);
-  g.ny = (int)rows.size();
-  g.nx = (int)cols.size();
+  g.win = hh::WinGrid{mr, wr - p.overlap[0], mc, wc - p.overlap[1]};
+  g.ny = (int)((nr - wr - 2 * mr) / g.win.rstep + 1);
+  g.nx = (int)((nc - wc - 2 * mc) / g.win.cstep + 1);
   g.x.resize(g.nx);
   g.y.resize(g.ny);
-  for (int j = 0; j < g.nx; ++j) g.x[j] = (float)((double)cols[j] + (wc - 1) / 2.0);
-  for (int i = 0; i < g.ny; ++i) g.y[i] = (float)((double)rows[i] + (wr - 1) / 2.0);
-  g.gmask.assign((size_t)g.ny * g.nx, 0);
+  for (int j = 0; j < g.nx; ++j) g.x[j] = (float)((double)(mc + 1 + (int64_t)j * g.win.cstep) + (wc - 1) / 2.0);
+  for (int i = 0; i < g.ny; ++i) g.y[i] = (float)((double)(mr + 1 + (int64_t)i * g.win.rstep) + (wr - 1) / 2.0);
   g.any_mask = false;
+  return HH_OK;
+}
+
+// The window list of the cells that gmask leaves.
+inline void grid_jobs(Grid& g) {
+  g.jobs.clear();
+  g.jobs.reserve(4 * (size_t)g.G());
+  for (int gj = 0; gj < g.nx; ++gj)
+    for (int gi = 0; gi < g.ny; ++gi)
+      if (!g.gmask[gi + (size_t)gj * g.ny]) {
+        const int32_t q[4] = {gi, gj, g.win.r0 + gi * g.win.rstep, g.win.c0 + gj * g.win.cstep};
+        g.jobs.insert(g.jobs.end(), q, q + 4);
+      }
+}
+
+inline hh_status make_grid(hh_ctx* ctx, int64_t nr, int64_t nc, const hh_pass_desc& p, const uint8_t* mask, double thr,
+                    Grid& g) {
+  HH_TRY(grid_axes(ctx, nr, nc, p, g));
+  const int wr = p.window[0], wc = p.window[1], sr = p.search[0], sc = p.search[1];
+  const int mr = (sr - wr) / 2, mc = (sc - wc) / 2;
+  g.gmask.assign((size_t)g.ny * g.nx, 0);
   if (mask) {
     for (int gj = 0; gj < g.nx; ++gj)
       for (int gi = 0; gi < g.ny; ++gi) {
-        const int64_t rs = rows[gi], cs = cols[gj];
+        const int64_t rs = g.win.r0 + (int64_t)gi * g.win.rstep, cs = g.win.c0 + (int64_t)gj * g.win.cstep;
         int64_t cw = 0, csr = 0;
         for (int j = 0; j < wc; ++j)
-          for (int i = 0; i < wr; ++i) cw += mask[(rs - 1 + i) + (cs - 1 + j) * nr] != 0;
+          for (int i = 0; i < wr; ++i) cw += mask[(rs + i) + (cs + j) * nr] != 0;
         const int64_t srs = rs - mr, scs = cs - mc;
         for (int j = 0; j < sc; ++j)
-          for (int i = 0; i < sr; ++i) csr += mask[(srs - 1 + i) + (scs - 1 + j) * nr] != 0;
+          for (int i = 0; i < sr; ++i) csr += mask[(srs + i) + (scs + j) * nr] != 0;
         const double fw = (double)cw / (double)(wr * wc), fs = (double)csr / (double)(sr * sc);
         const uint8_t m = fw >= thr || fs >= thr;
         g.gmask[gi + (size_t)gj * g.ny] = m;
         g.any_mask |= m != 0;
       }
   }
-  g.jobs.clear();
-  for (int gj = 0; gj < g.nx; ++gj)
-    for (int gi = 0; gi < g.ny; ++gi)
-      if (!g.gmask[gi + (size_t)gj * g.ny]) {
-        g.jobs.push_back(gi);
-        g.jobs.push_back(gj);
-        g.jobs.push_back((int32_t)(rows[gi] - 1));
-        g.jobs.push_back((int32_t)(cols[gj] - 1));
-      }
+  grid_jobs(g);
   return HH_OK;
 }
 
@@ -618,25 +634,133 @@ inline hh_status validate_device(hh_ctx* ctx, const hh_pass_desc& p, int ny, int
                           const float* alt_u, const float* alt_v, int nalt, bool force_replace) {
   cudaStream_t s = ctx->stream;
   const int64_t G = (int64_t)ny * nx;
-  HH_CK(cudaMemsetAsync(outl, 0, G, s));
-  const uint8_t* excl = any_mask ? gmask : nullptr;
-  if (p.uod_enable) HH_K(HH_K_VECTOR, 1, 0, 48 * G, G, hh::launch_uod(u, v, ny, nx, p.uod_threshold, p.uod_neighborhood, 0.1, excl, outl, 1, s));
-  if (p.min_peak_ratio > 1) HH_K(HH_K_VECTOR, 1, 0, 5 * G, G, hh::launch_flag_ratio(ratio, G, p.min_peak_ratio, outl, s));
-  for (int q = 0; q < p.n_validators; ++q) {
-    const hh_validator& vd = p.validators[q];
-    if (vd.kind == HH_VAL_PEAK_RATIO) HH_K(HH_K_VECTOR, 1, 0, 5 * G, G, hh::launch_flag_ratio(ratio, G, vd.threshold, outl, s));
-    else if (vd.kind == HH_VAL_MOMENT) HH_K(HH_K_VECTOR, 1, 0, 5 * G, G, hh::launch_flag_moment(moment, G, vd.threshold, outl, s));
-    else if (vd.kind == HH_VAL_VELOCITY) HH_K(HH_K_VECTOR, 1, 0, 9 * G, G, hh::launch_flag_velocity(u, v, G, vd.vmin, vd.vmax, outl, s));
-    else if (vd.kind == HH_VAL_UOD)
-      HH_K(HH_K_VECTOR, 1, 0, 48 * G, G, hh::launch_uod(u, v, ny, nx, vd.threshold, vd.neighborhood, vd.epsilon, excl, outl, 1, s));
+  const uint8_t* gm = any_mask ? gmask : nullptr;
+  hh::FlagRules r{p.uod_enable, p.uod_neighborhood, p.uod_threshold, p.min_peak_ratio, p.n_validators};
+  std::copy(p.validators, p.validators + p.n_validators, r.val);
+  const bool subst = alt_u && nalt > 0;
+  HH_K(HH_K_VECTOR, 1, 0, 48 * G, G, hh::launch_flags(u, v, ratio, moment, ny, nx, r, gm, outl, subst ? outl2 : nullptr, s));
+  if (subst)
+    HH_K(HH_K_VECTOR, 1, 0, (10 + 8 * nalt) * G, G,
+         hh::launch_substitute(u, v, outl2, outl, gm, alt_u, alt_v, nalt, ny, nx, p.uod_neighborhood, p.uod_threshold, s));
+  if (force_replace || p.replace_outliers)
+    HH_K(HH_K_VECTOR, 1, 0, 10 * G, G, hh::launch_replace(u, v, outl, gm, ny, nx, 1, s));
+  return HH_OK;
+}
+
+// The grids of every pass and, with an image mask on the device, their grid
+// masks and window lists: counted on the device, one copy back for all passes.
+inline hh_status pass_grids(hh_ctx* ctx, int64_t nr, int64_t nc, const hh_pass_desc* passes, int np, const uint8_t* dmask,
+                            double thr, std::vector<Grid>& grids) {
+  grids.assign(np, Grid());
+  int64_t tot = 0;
+  for (int k = 0; k < np; ++k) {
+    HH_TRY(grid_axes(ctx, nr, nc, passes[k], grids[k]));
+    tot += grids[k].G();
   }
-  if (any_mask) HH_K(HH_K_VECTOR, 1, 0, 2 * G, G, hh::launch_mask_flags(outl, gmask, G, s));
-  if (alt_u && nalt > 0) {
-    HH_K(HH_K_VECTOR, 1, 0, (10 + 8 * nalt) * G, G, hh::launch_substitute(u, v, outl, outl2, gmask, alt_u, alt_v, nalt, ny, nx, p.uod_neighborhood,
-                                p.uod_threshold, s));
-    HH_CK(cudaMemcpyAsync(outl, outl2, G, cudaMemcpyDeviceToDevice, s));
+  if (!dmask) return HH_OK;
+  uint8_t* d;
+  HH_TRY(buf(ctx, "gmask_all", tot, &d));
+  int64_t off = 0;
+  for (int k = 0; k < np; ++k) {
+    const hh_pass_desc& p = passes[k];
+    const Grid& g = grids[k];
+    HH_K(HH_K_VECTOR, 1, 0, g.G(), g.G(),
+         hh::launch_mask_grid(dmask, nr, g.ny, g.nx, g.win, p.window[0], p.window[1], (p.search[0] - p.window[0]) / 2,
+                              (p.search[1] - p.window[1]) / 2, thr, d + off, ctx->stream));
+    off += g.G();
   }
-  if (force_replace || p.replace_outliers) HH_K(HH_K_VECTOR, 1, 0, 10 * G, G, hh::launch_replace(u, v, outl, gmask, ny, nx, 1, s));
+  std::vector<uint8_t> h(tot);
+  HH_CK(cudaMemcpyAsync(h.data(), d, tot, cudaMemcpyDeviceToHost, ctx->stream));
+  HH_CK(cudaStreamSynchronize(ctx->stream));
+  off = 0;
+  for (Grid& g : grids) {
+    g.gmask.assign(h.begin() + off, h.begin() + off + g.G());
+    g.any_mask = std::any_of(g.gmask.begin(), g.gmask.end(), [](uint8_t m) { return m != 0; });
+    if (g.any_mask) grid_jobs(g);
+    off += g.G();
+  }
+  return HH_OK;
+}
+// windows of a grid from pass_grids
+inline int64_t grid_njobs(const Grid& g) { return g.any_mask ? (int64_t)g.jobs.size() / 4 : g.G(); }
+// its window list and grid mask on the device (the mask only where a cell is masked)
+inline hh_status stage_grid(hh_ctx* ctx, const Grid& g, int32_t* djobs, uint8_t* gm) {
+  cudaStream_t s = ctx->stream;
+  if (!g.any_mask) {
+    HH_K(HH_K_VECTOR, 1, 0, 16 * g.G(), g.G(), hh::launch_make_jobs(djobs, g.ny, g.nx, g.win, s));
+    return HH_OK;
+  }
+  HH_CK(cudaMemcpyAsync(djobs, g.jobs.data(), g.jobs.size() * sizeof(int32_t), cudaMemcpyHostToDevice, s));
+  HH_CK(cudaMemcpyAsync(gm, g.gmask.data(), g.G(), cudaMemcpyHostToDevice, s));
+  return HH_OK;
+}
+// predictor nodes of grid g
+inline hh::PredGrid pred_grid(const Grid& g) {
+  return hh::PredGrid{g.ny, g.nx, g.y[0], g.ny > 1 ? g.y[1] - g.y[0] : 1.f, g.x[0], g.nx > 1 ? g.x[1] - g.x[0] : 1.f};
+}
+// predictor (u, v) on nodes pg, wanted on grid g
+inline hh::NodePred node_pred(const float* u, const float* v, const hh::PredGrid& pg, const Grid& g) {
+  const hh::PredGrid n = pred_grid(g);
+  return hh::NodePred{u, v, pg, n.y0, n.ysp, n.x0, n.xsp};
+}
+
+// Device storage of the final fields as one block of G cells per field, in
+// the order u, v, ratio, moment, flags (a byte each), uncertainties: a result
+// that fits the context's page-locked block comes back in one copy.
+struct ResultBlock {
+  float *u, *v, *ratio, *moment, *uncu, *uncv;
+  uint8_t* outl;
+};
+inline hh_status result_block(hh_ctx* ctx, int64_t G, ResultBlock& r) {
+  const int64_t fw = (G + 3) / 4;  // words of the flags
+  HH_TRY(buf(ctx, "result", (size_t)(6 * G + fw), &r.u));
+  r.v = r.u + G;
+  r.ratio = r.v + G;
+  r.moment = r.ratio + G;
+  r.outl = reinterpret_cast<uint8_t*>(r.moment + G);
+  r.uncu = r.moment + G + fw;
+  r.uncv = r.uncu + G;
+  return HH_OK;
+}
+// G: cells the block was laid out for; unc: whether uncertainties were estimated (else they are NaN)
+inline hh_status read_results(hh_ctx* ctx, const Grid& g, const ResultBlock& r, int64_t Gb, bool unc, hh_result* out) {
+  cudaStream_t s = ctx->stream;
+  const int64_t G = g.G();
+  out->ny = g.ny;
+  out->nx = g.nx;
+  if (out->x) memcpy(out->x, g.x.data(), g.nx * sizeof(float));
+  if (out->y) memcpy(out->y, g.y.data(), g.ny * sizeof(float));
+  struct Field {
+    void* dst;
+    const void* src;
+    size_t bytes;
+  } f[7] = {{out->u, r.u, G * sizeof(float)},
+            {out->v, r.v, G * sizeof(float)},
+            {out->peak_ratio, r.ratio, G * sizeof(float)},
+            {out->correlation_moment, r.moment, G * sizeof(float)},
+            {out->outliers, r.outl, (size_t)G},
+            {unc ? out->uncertainty_u : nullptr, r.uncu, G * sizeof(float)},
+            {unc ? out->uncertainty_v : nullptr, r.uncv, G * sizeof(float)}};
+  const char* base = reinterpret_cast<const char*>(r.u);
+  const size_t total = (unc ? 6 * Gb + (Gb + 3) / 4 : 4 * Gb + (Gb + 3) / 4) * sizeof(float);
+  if (total <= HH_PINNED_BYTES) {
+    HH_CK(cudaMemcpyAsync(ctx->pinned, base, total, cudaMemcpyDeviceToHost, s));
+    HH_CK(cudaStreamSynchronize(s));
+    const char* h = reinterpret_cast<const char*>(ctx->pinned);
+    for (const Field& q : f)
+      if (q.dst) memcpy(q.dst, h + (static_cast<const char*>(q.src) - base), q.bytes);
+  } else {
+    for (const Field& q : f)
+      if (q.dst) HH_CK(cudaMemcpyAsync(q.dst, q.src, q.bytes, cudaMemcpyDeviceToHost, s));
+    HH_CK(cudaStreamSynchronize(s));
+  }
+  if (!unc)
+    for (float* q : {out->uncertainty_u, out->uncertainty_v})
+      if (q) std::fill(q, q + G, std::nanf(""));
+  if (out->mask) {
+    if (g.any_mask) memcpy(out->mask, g.gmask.data(), G);
+    else memset(out->mask, 0, G);
+  }
   return HH_OK;
 }
 

@@ -32,20 +32,24 @@ extern "C" hh_status hh_run_ensemble(hh_ctx* ctx, const hh_batch_pair* pairs, in
   }
   const bool device_inputs = (flags & HH_BATCH_DEVICE_INPUTS) != 0;
   cudaStream_t s = ctx->stream;
-  std::vector<Grid> grids(np);
+  uint8_t* dmask = nullptr;
+  if (hmask) {
+    HH_TRY(buf(ctx, "ens_mask", (size_t)P, &dmask));
+    HH_CK(cudaMemcpyAsync(dmask, hmask, (size_t)P, cudaMemcpyHostToDevice, s));
+  }
+  std::vector<Grid> grids;
+  HH_TRY(pass_grids(ctx, nr, nc, passes, np, dmask, thr, grids));
   int64_t Gmax = 1, Jmax = 1, accmax = 1;
   int nalt_max = 0;
   for (int k = 0; k < np; ++k) {
-    HH_TRY(make_grid(ctx, nr, nc, passes[k], hmask, thr, grids[k]));
-    const int64_t nj = (int64_t)grids[k].jobs.size() / 4;
+    const int64_t nj = grid_njobs(grids[k]);
     const int64_t PL = (int64_t)fft_rows(passes[k]) * fft_cols(passes[k]);
-    Gmax = std::max<int64_t>(Gmax, (int64_t)grids[k].ny * grids[k].nx);
+    Gmax = std::max<int64_t>(Gmax, grids[k].G());
     Jmax = std::max<int64_t>(Jmax, nj);
     accmax = std::max<int64_t>(accmax, nj * PL);
     nalt_max = std::max(nalt_max, passes[k].n_peaks - 1);
   }
   float *dA = nullptr, *dB = nullptr, *coefA, *coefB, *warpA, *warpB, *acc;
-  uint8_t* dmask = nullptr;
   double* stats;
   bool any_u16 = false;
   for (int q = 0; q < npairs; ++q) any_u16 |= pairs[q].format != HH_PIX_F32;
@@ -58,28 +62,21 @@ extern "C" hh_status hh_run_ensemble(hh_ctx* ctx, const hh_batch_pair* pairs, in
     HH_TRY(buf(ctx, "ens_A16", (size_t)P, &d16A));
     HH_TRY(buf(ctx, "ens_B16", (size_t)P, &d16B));
   }
-  if (hmask) {
-    HH_TRY(buf(ctx, "ens_mask", (size_t)P, &dmask));
-    HH_CK(cudaMemcpyAsync(dmask, hmask, (size_t)P, cudaMemcpyHostToDevice, s));
-  }
   HH_TRY(buf(ctx, "coefA", (size_t)(nr + 2) * (nc + 2), &coefA));
   HH_TRY(buf(ctx, "coefB", (size_t)(nr + 2) * (nc + 2), &coefB));
   HH_TRY(buf(ctx, "warpA", (size_t)P, &warpA));
   HH_TRY(buf(ctx, "warpB", (size_t)P, &warpB));
   HH_TRY(buf(ctx, "ens_acc", (size_t)accmax, &acc));
   HH_TRY(buf(ctx, "ens_stats", (size_t)Jmax * 88, &stats));
-  float *u, *v, *resu, *resv, *ratio, *moment, *uncu, *uncv, *altu = nullptr, *altv = nullptr, *predu, *predv, *predw_u,
-        *predw_v, *dx, *dy;
-  uint8_t *outl, *outl2, *gm;
+  ResultBlock rb;
+  HH_TRY(result_block(ctx, Gmax, rb));
+  float *u = rb.u, *v = rb.v, *ratio = rb.ratio, *moment = rb.moment, *uncu = rb.uncu, *uncv = rb.uncv;
+  uint8_t* outl = rb.outl;
+  float *resu, *resv, *altu = nullptr, *altv = nullptr, *predu, *predv, *predw_u, *predw_v;
+  uint8_t *outl2, *gm;
   int32_t* djobs;
-  HH_TRY(buf(ctx, "u", Gmax, &u));
-  HH_TRY(buf(ctx, "v", Gmax, &v));
   HH_TRY(buf(ctx, "resu", Gmax, &resu));
   HH_TRY(buf(ctx, "resv", Gmax, &resv));
-  HH_TRY(buf(ctx, "ratio", Gmax, &ratio));
-  HH_TRY(buf(ctx, "moment", Gmax, &moment));
-  HH_TRY(buf(ctx, "uncu", Gmax, &uncu));
-  HH_TRY(buf(ctx, "uncv", Gmax, &uncv));
   if (nalt_max > 0) {
     HH_TRY(buf(ctx, "altu", Gmax * nalt_max, &altu));
     HH_TRY(buf(ctx, "altv", Gmax * nalt_max, &altv));
@@ -88,9 +85,6 @@ extern "C" hh_status hh_run_ensemble(hh_ctx* ctx, const hh_batch_pair* pairs, in
   HH_TRY(buf(ctx, "predv", Gmax, &predv));
   HH_TRY(buf(ctx, "predwu", Gmax, &predw_u));
   HH_TRY(buf(ctx, "predwv", Gmax, &predw_v));
-  HH_TRY(buf(ctx, "gx", Gmax, &dx));
-  HH_TRY(buf(ctx, "gy", Gmax, &dy));
-  HH_TRY(buf(ctx, "outl", Gmax, &outl));
   HH_TRY(buf(ctx, "outl2", Gmax, &outl2));
   HH_TRY(buf(ctx, "gmask", Gmax, &gm));
   HH_TRY(buf(ctx, "jobs", 4 * Jmax, &djobs));
@@ -113,7 +107,7 @@ extern "C" hh_status hh_run_ensemble(hh_ctx* ctx, const hh_batch_pair* pairs, in
     const bool force_replace = k < np - 1;
     const int ny = g.ny, nx = g.nx;
     const int64_t G = (int64_t)ny * nx;
-    const int64_t njobs = (int64_t)g.jobs.size() / 4;
+    const int64_t njobs = grid_njobs(g);
     const int W = p.window[0], NR = fft_rows(p), NC = fft_cols(p);
     const int64_t PL = (int64_t)NR * NC;
     const int nalt = p.n_peaks - 1;
@@ -122,40 +116,14 @@ extern "C" hh_status hh_run_ensemble(hh_ctx* ctx, const hh_batch_pair* pairs, in
     HH_TRY(get_tables(ctx, p, tb));
     if (k > 0) {  // build_predictor from the previous pass's result (src/pipeline.jl:454-464)
       const Grid& pgd = grids[k - 1];
-      const int64_t Gp = (int64_t)pgd.ny * pgd.nx;
-      HH_CK(cudaMemcpyAsync(predw_u, u, Gp * sizeof(float), cudaMemcpyDeviceToDevice, s));
-      HH_CK(cudaMemcpyAsync(predw_v, v, Gp * sizeof(float), cudaMemcpyDeviceToDevice, s));
-      if (pgd.any_mask) {
-        HH_CK(cudaMemcpyAsync(gm, pgd.gmask.data(), Gp, cudaMemcpyHostToDevice, s));
-        HH_K(HH_K_VECTOR, 1, 0, 10 * Gp, Gp, hh::launch_replace(predw_u, predw_v, nullptr, gm, pgd.ny, pgd.nx, 0, s));
-      }
-      if (smoothing) {
-        HH_K(HH_K_VECTOR, 1, 0, 8 * Gp, Gp, hh::launch_smooth(predw_u, pgd.ny, pgd.nx, predu, s));
-        HH_K(HH_K_VECTOR, 1, 0, 8 * Gp, Gp, hh::launch_smooth(predw_v, pgd.ny, pgd.nx, predv, s));
-        pred_src_u = predu;
-        pred_src_v = predv;
-      } else {
-        pred_src_u = predw_u;
-        pred_src_v = predw_v;
-      }
-      pg.gny = pgd.ny;
-      pg.gnx = pgd.nx;
-      pg.y0 = pgd.y[0];
-      pg.x0 = pgd.x[0];
-      pg.ysp = pgd.ny > 1 ? pgd.y[1] - pgd.y[0] : 1.f;
-      pg.xsp = pgd.nx > 1 ? pgd.x[1] - pgd.x[0] : 1.f;
+      HH_K(HH_K_VECTOR, 1, 0, 24 * pgd.G(), pgd.G(),
+           hh::launch_predictor(u, v, pgd.any_mask ? gm : nullptr, pgd.ny, pgd.nx, smoothing, predw_u, predw_v, predu, predv,
+                                nullptr, nullptr, s));
+      pred_src_u = smoothing ? predu : predw_u;
+      pred_src_v = smoothing ? predv : predw_v;
+      pg = pred_grid(pgd);
     }
-    HH_CK(cudaMemcpyAsync(djobs, g.jobs.data(), g.jobs.size() * sizeof(int32_t), cudaMemcpyHostToDevice, s));
-    HH_CK(cudaMemcpyAsync(gm, g.gmask.data(), G, cudaMemcpyHostToDevice, s));
-    HH_CK(cudaMemcpyAsync(dx, g.x.data(), nx * sizeof(float), cudaMemcpyHostToDevice, s));
-    HH_CK(cudaMemcpyAsync(dy, g.y.data(), ny * sizeof(float), cudaMemcpyHostToDevice, s));
-    // the shared predictor's node values (zero without one)
-    if (k > 0) {
-      HH_K(HH_K_VECTOR, 1, 0, 8 * G, G, hh::launch_node_values(pred_src_u, pred_src_v, pg, dy, ny, dx, nx, u, v, s));
-    } else {
-      HH_CK(cudaMemsetAsync(u, 0, G * sizeof(float), s));
-      HH_CK(cudaMemsetAsync(v, 0, G * sizeof(float), s));
-    }
+    HH_TRY(stage_grid(ctx, g, djobs, gm));
     HH_CK(cudaMemsetAsync(acc, 0, (size_t)njobs * PL * sizeof(float), s));
     if (unc) HH_CK(cudaMemsetAsync(stats, 0, (size_t)njobs * 88 * sizeof(double), s));
     for (int q = 0; q < npairs; ++q) {
@@ -240,11 +208,9 @@ extern "C" hh_status hh_run_ensemble(hh_ctx* ctx, const hh_batch_pair* pairs, in
         return fail(ctx, HH_ERR_STATE, "ensemble reducer failed in pass " + std::to_string(k + 1));
     }
     // ensemble_analyze! (src/ensemble.jl:273-305): one analysis of every summed plane
-    HH_K(HH_K_VECTOR, 1, 0, 4 * G, G, hh::launch_fill(uncu, NaN, G, s));
-    HH_K(HH_K_VECTOR, 1, 0, 4 * G, G, hh::launch_fill(uncv, NaN, G, s));
-    if (nalt > 0) {
-      HH_K(HH_K_VECTOR, 1, 0, 4 * G * nalt, G, hh::launch_fill(altu, NaN, G * nalt, s));
-      HH_K(HH_K_VECTOR, 1, 0, 4 * G * nalt, G, hh::launch_fill(altv, NaN, G * nalt, s));
+    if (unc && g.any_mask) {  // a masked cell has no estimate
+      HH_K(HH_K_VECTOR, 1, 0, 4 * G, G, hh::launch_fill(uncu, NaN, G, s));
+      HH_K(HH_K_VECTOR, 1, 0, 4 * G, G, hh::launch_fill(uncv, NaN, G, s));
     }
     if (njobs > 0) {
       hh::AnalyzeArgs aa{};
@@ -270,29 +236,14 @@ extern "C" hh_status hh_run_ensemble(hh_ctx* ctx, const hh_batch_pair* pairs, in
     }
     HH_K(HH_K_VECTOR, 1, 0, (28 + 8 * nalt) * G, G,
          hh::launch_combine(u, v, resu, resv, ratio, moment, nalt > 0 ? altu : nullptr, nalt > 0 ? altv : nullptr, nalt,
-                            g.any_mask ? gm : nullptr, G, nullptr, nullptr, s));
+                            g.any_mask ? gm : nullptr, ny, nx,
+                            k > 0 ? node_pred(pred_src_u, pred_src_v, pg, g) : hh::NodePred{}, nullptr, nullptr, s));
     HH_TRY(validate_device(ctx, p, ny, nx, u, v, ratio, moment, outl, outl2, gm, g.any_mask,
                            nalt > 0 ? altu : nullptr, nalt > 0 ? altv : nullptr, nalt, force_replace));
     HH_CK(cudaEventRecord(ctx->events[k + 1], s));
   }
-  const Grid& g = grids[np - 1];
-  const int64_t G = (int64_t)g.ny * g.nx;
-  if (out) {
-    out->ny = g.ny;
-    out->nx = g.nx;
-    if (out->x) memcpy(out->x, g.x.data(), g.nx * sizeof(float));
-    if (out->y) memcpy(out->y, g.y.data(), g.ny * sizeof(float));
-    if (out->u) HH_CK(cudaMemcpyAsync(out->u, u, G * sizeof(float), cudaMemcpyDeviceToHost, s));
-    if (out->v) HH_CK(cudaMemcpyAsync(out->v, v, G * sizeof(float), cudaMemcpyDeviceToHost, s));
-    if (out->peak_ratio) HH_CK(cudaMemcpyAsync(out->peak_ratio, ratio, G * sizeof(float), cudaMemcpyDeviceToHost, s));
-    if (out->correlation_moment)
-      HH_CK(cudaMemcpyAsync(out->correlation_moment, moment, G * sizeof(float), cudaMemcpyDeviceToHost, s));
-    if (out->uncertainty_u) HH_CK(cudaMemcpyAsync(out->uncertainty_u, uncu, G * sizeof(float), cudaMemcpyDeviceToHost, s));
-    if (out->uncertainty_v) HH_CK(cudaMemcpyAsync(out->uncertainty_v, uncv, G * sizeof(float), cudaMemcpyDeviceToHost, s));
-    if (out->outliers) HH_CK(cudaMemcpyAsync(out->outliers, outl, G, cudaMemcpyDeviceToHost, s));
-    if (out->mask) memcpy(out->mask, g.gmask.data(), G);
-  }
-  HH_CK(cudaStreamSynchronize(s));
+  if (out) HH_TRY(read_results(ctx, grids[np - 1], rb, Gmax, passes[np - 1].uncertainty != 0, out));
+  else HH_CK(cudaStreamSynchronize(s));
   for (int k = 0; k < np; ++k) HH_CK(cudaEventElapsedTime(&ctx->pass_ms[k], ctx->events[k], ctx->events[k + 1]));
   return flush_profile(ctx);
 }

@@ -3,6 +3,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "hammerhead_b200.h"
+
 namespace hh {
 
 struct BPair;
@@ -136,16 +138,38 @@ cudaError_t launch_node_values(const float* pu, const float* pv, PredGrid g, con
                                const float* x, int32_t nx, float* u, float* v, cudaStream_t s);
 
 // --- vector-grid kernels -----------------------------------------------------
+// a predictor on nodes (u, v) and the grid it is wanted on: node (gi, gj) at
+// (y0 + gi ysp, x0 + gj xsp); u == nullptr: no predictor
+struct NodePred {
+  const float* u;
+  const float* v;
+  PredGrid g;
+  float y0, ysp, x0, xsp;
+};
+// validation rules of a pass (hh_pass_desc)
+struct FlagRules {
+  int32_t uod, uod_nb;
+  double uod_thr, min_ratio;
+  int32_t nval;
+  hh_validator val[HH_MAX_VALIDATORS];
+};
+// the windows of a grid: 0-based first pixel of window (gi, gj) at
+// (r0 + gi rstep, c0 + gj cstep)
+struct WinGrid {
+  int32_t r0, rstep, c0, cstep;
+};
 cudaError_t launch_combine(float* u, float* v, const float* resu, const float* resv, float* ratio, float* moment,
-                           float* alt_u, float* alt_v, int32_t nalt, const uint8_t* gmask, int64_t G,
-                           float* meas_u, float* meas_v, cudaStream_t s);
+                           float* alt_u, float* alt_v, int32_t nalt, const uint8_t* gmask, int32_t ny, int32_t nx,
+                           const NodePred& pr, float* meas_u, float* meas_v, cudaStream_t s);
+cudaError_t launch_flags(const float* u, const float* v, const float* ratio, const float* moment, int32_t ny, int32_t nx,
+                         const FlagRules& r, const uint8_t* gmask, uint8_t* flags, uint8_t* flags2, cudaStream_t s);
+cudaError_t launch_predictor(const float* u, const float* v, const uint8_t* gmask, int32_t ny, int32_t nx, bool smoothing,
+                             float* wu, float* wv, float* ou, float* ov, float* prev_u, float* prev_v, cudaStream_t s);
+cudaError_t launch_make_jobs(int32_t* jobs, int32_t ny, int32_t nx, const WinGrid& w, cudaStream_t s);
+cudaError_t launch_mask_grid(const uint8_t* mask, int64_t nr, int32_t ny, int32_t nx, const WinGrid& w, int32_t wr,
+                             int32_t wc, int32_t mr, int32_t mc, double thr, uint8_t* gmask, cudaStream_t s);
 cudaError_t launch_uod(const float* u, const float* v, int32_t ny, int32_t nx, double thr, int32_t nb, double eps,
                        const uint8_t* exclude, uint8_t* flags, int32_t or_into, cudaStream_t s);
-cudaError_t launch_flag_ratio(const float* ratio, int64_t G, double thr, uint8_t* flags, cudaStream_t s);
-cudaError_t launch_flag_moment(const float* moment, int64_t G, double thr, uint8_t* flags, cudaStream_t s);
-cudaError_t launch_flag_velocity(const float* u, const float* v, int64_t G, double vmin, double vmax,
-                                 uint8_t* flags, cudaStream_t s);
-cudaError_t launch_mask_flags(uint8_t* flags, const uint8_t* gmask, int64_t G, cudaStream_t s);
 cudaError_t launch_substitute(float* u, float* v, const uint8_t* outl_in, uint8_t* outl_out, const uint8_t* gmask,
                               const float* alt_u, const float* alt_v, int32_t nalt, int32_t ny, int32_t nx,
                               int32_t er, double thr, cudaStream_t s);

@@ -19,7 +19,7 @@ from . import _lib
 from ._lib import ArgumentError, DimensionMismatch
 from .params import PIVParameters, effort_schedule
 from .batch import _pixel_format
-from .pipeline import PIVResult, PIVWorkspace, _is_device_tensor, check_backend_params, pass_grid
+from .pipeline import PIVResult, PIVWorkspace, _grid_shape, _is_device_tensor, check_backend_params
 
 _FIELDS = ("u", "v", "peak_ratio", "correlation_moment", "uncertainty_u", "uncertainty_v")
 
@@ -190,8 +190,7 @@ def _prepare(pairs, params, effort, predictor_smoothing, mask, mask_threshold, p
 def _run(prep, workspace, scale, reducer):
     shape, passes, descs, m = prep["shape"], prep["passes"], prep["descs"], prep["mask"]
     mask_threshold, device = prep["mask_threshold"], prep["device"]
-    x, y, _, _ = pass_grid(shape, passes[-1], None, mask_threshold)
-    ny, nx = len(y), len(x)
+    ny, nx = _grid_shape(shape[0], shape[1], descs[-1])
     out = {k: np.empty((ny, nx), np.float32, order="F") for k in _FIELDS}
     outl = np.empty((ny, nx), np.uint8, order="F")
     gm = np.empty((ny, nx), np.uint8, order="F")

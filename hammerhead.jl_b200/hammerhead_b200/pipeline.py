@@ -121,6 +121,7 @@ def check_backend_params(passes):
     not implement before any work (src/ka_backend.jl:13-29)."""
     descs = (_lib.hh_pass_desc * len(passes))(*[p.to_desc() for p in passes])
     _lib.check(_lib.lib().hh_check_backend_params(descs, len(passes)))
+    return descs
 
 
 def pass_grid(imgsize, params, mask=None, mask_threshold=0.5):
@@ -140,6 +141,14 @@ def pass_grid(imgsize, params, mask=None, mask_threshold=0.5):
                               ctypes.byref(nx), _lib.fptr(x), _lib.fptr(y), _lib.u8ptr(gm), _lib.i32ptr(jobs),
                               ctypes.byref(nj)))
     return x, y, gm.astype(bool), jobs[: nj.value]
+
+
+def _grid_shape(nr, nc, desc):
+    """(ny, nx) of a pass's grid."""
+    ny, nx = ctypes.c_int32(), ctypes.c_int32()
+    _lib.check(_lib.lib().hh_pass_grid(nr, nc, ctypes.byref(desc), None, 0.5, ctypes.byref(ny), ctypes.byref(nx), None,
+                                       None, None, None, None))
+    return ny.value, nx.value
 
 
 def _is_device_tensor(a):
@@ -177,7 +186,7 @@ def run_piv(imgA, imgB, passes=None, *, effort=None, backend="b200", uncertainty
                             "build the workspace with the same `backend`")
     if not passes:
         raise ArgumentError("at least one pass is required")
-    check_backend_params(passes)
+    descs = check_backend_params(passes)
     if tuple(imgA.shape) != tuple(imgB.shape):
         raise DimensionMismatch(f"images must have the same size, got {tuple(imgA.shape)} and {tuple(imgB.shape)}")
     if len(imgA.shape) != 2:
@@ -191,8 +200,7 @@ def run_piv(imgA, imgB, passes=None, *, effort=None, backend="b200", uncertainty
     try:
         nr, nc = int(imgA.shape[0]), int(imgA.shape[1])
         final = passes[-1]
-        x, y, _, _ = pass_grid((nr, nc), final, None, mask_threshold)
-        ny, nx = len(y), len(x)
+        ny, nx = _grid_shape(nr, nc, descs[-1])
         out = {k: np.empty((ny, nx), np.float32, order="F") for k in
                ("u", "v", "peak_ratio", "correlation_moment", "uncertainty_u", "uncertainty_v")}
         outl = np.empty((ny, nx), np.uint8, order="F")
@@ -203,7 +211,6 @@ def run_piv(imgA, imgB, passes=None, *, effort=None, backend="b200", uncertainty
                              _lib.fptr(out["peak_ratio"]), _lib.fptr(out["correlation_moment"]),
                              _lib.fptr(out["uncertainty_u"]), _lib.fptr(out["uncertainty_v"]), _lib.u8ptr(outl),
                              _lib.u8ptr(gm))
-        descs = (_lib.hh_pass_desc * len(passes))(*[p.to_desc() for p in passes])
         L = _lib.lib()
         if _is_device_tensor(imgA):
             for t in (imgA, imgB) + ((mask,) if mask is not None else ()):

@@ -313,7 +313,7 @@ __global__ void __launch_bounds__(NCC_PR) ncc_pixel_kernel(const NccArgs a) {
 //    rows, then each node its columns. (A warp per node read every pixel of a
 //    node's support for itself, a third of its lanes idle, and formed the
 //    weights again for each node: 48 us at 1024^2 against 21 us.)
-constexpr int NODE_R = 16, NODE_C = 8, NODE_K = 32, NODE_THREADS = 256;
+constexpr int NODE_R = 16, NODE_C = 2, NODE_K = 32, NODE_THREADS = 256;
 struct Reach {
   int64_t lo, hi;  // 1-based pixels whose stencil may reach the node
 };
@@ -336,6 +336,7 @@ __global__ void __launch_bounds__(NODE_THREADS) ncc_node_kernel(const NccArgs a)
   // this thread's node and component in the second step
   const int ny = threadIdx.x % NODE_R, nx = threadIdx.x / NODE_R % NODE_C, comp = threadIdx.x / (NODE_R * NODE_C);
   const int gx = gx0 + nx;
+  const bool node = comp < 2 && gy0 + ny < a.gny && gx < a.gnx;
   const Reach cr = reach_of(min(gx, a.gnx - 1), a.gnx, a.x0, a.xsp, a.nc);
   double acc = 0.0;
   for (int64_t cb = c_lo; cb <= c_hi; cb += NODE_K) {
@@ -358,13 +359,13 @@ __global__ void __launch_bounds__(NODE_THREADS) ncc_node_kernel(const NccArgs a)
     }
     __syncthreads();
     const int k0 = (int)max((int64_t)0, cr.lo - cb), k1 = (int)min((int64_t)NODE_K - 1, cr.hi - cb);
-    for (int k = k0; k <= k1; ++k) {
+    for (int k = k0; node && k <= k1; ++k) {
       const float w = cell_w(a.cells, a.nr + cb + k - 1, gx, a.gnx);
       if (w != 0.f) acc += (double)w * t[comp][k][ny];
     }
     __syncthreads();
   }
-  if (gy0 + ny < a.gny && gx < a.gnx) a.grad[comp * G + (gy0 + ny) + (int64_t)gx * a.gny] = (float)acc;
+  if (node) a.grad[comp * G + (gy0 + ny) + (int64_t)gx * a.gny] = (float)acc;
 }
 
 // loss = -sum of the tiles' sums (one CTA)

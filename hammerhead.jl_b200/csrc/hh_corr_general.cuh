@@ -9,9 +9,14 @@
 //     factors up to 61 (FFTW plans any size; 2, 3 and 5 cover the usual ones);
 //   - rectangular windows and search areas (window_size / search_area_size
 //     tuples, src/types.jl:254-257), padded or not.
-// One CTA per window (grid-stride over jobs) works on its own slice of a
-// global scratch buffer -- the complex plane and the real correlation plane,
-// about 0.8 MB for a 256 x 256 plane, so 148 slices stay resident in L2:
+// Planes that fit a CTA's shared memory twice run on the kernel of
+// hh_corr_plane.cuh. One CTA per window (grid-stride over jobs) works on its
+// own slice of a global scratch buffer, which stays in L2: the complex plane
+// holds the data columns, then the kept lags' columns, the real plane the
+// kept lags only (the box), 0.3 MB for a padded 128 px window instead of the
+// 0.8 MB of both whole planes, so two 256-thread CTAs per SM work on their
+// windows side by side and cover each other's barriers and L2 latency (two
+// sweeps of 2048^2 at 128 px: 2.84 -> 2.30 ms against one CTA of 512 threads):
 //   1. window means in FP64 (masked pixels excluded), then the data columns
 //      of the packed plane Z = A + iB (mean-subtracted, apodized, zero-padded,
 //      load_windows!) transformed along the rows axis, built directly from the
@@ -30,9 +35,6 @@
 // exp(-2 pi i t / n) computed in double and rounded once.
 // (Included inside namespace hh, after analyze_group and cross_spectrum.)
 #pragma once
-
-constexpr int GC_THREADS = 512;
-constexpr int GC_WARPS = GC_THREADS / 32;
 
 // exp(-+2 pi i t / n) from the length-n table (inverse: the conjugate)
 __device__ __forceinline__ float2 gc_tw(const float2* tw, int t, bool inv) {
@@ -158,7 +160,11 @@ __device__ __forceinline__ void gc_fft16_n(float2* line, float2* tmp, int n, con
   }
 }
 
-__global__ void __launch_bounds__(GC_THREADS, 1) correlate_general_kernel(const CorrArgs a) {
+// THREADS per CTA; BOXED: the plane is zero outside its box, and not stored
+// there (else the box is the plane).
+template <int THREADS, bool BOXED>
+__global__ void __launch_bounds__(THREADS, 512 / THREADS) correlate_general_kernel(const CorrArgs a) {
+  constexpr int WARPS = THREADS / 32;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int NR = a.nfr, NC = a.nfc, wr = a.wr, wc = a.wc, sr = a.sr, sc = a.sc;
   // staged line strides (float2): room for the register form's padded exchange
@@ -169,37 +175,30 @@ __global__ void __launch_bounds__(GC_THREADS, 1) correlate_general_kernel(const 
   const size_t lines_b = a.gc_smem_lines;
   float2* buf0 = reinterpret_cast<float2*>(smem_raw);
   float2* buf1 = reinterpret_cast<float2*>(smem_raw + lines_b / 2);
-  double* part = reinterpret_cast<double*>(smem_raw + lines_b);  // GC_WARPS x 4
-  uint32_t* red = reinterpret_cast<uint32_t*>(part + 4 * GC_WARPS);
-  float* s_vals = reinterpret_cast<float*>(red + GC_WARPS * 2 * KMAX);
+  double* part = reinterpret_cast<double*>(smem_raw + lines_b);  // WARPS x 4
+  uint32_t* red = reinterpret_cast<uint32_t*>(part + 4 * WARPS);
+  float* s_vals = reinterpret_cast<float*>(red + WARPS * 2 * KMAX);
   int* s_locs = reinterpret_cast<int*>(s_vals + KMAX);
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int K = a.npeaks > 2 ? a.npeaks : 2;
   const int64_t P = (int64_t)NR * NC;
-  float2* Z = a.gscr + (int64_t)blockIdx.x * a.gscr_stride;  // complex plane, column-major, ld NR
-  float* R = reinterpret_cast<float*>(Z + P);                 // real plane, column-major, ld NR
-  const int oar = (sr - wr) / 2, oac = (sc - wc) / 2;  // frame-A window inside the search area
-  const bool search = sr != wr || sc != wc;
-  const float scale = 1.0f / (float)P;
   // rows / columns of the fftshifted plane that can be nonzero; outside this
   // box the gain (or the kept-lag restriction) makes the plane exactly zero,
   // so its columns skip the last inverse transform and the peak scan covers
   // the box (plus the last pixel, the one place outside where a zero can be
   // a regional maximum), as in the fused kernels
   const int rlo = a.gc_box[0], rhi = a.gc_box[1], clo = a.gc_box[2], chi = a.gc_box[3];
-  const ScanPlan sp = scan_plan(tid, GC_THREADS, rlo, rhi, clo, chi);
+  const int nbox = chi - clo + 1, zcols = sc > nbox ? sc : nbox;
+  const int ldb = (rhi - rlo + 1) | 1;  // real plane: column js at js * ldb, row is (both fftshifted)
+  // complex plane, column-major, ld NR: data columns j, after step 2 box columns js - clo
+  float2* Z = a.gscr + (int64_t)blockIdx.x * a.gscr_stride;
+  float* R = reinterpret_cast<float*>(Z + (int64_t)zcols * NR) - ((int64_t)clo * ldb + rlo);
+  const int oar = (sr - wr) / 2, oac = (sc - wc) / 2;  // frame-A window inside the search area
+  const bool search = sr != wr || sc != wc;
+  const float scale = 1.0f / (float)P;
+  const ScanPlan sp = scan_plan(tid, THREADS, rlo, rhi, clo, chi);
   PeakOut po{a.du, a.dv, a.ratio, a.moment, a.alt_u, a.alt_v, a.nalt, a.G, a.packed, a.locs};
-
-  // the real plane outside the box's columns is zero for every window of
-  // this launch (the box is the launch's): cleared once here, never rewritten
-  for (int c = warp; c < NC; c += GC_WARPS) {
-    const int js = c;
-    if (js >= clo && js <= chi) continue;
-    float* rc = R + (int64_t)js * NR;
-    for (int i = lane; i < NR; i += 32) rc[i] = 0.f;
-  }
-  __syncthreads();
 
   for (int64_t job = blockIdx.x; job < a.njobs; job += gridDim.x) {
     int rs, cs;
@@ -232,35 +231,51 @@ __global__ void __launch_bounds__(GC_THREADS, 1) correlate_general_kernel(const 
     // search-area origin: the window's origin less the centring offset
     const int64_t r0 = (int64_t)rs - oar, c0 = (int64_t)cs - oac;
 
-    // ---- 1a. means over the unmasked pixels (FP64, one rounding)
-    double sa = 0.0, sb = 0.0, na = 0.0, nb = 0.0;
-    for (int j = warp; j < sc; j += GC_WARPS)  // warps on columns, lanes down the rows
-      for (int i = lane; i < sr; i += 32) {
-        const int64_t off = (r0 + i) + (c0 + j) * ld;
-        if (M && __ldg(M + off)) continue;
-        sb += (double)__ldg(B + off);
-        nb += 1.0;
-        if ((unsigned)(i - oar) < (unsigned)wr && (unsigned)(j - oac) < (unsigned)wc) {
-          sa += (double)__ldg(A + off);
-          na += 1.0;
+    // ---- 1a. means over the unmasked pixels (FP64, one rounding); the loads
+    //      are predicated, so that those of several pixels are in flight
+    double sa = 0.0, sb = 0.0;
+    int na = 0, nb = 0;
+    for (int j = warp; j < sc; j += WARPS) {  // warps on columns, lanes down the rows
+      const bool cina = (unsigned)(j - oac) < (unsigned)wc;
+      for (int ib = lane; ib < sr + lane; ib += 128) {
+        float va[4], vb[4];
+        uint8_t mk[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int i = ib + 32 * u;
+          const bool in = i < sr;
+          const int64_t off = (r0 + i) + (c0 + j) * ld;
+          va[u] = ld_keep_if(A + off, in && cina && (unsigned)(i - oar) < (unsigned)wr);
+          vb[u] = ld_keep_if(B + off, in);
+          mk[u] = ld_stream_if(M + off, in && M);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int i = ib + 32 * u;
+          const bool on = i < sr && !mk[u], ina = on && cina && (unsigned)(i - oar) < (unsigned)wr;
+          sb += (double)(on ? vb[u] : 0.f);
+          sa += (double)(ina ? va[u] : 0.f);
+          nb += on;
+          na += ina;
         }
       }
+    }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
       sa += __shfl_xor_sync(0xffffffffu, sa, o);
       sb += __shfl_xor_sync(0xffffffffu, sb, o);
-      na += __shfl_xor_sync(0xffffffffu, na, o);
-      nb += __shfl_xor_sync(0xffffffffu, nb, o);
     }
+    na = __reduce_add_sync(0xffffffffu, na);
+    nb = __reduce_add_sync(0xffffffffu, nb);
     if (lane == 0) {
       part[4 * warp] = sa;
       part[4 * warp + 1] = sb;
-      part[4 * warp + 2] = na;
-      part[4 * warp + 3] = nb;
+      part[4 * warp + 2] = (double)na;
+      part[4 * warp + 3] = (double)nb;
     }
     __syncthreads();
     double ta = 0.0, tb = 0.0, tna = 0.0, tnb = 0.0;
-    for (int w = 0; w < GC_WARPS; ++w) {
+    for (int w = 0; w < WARPS; ++w) {
       ta += part[4 * w];
       tb += part[4 * w + 1];
       tna += part[4 * w + 2];
@@ -283,22 +298,21 @@ __global__ void __launch_bounds__(GC_THREADS, 1) correlate_general_kernel(const 
         float2* l0 = wbuf + (regR ? hw * 2 * LDR : 0);
         float2* l1 = l0 + LDR;
         if (act) {
+          const int ja = j - oac;
+          const bool cina = (unsigned)ja < (unsigned)wc;
 #pragma unroll 4
           for (int i = i0; i < NR; i += st) {
+            const int ia = i - oar;
+            const bool in = i < sr && !bad, ina = in && cina && (unsigned)ia < (unsigned)wr;
+            const int64_t off = (r0 + i) + (c0 + j) * ld;
+            const float va = ld_keep_if(A + off, ina), vb = ld_keep_if(B + off, in);
+            const float ap = ld_keep_if(a.apod + ia + ja * wr, ina);
+            const bool mk = ld_stream_if(M + off, in && M) != 0;
             float2 z = make_float2(0.f, 0.f);
-            if (i < sr && !bad) {
-              const int64_t off = (r0 + i) + (c0 + j) * ld;
-              if (!(M && __ldg(M + off))) {
-                const int ia = i - oar, ja = j - oac;
-                const bool ina = (unsigned)ia < (unsigned)wr && (unsigned)ja < (unsigned)wc;
-                if (search) {
-                  z.y = __ldg(B + off) - mb;
-                  if (ina) z.x = __ldg(a.apod + ia + ja * wr) * (__ldg(A + off) - ma);
-                } else {
-                  const float ap = __ldg(a.apod + i + j * wr);
-                  z = make_float2(ap * (__ldg(A + off) - ma), ap * (__ldg(B + off) - mb));
-                }
-              }
+            if (in && !mk) {
+              // rounded here, whether or not the transform adds to it next
+              if (ina) z.x = __fmul_rn(ap, __fsub_rn(va, ma));
+              z.y = search ? __fsub_rn(vb, mb) : __fmul_rn(ap, __fsub_rn(vb, mb));
             }
             l0[i] = z;
           }
@@ -326,7 +340,7 @@ __global__ void __launch_bounds__(GC_THREADS, 1) correlate_general_kernel(const 
       for (int l0 = lane; l0 < 2 * nh; l0 += 32) {
         const int ra = h0 + (l0 >> 1), row = (l0 & 1) ? (NR - ra) % NR : ra;
 #pragma unroll 8
-        for (int j = warp; j < NC; j += GC_WARPS)
+        for (int j = warp; j < NC; j += WARPS)
           buf0[l0 * LDC + j] = j < sc ? Z[(int64_t)j * NR + row] : make_float2(0.f, 0.f);
       }
       __syncthreads();
@@ -334,14 +348,14 @@ __global__ void __launch_bounds__(GC_THREADS, 1) correlate_general_kernel(const 
         const int l = 2 * warp + hw;
         gc_fft16_n<false>(buf0 + l * LDC, buf1 + l * LDC, NC, a.twc, hl, l < 2 * nh);
       } else {
-        for (int l = warp; l < 2 * nh; l += GC_WARPS)
+        for (int l = warp; l < 2 * nh; l += WARPS)
           gc_line(buf0 + l * LDC, buf1 + l * LDC, NC, a.gc_radix_c, a.gc_nst_c, a.twc, false, lane);
       }
       __syncthreads();
       // the register form leaves its result in place
       float2* fz = (!regC && (a.gc_nst_c & 1)) ? buf1 : buf0;  // forward rows
       float2* sz = (!regC && (a.gc_nst_c & 1)) ? buf0 : buf1;  // spectrum rows
-      for (int l = warp; l < 2 * nh; l += GC_WARPS) {
+      for (int l = warp; l < 2 * nh; l += WARPS) {
         const int ra = h0 + (l >> 1), row = (l & 1) ? (NR - ra) % NR : ra;
         const float2* Za = fz + l * LDC;          // this row
         const float2* Zb = fz + (l ^ 1) * LDC;    // its partner row (-r)
@@ -355,7 +369,7 @@ __global__ void __launch_bounds__(GC_THREADS, 1) correlate_general_kernel(const 
         const int l = 2 * warp + hw;
         gc_fft16_n<true>(sz + l * LDC, fz + l * LDC, NC, a.twc, hl, l < 2 * nh);
       } else {
-        for (int l = warp; l < 2 * nh; l += GC_WARPS)
+        for (int l = warp; l < 2 * nh; l += WARPS)
           gc_line(sz + l * LDC, fz + l * LDC, NC, a.gc_radix_c, a.gc_nst_c, a.twc, true, lane);
       }
       __syncthreads();
@@ -364,20 +378,16 @@ __global__ void __launch_bounds__(GC_THREADS, 1) correlate_general_kernel(const 
         const int ra = h0 + (l0 >> 1), row = (l0 & 1) ? (NR - ra) % NR : ra;
         if ((l0 & 1) && row == ra) continue;  // a self-paired row (0, NR/2) is written once
 #pragma unroll 4
-        for (int j = warp; j < NC; j += GC_WARPS) {
-          const int js = j + NC / 2 < NC ? j + NC / 2 : j + NC / 2 - NC;
-          if (js < clo || js > chi) continue;  // a column that step 3 writes as zeros
-          Z[(int64_t)j * NR + row] = iz[l0 * LDC + j];
+        for (int b = warp; b < nbox; b += WARPS) {  // the box's columns (fftshifted clo + b)
+          const int js = clo + b, j = js >= NC / 2 ? js - NC / 2 : js - NC / 2 + NC;
+          Z[(int64_t)b * NR + row] = iz[l0 * LDC + j];
         }
       }
       __syncthreads();
     }
 
-    // ---- 3. columns back, then |.| / (nr nc), fftshift, gain, kept lags;
-    //      columns whose shifted position lies outside the box are zero
-    //      (those columns were cleared at the start of the launch)
-    const int nbox = chi - clo + 1;
-    //      the box's columns, one warp each: unshifted column j = (js - NC/2) mod NC
+    // ---- 3. the box's columns back, one warp each, then |.| / (nr nc),
+    //      fftshift, gain, kept lags, for the box's rows
     if (warp < a.gc_col_warps) {
       const int lpw = regR ? 2 : 1;
       float2* wbuf = buf0 + (size_t)warp * 2 * lpw * LDR;
@@ -387,9 +397,9 @@ __global__ void __launch_bounds__(GC_THREADS, 1) correlate_general_kernel(const 
         const int i0 = regR ? hl : lane, st = regR ? 16 : 32;
         float2* l0 = wbuf + (regR ? hw * 2 * LDR : 0);
         float2* l1 = l0 + LDR;
-        const int js = clo + (act ? b : 0), j = (js + NC - NC / 2) % NC;
+        const int js = clo + (act ? b : 0);
         if (act) {
-          const float2* zc = Z + (int64_t)j * NR;
+          const float2* zc = Z + (int64_t)b * NR;
 #pragma unroll 8
           for (int i = i0; i < NR; i += st) l0[i] = zc[i];
         }
@@ -397,17 +407,16 @@ __global__ void __launch_bounds__(GC_THREADS, 1) correlate_general_kernel(const 
         const float2* res = l0;
         if (regR) gc_fft16_n<true>(l0, l1, NR, a.twr, hl, act);
         else res = gc_line(l0, l1, NR, a.gc_radix_r, a.gc_nst_r, a.twr, true, lane);
-        float* rc = R + (int64_t)js * NR;
-        const bool colkept = !search || abs(js - NC / 2) <= oac;
-        if (act)
-        for (int i = i0; i < NR; i += st) {
-          const float2 c = res[i];
-          const int is = i + NR / 2 < NR ? i + NR / 2 : i + NR / 2 - NR;  // fftshifted row
-          float v = hypotf(c.x * scale, c.y * scale);
-          if (a.gain) v *= __ldg(a.gain + is + (int64_t)js * NR);
-          if (!colkept || (search && abs(is - NR / 2) > oar)) v = 0.f;
-          if (bad) v = __int_as_float(0x7fc00000);
-          rc[is] = v;
+        float* rc = R + (int64_t)js * ldb;
+        if (act) {
+#pragma unroll 2
+          for (int is = rlo + i0; is <= rhi; is += st) {
+            const float2 c = res[is >= NR / 2 ? is - NR / 2 : is - NR / 2 + NR];  // fftshifted row is
+            float v = hypotf(c.x * scale, c.y * scale);
+            if (a.gain) v *= __ldg(a.gain + is + (int64_t)js * NR);
+            if (bad) v = __int_as_float(0x7fc00000);
+            rc[is] = v;
+          }
         }
         __syncwarp();
       }
@@ -417,15 +426,30 @@ __global__ void __launch_bounds__(GC_THREADS, 1) correlate_general_kernel(const 
     // ---- 4. plane out (correlation_planes / ensemble sums) and analysis
     if (a.planes) {  // a window holding NaN or Inf has a NaN plane, as in the reference
       float* dst = a.planes + job * P;
-      for (int64_t e = tid; e < P; e += GC_THREADS) {
-        const float v = bad ? __int_as_float(0x7fc00000) : R[e];
+      for (int64_t e = tid; e < P; e += THREADS) {
+        const int is = (int)(e % NR), js = (int)(e / NR);
+        const bool in = !BOXED || (is >= rlo && is <= rhi && js >= clo && js <= chi);
+        const float v = bad ? __int_as_float(0x7fc00000) : (in ? R[(int64_t)js * ldb + is] : 0.f);
         dst[e] = a.accumulate ? dst[e] + v : v;
       }
     }
     if (!a.accumulate) {
-      analyze_group(R, NR, NC, NR, K, a.npeaks, a.finder, a.subpixel, tid, GC_THREADS, red, true, s_vals, s_locs,
-                    gid, job, &pw, bad, 0, sp, nullptr, 0);
+      analyze_group<0, BOXED>(R, NR, NC, ldb, K, a.npeaks, a.finder, a.subpixel, tid, THREADS, red, true, s_vals, s_locs,
+                              gid, job, &pw, bad, 0, sp, nullptr, 0);
     }
-    __syncthreads();  // the scratch plane and shared buffers are reused by the CTA's next window
+    __syncthreads();  // the planes and shared buffers are reused by the CTA's next window
   }
+}
+
+template <int THREADS, bool BOXED> static cudaError_t launch_general(const CorrArgs& a, cudaStream_t s) {
+  static bool attr = false;  // raised to the device's limit once: launches of different shapes may share a graph
+  if (!attr) {
+    cudaError_t e = cudaFuncSetAttribute(correlate_general_kernel<THREADS, BOXED>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    if (e != cudaSuccess) return e;
+    attr = true;
+  }
+  const int64_t grid = a.njobs < a.gscr_slices ? a.njobs : a.gscr_slices;
+  correlate_general_kernel<THREADS, BOXED><<<(unsigned)grid, THREADS, a.gc_smem_bytes, s>>>(a);
+  return cudaGetLastError();
 }

@@ -43,6 +43,13 @@ __device__ __forceinline__ uint8_t ld_stream_if(const uint8_t* p, bool on) {
       : "=h"(v) : "l"(p), "r"((int)on));
   return (uint8_t)v;
 }
+__device__ __forceinline__ float ld_keep_if(const float* p, bool on) {
+  float v;
+  asm("{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %2, 0;\n\tmov.f32 %0, 0f00000000;\n\t"
+      "@p ld.global.nc.f32 %0, [%1];\n\t}"
+      : "=f"(v) : "l"(p), "r"((int)on));
+  return v;
+}
 __device__ __forceinline__ float ld_keep(const float* p) {
   float v;
   asm("ld.global.nc.L1::evict_last.f32 %0, [%1];" : "=f"(v) : "l"(p));
@@ -211,12 +218,12 @@ struct PlaneAcc {
   int ld;
   __device__ __forceinline__ float operator()(int i, int j) const { return p[j * ld + i]; }
 };
-// a plane that is zero, and not stored, outside rows and columns [lo, hi]
+// a plane that is zero, and not stored, outside rows [rlo, rhi] x columns [clo, chi]
 struct BoxAcc {
   const float* p;
-  int ld, lo, hi;
+  int ld, rlo, rhi, clo, chi;
   __device__ __forceinline__ float operator()(int i, int j) const {
-    return i >= lo && i <= hi && j >= lo && j <= hi ? p[j * ld + i] : 0.f;
+    return i >= rlo && i <= rhi && j >= clo && j <= chi ? p[j * ld + i] : 0.f;
   }
 };
 struct RecAcc {
@@ -620,8 +627,8 @@ __device__ __forceinline__ void scan_rows(TK& tk, const float* R, int ldr, int K
 
 // FN > 0: an FN x FN plane of a fused kernel with its row maxima (scan_rows);
 // FN = 0: any plane, by column strips. BOXED: the plane is zero, and not
-// stored, outside the box [rlo, rhi] x [clo, chi] (square, and away from the
-// plane's edges).
+// stored, outside the box [rlo, rhi] x [clo, chi], which leaves at least the
+// plane's last row and column out.
 template <int KC, int FN, bool BOXED>
 __device__ __forceinline__ void analyze_body(const float* R, int nr, int nc, int ldr, int K, int npeaks, int finder,
                                              int subpixel, int gtid, int gsize, uint32_t* red, bool active,
@@ -635,7 +642,7 @@ __device__ __forceinline__ void analyze_body(const float* R, int nr, int nc, int
   const bool scan = active && !poison;
   const int gwarp = gtid >> 5, nwarps = gsize >> 5;
   const int P = nr * nc;
-  const BoxAcc box{R, ldr, rlo, rhi};
+  const BoxAcc box{R, ldr, rlo, rhi, clo, chi};
   auto at = [&](int i, int j) { return BOXED ? box(i, j) : R[j * ldr + i]; };
   int nfound = 0;
   if (finder == 0) {
@@ -683,8 +690,9 @@ __device__ __forceinline__ void analyze_body(const float* R, int nr, int nc, int
     }
     if (scan && gtid == 0 && (rhi < nr - 1 || chi < nc - 1)) {  // the last pixel, outside the box
       const int r = nr - 1, c = nc - 1;
-      if (BOXED) tk.insert(fkey(0.f), ~(uint32_t)(r + c * nr), K);  // a zero among zeros
-      else if (is_local_max(R, nr, nc, ldr, r, c, R[c * ldr + r]))
+      if (BOXED) {  // a zero; its neighbours are zeros too but for a box that reaches the diagonal one
+        if (!(at(r - 1, c - 1) > 0.f)) tk.insert(fkey(0.f), ~(uint32_t)(r + c * nr), K);
+      } else if (is_local_max(R, nr, nc, ldr, r, c, R[c * ldr + r]))
         tk.insert(fkey(R[c * ldr + r]), ~(uint32_t)(r + c * nr), K);
     }
     // Merge: each warp takes its K best from its threads' lists by shuffle
@@ -799,7 +807,7 @@ __device__ __forceinline__ void analyze_body(const float* R, int nr, int nc, int
   }
   if (gtid == 0) {
     if constexpr (BOXED)
-      peak_outputs(BoxSrc{{R, ldr, rlo, rhi}}, nr, nc, K, npeaks, subpixel, nfound, s_vals, s_locs, grid_id, job, *o);
+      peak_outputs(BoxSrc{{R, ldr, rlo, rhi, clo, chi}}, nr, nc, K, npeaks, subpixel, nfound, s_vals, s_locs, grid_id, job, *o);
     else
       peak_outputs(PlaneSrc{R, ldr}, nr, nc, K, npeaks, subpixel, nfound, s_vals, s_locs, grid_id, job, *o);
   }

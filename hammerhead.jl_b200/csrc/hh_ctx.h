@@ -469,29 +469,68 @@ inline hh_status gcorr_setup(hh_ctx* ctx, const hh_pass_desc& p, CorrArgs& ca) {
                     std::to_string(ca.nfc));
   HH_TRY(gc_twiddles(ctx, ca.nfr, &ca.twr));
   HH_TRY(gc_twiddles(ctx, ca.nfc, &ca.twc));
-  // columns passes: per warp one line (two, one per half-warp, for the
-  // register-form lengths 32..256), two buffers per line, as many warps (of
-  // 16) as fit; rows pass: chunks of row pairs, two buffers each. Lines are
-  // staged with 16 elements of padding (the register form's exchange).
-  const size_t ldr = (size_t)ca.nfr + 16, ldc = (size_t)ca.nfc + 16;
-  const int lpw = gc_reg_length(ca.nfr) ? 2 : 1;
-  ca.gc_col_warps = std::max(1, std::min(16, (int)(GC_SMEM_LINES / (2 * lpw * ldr * sizeof(float2)))));
-  ca.gc_chunk_c = std::max(2, std::min(32, (int)(GC_SMEM_LINES / (2 * ldc * sizeof(float2)))) & ~1);
-  const size_t lines = std::max((size_t)ca.gc_col_warps * lpw * ldr, (size_t)ca.gc_chunk_c * ldc);
-  ca.gc_smem_lines = (int64_t)(2 * lines * sizeof(float2));
-  const int64_t P = (int64_t)ca.nfr * ca.nfc;
-  ca.gscr_stride = (P + (P + 1) / 2 + 31) & ~(int64_t)31;  // complex plane + real plane, 256-byte aligned slices
-  ca.gscr_slices = ctx->num_sms;
   Tables tb;
   HH_TRY(get_tables(ctx, p, tb));
   ca.gc_box[0] = tb.rlo;
   ca.gc_box[1] = tb.rhi;
   ca.gc_box[2] = tb.clo;
   ca.gc_box[3] = tb.chi;
+  // columns passes: per warp one line (two, one per half-warp, for the
+  // register-form lengths 32..256), two buffers per line, as many warps as
+  // fit; rows pass: chunks of row pairs, two buffers each, at most two lines
+  // per warp. Lines are staged with 16 elements of padding (the register
+  // form's exchange). The complex plane holds the data columns, later the
+  // box's, the real plane the box.
+  const size_t ldr = (size_t)ca.nfr + 16, ldc = (size_t)ca.nfc + 16;
+  const int lpw = gc_reg_length(ca.nfr) ? 2 : 1;
+  const int64_t nboxc = tb.chi - tb.clo + 1, ldb = (tb.rhi - tb.rlo + 1) | 1;
+  const int64_t zf = std::max<int64_t>(p.search[1], nboxc) * ca.nfr;  // float2
+  const size_t planes = (size_t)zf * sizeof(float2) + (size_t)(nboxc * ldb) * sizeof(float);
+  // An SM has 228 KB of shared memory, 1 KB of it taken per CTA, and registers
+  // for 6, 2 or 1 CTAs of 128, 256 or 512 threads. The smallest CTA whose
+  // planes leave room for 4, 2 or 1 of it: a window is then slower, but several
+  // cover each other's barriers (6 CTAs of 128 threads against 4: 0.33 and
+  // 0.35 ms for 8001 windows of 24 x 16, padded).
+  constexpr size_t SM = 228 * 1024, CTA = 1024;
+  int per_sm = 0;
+  for (int t : {128, 256, 512}) {
+    const size_t b = hh::gcorr_plane_smem(ca.nfr, ca.nfc, tb.rhi - tb.rlo + 1, nboxc, t);
+    if (b > SM * t / 512 - CTA) continue;
+    per_sm = t == 128 ? std::min<int>(hh::gcorr_plane_ctas, (int)(SM / (b + CTA))) : 512 / t;
+    ca.gc_threads = t;
+    ca.gc_in_smem = 1;
+    ca.gc_smem_bytes = b;
+    break;
+  }
+  if (!per_sm) {
+    // Planes that fit no CTA's shared memory go to L2: 256 threads and two
+    // CTAs per SM while their line buffers fit twice, and the slices together
+    // stay within L2 (2.84 -> 2.30 ms for two sweeps of 256 x 256 planes at
+    // 2048^2); else one CTA of 512.
+    auto shape = [&](int threads) {
+      const int warps = threads / 32;
+      ca.gc_threads = threads;
+      ca.gc_in_smem = 0;
+      ca.gc_col_warps = std::max(1, std::min(warps, (int)(GC_SMEM_LINES / (2 * lpw * ldr * sizeof(float2)))));
+      ca.gc_chunk_c = std::max(2, std::min(2 * warps, (int)(GC_SMEM_LINES / (2 * ldc * sizeof(float2)))) & ~1);
+      const size_t lines = std::max((size_t)ca.gc_col_warps * lpw * ldr, (size_t)ca.gc_chunk_c * ldc);
+      ca.gc_smem_lines = (int64_t)(2 * lines * sizeof(float2));
+      ca.gc_smem_bytes = ca.gc_smem_lines + hh::gcorr_smem_extra(warps);
+      return (size_t)ca.gc_smem_bytes;
+    };
+    per_sm = 2;
+    if (shape(256) > SM / 2 - CTA || 2 * ctx->num_sms * planes > (size_t)110 << 20) {
+      per_sm = 1;
+      shape(512);
+    }
+  }
+  ca.gscr_slices = per_sm * ctx->num_sms;
+  ca.gscr_stride = ca.gc_in_smem ? 0 : (zf + (nboxc * ldb + 1) / 2 + 31) & ~(int64_t)31;  // 256-byte aligned slices
   return HH_OK;
 }
 inline hh_status gcorr_prepare(hh_ctx* ctx, const hh_pass_desc& p, CorrArgs& ca) {
   HH_TRY(gcorr_setup(ctx, p, ca));
+  if (ca.gc_in_smem) return HH_OK;
   return buf(ctx, "gcorr_scratch", (size_t)ca.gscr_slices * ca.gscr_stride, &ca.gscr);
 }
 

@@ -68,7 +68,8 @@ struct CorrArgs {
   float* rec;
   // general-shape path (correlate_general_kernel): window wr x wc, search
   // area sr x sc, FFT plane nfr x nfc; gscr holds one scratch slice of
-  // gscr_stride float2 per CTA (complex plane + real plane); twr / twc the
+  // gscr_stride float2 per CTA (complex and real plane; none when they live in
+  // shared memory), gscr_slices is the number of CTAs; twr / twc the
   // twiddle tables exp(-2 pi i t / n) of the two lengths and their radix
   // plans; the line buffers' layout and shared bytes
   int32_t wr, wc, sr, sc, nfr, nfc;
@@ -81,6 +82,8 @@ struct CorrArgs {
   int32_t gc_nst_r, gc_nst_c;
   int32_t gc_col_warps, gc_chunk_c;  // warps of the columns passes (one line each); rows-pass lines per chunk
   int64_t gc_smem_lines;
+  int32_t gc_threads, gc_in_smem;  // threads per CTA; whether the planes live in shared memory
+  int64_t gc_smem_bytes;           // shared memory per CTA
   // fftshifted rows [0], [1] and columns [2], [3] outside which the plane is
   // zero (overlap-gain support or kept search lags; the whole plane otherwise)
   int32_t gc_box[4];
@@ -95,12 +98,18 @@ bool correlate_supported(int N, int W);
 // The general-shape correlation (any FFT lengths, rectangular windows and
 // search areas): a.wr .. a.gc_smem_lines set by the host (gcorr_prepare).
 cudaError_t launch_correlate_general(const CorrArgs& a, cudaStream_t s);
+// shared memory of a general-shape CTA beside its line buffers and planes
+__host__ __device__ constexpr size_t gcorr_smem_extra(int warps) {
+  return warps * (4 * sizeof(double) + 2 * KMAX * sizeof(uint32_t)) + KMAX * (sizeof(float) + 2 * sizeof(int)) + 64;
+}
+// CTAs of 128 threads per SM of the kernel that holds the planes in shared
+// memory (hh_corr_plane.cuh), and its shared memory per CTA
+constexpr int gcorr_plane_ctas = 6;
+size_t gcorr_plane_smem(int nr, int nc, int box_rows, int box_cols, int threads);
 // Radix plan of an FFT length (factors 4, 2, then odd primes <= 61);
 // returns the stage count, or -1 when a factor exceeds 61 or there are more
 // than 24 stages.
 int gcorr_radix_plan(int n, int8_t* radix);
-// Shared bytes the general kernel needs beyond its line buffers.
-size_t gcorr_smem_extra();
 size_t correlate_record_words(int npeaks);  // per job
 size_t correlate_smem_bytes(int N, int W);
 

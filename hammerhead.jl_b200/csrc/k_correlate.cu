@@ -8,6 +8,8 @@ namespace hh {
 // the general-shape kernel (any FFT lengths, rectangular windows, planes
 // larger than a CTA's shared memory)
 #include "hh_corr_general.cuh"
+// ... and the same with the plane in shared memory
+#include "hh_corr_plane.cuh"
 
 // Device analysis of caller-supplied planes (one CTA of 128 threads each).
 // The plane is staged in shared memory when it fits (in_smem), else read in
@@ -79,6 +81,10 @@ cudaError_t launch_peak_epilogue(const CorrArgs& a, int N, cudaStream_t s, int n
   return cudaGetLastError();
 }
 
+size_t gcorr_plane_smem(int nr, int nc, int box_rows, int box_cols, int threads) {
+  return plane_smem(nr, nc, box_rows, box_cols, threads / 32);
+}
+
 size_t correlate_record_words(int npeaks) { return (size_t)rec_words(npeaks > 2 ? npeaks : 2); }
 
 #define HH_CORR_SIZES(X) X(16) X(24) X(32) X(48) X(64) X(96) X(128)
@@ -134,26 +140,24 @@ int gcorr_radix_plan(int n, int8_t* radix) {
   return n == 1 ? ns : -1;
 }
 
-size_t gcorr_smem_extra() {
-  return 4 * GC_WARPS * sizeof(double) + GC_WARPS * 2 * KMAX * sizeof(uint32_t) + KMAX * sizeof(float) +
-         2 * KMAX * sizeof(int) + 64;
-}
-
 cudaError_t launch_correlate_general(const CorrArgs& a, cudaStream_t s) {
   if (a.njobs <= 0) return cudaSuccess;
-  if (!a.gscr || !a.twr || !a.twc || a.gscr_slices < 1 || a.gc_col_warps < 1 || a.gc_col_warps > GC_WARPS ||
-      a.gc_chunk_c < 2)
+  if (!a.twr || !a.twc || a.gscr_slices < 1 || a.gc_smem_bytes > 227 * 1024) return cudaErrorInvalidValue;
+  if (!a.gc_in_smem && (!a.gscr || a.gc_col_warps < 1 || a.gc_col_warps > a.gc_threads / 32 || a.gc_chunk_c < 2))
     return cudaErrorInvalidValue;
-  const size_t sm = (size_t)a.gc_smem_lines + gcorr_smem_extra();
-  static size_t attr = 0;
-  if (sm > attr) {
-    cudaError_t e = cudaFuncSetAttribute(correlate_general_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (e != cudaSuccess) return e;
-    attr = sm;
-  }
-  const int64_t grid = a.njobs < a.gscr_slices ? a.njobs : a.gscr_slices;
-  correlate_general_kernel<<<(unsigned)grid, GC_THREADS, sm, s>>>(a);
-  return cudaGetLastError();
+  const bool boxed = a.gc_box[0] > 0 || a.gc_box[2] > 0 || a.gc_box[1] < a.nfr - 1 || a.gc_box[3] < a.nfc - 1;
+  // a box smaller than the plane leaves its last row and column out
+  if (boxed && (a.gc_box[1] > a.nfr - 2 || a.gc_box[3] > a.nfc - 2)) return cudaErrorInvalidValue;
+  if (a.gc_in_smem) switch (a.gc_threads) {
+      case 128: return boxed ? launch_plane<128, true>(a, s) : launch_plane<128, false>(a, s);
+      case 256: return boxed ? launch_plane<256, true>(a, s) : launch_plane<256, false>(a, s);
+      case 512: return boxed ? launch_plane<512, true>(a, s) : launch_plane<512, false>(a, s);
+    }
+  else switch (a.gc_threads) {
+      case 256: return boxed ? launch_general<256, true>(a, s) : launch_general<256, false>(a, s);
+      case 512: return boxed ? launch_general<512, true>(a, s) : launch_general<512, false>(a, s);
+    }
+  return cudaErrorInvalidValue;
 }
 
 cudaError_t launch_analyze_planes(const AnalyzeArgs& a, cudaStream_t s) {

@@ -87,3 +87,46 @@ def test_default_equals_alternative_shape(fft, padding, method):
     for k in (0, 2):
         for x, y in zip(got[k], got[k + 1]):
             np.testing.assert_array_equal(x, y)
+
+
+@pytest.mark.parametrize("window,search", [((24, 16), None), ((48, 32), None), ((12, 20), None), ((14, 22), None),
+                                           ((9, 26), None), ((64, 4), None), ((4, 34), None), ((50, 10), None),
+                                           ((128, 40), None), ((16, 12), (24, 30)), ((100, 128), None)])
+@pytest.mark.parametrize("method", ["cross", "phase"])
+def test_general_shapes_vs_fp64(window, search, method):
+    """General shapes (prime factors 2 to 17, register and Stockham lengths,
+    planes for every CTA size): the unpadded plane against numpy in FP64
+    (within 2e-5 of the peak), and the peaks against the plane analysis, bit for bit."""
+    import hammerhead_b200 as hb
+    from hammerhead_b200 import hooks
+
+    s = search or window
+    rng = np.random.default_rng(sum(window))
+    n, m = s[0] + 7, 2 * s[1] + 3
+    A, B = rng.random((2, n, m)).astype(np.float32)
+    p = hb.PIVParameters(window_size=window, search_area_size=s, overlap=0, correlation_method=method, n_peaks=4)
+    _, _, _, jobs = hb.pass_grid((n, m), p)
+    with hb.piv_workspace() as ws:
+        d = hooks.DeviceSession(ws)
+        d.stage_pair(A, B)
+        planes = d.correlation_planes(p, jobs)
+        out, locs, _ = d.process_windows(p, jobs, want_locs=True)
+        if s[0] * s[1] * 4 <= 180 * 1024:
+            ref, rlocs = hooks.analyze_planes(ws, planes, 4)
+            np.testing.assert_array_equal(locs, rlocs)
+            np.testing.assert_array_equal(out, ref)
+    if method == "phase":  # bins of small magnitude: no bound on the plane by its peak
+        return
+    o = [(s[k] - window[k]) // 2 for k in range(2)]
+    for j, (_, _, rs, cs) in enumerate(jobs):
+        r, c = rs - 1, cs - 1
+        a = np.zeros(s)
+        w = A[r:r + window[0], c:c + window[1]].astype(float)
+        a[o[0]:o[0] + window[0], o[1]:o[1] + window[1]] = w - w.mean()
+        b = B[r - o[0]:r - o[0] + s[0], c - o[1]:c - o[1] + s[1]].astype(float)
+        S = np.conj(np.fft.fft2(a)) * np.fft.fft2(b - b.mean())
+        R = np.fft.fftshift(np.abs(np.fft.ifft2(S)))
+        if search:
+            keep = [np.abs(np.arange(s[k]) - s[k] // 2) <= o[k] for k in range(2)]
+            R = R * (keep[0][:, None] & keep[1][None])
+        assert np.abs(planes[j] - R).max() <= 2e-5 * R.max()

@@ -540,13 +540,13 @@ inline hh_status gcorr_prepare(hh_ctx* ctx, const hh_pass_desc& p, CorrArgs& ca)
 inline void uq_setup(hh_ctx* ctx, int wr, int wc, hh::UQArgs& ua) {
   ua.W = wr;
   ua.Wc = wc;
-  if (!hh::uq_general(wr, wc)) return;
+  if (!hh::uq_general_scratch(wr, wc)) return;
   ua.gscr_stride = hh::uq_general_stride(wr, wc);
   ua.gscr_slices = 4 * ctx->num_sms;
 }
 inline hh_status uq_prepare(hh_ctx* ctx, int wr, int wc, hh::UQArgs& ua) {
   uq_setup(ctx, wr, wc, ua);
-  if (!hh::uq_general(wr, wc)) return HH_OK;
+  if (!hh::uq_general_scratch(wr, wc)) return HH_OK;
   return buf(ctx, "uq_scratch", (size_t)ua.gscr_slices * ua.gscr_stride, &ua.gscr);
 }
 

@@ -231,6 +231,7 @@ cudaError_t launch_uq(const UQArgs& a, cudaStream_t s, int num_sms);
 // Does this window shape run the general (global-scratch) form, and how many
 // doubles does one window's scratch slice take?
 bool uq_general(int wr, int wc);
+bool uq_general_scratch(int wr, int wc);  // ... and does it need the scratch (else shared memory)?
 int64_t uq_general_stride(int wr, int wc);
 // finalize_uncertainty of pooled statistics (88 per job) into grid cells
 cudaError_t launch_uq_finalize(const double* stats, const int32_t* jobs, int64_t njobs, int32_t ny, float* unc_u,

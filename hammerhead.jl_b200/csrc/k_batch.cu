@@ -98,7 +98,7 @@ __global__ void b_flags_kernel(const BPair* __restrict__ bp, int npairs, const i
 }
 
 // secondary-peak substitution (src/quality.jl:307-351): outl -> outl2
-__global__ void b_substitute_kernel(const BPair* __restrict__ bp, int npairs, const int32_t* __restrict__ done, int it,
+__global__ void __launch_bounds__(128, 3) b_substitute_kernel(const BPair* __restrict__ bp, int npairs, const int32_t* __restrict__ done, int it,
                                     int64_t gtot, BGrid g) {
   B_STRIDE(k, gtot) {
     B_CELL(k, p, b, l)
@@ -120,49 +120,28 @@ __global__ void b_replace_kernel(const BPair* __restrict__ bp, int npairs, const
     const uint8_t* fl = g.outl2 + o;
     if (!repl_invalid(fl, b.gmask, l)) continue;
     float nu = g.u[o + l], nv = g.v[o + l];
-    replace_cell(g.u + o, g.v + o, fl, b.gmask, b.ny, b.nx, (int)(l % b.ny), (int)(l / b.ny), nu, nv);
+    // a masked cell ends as NaN and no other cell reads it
     if (b.gmask && b.gmask[l]) nu = nv = f_nan();
+    else replace_cell(g.u + o, g.v + o, fl, b.gmask, b.ny, b.nx, (int)(l % b.ny), (int)(l / b.ny), nu, nv);
     g.u[o + l] = nu;
     g.v[o + l] = nv;
   }
 }
 
-// field_change (src/pipeline.jl:849-866), one CTA per pair; a pair whose
+// field_change (src/pipeline.jl:849-866), one cluster per pair; a pair whose
 // change falls below convergence_tol is marked done.
-constexpr int BFC_THREADS = 1024;
-
-__global__ void __launch_bounds__(BFC_THREADS) b_field_change_kernel(const BPair* __restrict__ bp, int32_t* done, int it,
-                                                                     BGrid g) {
-  __shared__ uint32_t hist[256];
-  __shared__ uint32_t s_bucket;
-  __shared__ int64_t s_k;
-  __shared__ unsigned long long s_n;
-  const int p = blockIdx.x;
+__global__ void __cluster_dims__(FC_CLUSTER, 1, 1) __launch_bounds__(FC_THREADS)
+    b_field_change_kernel(const BPair* __restrict__ bp, int32_t* done, int it, BGrid g) {
+  __shared__ FieldChangeSmem sm;
+  const int p = blockIdx.x / FC_CLUSTER;
   const BPair& b = bp[p];
-  if (!bp_live(b, it, done, p) || !(it < b.maxit) || !(b.tol > 0)) return;  // uniform across the CTA
-  const int64_t G = (int64_t)b.ny * b.nx, o = b.goff;
-  uint32_t* keys = g.keys + o;
-  if (threadIdx.x == 0) s_n = 0;
-  __syncthreads();
-  unsigned long long n_local = 0;
-  for (int64_t i = threadIdx.x; i < G; i += blockDim.x) {
-    bool counts;
-    keys[i] = change_key(g.u[o + i], g.v[o + i], g.prev_u[o + i], g.prev_v[o + i], b.gmask && b.gmask[i], counts);
-    n_local += counts;
-  }
-  atomicAdd(&s_n, n_local);
-  __syncthreads();
-  const int64_t n = (int64_t)s_n;
-  float change = 0.f;
-  if (n > 0) {
-    int64_t ka, kb;
-    double gq;
-    quantile95_index(n, ka, kb, gq);
-    const uint32_t a = cta_radix_select(keys, G, ka, hist, &s_bucket, &s_k);
-    const uint32_t c = kb == ka ? a : cta_radix_select(keys, G, kb, hist, &s_bucket, &s_k);
-    change = quantile95_value(a, c, gq);
-  }
-  if (threadIdx.x == 0 && (double)change < b.tol) done[p] = 1;
+  if (!bp_live(b, it, done, p) || !(it < b.maxit) || !(b.tol > 0)) return;  // uniform across the cluster
+  const int64_t o = b.goff;
+  const float change = cluster_field_change(sm, (int64_t)b.ny * b.nx, g.keys + o, [&](int64_t i, bool& counts) {
+    return change_key(g.u[o + i], g.v[o + i], g.prev_u[o + i], g.prev_v[o + i], b.gmask && b.gmask[i], counts);
+  });
+  // every CTA has read done[p]: the cluster has met since
+  if (blockIdx.x % FC_CLUSTER == 0 && threadIdx.x == 0 && (double)change < b.tol) done[p] = 1;
 }
 
 cudaError_t launch_b_vector(const BPair* bp, int npairs, int32_t* done, int it, int64_t gtot, const BGrid& g,
@@ -181,7 +160,7 @@ cudaError_t launch_b_vector(const BPair* bp, int npairs, int32_t* done, int it, 
     ++n;
   }
   if (any_tol && it >= 2 && it < max_maxit) {
-    b_field_change_kernel<<<npairs, BFC_THREADS, 0, s>>>(bp, done, it, g);
+    b_field_change_kernel<<<npairs * FC_CLUSTER, FC_THREADS, 0, s>>>(bp, done, it, g);
     ++n;
   }
   if (nlaunch) *nlaunch = n;

@@ -117,7 +117,7 @@ cudaError_t launch_flags(const float* u, const float* v, const float* ratio, con
   return cudaGetLastError();
 }
 
-__global__ void substitute_kernel(float* u, float* v, const uint8_t* outl_in, uint8_t* outl_out, const uint8_t* gmask,
+__global__ void __launch_bounds__(128, 3) substitute_kernel(float* u, float* v, const uint8_t* outl_in, uint8_t* outl_out, const uint8_t* gmask,
                                   const float* alt_u, const float* alt_v, int32_t nalt, int32_t ny, int32_t nx,
                                   int32_t er, double thr) {
   GRID_STRIDE(k, (int64_t)ny * nx)
@@ -138,8 +138,9 @@ __global__ void replace_kernel(float* u, float* v, const uint8_t* flags, const u
   GRID_STRIDE(k, (int64_t)ny * nx) {
     if (!repl_invalid(flags, gmask, k)) continue;
     float nu = u[k], nvv = v[k];
-    replace_cell(u, v, flags, gmask, ny, nx, (int)(k % ny), (int)(k / ny), nu, nvv);
+    // a masked cell that ends as NaN is not searched for (no other cell reads it)
     if (nan_mask && gmask && gmask[k]) nu = nvv = f_nan();
+    else replace_cell(u, v, flags, gmask, ny, nx, (int)(k % ny), (int)(k / ny), nu, nvv);
     u[k] = nu;
     v[k] = nvv;
   }
@@ -240,42 +241,21 @@ cudaError_t launch_mask_grid(const uint8_t* mask, int64_t nr, int32_t ny, int32_
   return cudaGetLastError();
 }
 
-// field_change (src/pipeline.jl:849-866): one CTA, keys in scratch.
-constexpr int FC_THREADS = 1024;
-
-__global__ void __launch_bounds__(FC_THREADS) field_change_kernel(const float* u, const float* v, const float* pu,
-                                                                  const float* pv, const uint8_t* gmask, int64_t G,
-                                                                  uint32_t* keys, float* out) {
-  __shared__ uint32_t hist[256];
-  __shared__ uint32_t s_bucket;
-  __shared__ int64_t s_k;
-  __shared__ unsigned long long s_n;
-  if (threadIdx.x == 0) s_n = 0;
-  __syncthreads();
-  unsigned long long n_local = 0;
-  for (int64_t i = threadIdx.x; i < G; i += blockDim.x) {
-    bool counts;
-    keys[i] = change_key(u[i], v[i], pu[i], pv[i], gmask && gmask[i], counts);
-    n_local += counts;
-  }
-  atomicAdd(&s_n, n_local);
-  __syncthreads();
-  const int64_t n = (int64_t)s_n;
-  if (n == 0) {
-    if (threadIdx.x == 0) *out = 0.f;
-    return;
-  }
-  int64_t ka, kb;
-  double g;
-  quantile95_index(n, ka, kb, g);
-  const uint32_t a = cta_radix_select(keys, G, ka, hist, &s_bucket, &s_k);
-  const uint32_t b = kb == ka ? a : cta_radix_select(keys, G, kb, hist, &s_bucket, &s_k);
-  if (threadIdx.x == 0) *out = quantile95_value(a, b, g);
+// field_change (src/pipeline.jl:849-866): one cluster, keys in scratch.
+__global__ void __cluster_dims__(FC_CLUSTER, 1, 1) __launch_bounds__(FC_THREADS)
+    field_change_kernel(const float* u, const float* v, const float* pu, const float* pv, const uint8_t* gmask,
+                        int64_t G, uint32_t* keys, float* out) {
+  __shared__ FieldChangeSmem sm;
+  const float change = cluster_field_change(sm, G, keys, [&](int64_t i, bool& counts) {
+    return change_key(u[i], v[i], pu[i], pv[i], gmask && gmask[i], counts);
+  });
+  if (blockIdx.x == 0 && threadIdx.x == 0) *out = change;
 }
 
 cudaError_t launch_field_change(const float* u, const float* v, const float* pu, const float* pv, const uint8_t* gmask,
                                 int64_t G, float* scratch, float* out, cudaStream_t s) {
-  field_change_kernel<<<1, FC_THREADS, 0, s>>>(u, v, pu, pv, gmask, G, reinterpret_cast<uint32_t*>(scratch), out);
+  field_change_kernel<<<FC_CLUSTER, FC_THREADS, 0, s>>>(u, v, pu, pv, gmask, G, reinterpret_cast<uint32_t*>(scratch),
+                                                        out);
   return cudaGetLastError();
 }
 

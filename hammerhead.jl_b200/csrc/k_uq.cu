@@ -27,9 +27,10 @@ struct UQOffsets {
   // (dr = 1..4), else 4 + 9 (dc - 1) + (dr + 4)
   int8_t nat2ring[40];
 };
-static UQOffsets make_offsets() {
+constexpr int uq_natural(int dr, int dc) { return dc == 0 ? dr - 1 : 4 + 9 * (dc - 1) + (dr + 4); }
+static constexpr UQOffsets make_offsets() {
   UQOffsets o{};
-  int tmp[40][2], n = 0;
+  int tmp[40][2] = {}, n = 0;
   for (int dc = 0; dc <= 4; ++dc)
     for (int dr = (dc == 0 ? 1 : -4); dr <= 4; ++dr) {
       tmp[n][0] = dr;
@@ -52,16 +53,29 @@ static UQOffsets make_offsets() {
   o.ring_start[4] = 40;
   for (int k2 = 0; k2 < 40; ++k2) {
     const int dr = o.dr[k2], dc = o.dc[k2];
-    const int n = dc == 0 ? dr - 1 : 4 + 9 * (dc - 1) + (dr + 4);
-    o.nat2ring[n] = (int8_t)k2;
+    o.nat2ring[uq_natural(dr, dc)] = (int8_t)k2;
   }
   return o;
 }
 
+// sigma from the peak's three correlation values and the variance sum s2
+__device__ __forceinline__ float uq_sigma(double C0, double Cp, double Cm, double s2) {
+  const double sdc = sqrt(fmax(s2, 0.0));
+  const double Cpm = __dadd_rn(Cp, Cm) / 2.0;
+  const double lo = __dsub_rn(Cpm, sdc / 2.0), hi = __dadd_rn(Cpm, sdc / 2.0);
+  if (!(C0 > 0 && lo > 0)) return __int_as_float(0x7fc00000);
+  const double lhi = log(hi), llo = log(lo);
+  const double denom = __dsub_rn(__dsub_rn(__dmul_rn(2.0, log(C0)), lhi), llo);
+  if (!(denom > 0)) return __int_as_float(0x7fc00000);
+  return (float)(__dsub_rn(lhi, llo) / __dmul_rn(2.0, denom));
+}
+
+static __constant__ const UQOffsets UQ_TABLES = make_offsets();
+
 // finalize_uncertainty (src/uncertainty.jl:162-179). The doubled covariance
 // sums enter S00 one ring at a time (each ring summed in its own order, then
-// added), the arithmetic of the lane-parallel form uq_finalize_seg, so every
-// kernel gives a window the same sigma from the same statistics.
+// added), the arithmetic of uq_finalize_natural, so every kernel gives a window
+// the same sigma from the same statistics.
 __device__ __forceinline__ float uq_finalize(const double* s, const UQOffsets& o) {
   const double C0 = s[0], Cp = s[1], Cm = s[2], S00 = s[3];
   double s2 = S00;
@@ -74,14 +88,7 @@ __device__ __forceinline__ float uq_finalize(const double* s, const UQOffsets& o
     if (mx < __dmul_rn(0.05, S00)) break;
     s2 = __dadd_rn(s2, rsum);
   }
-  const double sdc = sqrt(fmax(s2, 0.0));
-  const double Cpm = __dadd_rn(Cp, Cm) / 2.0;
-  const double lo = __dsub_rn(Cpm, sdc / 2.0), hi = __dadd_rn(Cpm, sdc / 2.0);
-  if (!(C0 > 0 && lo > 0)) return __int_as_float(0x7fc00000);
-  const double lhi = log(hi), llo = log(lo);
-  const double denom = __dsub_rn(__dsub_rn(__dmul_rn(2.0, log(C0)), lhi), llo);
-  if (!(denom > 0)) return __int_as_float(0x7fc00000);
-  return (float)(__dsub_rn(lhi, llo) / __dmul_rn(2.0, denom));
+  return uq_sigma(C0, Cp, Cm, s2);
 }
 
 // One CTA (4 warps) per window. Every reduction runs across lanes: the
@@ -263,10 +270,18 @@ __global__ void __launch_bounds__(UQ_THREADS) uq_kernel(const UQArgs a, const UQ
 // per-lane partials. Same FP32 operations as uq_kernel, FP64 sums.
 // When dC has at most 16 columns (W <= 17) a warp serves two windows, one
 // per 16-lane segment (shuffles of width 16), so no lane idles for want of
-// a column. Window means are one warp's job per window (all 32 lanes), and
-// finalize_uncertainty is spread over the first lanes of each window (ring
-// maxima and sums on lanes 0-3, one logarithm each on lanes 0-2).
+// a column. Window means are one warp's job per window (all 32 lanes).
+//
+// What bounds it: instructions issued, of which the covariance FMAs are about
+// a quarter (60 % of the issue slots busy at 16 warps per SM; the FP64 pipe 35
+// %). So the totals of PEND windows are kept and finalized together, a lane
+// per window and component (ring sums, square root and logarithms for one
+// window cost a warp as much as for 32), mask bytes are handled only for
+// windows that have a mask, and the pixel loops step by constants. 16 px: 4.2
+// ns a window with a finalization per window, 3.4 now; 24 px: 12.2 and 10.4;
+// 32 px: 15.7 and 14.1.
 constexpr int UQW_THREADS = 128;  // two warp pairs (u, v)
+constexpr int TOT_LD = 45;        // doubles per pending component (odd: a lane each without conflicts)
 
 template <int W> struct UQWCfg {
   static constexpr int LD = W + 1;  // odd column stride: conflict-free column and row walks
@@ -274,13 +289,14 @@ template <int W> struct UQWCfg {
   static constexpr int WPW = M <= 16 ? 2 : 1;  // windows per warp
   static constexpr int SEG = 32 / WPW;         // lanes per window
   static constexpr int NWIN = 2 * WPW;         // windows per CTA
+  static constexpr int PEND = W == 24 ? 4 : 8;  // window components a warp finalizes together (4 CTAs per SM at 24 px)
   // the smoothed field of one window component: column c at c * DLD doubles.
   // DLD = W + 2 is 2 mod 4 (W is a multiple of 4), so the 16-byte row pairs
   // that 8 consecutive lanes read from 8 consecutive columns fall in distinct
-  // bank groups. Columns SEG .. SEG+3 stay zero: the lag partners of the last
-  // lanes.
+  // bank groups. Columns M .. M+3 stay zero: the lag partners of the last
+  // columns (lanes past M read the last column's partners, times zero).
   static constexpr int DLD = W + 2;
-  static constexpr int DCOLS = SEG + 4;
+  static constexpr int DCOLS = M + 4;
   static constexpr size_t dd_bytes = (size_t)DCOLS * DLD * sizeof(double);
   // window buffers of consecutive slots start 16 banks apart (64 bytes mod
   // 128), so the two windows of a warp do not meet in one bank
@@ -292,15 +308,14 @@ template <int W> struct UQWCfg {
   static constexpr bool PREFETCH = W <= 24;
   static constexpr int NBUF = PREFETCH ? 2 : 1;
   static constexpr size_t up128(size_t x) { return (x + 127) / 128 * 128; }
-  // shared memory: smoothed fields (4 warps x WPW), totals (4 x WPW x 44),
-  // window buffers, per-warp sums for the window means, apodization, offset
-  // tables
+  // shared memory: smoothed fields (4 warps x WPW), the pending windows' totals
+  // and grid cells (per warp), window buffers, per-warp sums for the window
+  // means and the slots' mask flags, apodization
   static constexpr size_t off_tot = up128(4 * WPW * dd_bytes);
-  static constexpr size_t off_win = up128(off_tot + 4 * WPW * 44 * sizeof(double));
+  static constexpr size_t off_win = up128(off_tot + 4 * PEND * (TOT_LD + 1) * sizeof(double));
   static constexpr size_t off_mean = up128(off_win + NBUF * NWIN * win_bytes);
-  static constexpr size_t off_apod = up128(off_mean + 4 * 3 * sizeof(double));
-  static constexpr size_t off_offs = up128(off_apod + (size_t)W * W * sizeof(float));
-  static constexpr size_t smem() { return off_offs + sizeof(UQOffsets) + 16; }
+  static constexpr size_t off_apod = up128(off_mean + (4 * 3 + NWIN) * sizeof(double));
+  static constexpr size_t smem() { return off_apod + (size_t)W * W * sizeof(float); }
   static constexpr int MINB = W <= 24 ? 4 : 3;  // CTAs per SM the register budget is sized for
 };
 
@@ -340,41 +355,28 @@ template <int N, int O> __device__ __forceinline__ void seg_tsum(double* v, int 
   }
 }
 
-// finalize_uncertainty (src/uncertainty.jl:162-179) of one window component
-// from its 44 statistics in ring order (shared memory, visible to the
-// segment), spread over the segment's first lanes: lane j < 4 forms ring
-// j+1's maximum and doubled sum, lanes 0, 1, 2 one logarithm each. The
-// result is valid on every lane of the segment.
-template <int SEG> __device__ __forceinline__ float uq_finalize_seg(const double* s, const UQOffsets& o, int c) {
-  constexpr unsigned FULL = 0xffffffffu;
-  const int lb = (int)(threadIdx.x & 31) & ~(SEG - 1);  // the segment's first lane
-  double mx = -INFINITY, rsum = 0.0;
-  if (c < 4)
-    for (int k = o.ring_start[c]; k < o.ring_start[c + 1]; ++k) {
-      const double x = s[4 + k];
-      mx = fmax(mx, x);
-      rsum = fma(2.0, x, rsum);
-    }
-  const double C0 = s[0], Cp = s[1], Cm = s[2], S00 = s[3];
-  const double thr = __dmul_rn(0.05, S00);
+// uq_finalize of one window component from its 44 totals in natural order
+// (C0, C+, C-, S00, then lag n at 4 + n); the table folds into immediate
+// offsets.
+__device__ __forceinline__ float uq_finalize_natural(const double* s) {
+  constexpr UQOffsets o = make_offsets();
+  const double S00 = s[3], thr = __dmul_rn(0.05, S00);
   double s2 = S00;
   bool go = true;
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const double m = __shfl_sync(FULL, mx, lb + j);
-    const double t = __shfl_sync(FULL, rsum, lb + j);
-    go = go && !(m < thr);  // a ring below 5 % of S00 ends the sum (NaN does not)
-    if (go) s2 = __dadd_rn(s2, t);
+  for (int ring = 0; ring < 4; ++ring) {
+    double mx = -INFINITY, rsum = 0.0;
+#pragma unroll
+    for (int k = 0; k < 40; ++k)
+      if (k >= o.ring_start[ring] && k < o.ring_start[ring + 1]) {
+        const double x = s[4 + uq_natural(o.dr[k], o.dc[k])];
+        mx = fmax(mx, x);
+        rsum = fma(2.0, x, rsum);
+      }
+    go = go && !(mx < thr);  // a ring below 5 % of S00 ends the sum (NaN does not)
+    if (go) s2 = __dadd_rn(s2, rsum);
   }
-  const double sdc = sqrt(fmax(s2, 0.0));
-  const double Cpm = __dmul_rn(__dadd_rn(Cp, Cm), 0.5);
-  const double lo = __dsub_rn(Cpm, __dmul_rn(sdc, 0.5)), hi = __dadd_rn(Cpm, __dmul_rn(sdc, 0.5));
-  const double lg = log(c == 0 ? C0 : (c == 1 ? hi : lo));
-  const double lC0 = __shfl_sync(FULL, lg, lb), lhi = __shfl_sync(FULL, lg, lb + 1), llo = __shfl_sync(FULL, lg, lb + 2);
-  if (!(C0 > 0 && lo > 0)) return __int_as_float(0x7fc00000);
-  const double denom = __dsub_rn(__dsub_rn(__dmul_rn(2.0, lC0), lhi), llo);
-  if (!(denom > 0)) return __int_as_float(0x7fc00000);
-  return (float)(__dsub_rn(lhi, llo) / __dmul_rn(2.0, denom));
+  return uq_sigma(s[0], s[1], s[2], s2);
 }
 
 // Where window `job` comes from: on = the window is estimated in this launch.
@@ -419,31 +421,47 @@ __device__ __forceinline__ void cp_async4(void* dst, const void* src) {
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_prev() { asm volatile("cp.async.wait_group 1;\n" ::: "memory"); }
 
+// f(p, q) for the pixels k = t, t + NT, ... of a W x W window (k = p + q W)
+template <int W, int NT, class F> __device__ __forceinline__ void uq_each(int t, const F& f) {
+  if constexpr (NT % W == 0) {
+    constexpr int N = (W * W + NT - 1) / NT;
+    const int p0 = t % W, q0 = t / W;
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+      if ((i + 1) * NT <= W * W || t + i * NT < W * W) f(p0, q0 + i * (NT / W));
+  } else {
+#pragma unroll 3
+    for (int k = t; k < W * W; k += NT) f(k % W, k / W);
+  }
+}
+
 template <int W>
-__global__ void __launch_bounds__(UQW_THREADS, UQWCfg<W>::MINB) uq_warp_kernel(const UQArgs a, const UQOffsets o) {
+__global__ void __launch_bounds__(UQW_THREADS, UQWCfg<W>::MINB) uq_warp_kernel(const UQArgs a) {
   using C = UQWCfg<W>;
   constexpr int LD = C::LD, M = C::M, WPW = C::WPW, SEG = C::SEG, NWIN = C::NWIN, DLD = C::DLD;
+  constexpr int MW = 4 / NWIN;      // warps that form a window's means
+  constexpr int NT = 2 * SEG;       // threads of a window (= 32 MW)
+  constexpr int FB = C::PEND / WPW;  // iterations between finalizations
+  static_assert(NT == 32 * MW, "");
   constexpr unsigned FULL = 0xffffffffu;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   unsigned char* wbase = smem_raw + C::off_win;
   double* msum = reinterpret_cast<double*>(smem_raw + C::off_mean);  // per warp: its share of (sum A, sum B, count)
+  int* smask = reinterpret_cast<int*>(msum + 12);                    // per slot: the window has a mask
   float* sap = reinterpret_cast<float*>(smem_raw + C::off_apod);    // the apodization window
-  // the offset tables in shared memory (indexed at run time; a parameter
-  // struct indexed that way would be copied to local memory)
-  UQOffsets& so = *reinterpret_cast<UQOffsets*>(smem_raw + C::off_offs);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int comp = warp & 1, seg = lane / SEG, c = lane % SEG;
   const int slot = (warp >> 1) * WPW + seg;  // window of this lane
-  const int ts = comp * SEG + c;             // this lane among the 2*SEG threads of its window
+  const int ts = comp * SEG + c;             // this lane among the NT threads of its window
   double* dsm = reinterpret_cast<double*>(smem_raw + (size_t)(warp * WPW + seg) * C::dd_bytes);  // this segment's field
-  double* tot = reinterpret_cast<double*>(smem_raw + C::off_tot) + (warp * WPW + seg) * 44;      // its 44 totals
-  if (tid == 0) so = o;
+  double* pend = reinterpret_cast<double*>(smem_raw + C::off_tot) + warp * C::PEND * (TOT_LD + 1);  // totals
+  long long* pcell = reinterpret_cast<long long*>(pend + C::PEND * TOT_LD);  // their grid cells (< 0: none)
   for (int k = tid; k < W * W; k += UQW_THREADS) sap[k] = __ldg(a.apod + k);
-  {  // the zero columns past each segment's lanes (never written again)
+  {  // the zero columns past each field's columns (never written again)
     double* d0 = reinterpret_cast<double*>(smem_raw + (size_t)(warp * WPW) * C::dd_bytes);
     for (int k = lane; k < WPW * 4 * DLD; k += 32) {
       const int g = k / (4 * DLD), e = k % (4 * DLD);
-      d0[(size_t)g * (C::dd_bytes / sizeof(double)) + SEG * DLD + e] = 0.0;
+      d0[(size_t)g * (C::dd_bytes / sizeof(double)) + M * DLD + e] = 0.0;
     }
   }
   __syncthreads();
@@ -452,13 +470,16 @@ __global__ void __launch_bounds__(UQW_THREADS, UQWCfg<W>::MINB) uq_warp_kernel(c
   auto prefetch = [&](const UQSrc& q0, int ph) {
     float* pa = reinterpret_cast<float*>(wbase + (ph * NWIN + slot) * C::win_bytes);
     float* pb = pa + LD * W;
-    if (q0.on)
-      for (int k = ts; k < W * W; k += 2 * SEG) {
-        const int p = k % W, q = k / W;
-        const int64_t off = (int64_t)(q0.rs + p) + (int64_t)(q0.cs + q) * q0.ld;
-        cp_async4(pa + p + q * LD, q0.A + off);
-        cp_async4(pb + p + q * LD, q0.B + off);
-      }
+    if (q0.on) {
+      const int64_t o0 = (int64_t)q0.rs + (int64_t)q0.cs * q0.ld;
+      const float* A0 = q0.A + o0;
+      const float* B0 = q0.B + o0;
+      uq_each<W, NT>(ts, [&](int p, int q) {
+        const int64_t off = p + q * q0.ld;
+        cp_async4(pa + p + q * LD, A0 + off);
+        cp_async4(pb + p + q * LD, B0 + off);
+      });
+    }
   };
   int iter = 0;
   int64_t base = (int64_t)blockIdx.x * NWIN;
@@ -478,16 +499,13 @@ __global__ void __launch_bounds__(UQW_THREADS, UQWCfg<W>::MINB) uq_warp_kernel(c
     // ---- the window's source (uniform within the window's lanes)
     const UQSrc nxt = uq_src(a, base + stride + slot);
     const bool on = src.on;
-    const float* A = src.A;
-    const float* B = src.B;
-    const uint8_t* Mk = src.M;
-    const int64_t ld = src.ld, gid = src.gid;
-    const int rs = src.rs, cs = src.cs;
     // with two windows per warp every lane runs the arithmetic below (the
     // shuffles span the warp, whose windows may differ in `on`); a window
-    // that is off computes on zeros and writes nothing. With one window per
-    // warp `on` is uniform and an idle warp pair skips the work.
+    // that is off computes on whatever its buffers hold and writes nothing.
+    // With one window per warp `on` is uniform and an idle pair skips the work.
     const bool run = WPW == 1 ? on : true;
+    const int64_t o0 = (int64_t)src.rs + (int64_t)src.cs * src.ld;
+    const bool masked = on && src.M;
     if (C::PREFETCH) {
       // the next windows go to the other buffer set while these are reduced
       // (that set was last read in the previous iteration, before its final
@@ -495,81 +513,78 @@ __global__ void __launch_bounds__(UQW_THREADS, UQWCfg<W>::MINB) uq_warp_kernel(c
       prefetch(nxt, ph ^ 1);  // nothing for a window past the last job (nxt.on is false)
       cp_async_commit();
       cp_async_wait_prev();
-      if (run)
-        for (int k = ts; k < W * W; k += 2 * SEG) {
-          const int p = k % W, q = k / W;
-          uint8_t mk = 1;
-          if (on) {
-            mk = Mk ? __ldg(Mk + (int64_t)(rs + p) + (int64_t)(cs + q) * ld) : 0;
-          } else {
-            wa[p + q * LD] = 0.f;
-            wb[p + q * LD] = 0.f;
-          }
-          mf[k] = mk;
-        }
-    } else if (run) {
-      for (int k = ts; k < W * W; k += 2 * SEG) {
-        const int p = k % W, q = k / W;
-        float va = 0.f, vb = 0.f;
-        uint8_t mk = 1;
-        if (on) {
-          const int64_t off = (int64_t)(rs + p) + (int64_t)(cs + q) * ld;
-          va = __ldg(A + off);
-          vb = __ldg(B + off);
-          mk = Mk ? __ldg(Mk + off) : 0;
-        }
-        wa[p + q * LD] = va;
-        wb[p + q * LD] = vb;
-        mf[k] = mk;
-      }
+    } else if (on) {
+      const float* A0 = src.A + o0;
+      const float* B0 = src.B + o0;
+      uq_each<W, NT>(ts, [&](int p, int q) {
+        const int64_t off = p + q * src.ld;
+        wa[p + q * LD] = __ldg(A0 + off);
+        wb[p + q * LD] = __ldg(B0 + off);
+      });
     }
+    if (masked) {
+      const uint8_t* M0 = src.M + o0;
+      uq_each<W, NT>(ts, [&](int p, int q) { mf[p + q * W] = __ldg(M0 + p + q * src.ld); });
+    }
+    if (ts == 0) smask[slot] = masked;
     __syncthreads();
-    // ---- window means (load_uncertainty_windows!), FP64: MW = 4 / NWIN warps
-    //      per window slot, each summing its share of the pixels over all its
-    //      lanes (a slot whose window is off and was not loaded yields values
-    //      nobody reads)
+    // ---- window means (load_uncertainty_windows!), FP64: MW warps per window
+    //      slot, each summing its share of the pixels over all its lanes (a
+    //      slot whose window is off yields values nobody reads)
     {
-      constexpr int MW = 4 / NWIN;
       const int s = warp / MW, h = warp % MW;
       const float* pa = reinterpret_cast<const float*>(wbase + (ph * NWIN + s) * C::win_bytes);
       const float* pb = pa + LD * W;
-      const uint8_t* pm = reinterpret_cast<const uint8_t*>(pb + LD * W);
-      double sa = 0.0, sb = 0.0, cnt = 0.0;
-#pragma unroll 4
-      for (int k = h * 32 + lane; k < W * W; k += 32 * MW)
-        if (!pm[k]) {
-          const int p = k % W, q = k / W;
+      double sa = 0.0, sb = 0.0;
+      if (!smask[s]) {
+        uq_each<W, NT>(h * 32 + lane, [&](int p, int q) {
           sa += (double)pa[p + q * LD];
           sb += (double)pb[p + q * LD];
-          cnt += 1.0;
-        }
+        });
+      } else {
+        const uint8_t* pm = reinterpret_cast<const uint8_t*>(pb + LD * W);
+        double cnt = 0.0;
+        uq_each<W, NT>(h * 32 + lane, [&](int p, int q) {
+          if (!pm[p + q * W]) {
+            sa += (double)pa[p + q * LD];
+            sb += (double)pb[p + q * LD];
+            cnt += 1.0;
+          }
+        });
+        cnt = seg_sum<32>(cnt);
+        if (lane == 0) msum[3 * warp + 2] = cnt;
+      }
       sa = seg_sum<32>(sa);
       sb = seg_sum<32>(sb);
-      cnt = seg_sum<32>(cnt);
       if (lane == 0) {
         msum[3 * warp] = sa;
         msum[3 * warp + 1] = sb;
-        msum[3 * warp + 2] = cnt;
       }
     }
     __syncthreads();  // the sums are visible, and every read of the raw values precedes the apodized writes
     if (run) {
-      constexpr int MW = 4 / NWIN;
-      double sa = 0.0, sb = 0.0, cnt = 0.0;
+      // the even lanes divide frame A's sum, the odd lanes frame B's
+      double sm = 0.0, cnt = (double)(W * W);
 #pragma unroll
-      for (int h = 0; h < MW; ++h) {
-        sa += msum[3 * (slot * MW + h)];
-        sb += msum[3 * (slot * MW + h) + 1];
-        cnt += msum[3 * (slot * MW + h) + 2];
+      for (int h = 0; h < MW; ++h) sm += msum[3 * (slot * MW + h) + (lane & 1)];
+      if (masked) {
+        cnt = 0.0;
+#pragma unroll
+        for (int h = 0; h < MW; ++h) cnt += msum[3 * (slot * MW + h) + 2];
       }
-      const float ma = cnt > 0 ? (float)(sa / cnt) : 0.f, mb = cnt > 0 ? (float)(sb / cnt) : 0.f;
-      for (int k = ts; k < W * W; k += 2 * SEG) {
-        const int p = k % W, q = k / W;
-        const float ap = sap[k];
+      const float mean = cnt > 0 ? (float)(sm / cnt) : 0.f;
+      const float other = __shfl_xor_sync(FULL, mean, 1);
+      const float ma = lane & 1 ? other : mean, mb = lane & 1 ? mean : other;
+      uq_each<W, NT>(ts, [&](int p, int q) {
+        const float ap = sap[p + q * W];
         const float va = wa[p + q * LD], vb = wb[p + q * LD];
-        wa[p + q * LD] = mf[k] ? 0.f : __fmul_rn(ap, __fsub_rn(va, ma));
-        wb[p + q * LD] = mf[k] ? 0.f : __fmul_rn(ap, __fsub_rn(vb, mb));
-      }
+        wa[p + q * LD] = __fmul_rn(ap, __fsub_rn(va, ma));
+        wb[p + q * LD] = __fmul_rn(ap, __fsub_rn(vb, mb));
+      });
+      if (masked)
+        uq_each<W, NT>(ts, [&](int p, int q) {
+          if (mf[p + q * W]) wa[p + q * LD] = wb[p + q * LD] = 0.f;
+        });
     }
     __syncthreads();
     if (run) {
@@ -608,28 +623,22 @@ __global__ void __launch_bounds__(UQW_THREADS, UQWCfg<W>::MINB) uq_warp_kernel(c
       const double mu = seg_sum<SEG>(fs[0] + fs[1]) * inv_n;
 #pragma unroll
       for (int r = 0; r < W; ++r) dd[r] = col ? dd[r] - mu : 0.0;
-      // this lane's column of the field into shared memory (lanes past M
-      // store zeros), for the neighbour-column reads of the covariance sums
+      // this lane's column of the field into shared memory, for the
+      // neighbour-column reads of the covariance sums
+      if (col)
 #pragma unroll
-      for (int r = 0; r < W; r += 2) *reinterpret_cast<double2*>(dsm + c * DLD + r) = make_double2(dd[r], dd[r + 1]);
+        for (int r = 0; r < W; r += 2) *reinterpret_cast<double2*>(dsm + c * DLD + r) = make_double2(dd[r], dd[r + 1]);
       // sums the per-lane partials v[0..N) of statistics first .. first+N-1
       // (natural order) over the window's lanes; the lanes holding totals
-      // store them in ring order
+      // store them
+      double* tot = pend + ((iter % FB) * WPW + seg) * TOT_LD;
       auto reduce_store = [&](double* v, auto n_tag, int first) {
         constexpr int N = decltype(n_tag)::value;
         int b = 0, n = N;
         seg_tsum<N, SEG / 2>(v, c, b, n);
 #pragma unroll
         for (int i = 0; i < tsum_slots(N, SEG); ++i)
-          if (i < n) {
-            const int st = first + b + i;
-            const int ri = st < 4 ? st : 4 + so.nat2ring[st - 4];
-            tot[ri] = v[i];
-            if (on && a.stats) {
-              if (a.accumulate) a.stats[job * 88 + comp * 44 + ri] += v[i];
-              else a.stats[job * 88 + comp * 44 + ri] = v[i];
-            }
-          }
+          if (i < n) tot[first + b + i] = v[i];
       };
       // ---- C0, C+, C-, S00 and the lag-(dr, 0) sums (registers only)
       {
@@ -655,7 +664,7 @@ __global__ void __launch_bounds__(UQW_THREADS, UQWCfg<W>::MINB) uq_warp_kernel(c
         for (int jj = 0; jj < 18; ++jj) acc[jj] = 0.0;
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
-          const double* xc = dsm + (c + dg + i) * DLD;
+          const double* xc = dsm + (min(c, M - 1) + dg + i) * DLD;
 #pragma unroll
           for (int r2 = 0; r2 < W; r2 += 2) {
             const double2 x2 = *reinterpret_cast<const double2*>(xc + r2);
@@ -672,12 +681,28 @@ __global__ void __launch_bounds__(UQW_THREADS, UQWCfg<W>::MINB) uq_warp_kernel(c
         }
         reduce_store(acc, std::integral_constant<int, 18>{}, 8 + 9 * (dg - 1));
       }
-      __syncwarp();  // the totals are visible to the segment
-      const float sg = uq_finalize_seg<SEG>(tot, so, c);
-      if (c == 0 && on && a.unc_u) (comp == 0 ? a.unc_u : a.unc_v)[gid] = sg;
+      if (a.stats) {
+        __syncwarp();  // the totals are visible to the segment
+        if (on)
+          for (int n = c; n < 44; n += SEG) {
+            const int ri = n < 4 ? n : 4 + UQ_TABLES.nat2ring[n - 4];
+            double* st = a.stats + job * 88 + comp * 44 + ri;
+            if (a.accumulate) *st += tot[n];
+            else *st = tot[n];
+          }
+      }
+    }
+    // ---- finalize_uncertainty (src/uncertainty.jl:162-179) of the last FB
+    //      iterations' windows, a lane each
+    if (c == 0) pcell[(iter % FB) * WPW + seg] = on ? (long long)src.gid : -1;
+    const bool last = base + stride >= a.njobs;
+    if (a.unc_u && (last || iter % FB == FB - 1)) {
+      __syncwarp();
+      if (lane < (iter % FB + 1) * WPW && pcell[lane] >= 0)
+        (comp == 0 ? a.unc_u : a.unc_v)[pcell[lane]] = uq_finalize_natural(pend + lane * TOT_LD);
     }
     src = nxt;
-    __syncthreads();  // the window buffers and fields are reused by the next iteration
+    __syncthreads();  // the window buffers, fields and totals are reused by the next iteration
   }
 }
 
@@ -878,7 +903,7 @@ __global__ void __launch_bounds__(UQ_THREADS) uq_general_kernel(const UQArgs a, 
   }
 }
 
-template <int W> static cudaError_t launch_uq_warp(const UQArgs& a, cudaStream_t s, int num_sms, const UQOffsets& offs) {
+template <int W> static cudaError_t launch_uq_warp(const UQArgs& a, cudaStream_t s, int num_sms) {
   using C = UQWCfg<W>;
   const size_t sm = C::smem();
   cudaError_t e = cudaFuncSetAttribute(uq_warp_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
@@ -890,7 +915,7 @@ template <int W> static cudaError_t launch_uq_warp(const UQArgs& a, cudaStream_t
   int64_t grid = (int64_t)per_sm * num_sms;
   const int64_t units = (a.njobs + C::NWIN - 1) / C::NWIN;
   if (grid > units) grid = units;
-  uq_warp_kernel<W><<<(unsigned)grid, UQW_THREADS, sm, s>>>(a, offs);
+  uq_warp_kernel<W><<<(unsigned)grid, UQW_THREADS, sm, s>>>(a);
   return cudaGetLastError();
 }
 
@@ -918,11 +943,11 @@ cudaError_t launch_uq(const UQArgs& a, cudaStream_t s, int num_sms) {
     return cudaGetLastError();
   }
   switch (a.W) {
-    case 8: return launch_uq_warp<8>(a, s, num_sms, offs);
-    case 12: return launch_uq_warp<12>(a, s, num_sms, offs);
-    case 16: return launch_uq_warp<16>(a, s, num_sms, offs);
-    case 24: return launch_uq_warp<24>(a, s, num_sms, offs);
-    case 32: return launch_uq_warp<32>(a, s, num_sms, offs);
+    case 8: return launch_uq_warp<8>(a, s, num_sms);
+    case 12: return launch_uq_warp<12>(a, s, num_sms);
+    case 16: return launch_uq_warp<16>(a, s, num_sms);
+    case 24: return launch_uq_warp<24>(a, s, num_sms);
+    case 32: return launch_uq_warp<32>(a, s, num_sms);
     default: break;
   }
   auto smem_of = [](int W) {

@@ -21,7 +21,7 @@
 // The 2-D transform runs each axis as an in-register radix-N1 pass and, for
 // N > 32, a second radix-N2 pass (N = N1*N2). The forward transform leaves
 // frequency k at position N2*(k % N1) + k / N1 along each axis; the spectrum
-// step reads pairs (k, -k) from there and the inverse takes that order back
+// is formed from pairs (k, -k) there and the inverse takes that order back
 // to natural order, so no bit-reversal pass exists anywhere.
 #pragma once
 #include "hh_corr_peaks.cuh"
@@ -112,7 +112,7 @@ template <int N, int W, bool SRCH = false, int VAR = 0> struct CorrCfg {
   static constexpr size_t PLANE_B = (size_t)PS * sizeof(float2);
   static constexpr size_t BASE_B = WPC * PLANE_B + WPC * (G / 32) * NPART * sizeof(double) + N * sizeof(float2) +
                                    WPC * (G / 32) * 2 * KMAX * sizeof(uint32_t) +
-                                   WPC * (KMAX * sizeof(float) + 2 * KMAX * sizeof(int)) + 3 * N * sizeof(int) +
+                                   WPC * (KMAX * sizeof(float) + 2 * KMAX * sizeof(int)) + N * sizeof(int) +
                                    (W == N ? WPC * N * sizeof(uint32_t) : 0) + 64;
   // The overlap gain is read by every window; from global memory its L1
   // lines are flushed by the window pixels (it took a third of the last
@@ -142,11 +142,7 @@ __global__ void __launch_bounds__(CorrCfg<N, W, SRCH, VAR>::NT, CorrCfg<N, W, SR
   uint32_t* red = reinterpret_cast<uint32_t*>(tw + N);
   float* s_vals = reinterpret_cast<float*>(red + WPC * (G / 32) * 2 * KMAX);
   int* s_locs = reinterpret_cast<int*>(s_vals + WPC * KMAX);
-  // per-axis storage tables (N2 > 1): frequency of storage slot a, storage
-  // slot of the negated frequency, canonical storage columns kq = 0..N/2
-  int* s_freq = reinterpret_cast<int*>(s_locs + WPC * 2 * KMAX);
-  int* s_neg = s_freq + N;
-  int* s_canon = s_neg + N;
+  int* s_canon = s_locs + WPC * 2 * KMAX;  // storage columns of kq = 0..N/2 (N2 > 1)
   uint32_t* s_rmax = reinterpret_cast<uint32_t*>(s_canon + N);  // per window: its plane's row maxima
   float* s_gain = reinterpret_cast<float*>(s_rmax + (W == N ? WPC * N : 0));  // (2Q + 1)^2 when C::BOXED
 
@@ -163,13 +159,7 @@ __global__ void __launch_bounds__(CorrCfg<N, W, SRCH, VAR>::NT, CorrCfg<N, W, SR
       sincospi(-2.0 * (double)m / (double)N, &sn, &cs);
       tw[m] = make_float2((float)cs, (float)sn);  // W_N^m = exp(-2 pi i m / N)
     }
-    for (int q = tid; q < N; q += NT) {
-      const int k = q / N2 + N1 * (q % N2);  // storage slot q holds frequency k
-      const int m = (N - k) % N;
-      s_freq[q] = k;
-      s_neg[q] = N2 * (m % N1) + m / N1;
-      if (q <= N / 2) s_canon[q] = N2 * (q % N1) + q / N1;
-    }
+    for (int q = tid; q <= N / 2; q += NT) s_canon[q] = N2 * (q % N1) + q / N1;
   }
   __syncthreads();  // the only CTA-wide barrier: from here on the window groups run independently
 
@@ -439,29 +429,14 @@ __global__ void __launch_bounds__(CorrCfg<N, W, SRCH, VAR>::NT, CorrCfg<N, W, SR
 #pragma unroll
       for (int k1 = 0; k1 < N1; ++k1) L[(N2 * k1 + n2) * LD] = x[k1];
     }
-    if (N2 > 1) {
-      grp_sync(bar, G);
-      for (int it = gt; it < N * N1; it += G) {
-        const int p = it % N, k1 = it / N;
-        float2* L = P + p + (N2 * k1) * LD;
-        float2 x[N2];
-#pragma unroll
-        for (int n2 = 0; n2 < N2; ++n2) x[n2] = L[n2 * LD];
-        RDFT<N2, false>::run(x, N2);
-#pragma unroll
-        for (int k2 = 0; k2 < N2; ++k2) L[k2 * LD] = x[k2];
-      }
-    }
     grp_sync(bar, G);
     // ---- stages 6-7: cross-power (or filtered phase) spectrum over Hermitian
     //      pairs (k, -k) and the inverse along p, on the canonical columns
     //      kq = 0..N/2 only (frequencies in storage order for N2 > 1, natural
-    //      order otherwise); the conjugate column -kq is then filled in as
-    //      conj of column kq. (i) The two self-paired columns (kq = 0, N/2)
-    //      pair rows within the column: their spectrum is formed first, in
-    //      place (for N <= 32 every canonical column is done here: folding
-    //      the spectrum into the single-pass inverse costs more registers
-    //      than the separate pass costs time).
+    //      order otherwise); column -kq is conj of column kq and is not stored.
+    //      For N <= 32 every canonical column's spectrum is formed in place
+    //      here: folding it into the single-pass inverse costs more registers
+    //      than the separate pass costs time.
     if constexpr (N2 == 1 && G <= N && N % G == 0) {
       // each thread owns rows ap = gt + j G (j < N / G) of every canonical
       // column; the columns are unrolled, so every address is the row's base
@@ -542,22 +517,82 @@ __global__ void __launch_bounds__(CorrCfg<N, W, SRCH, VAR>::NT, CorrCfg<N, W, SR
           }
       }
     } else {
-      // the two self-paired columns kq = 0 and N/2 (storage order)
+      // For N2 > 1 the second pass along q forms the spectrum from its own
+      // registers. Slot k2 of group k1 holds frequency k1 + N1 k2, canonical
+      // for k2 < N2/2 (and N2/2 of group 0); its negation is slot N2-1-k2 of
+      // group N1-k1 (slot N2-k2 of group 0 for group 0) in row -kp. So an item
+      // takes group ga of row ra and group gb = -ga of row rb = -ra, reads
+      // what it overwrites and nothing that another item writes: all rows for
+      // ga = 1 .. N1/2-1, and for ga = 0 and N1/2 (their own negations) a row
+      // of each pair, the self-negated rows 0 and N/2 together. Rows -ra of
+      // consecutive ra are consecutive too. A separate spectrum step read and
+      // wrote the whole plane once more: 12.8 ns per window at 48 points
+      // (padded) against 12.3; 64: 22.3 and 21.3; 96: 53.2 and 51.0; 128: 102 and 97.
+      constexpr int h2 = N2 / 2, HN = N1 / 2;
 #pragma unroll 1
-      for (int it = gt; it < 2 * N; it += G) {
-        const int ap = it % N, c = (it / N) * H;
-        const int aq = s_canon[c], bp = s_neg[ap], kp = s_freq[ap];
-        if (ap > bp) continue;  // its partner row does this pair
-        const float wk = method == 1 ? ld_keep(a.phasew + c * N + kp) : 1.f;
-        const float2 S = cross_spectrum(P[aq * LD + ap], P[aq * LD + bp], method, wk);
-        P[aq * LD + ap] = S;
-        P[aq * LD + bp] = make_float2(S.x, -S.y);
+      for (int it = gt; it < N * HN; it += G) {
+        int ga, gb, ra, rb;
+        bool self = false;
+        if (it < N * (HN - 1)) {
+          ga = 1 + it / N;
+          gb = N1 - ga;
+          ra = it % N;
+          rb = ra < N2 ? (N2 - ra) % N2 : N + N2 - 1 - ra;
+        } else {
+          const int e = it - N * (HN - 1), r = e % H;
+          ga = gb = e < H ? 0 : HN;
+          self = r == 0;  // rows 0 (kp = 0) and h2 (kp = N/2)
+          ra = r < h2 ? r : N2 + r - h2;
+          rb = self ? h2 : (ra < N2 ? N2 - ra : N + N2 - 1 - ra);
+        }
+        float2* La = P + ra + N2 * ga * LD;
+        float2* Lb = P + rb + N2 * gb * LD;
+        float2 xa[N2], xb[N2];
+#pragma unroll
+        for (int n2 = 0; n2 < N2; ++n2) {
+          xa[n2] = La[n2 * LD];
+          xb[n2] = Lb[n2 * LD];
+        }
+        RDFT<N2, false>::run(xa, N2);
+        RDFT<N2, false>::run(xb, N2);
+        // the filter weight of canonical column c = g + N1 k2 at row r
+        auto weight = [&](int g, int k2, int r) {
+          return method == 1 ? ld_keep(a.phasew + (g + N1 * k2) * N + r / N2 + N1 * (r % N2)) : 1.f;
+        };
+        if (ga != 0) {
+          auto pair = [&](const float2(&ya)[N2], const float2(&yb)[N2]) {
+#pragma unroll
+            for (int k2 = 0; k2 < h2; ++k2) {
+              La[k2 * LD] = cross_spectrum(xa[k2], ya[N2 - 1 - k2], method, weight(ga, k2, ra));
+              Lb[k2 * LD] = cross_spectrum(xb[k2], yb[N2 - 1 - k2], method, weight(gb, k2, rb));
+            }
+          };
+          if (self) pair(xa, xb);
+          else pair(xb, xa);
+        } else {
+          auto pair = [&](const float2(&ya)[N2], const float2(&yb)[N2]) {
+#pragma unroll
+            for (int k2 = 0; k2 <= h2; ++k2) {
+              const float2 S = cross_spectrum(xa[k2], ya[(N2 - k2) % N2], method, weight(0, k2, ra));
+              if (k2 != 0 && k2 != h2) {
+                La[k2 * LD] = S;
+                Lb[k2 * LD] = cross_spectrum(xb[k2], yb[(N2 - k2) % N2], method, weight(0, k2, rb));
+              } else if (!self) {  // columns 0 and N/2 are their own negations
+                La[k2 * LD] = S;
+                Lb[k2 * LD] = make_float2(S.x, -S.y);
+              } else {
+                const float2 T = cross_spectrum(xb[k2], yb[(N2 - k2) % N2], method, weight(0, k2, rb));
+                La[k2 * LD] = make_float2(S.x, -S.y);
+                Lb[k2 * LD] = make_float2(T.x, -T.y);
+              }
+            }
+          };
+          if (self) pair(xa, xb);
+          else pair(xb, xa);
+        }
       }
     }
     grp_sync(bar, G);
-    //      (ii) for N > 32 every other canonical column forms its spectrum
-    //      while it is read for its first inverse pass; its partner column
-    //      -kq is read only by it, and written only after the pass.
     if (N2 > 1) {
 #pragma unroll 1
       for (int it = gt; it < NC * N1; it += G) {
@@ -576,23 +611,10 @@ __global__ void __launch_bounds__(CorrCfg<N, W, SRCH, VAR>::NT, CorrCfg<N, W, SR
           c = it % NC;
           k1 = it / NC;
         }
-        const int aq = s_canon[c], bq = s_neg[aq];
-        float2* L = P + aq * LD + N2 * k1;
-        const float2* Lb = P + bq * LD;
-        // slot N2 k1 + k2 holds frequency k1 + N1 k2; its negation sits at
-        // slot N2 (N1 - k1) + N2 - 1 - k2 (k1 > 0), or N2 - k2 (k1 = 0, k2 > 0),
-        // or 0: the row base is per item, the offsets constants
-        const int nb0 = k1 == 0 ? N2 : N2 * (N1 - k1) + N2 - 1;
+        float2* L = P + s_canon[c] * LD + N2 * k1;
         float2 x[N2];
 #pragma unroll
-        for (int k2 = 0; k2 < N2; ++k2) {
-          x[k2] = L[k2];
-          if (aq != bq) {
-            const int neg = (k1 == 0 && k2 == 0) ? 0 : nb0 - k2;
-            const float wk = method == 1 ? ld_keep(a.phasew + c * N + k1 + N1 * k2) : 1.f;
-            x[k2] = cross_spectrum(x[k2], Lb[neg], method, wk);
-          }
-        }
+        for (int k2 = 0; k2 < N2; ++k2) x[k2] = L[k2];
         RDFT<N2, true>::run(x, N2);
 #pragma unroll
         for (int n2 = 1; n2 < N2; ++n2) {

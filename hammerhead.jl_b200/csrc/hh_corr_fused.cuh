@@ -70,13 +70,23 @@ template <int N, int W, bool SRCH = false, int VAR = 0> struct CorrCfg {
                                        : (VAR == 3 ? (MINB0 > 1 ? MINB0 - 1 : MINB_SH + 1) : MINB_SH);
   // the peak analysis inline (one window per CTA: its latency is the CTA's)
   static constexpr bool INLINE_ANALYSIS = N >= 96;
-  // Canonical column c sits at storage column N2 (c % N1) + c / N1, and with
-  // LD = N + 1 a 64-bit element's bank pair is (column + row) mod 16, so with
-  // N2 = 8 consecutive canonical columns (8 storage columns apart) share two
-  // bank pairs. The first inverse pass then walks c = N1 u + v with u
-  // fastest (a model of the pass's addresses: 1088 wavefronts instead of
-  // 2112 for 520 ideal at N = 128, 624 instead of 912 for 296 at N = 96).
-  static constexpr bool SPREAD7 = N2 == 8;
+  // Canonical column c = N1 u + v sits at storage column N2 v + u, and with
+  // LD = N + 1 a 64-bit element's bank pair is (column + row) mod 16: row slot
+  // N2 k1 + k2 of the first inverse pass along p falls on N2 (v + k1) + u + k2.
+  // Consecutive canonical columns share two (N2 = 8) or four (N2 = 4) bank
+  // pairs; with u fastest, half a warp covers u < N2/2 and 32 / N2 values of v,
+  // still two to a bank pair, since every term but u is a multiple of N2 or
+  // common. So every other run of 16 / N2 values of v swaps the halves of its
+  // groups: it takes slot k2 ^ N2/2 for k2, which turns the sign of the odd
+  // outputs (turned back in the twiddle) and leaves row N2 n1 + n2 of those
+  // columns at row slot N2 n1 + (n2 ^ N2/2), where the last axis looks for it
+  // (rot). For N2 = 6 the columns of u = 0 and 1 cover the bank pairs with v
+  // fastest, and those of u = 2 half of them. A model of the
+  // pass's addresses gives 1152 wavefronts at 128 points (ideal 1040, without
+  // the swap 2176), 672 at 96 (588; 1248), 288 at 64 (264; 880 in column
+  // order), 204 at 48 (150; 288 in column order).
+  static constexpr bool ROT = N2 == 4 || N2 == 8;
+  static __host__ __device__ constexpr int rot(int v) { return ROT ? (v / (16 / N2) & 1) * (N2 / 2) : 0; }
   // The spectrum is Hermitian, so the inverse transforms only the N/2 + 1
   // canonical columns along p and then rows p and p + N/2 together along q
   // (their outputs are real: one lands in the real part, one in the
@@ -597,32 +607,42 @@ __global__ void __launch_bounds__(CorrCfg<N, W, SRCH, VAR>::NT, CorrCfg<N, W, SR
 #pragma unroll 1
       for (int it = gt; it < NC * N1; it += G) {
         int c, k1;
-        if (C::SPREAD7) {  // c = N1 u + v with u fastest, then v, then k1; c = N/2 last
-          if (it < H * N1) {
-            constexpr int U = N2 / 2 > 0 ? N2 / 2 : 1;
-            const int u = it % U, w = it / U;
-            c = N1 * u + w % N1;
-            k1 = w / N1;
-          } else {
-            c = H;
-            k1 = it - H * N1;
-          }
+        if (it >= H * N1) {  // column N/2 last
+          c = H;
+          k1 = it - H * N1;
+        } else if (C::ROT) {
+          constexpr int U = N2 / 2 > 0 ? N2 / 2 : 1;
+          const int w = it / U;
+          c = N1 * (it % U) + w % N1;
+          k1 = w / N1;
+        } else if (N2 == 6) {  // columns of u = 0, 1, then those of u = 2
+          const bool lo = it < 2 * N1 * N1;
+          const int e = lo ? it : it - 2 * N1 * N1;
+          c = lo ? e % (2 * N1) : 2 * N1 + e % N1;
+          k1 = lo ? e / (2 * N1) : e / N1;
         } else {
-          c = it % NC;
-          k1 = it / NC;
+          c = it % H;
+          k1 = it / H;
         }
         float2* L = P + s_canon[c] * LD + N2 * k1;
+        const int swap = C::rot(c % N1);  // N2/2: the halves of the group change places
+        float2* L0 = L + swap;            // slots of k2 < N2/2
+        float2* L1 = L - swap;
+        const uint32_t sign = swap ? 0x80000000u : 0u;
         float2 x[N2];
 #pragma unroll
-        for (int k2 = 0; k2 < N2; ++k2) x[k2] = L[k2];
+        for (int k2 = 0; k2 < N2; ++k2) x[k2] = (k2 < N2 / 2 ? L0 : L1)[k2];
         RDFT<N2, true>::run(x, N2);
 #pragma unroll
         for (int n2 = 1; n2 < N2; ++n2) {
           const float2 t = tw[n2 * k1];
+          if (C::ROT && n2 % 2 == 1)  // the sign bits: a negated operand would change how the product is contracted
+            x[n2] = make_float2(__uint_as_float(__float_as_uint(x[n2].x) ^ sign),
+                                __uint_as_float(__float_as_uint(x[n2].y) ^ sign));
           x[n2] = cmul(x[n2], make_float2(t.x, -t.y));
         }
 #pragma unroll
-        for (int n2 = 0; n2 < N2; ++n2) L[n2] = x[n2];
+        for (int n2 = 0; n2 < N2; ++n2) (n2 < N2 / 2 ? L0 : L1)[n2] = x[n2];
       }
       grp_sync(bar, G);
     }
@@ -686,22 +706,22 @@ __global__ void __launch_bounds__(CorrCfg<N, W, SRCH, VAR>::NT, CorrCfg<N, W, SR
         const bool hasb = t + nh < nb, j0 = j == 0;
         const int pa = (blo + t + H) % N, pb = hasb ? (blo + t + nh + H) % N : pa;
         const int ga = N2 * j, gb = N2 * (j0 ? HN : N1 - j);
-        float2* La = P + pa;
-        const float2* Lb = P + pb;
+        // the rows' slots in the columns of groups j and N1 - j
+        const int kb = j0 ? HN : N1 - j, ta = C::rot(j), tb = C::rot(kb);
         float2 x1[N2], x2[N2], ma[h2 + 1], mb[h2];
-        auto row_pair = [&](int slot, float2& direct, float2& mirror) {
-          const float2 u = La[slot * LD];
-          const float2 v = hasb ? Lb[slot * LD] : make_float2(0.f, 0.f);
+        auto row_pair = [&](int slot, int t, float2& direct, float2& mirror) {
+          const float2 u = P[(pa ^ t) + slot * LD];
+          const float2 v = hasb ? P[(pb ^ t) + slot * LD] : make_float2(0.f, 0.f);
           direct = make_float2(u.x - v.y, u.y + v.x);
           mirror = make_float2(u.x + v.y, v.x - u.y);
         };
 #pragma unroll
         for (int k2 = 0; k2 < h2; ++k2) {
-          row_pair(ga + k2, x1[k2], ma[k2]);
-          row_pair(gb + k2, x2[k2], mb[k2]);
+          row_pair(ga + k2, ta, x1[k2], ma[k2]);
+          row_pair(gb + k2, tb, x2[k2], mb[k2]);
         }
         float2 mid = make_float2(0.f, 0.f);
-        if (j0) row_pair(h2, mid, ma[h2]);
+        if (j0) row_pair(h2, 0, mid, ma[h2]);
 #pragma unroll
         for (int k2 = h2; k2 < N2; ++k2) {
           const float2 own = k2 == h2 ? mid : ma[N2 - k2];
@@ -710,17 +730,16 @@ __global__ void __launch_bounds__(CorrCfg<N, W, SRCH, VAR>::NT, CorrCfg<N, W, SR
         }
         RDFT<N2, true>::run(x1, N2);
         RDFT<N2, true>::run(x2, N2);
-        const int kb = j0 ? HN : N1 - j;
 #pragma unroll
         for (int n2 = 1; n2 < N2; ++n2) {
-          const float2 ta = tw[n2 * j], tb = tw[n2 * kb];
-          x1[n2] = cmul(x1[n2], make_float2(ta.x, -ta.y));
-          x2[n2] = cmul(x2[n2], make_float2(tb.x, -tb.y));
+          const float2 wa = tw[n2 * j], wb = tw[n2 * kb];
+          x1[n2] = cmul(x1[n2], make_float2(wa.x, -wa.y));
+          x2[n2] = cmul(x2[n2], make_float2(wb.x, -wb.y));
         }
 #pragma unroll
         for (int n2 = 0; n2 < N2; ++n2) {
-          La[(ga + n2) * LD] = x1[n2];
-          La[(gb + n2) * LD] = x2[n2];
+          P[(pa ^ ta) + (ga + n2) * LD] = x1[n2];
+          P[(pa ^ tb) + (gb + n2) * LD] = x2[n2];
         }
       }
       grp_sync(bar, G);
@@ -747,7 +766,7 @@ __global__ void __launch_bounds__(CorrCfg<N, W, SRCH, VAR>::NT, CorrCfg<N, W, SR
             }
           } else {
 #pragma unroll
-            for (int k1 = 0; k1 < N1; ++k1) x[k1] = La[(N2 * k1 + n2) * LD];
+            for (int k1 = 0; k1 < N1; ++k1) x[k1] = P[(pa ^ C::rot(k1)) + (N2 * k1 + n2) * LD];
           }
           RDFT<N1, true>::run(x, N1);
           const int ps0 = blo + t, ps1 = blo + t + nh;  // fftshifted rows of pa and pb

@@ -31,7 +31,7 @@ struct BClass {
 };
 
 struct BSlot {
-  int64_t gtot = 0, ptot = 0;
+  int64_t gtot = 0, ptot = 0, dtot = 0;  // cells, and pixels and strips that deform
   int max_maxit = 0;
   bool any_nalt = false, any_replace = false, any_tol = false, any_keep = false, any_next = false;
   bool any_deform = false, any_pred0 = false;
@@ -228,7 +228,7 @@ static hh_status build_plan(hh_ctx* ctx, BPlan& P, const hh_batch_pair* pairs, i
     wcol[p] = WC;
     wrow[p] = WR;
     if (deforms[p]) {
-      Wt += (nr * nc + 3) / 4 * 4;  // 16-byte aligned per pair: the deformation stores pixel quads
+      Wt += (nr * nc + 3) / 4 * 4;  // 16-byte aligned per pair
       Q += (nr + 2) * (nc + 2);
       WC += (nc + 31) / 32 * hh::b_nseg(nr + 2);  // column tiles x segments
       WR += (nr + 2 + 31) / 32 * hh::b_nseg(nc + 2);  // 32-row groups x segments
@@ -289,7 +289,7 @@ static hh_status build_plan(hh_ctx* ctx, BPlan& P, const hh_batch_pair* pairs, i
   for (int k = 0; k < nslots; ++k) {
     BSlot& S = P.slots[k];
     std::map<std::tuple<int, int, int, int, int, int, int, int, int, int, int, int>, int> cls;
-    int64_t coff = 0, pcoff = 0;
+    int64_t coff = 0, dcoff = 0;
     for (int p = 0; p < npairs; ++p) {
       const hh_batch_pair& q = pairs[p];
       const hh_pass_desc* ps = passes + so[P.sched[p]];
@@ -305,7 +305,7 @@ static hh_status build_plan(hh_ctx* ctx, BPlan& P, const hh_batch_pair* pairs, i
       b.aoff = aoff[p];
       b.roff = roff[p];
       b.coff = coff;
-      b.pcoff = pcoff;
+      b.dcoff = dcoff;
       b.deforms = deforms[p];
       b.coefA = P.coefA + qoff[p];
       b.coefB = P.coefB + qoff[p];
@@ -363,7 +363,10 @@ static hh_status build_plan(hh_ctx* ctx, BPlan& P, const hh_batch_pair* pairs, i
       b.tol = pd.convergence_tol;
       const int64_t Gk = (int64_t)gr.ny * gr.nx;
       coff += Gk;
-      if (deforms[p]) pcoff += (q.nr * q.nc + 3) / 4 * 4;  // quads of pixels never straddle two pairs
+      if (deforms[p]) {
+        dcoff += hh::deform_strips(q.nr, q.nc);
+        S.ptot += q.nr * q.nc;
+      }
       S.max_maxit = std::max(S.max_maxit, (int)pd.max_iterations);
       S.any_nalt |= b.nalt > 0;
       S.any_replace |= b.replace != 0;
@@ -408,7 +411,7 @@ static hh_status build_plan(hh_ctx* ctx, BPlan& P, const hh_batch_pair* pairs, i
       }
     }
     S.gtot = coff;
-    S.ptot = pcoff;
+    S.dtot = dcoff;
     for (auto& c : S.classes) {
       c.njobs = (int64_t)c.hjobs.size() / 4;
       void* d = nullptr;
@@ -468,7 +471,7 @@ static hh_status issue(hh_ctx* ctx, BPlan& P) {
                                     P.d_slot_sweeps + (size_t)k * np, s));
       charge(HH_K_VECTOR, k, it, -1, 0);
       if (S.any_deform && (it > 1 || S.any_pred0)) {
-        HH_K(HH_K_DEFORM, 1, 120 * Ps, 16 * Ps, S.ptot, hh::launch_b_deform(T, np, P.d_done, it, S.ptot, pu, pv, s));
+        HH_K(HH_K_DEFORM, 1, 120 * Ps, 16 * Ps, S.ptot, hh::launch_b_deform(T, np, P.d_done, it, S.dtot, pu, pv, s));
         charge(HH_K_DEFORM, k, it, -1, 0);
       }
       for (size_t ci = 0; ci < S.classes.size(); ++ci) {

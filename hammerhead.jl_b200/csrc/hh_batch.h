@@ -11,7 +11,7 @@
 // it, it <= max_iterations, and it has not converged (done[p]).
 //
 // Kernels of a slot iterate over slot-compact index spaces (coff: cells of
-// the pairs that have the slot; pcoff: their pixels) and find the owning
+// the pairs that have the slot; dcoff: the strips of those that deform) and find the owning
 // pair by binary search, so one launch covers every pair and pairs of
 // uneven size cost nothing extra. Everything a kernel needs about a pair is
 // read from this table at run time, so a captured graph stays valid when
@@ -47,7 +47,7 @@ struct BPair {
   int64_t goff;   // cell storage offset
   int64_t aoff;   // alternatives storage offset (nalt planes of ny*nx cells)
   int64_t coff;   // slot-compact cell offset
-  int64_t pcoff;  // slot-compact pixel offset (a multiple of 4)
+  int64_t dcoff;  // slot-compact offset of its deformation strips
   int64_t roff;   // offset of the pair's final-pass result
   int32_t ny, nx;      // this slot's grid (0 when the slot does not exist)
   int32_t pgny, pgnx;  // previous slot's grid (predictor of sweep 1)
@@ -105,7 +105,7 @@ cudaError_t launch_b_prefilter(const BPair* bp, int npairs, int64_t qtot, int64_
 cudaError_t launch_b_sweep_begin(const BPair* bp, int npairs, const int32_t* done, int it, int64_t gtot,
                                  const float* pu, const float* pv, float* u, float* v, float* uncu, float* uncv,
                                  int32_t* sweeps, int32_t* slot_sweeps, cudaStream_t s);
-cudaError_t launch_b_deform(const BPair* bp, int npairs, const int32_t* done, int it, int64_t ptot, const float* pu,
+cudaError_t launch_b_deform(const BPair* bp, int npairs, const int32_t* done, int it, int64_t stot, const float* pu,
                             const float* pv, cudaStream_t s);
 struct BGrid {  // concatenated grid arrays, indexed by goff + cell
   float *u, *v, *resu, *resv, *ratio, *moment, *alt_u, *alt_v, *meas_u, *meas_v;

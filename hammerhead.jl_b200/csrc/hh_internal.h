@@ -141,6 +141,7 @@ struct PredGrid {
   int32_t gny, gnx;
   float y0, ysp, x0, xsp;
 };
+int64_t deform_strips(int64_t nr, int64_t nc);  // warps' work items of a deformation
 cudaError_t launch_deform(const float* CA, const float* CB, int64_t nr, int64_t nc, const float* pu,
                           const float* pv, PredGrid g, float* wA, float* wB, cudaStream_t s);
 cudaError_t launch_node_values(const float* pu, const float* pv, PredGrid g, const float* y, int32_t ny,

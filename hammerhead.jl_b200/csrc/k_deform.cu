@@ -8,8 +8,8 @@
 //   c_{n-2} = b_{n-2} and a constant-coefficient tridiagonal system, solved
 //   by the Thomas algorithm with the line-independent elimination factors
 //   precomputed once. Separable: every column, then every row.
-// deform: one thread per output pixel evaluates the predictor by bilinear
-//   interpolation with flat extrapolation (Gridded(Linear()) + Flat(),
+// deform: a lane per image row, stepping along the columns, evaluates the
+//   predictor by bilinear interpolation with flat extrapolation (Gridded(Linear()) + Flat(),
 //   src/pipeline.jl:561-600) and samples both coefficient arrays with the
 //   4x4 cubic B-spline at -+ half the displacement, zero outside the image
 //   (deform_columns!, src/pipeline.jl:957-965; _ka_deform!,
@@ -69,60 +69,169 @@ cudaError_t launch_bspline_factors(int64_t n, float* cp, float* inv, cudaStream_
 }
 
 // ---------------------------------------------------------------------------
-// Interpolations' cubic B-spline weights at fractional offset d.
-__device__ __forceinline__ void cubw(float d, float* w) {
-  const float x3 = FM(FM(d, d), d), c = FS(1.f, d), c3 = FM(FM(c, c), c);
-  const float two3 = kTwoThirds;
-  w[0] = div6(c3);
-  w[1] = FA(FS(two3, FM(d, d)), FM(x3, 0.5f));
-  w[2] = FA(FS(two3, FM(c, c)), FM(c3, 0.5f));
-  w[3] = div6(x3);
+// Two floats in one register pair: the frames' samples A and B, or the
+// predictor's components u and v, go through the same arithmetic, and the
+// packed instructions issue it once for both. Each half is rounded to nearest
+// like the scalar operation.
+struct F2 {
+  unsigned long long v;
+};
+__device__ __forceinline__ F2 pk(float a, float b) {
+  F2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void unpk(F2 x, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(x.v)); }
+__device__ __forceinline__ F2 add2(F2 a, F2 b) {
+  F2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 sub2(F2 a, F2 b) {
+  F2 r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
+  F2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+__device__ __forceinline__ F2 both(float x) { return pk(x, x); }
+// Packed products, each rounded by itself: the assembler contracts a packed
+// multiplication and the addition that uses it into one rounding, so a product
+// is the fused operation with an addend of -0 that only the launch knows.
+struct Mul2 {
+  F2 zero;
+  __device__ __forceinline__ F2 operator()(F2 a, F2 b) const { return fma2(a, b, zero); }
+};
+// div6 of both halves (its remainder step as q0 * -6 + x, the same product)
+__device__ __forceinline__ F2 div6_2(const Mul2& mul2, F2 x) {
+  const F2 r = both(k_sixth()), q0 = mul2(x, r);
+  return fma2(fma2(q0, both(-6.0f), x), r, q0);
+}
+// Interpolations' cubic B-spline weights at fractional offsets d.
+__device__ __forceinline__ void cubw2(const Mul2& mul2, F2 d, F2* w) {
+  const F2 d2 = mul2(d, d), x3 = mul2(d2, d), c = sub2(both(1.f), d), c2 = mul2(c, c), c3 = mul2(c2, c);
+  const F2 two3 = both(kTwoThirds), half = both(0.5f);
+  w[0] = div6_2(mul2, c3);
+  w[1] = add2(sub2(two3, d2), mul2(x3, half));
+  w[2] = add2(sub2(two3, c2), mul2(c3, half));
+  w[3] = div6_2(mul2, x3);
 }
 
-__device__ __forceinline__ float bspline_eval(const float* C, int64_t nr, int64_t nc, float yy, float xx) {
-  if (yy < 1.f || yy > (float)nr || xx < 1.f || xx > (float)nc) return 0.f;
-  int64_t iy = (int64_t)floorf(yy);
-  if (iy > nr - 1) iy = nr - 1;
-  int64_t ix = (int64_t)floorf(xx);
-  if (ix > nc - 1) ix = nc - 1;
-  float wy[4], wx[4];
-  cubw(FS(yy, (float)iy), wy);
-  cubw(FS(xx, (float)ix), wx);
-  const int64_t ld = nr + 2;
-  const float* base = C + (iy - 1) + (ix - 1) * ld;
-  float s = 0.f;
-#pragma unroll
-  for (int a = 0; a < 4; ++a) {
-    float t = 0.f;
-#pragma unroll
-    for (int b = 0; b < 4; ++b) t = FA(t, FM(wx[b], __ldg(base + a + b * ld)));
-    s = FA(s, FM(wy[a], t));
-  }
-  return s;
+// where coordinate q of a sample starts on an axis of n pixels: the cell's
+// first coefficient, and whether the sample is inside the image. A sample
+// outside reads the nearest cell and counts as zero.
+__device__ __forceinline__ int spline_cell(float q, int n, bool& in) {
+  in = !(q < 1.f || q > (float)n);
+  return min(__float2int_rd(fminf(fmaxf(q, 1.f), (float)n)), n - 1);
 }
 
-__global__ void __launch_bounds__(256) deform_kernel(const float* __restrict__ CA, const float* __restrict__ CB,
-                                                     int64_t nr, int64_t nc, const float* __restrict__ pu,
-                                                     const float* __restrict__ pv, PredGrid g, float* wA, float* wB) {
-  const int64_t total = nr * nc;
-  const bool small = total <= 0x7fffffff;
-  for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < total; k += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t r = small ? (int64_t)((uint32_t)k % (uint32_t)nr) : k % nr;
-    const int64_t c = small ? (int64_t)((uint32_t)k / (uint32_t)nr) : k / nr;
-    const float R = (float)(r + 1), Cc = (float)(c + 1);
-    const float du2 = FM(bilinear(pu, g, R, Cc), 0.5f);
-    const float dv2 = FM(bilinear(pv, g, R, Cc), 0.5f);
-    wA[k] = bspline_eval(CA, nr, nc, FS(R, dv2), FS(Cc, du2));
-    wB[k] = bspline_eval(CB, nr, nc, FA(R, dv2), FA(Cc, du2));
+// One warp deforms both frames on DEF_ROWS rows from row r0 and the columns
+// [c0, c1): a lane per row, stepping along the columns, so that every load and
+// store of the warp runs down one column. The predictor's cell and fraction are
+// formed once per row and, a lane each, once per column; its corner values are
+// loaded where the columns enter a new cell.
+//
+// What bounds it: the latency of a column's chain (coordinates, 32 loads, the
+// sums) at 24 warps per SM, then instructions issued (61 % of the slots): a
+// pixel needs two samples of 16 coefficients, whose products and sums may not
+// be fused (they are the CPU restatement's), and four cubic weights, some 270
+// instructions in packed form. 2048 x 2048: a thread per pixel with its own
+// divisions and 64-bit indices took 79 us; four rows per thread, whose loads
+// touch four lines each, 70; this takes 52. Strips of 8 columns: 16 and 32 are
+// as fast there (51, 59 us) but leave too few warps at 512 x 512 (8, 13, 24
+// us); 64 registers for 32 warps per SM spill and gain nothing (51 us).
+constexpr int DEF_ROWS = 32, DEF_COLS = 8;  // DEF_COLS <= 32: a lane per column
+__device__ __forceinline__ void deform_strip(const float* __restrict__ CA, const float* __restrict__ CB, int nr, int nc,
+                                             const float* __restrict__ pu, const float* __restrict__ pv,
+                                             const PredGrid& g, float* __restrict__ wA, float* __restrict__ wB, int r0,
+                                             int c0, int c1, float minus_zero) {
+  const Mul2 mul2{both(minus_zero)};
+  const int lane = threadIdx.x & 31;
+  const int r = min(r0 + lane, nr - 1);
+  const bool store = r0 + lane < nr;
+  const int64_t ld = (int64_t)nr + 2;
+  const float R = (float)(r + 1);
+  int iy, ixl;
+  float dy, dxl;
+  lin_axis(R, g.y0, g.ysp, g.gny, iy, dy);
+  lin_axis((float)(min(c0 + lane, nc - 1) + 1), g.x0, g.xsp, g.gnx, ixl, dxl);
+  const int iy2 = g.gny == 1 ? iy : iy + 1;
+  const F2 dy2 = both(dy), ey2 = both(FS(1.f, dy)), half = both(0.5f);
+  F2 f00 = both(0.f), f01 = f00, f10 = f00, f11 = f00;
+  int held = -1;
+  for (int c = c0; c < c1; ++c) {
+    const int ix = __shfl_sync(0xffffffffu, ixl, c - c0);
+    const float dx = __shfl_sync(0xffffffffu, dxl, c - c0);
+    if (ix != held) {  // uniform
+      held = ix;
+      const int64_t q0 = (int64_t)ix * g.gny, q1 = (int64_t)(g.gnx == 1 ? ix : ix + 1) * g.gny;
+      f00 = pk(pu[iy + q0], pv[iy + q0]);
+      f01 = pk(pu[iy + q1], pv[iy + q1]);
+      f10 = pk(pu[iy2 + q0], pv[iy2 + q0]);
+      f11 = pk(pu[iy2 + q1], pv[iy2 + q1]);
+    }
+    const F2 dx2 = both(dx), ex2 = both(FS(1.f, dx));
+    const F2 a = add2(mul2(ex2, f00), mul2(dx2, f01)), b = add2(mul2(ex2, f10), mul2(dx2, f11));
+    float du, dv;  // half the displacement
+    unpk(mul2(add2(mul2(ey2, a), mul2(dy2, b)), half), du, dv);
+    const float Cc = (float)(c + 1);
+    const float ya = FS(R, dv), yb = FA(R, dv), xa = FS(Cc, du), xb = FA(Cc, du);
+    bool inya, inyb, inxa, inxb;
+    const int iya = spline_cell(ya, nr, inya), iyb = spline_cell(yb, nr, inyb);
+    const int ixa = spline_cell(xa, nc, inxa), ixb = spline_cell(xb, nc, inxb);
+    const float* ca = CA + (iya - 1) + (ixa - 1) * ld;
+    const float* cb = CB + (iyb - 1) + (ixb - 1) * ld;
+    F2 wy[4], wx[4], t[4];
+    cubw2(mul2, sub2(pk(ya, yb), pk((float)iya, (float)iyb)), wy);
+    cubw2(mul2, sub2(pk(xa, xb), pk((float)ixa, (float)ixb)), wx);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const F2 m = mul2(wx[j], pk(__ldg(ca + i + j * ld), __ldg(cb + i + j * ld)));
+        t[i] = j == 0 ? m : add2(t[i], m);
+      }
+    }
+    F2 s = mul2(wy[0], t[0]);
+#pragma unroll
+    for (int i = 1; i < 4; ++i) s = add2(s, mul2(wy[i], t[i]));
+    float sa, sb;
+    unpk(s, sa, sb);
+    if (store) {
+      const int64_t k = r + (int64_t)c * nr;
+      wA[k] = inya && inxa ? sa : 0.f;
+      wB[k] = inyb && inxb ? sb : 0.f;
+    }
   }
 }
+
+// strips of an image: DEF_ROWS rows (fastest) by DEF_COLS columns
+__host__ __device__ static inline int64_t def_row_strips(int64_t nr) { return (nr + DEF_ROWS - 1) / DEF_ROWS; }
+
+__global__ void __launch_bounds__(256, 3) deform_kernel(const float* __restrict__ CA, const float* __restrict__ CB, int nr,
+                                                     int nc, const float* __restrict__ pu,
+                                                     const float* __restrict__ pv, PredGrid g, float* wA, float* wB,
+                                                        float minus_zero) {
+  const int64_t rs = def_row_strips(nr), total = rs * ((nc + DEF_COLS - 1) / DEF_COLS);
+  for (int64_t k = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; k < total; k += ((int64_t)gridDim.x * blockDim.x) >> 5) {
+    const int c0 = (int)(k / rs) * DEF_COLS;
+    deform_strip(CA, CB, nr, nc, pu, pv, g, wA, wB, (int)(k % rs) * DEF_ROWS, c0, min(c0 + DEF_COLS, nc), minus_zero);
+  }
+}
+
+int64_t deform_strips(int64_t nr, int64_t nc) { return def_row_strips(nr) * ((nc + DEF_COLS - 1) / DEF_COLS); }
 
 cudaError_t launch_deform(const float* CA, const float* CB, int64_t nr, int64_t nc, const float* pu,
                           const float* pv, PredGrid g, float* wA, float* wB, cudaStream_t s) {
-  const int64_t total = nr * nc;
-  int64_t blocks = (total + 255) / 256;
+  // a strip forms the predictor's axis cells once, so longer strips are
+  // cheaper; DEF_COLS columns leave a 1024 x 1024 image as many warps as the
+  // chip holds
+  int64_t blocks = (deform_strips(nr, nc) + 7) / 8;
   if (blocks > 148 * 32) blocks = 148 * 32;
-  deform_kernel<<<(unsigned)blocks, 256, 0, s>>>(CA, CB, nr, nc, pu, pv, g, wA, wB);
+  deform_kernel<<<(unsigned)blocks, 256, 0, s>>>(CA, CB, (int)nr, (int)nc, pu, pv, g, wA, wB, -0.0f);
   return cudaGetLastError();
 }
 
@@ -629,77 +738,26 @@ cudaError_t launch_b_sweep_begin(const BPair* bp, int npairs, const int32_t* don
   return cudaGetLastError();
 }
 
-// Four consecutive pixels (a quad; pairs start on multiples of 4 in the
-// slot-compact index and in the warped arrays) per thread: the pair lookup,
-// the pair's fields, the pixel index division and the predictor's column
-// interpolation are done once per quad (again only where the quad wraps to
-// the next column), and a full quad is stored as one 16-byte vector.
-__global__ void __launch_bounds__(256) b_deform_kernel(const BPair* __restrict__ bp, int npairs,
-                                                       const int32_t* __restrict__ done, int it, int64_t ptot,
-                                                       const float* __restrict__ pu, const float* __restrict__ pv) {
-  B_STRIDE(t, (ptot + 3) / 4) {
-    const int64_t k = 4 * t;
-    const int p = bp_find<&BPair::pcoff>(bp, npairs, k);
+// Strips (deform_strip) of every pair that deforms, a warp each; the pair of a
+// strip is looked up once.
+__global__ void __launch_bounds__(256, 3) b_deform_kernel(const BPair* __restrict__ bp, int npairs,
+                                                       const int32_t* __restrict__ done, int it, int64_t stot,
+                                                       const float* __restrict__ pu, const float* __restrict__ pv, float minus_zero) {
+  for (int64_t k = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; k < stot; k += ((int64_t)gridDim.x * blockDim.x) >> 5) {
+    const int p = bp_find<&BPair::dcoff>(bp, npairs, k);
     const BPair& b = bp[p];
-    const int64_t l0 = k - b.pcoff, npx = b.nr * b.nc;
-    if (!bp_live(b, it, done, p) || !(it > 1 || b.has_pred0) || !b.deforms || l0 >= npx) continue;
-    const PredGrid g = b_pred_grid(b, it);
-    const float* fu = pu + b.goff;
-    const float* fv = pv + b.goff;
-    const int64_t nr = b.nr, nc = b.nc;
-    int64_t r, c;
-    if (npx <= 0x7fffffff) {  // 32-bit division when the pair's pixel index fits
-      r = (uint32_t)l0 % (uint32_t)nr;
-      c = (uint32_t)l0 / (uint32_t)nr;
-    } else {
-      r = l0 % nr;
-      c = l0 / nr;
-    }
-    float wa[4], wb[4];
-    int ix = 0;
-    float dx = 0.f;
-    int64_t cx = -1;  // column whose x interpolation (ix, dx) is held
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      wa[j] = wb[j] = 0.f;
-      if (l0 + j < npx) {
-        int64_t rj = r + j, cj = c;
-        while (rj >= nr) {  // the quad wraps to the next column
-          rj -= nr;
-          ++cj;
-        }
-        const float R = (float)(rj + 1), Cc = (float)(cj + 1);
-        if (cj != cx) {
-          lin_axis(Cc, g.x0, g.xsp, g.gnx, ix, dx);
-          cx = cj;
-        }
-        int iy;
-        float dy;
-        lin_axis(R, g.y0, g.ysp, g.gny, iy, dy);
-        const float du2 = FM(bilinear_at(fu, g, iy, dy, ix, dx), 0.5f);
-        const float dv2 = FM(bilinear_at(fv, g, iy, dy, ix, dx), 0.5f);
-        wa[j] = bspline_eval(b.coefA, nr, nc, FS(R, dv2), FS(Cc, du2));
-        wb[j] = bspline_eval(b.coefB, nr, nc, FA(R, dv2), FA(Cc, du2));
-      }
-    }
-    if (l0 + 3 < npx) {
-      *reinterpret_cast<float4*>(b.warpA + l0) = make_float4(wa[0], wa[1], wa[2], wa[3]);
-      *reinterpret_cast<float4*>(b.warpB + l0) = make_float4(wb[0], wb[1], wb[2], wb[3]);
-    } else {
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-        if (l0 + j < npx) {
-          b.warpA[l0 + j] = wa[j];
-          b.warpB[l0 + j] = wb[j];
-        }
-    }
+    if (!bp_live(b, it, done, p) || !(it > 1 || b.has_pred0) || !b.deforms) continue;  // uniform across the warp
+    const int64_t l = k - b.dcoff, rs = def_row_strips(b.nr);
+    const int c0 = (int)(l / rs) * DEF_COLS;
+    deform_strip(b.coefA, b.coefB, (int)b.nr, (int)b.nc, pu + b.goff, pv + b.goff, b_pred_grid(b, it), b.warpA, b.warpB,
+                 (int)(l % rs) * DEF_ROWS, c0, min(c0 + DEF_COLS, (int)b.nc), minus_zero);
   }
 }
 
-cudaError_t launch_b_deform(const BPair* bp, int npairs, const int32_t* done, int it, int64_t ptot, const float* pu,
+cudaError_t launch_b_deform(const BPair* bp, int npairs, const int32_t* done, int it, int64_t stot, const float* pu,
                             const float* pv, cudaStream_t s) {
-  if (ptot <= 0) return cudaSuccess;
-  b_deform_kernel<<<b_blocks((ptot + 3) / 4, 32), 256, 0, s>>>(bp, npairs, done, it, ptot, pu, pv);
+  if (stot <= 0) return cudaSuccess;
+  b_deform_kernel<<<b_blocks(stot * 32, 32), 256, 0, s>>>(bp, npairs, done, it, stot, pu, pv, -0.0f);
   return cudaGetLastError();
 }
 

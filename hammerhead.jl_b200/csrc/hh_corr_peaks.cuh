@@ -835,9 +835,9 @@ __device__ __noinline__ void analyze_group(const float* R, int nr, int nc, int l
 // (spectrum!, src/correlators.jl:266-279); the phase method divides by
 // |S| + eps(Float32) and applies the spectral filter weight wk.
 __device__ __forceinline__ float2 cross_spectrum(float2 X, float2 Zm, int method, float wk) {
-  const float2 Y = make_float2(Zm.x, -Zm.y);
-  const float Ar = 0.5f * (X.x + Y.x), Ai = 0.5f * (X.y + Y.y);
-  const float Br = 0.5f * (X.y - Y.y), Bi = -0.5f * (X.x - Y.x);
+  const float2 s = cadd2(X, Zm), d = csub2(X, Zm);
+  const float Ar = 0.5f * s.x, Ai = 0.5f * d.y;
+  const float Br = 0.5f * s.y, Bi = -0.5f * d.x;
   float2 S = cmul(make_float2(Ar, -Ai), make_float2(Br, Bi));
   if (method == 1) {
     const float den = hypotf(S.x, S.y) + 1.1920929e-7f;

@@ -24,8 +24,8 @@
 // mask's bytes are gathered apart): with one per pixel the loads went out one
 // by one, and a third of a warp's time was the wait for them (32-point padded
 // windows 4.6 -> 3.5 ns, unpadded 12.1 -> 7.3). Bound by issue and latency
-// (2.5 k warp instructions per padded 16 px window, half the issue slots
-// used); times beside the dispatch in launch_corr_nw.
+// (half the issue slots used at 16 to 20 warps per SM; complex sums are packed
+// instructions, cadd2); times beside the dispatch in launch_corr_nw.
 #pragma once
 #include "hh_corr_peaks.cuh"
 
@@ -42,7 +42,7 @@ template <int N, int W> struct SegCfg {
   static constexpr int COLS = W > H ? W : H;
   // the windows of a half-warp (64-bit accesses) and of a warp (32-bit ones) start 16 banks apart
   static constexpr int PS = (COLS * LD + 15) / 16 * 16 + 8;
-  static constexpr int MINB = W == 32 ? 3 : 4;
+  static constexpr int MINB = W == 32 ? 3 : (N == 16 ? 5 : 4);
   static constexpr size_t off_apod = (size_t)WIN * PS * sizeof(float2);
   static constexpr size_t off_gain = off_apod + (size_t)W * (W + 1) * sizeof(float);
   static constexpr size_t off_rmax = off_gain + (BOXED ? (2 * Q + 1) * (2 * Q + 1) * sizeof(float) : 0);

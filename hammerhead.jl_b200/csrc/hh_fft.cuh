@@ -19,6 +19,23 @@ __device__ __forceinline__ float2 csub(float2 a, float2 b) { return make_float2(
 __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
   return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
+// a + b and a - b of complex values as one packed instruction; each part is
+// rounded like the scalar operation. Not for operands that are products: those
+// the compiler contracts with the scalar addition (RDFT<3>), and not where an
+// operand's parts change places (mul_mi), which the packed form would have to
+// move first.
+__device__ __forceinline__ float2 cadd2(float2 a, float2 b) {
+  float2 r;
+  asm("{.reg .b64 p, q; mov.b64 p, {%2, %3}; mov.b64 q, {%4, %5}; add.rn.f32x2 p, p, q; mov.b64 {%0, %1}, p;}"
+      : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return r;
+}
+__device__ __forceinline__ float2 csub2(float2 a, float2 b) {
+  float2 r;
+  asm("{.reg .b64 p, q; mov.b64 p, {%2, %3}; mov.b64 q, {%4, %5}; sub.rn.f32x2 p, p, q; mov.b64 {%0, %1}, p;}"
+      : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return r;
+}
 // multiply by -i (forward) or +i (inverse)
 template <bool INV> __device__ __forceinline__ float2 mul_mi(float2 v) {
   return INV ? make_float2(-v.y, v.x) : make_float2(v.y, -v.x);
@@ -45,7 +62,7 @@ template <bool INV> struct RDFT<2, INV> {
   static __device__ __forceinline__ void run(float2* x, int nz = 2) {
     if (nz <= 0) return;
     if (nz == 1) { x[1] = x[0]; return; }
-    float2 a = cadd(x[0], x[1]), b = csub(x[0], x[1]);
+    float2 a = cadd2(x[0], x[1]), b = csub2(x[0], x[1]);
     x[0] = a;
     x[1] = b;
   }
@@ -79,18 +96,18 @@ template <bool INV> struct RDFT<4, INV> {
       a0 = a1 = x[0];
       b0 = b1 = x[1];
     } else {
-      a0 = cadd(x[0], x[2]);
-      a1 = csub(x[0], x[2]);
+      a0 = cadd2(x[0], x[2]);
+      a1 = csub2(x[0], x[2]);
       if (nz == 3) {
         b0 = b1 = x[1];
       } else {
-        b0 = cadd(x[1], x[3]);
-        b1 = csub(x[1], x[3]);
+        b0 = cadd2(x[1], x[3]);
+        b1 = csub2(x[1], x[3]);
       }
     }
     float2 jb = mul_mi<INV>(b1);
-    x[0] = cadd(a0, b0);
-    x[2] = csub(a0, b0);
+    x[0] = cadd2(a0, b0);
+    x[2] = csub2(a0, b0);
     x[1] = cadd(a1, jb);
     x[3] = csub(a1, jb);
   }

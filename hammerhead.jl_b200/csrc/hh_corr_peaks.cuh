@@ -360,10 +360,12 @@ struct RecSrc {
 // The per-window outputs from the peaks found (analyze_plane!'s tail,
 // src/correlators.jl:459-468): the primary refined by the chosen subpixel
 // method, displacement from the plane centre, peak ratio and moment; the
-// alternatives 1..npeaks-1 refined by gauss3; 1-based peak locations.
+// alternatives 1..npeaks-1 refined by gauss3; 1-based peak locations. Of the K
+// peaks only [m0, m1) are handled (vals and locs[2 m0 ..] are read).
 template <class Src>
 __device__ void peak_outputs(const Src& src, int nr, int nc, int K, int npeaks, int subpixel, int nfound,
-                             const float* vals, const int* locs, int64_t grid_id, int64_t job, const PeakOut& o) {
+                             const float* vals, const int* locs, int64_t grid_id, int64_t job, const PeakOut& o,
+                             int m0, int m1) {
   int found = 0;
   if (nfound > 0) {
     found = 1;
@@ -373,7 +375,7 @@ __device__ void peak_outputs(const Src& src, int nr, int nc, int K, int npeaks, 
   const int cr = nr / 2 + 1, cc = nc / 2 + 1;
   const int mmax = found < npeaks ? found : npeaks;  // peaks 1..mmax carry results
   float* pk = o.packed ? o.packed + job * (int64_t)(5 + 2 * (K - 1)) : nullptr;
-  for (int m = 0; m < K; ++m) {
+  for (int m = m0; m < m1; ++m) {
     float ref[2] = {NaN, NaN};
     if (m < found && (m == 0 || m < mmax)) {
       const int pr = locs[2 * m], pc = locs[2 * m + 1];
@@ -807,9 +809,9 @@ __device__ __forceinline__ void analyze_body(const float* R, int nr, int nc, int
   }
   if (gtid == 0) {
     if constexpr (BOXED)
-      peak_outputs(BoxSrc{{R, ldr, rlo, rhi, clo, chi}}, nr, nc, K, npeaks, subpixel, nfound, s_vals, s_locs, grid_id, job, *o);
+      peak_outputs(BoxSrc{{R, ldr, rlo, rhi, clo, chi}}, nr, nc, K, npeaks, subpixel, nfound, s_vals, s_locs, grid_id, job, *o, 0, K);
     else
-      peak_outputs(PlaneSrc{R, ldr}, nr, nc, K, npeaks, subpixel, nfound, s_vals, s_locs, grid_id, job, *o);
+      peak_outputs(PlaneSrc{R, ldr}, nr, nc, K, npeaks, subpixel, nfound, s_vals, s_locs, grid_id, job, *o, 0, K);
   }
 }
 

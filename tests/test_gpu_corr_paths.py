@@ -130,3 +130,24 @@ def test_general_shapes_vs_fp64(window, search, method):
             keep = [np.abs(np.arange(s[k]) - s[k] // 2) <= o[k] for k in range(2)]
             R = R * (keep[0][:, None] & keep[1][None])
         assert np.abs(planes[j] - R).max() <= 2e-5 * R.max()
+
+
+@pytest.mark.parametrize("n_peaks", [1, 2, 4, 8])
+def test_epilogue_split_and_whole(ws, hb, n_peaks):
+    """A thread per window and peak below 32768 windows, one per window above:
+    the same windows through both, every packed value alike."""
+    from hammerhead_b200 import hooks, synthetic
+
+    A, B = synthetic.particle_pair((420, 400), synthetic.uniform_flow(1.4, -0.8), seed=21, ppp=0.02)
+    A[100:140, 100:140] = B[100:140, 100:140] = 0.25  # windows without a peak
+    p = hb.PIVParameters(window_size=16, overlap=14, padding=False, apodization="none", n_peaks=n_peaks)
+    jobs = hb.pass_grid(A.shape, p)[3]
+    jobs = np.concatenate([jobs, jobs[:: -1]])
+    assert len(jobs) > 32768
+    sess = hooks.DeviceSession(ws)
+    sess.stage_pair(A, B)
+    whole, wlocs, _ = sess.process_windows(p, jobs, want_locs=True)
+    for i in (0, len(jobs) // 2, len(jobs) - 1000):
+        part, plocs, _ = sess.process_windows(p, jobs[i:i + 1000], want_locs=True)
+        np.testing.assert_array_equal(part, whole[i:i + 1000])
+        np.testing.assert_array_equal(plocs, wlocs[i:i + 1000])

@@ -263,16 +263,17 @@ __global__ void __launch_bounds__(NCC_PR) ncc_pixel_kernel(const NccArgs a) {
     cw[threadIdx.x] = span_at(c0 + threadIdx.x, a.W, a.step, a.wx);
   }
   __syncthreads();
-  if (r >= a.nr) return;
-  const Cell y = cell_at((float)(r + 1), a.y0, a.ysp, a.gny);
-  // the rows' and columns' cells, for the node kernel
-  if (blockIdx.y == 0) {
-    a.cells[2 * r] = y.i;
-    a.cells[2 * r + 1] = __float_as_int(y.d);
-  }
+  // the rows' and columns' cells, for the node kernel (the columns' also where
+  // the image has fewer rows than the block has columns)
   if (blockIdx.x == 0 && threadIdx.x < nc) {
     a.cells[2 * (a.nr + c0 + threadIdx.x)] = cx[threadIdx.x].i;
     a.cells[2 * (a.nr + c0 + threadIdx.x) + 1] = __float_as_int(cx[threadIdx.x].d);
+  }
+  if (r >= a.nr) return;
+  const Cell y = cell_at((float)(r + 1), a.y0, a.ysp, a.gny);
+  if (blockIdx.y == 0) {
+    a.cells[2 * r] = y.i;
+    a.cells[2 * r + 1] = __float_as_int(y.d);
   }
   const Span rw = span_at(r, a.W, a.step, a.wy);
   // dL/da = sum_j -(b - bbar_j) inv_j + ca_j (a - abar_j) over the windows j

@@ -1,0 +1,27 @@
+"""The adjoint at the edges of its launches' ranges, against the oracle's FP64
+loss and analytic gradient (the tolerances of the differentiation case: 1e-5
+relative on the loss, 1e-3 relative L2 on dL/dP)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _agrees(hb, orc, ws, A, B, P, grid, window, overlap):
+    L, g = hb.NCCLoss(A, B, window=window, overlap=overlap, workspace=ws).value_and_grad(P, grid)
+    cA, cB = orc.prefilter(A, dtype=np.float64), orc.prefilter(B, dtype=np.float64)
+    wins = orc.ncc_windows(A.shape, window, overlap)
+    L64, g64 = orc.ncc_loss_grad(cA, cB, A.shape, P.astype(np.float64), grid, windows=wins, window=window, nthreads=8)
+    assert abs(L - L64) <= 1e-5 * abs(L64)
+    assert np.linalg.norm(g - g64) <= 1e-3 * np.linalg.norm(g64)
+
+
+@pytest.mark.parametrize("rows,window,overlap", [(2, 2, 0), (4, 4, 2), (5, 3, 1), (7, 6, 3), (8, 8, 4), (9, 8, 6)])
+def test_few_rows(hb, orc, ws, rows, window, overlap):
+    """Images with fewer rows than the pixel kernel's block has columns (8)."""
+    rng = np.random.default_rng(rows)
+    A = rng.random((rows, 61)).astype(np.float32)
+    B = (A + 0.2 * rng.random(A.shape)).astype(np.float32)
+    P = rng.normal(0.0, 0.2, (2, 9, 2)).astype(np.float32)
+    grid = (1.5, rows - 2.0 if rows > 2 else 1.0, 2.0, 7.0)
+    _agrees(hb, orc, ws, A, B, P, grid, window, overlap)

@@ -133,6 +133,17 @@ __device__ __forceinline__ void deformed(const NccArgs& a, int64_t r, int64_t c,
   vb = bs_sample<GRAD>(a.CB, a.nr, a.nc, __fadd_rn(R, v2), __fadd_rn(Cc, u2), by, bx);
 }
 
+// The CTA's place in a two-dimensional arrangement of nx (first axis, fastest)
+// by as many as there are. The launches are one-dimensional: a grid's second
+// dimension ends at 65535, which image columns and node columns may pass.
+struct Block {
+  int x, y;
+};
+__device__ __forceinline__ Block block_of(int64_t nx) {
+  const int n = (int)nx;
+  return Block{(int)blockIdx.x % n, (int)blockIdx.x / n};
+}
+
 constexpr int NCC_THREADS = 256;
 
 __device__ __forceinline__ double block_sum(double v, double* red) {
@@ -175,7 +186,8 @@ __global__ void __launch_bounds__(NCC_THREADS) ncc_tile_kernel(const NccArgs a) 
   Cell* cx = ry + side;
   double* part = reinterpret_cast<double*>(cx + side);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int jr0 = blockIdx.x * TW, jc0 = blockIdx.y * TW;
+  const Block b = block_of((a.wy + TW - 1) / TW);
+  const int jr0 = b.x * TW, jc0 = b.y * TW;
   const int ty = min(TW, a.wy - jr0), tx = min(TW, a.wx - jc0);           // windows of this tile
   const int rt = W + (ty - 1) * a.step, ct = W + (tx - 1) * a.step;       // its pixels
   const int64_t r0 = (int64_t)jr0 * a.step, c0 = (int64_t)jc0 * a.step;
@@ -239,7 +251,7 @@ __global__ void __launch_bounds__(NCC_THREADS) ncc_tile_kernel(const NccArgs a) 
   if (tid == 0) {
     double t = 0.0;
     for (int k = 0; k < NCC_THREADS / 32; ++k) t += part[k];
-    a.wstat[6 * (int64_t)a.wy * a.wx + blockIdx.x + (int64_t)blockIdx.y * gridDim.x] = t;
+    a.wstat[6 * (int64_t)a.wy * a.wx + blockIdx.x] = t;
   }
 }
 
@@ -256,7 +268,8 @@ __device__ __forceinline__ Span span_at(int64_t p, int W, int step, int nw) {
 __global__ void __launch_bounds__(NCC_PR) ncc_pixel_kernel(const NccArgs a) {
   __shared__ Cell cx[NCC_PC];
   __shared__ Span cw[NCC_PC];
-  const int64_t P = a.nr * a.nc, r = (int64_t)blockIdx.x * NCC_PR + threadIdx.x, c0 = (int64_t)blockIdx.y * NCC_PC;
+  const Block b = block_of((a.nr + NCC_PR - 1) / NCC_PR);
+  const int64_t P = a.nr * a.nc, r = (int64_t)b.x * NCC_PR + threadIdx.x, c0 = (int64_t)b.y * NCC_PC;
   const int nc = (int)min((int64_t)NCC_PC, a.nc - c0);
   if (threadIdx.x < nc) {
     cx[threadIdx.x] = cell_at((float)(c0 + threadIdx.x + 1), a.x0, a.xsp, a.gnx);
@@ -265,13 +278,13 @@ __global__ void __launch_bounds__(NCC_PR) ncc_pixel_kernel(const NccArgs a) {
   __syncthreads();
   // the rows' and columns' cells, for the node kernel (the columns' also where
   // the image has fewer rows than the block has columns)
-  if (blockIdx.x == 0 && threadIdx.x < nc) {
+  if (b.x == 0 && threadIdx.x < nc) {
     a.cells[2 * (a.nr + c0 + threadIdx.x)] = cx[threadIdx.x].i;
     a.cells[2 * (a.nr + c0 + threadIdx.x) + 1] = __float_as_int(cx[threadIdx.x].d);
   }
   if (r >= a.nr) return;
   const Cell y = cell_at((float)(r + 1), a.y0, a.ysp, a.gny);
-  if (blockIdx.y == 0) {
+  if (b.y == 0) {
     a.cells[2 * r] = y.i;
     a.cells[2 * r + 1] = __float_as_int(y.d);
   }
@@ -331,7 +344,8 @@ __device__ __forceinline__ float cell_w(const int* cells, int64_t p, int g, int 
 __global__ void __launch_bounds__(NODE_THREADS) ncc_node_kernel(const NccArgs a) {
   __shared__ double t[2][NODE_K][NODE_R + 1];
   const int64_t G = (int64_t)a.gny * a.gnx, P = a.nr * a.nc;
-  const int gy0 = blockIdx.x * NODE_R, gx0 = blockIdx.y * NODE_C;
+  const Block b = block_of((a.gny + NODE_R - 1) / NODE_R);
+  const int gy0 = b.x * NODE_R, gx0 = b.y * NODE_C;
   const int64_t c_lo = reach_of(gx0, a.gnx, a.x0, a.xsp, a.nc).lo;
   const int64_t c_hi = reach_of(min(gx0 + NODE_C, a.gnx) - 1, a.gnx, a.x0, a.xsp, a.nc).hi;
   // this thread's node and component in the second step
@@ -389,15 +403,16 @@ cudaError_t launch_ncc_loss_grad(const NccArgs& a, cudaStream_t s) {
   cudaError_t e = cudaFuncSetAttribute(ncc_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)(NCC_SIDE * (NCC_SIDE + 1) * sizeof(float2) + 4096));
   if (e != cudaSuccess) return e;
+  auto blocks = [](int64_t n, int per) { return (n + per - 1) / per; };
   const int TW = tile_windows(a.W, a.step);
-  const dim3 tiles((a.wy + TW - 1) / TW, (a.wx + TW - 1) / TW);
-  ncc_tile_kernel<<<tiles, NCC_THREADS, sm, s>>>(a);
-  ncc_loss_kernel<<<1, NCC_THREADS, 0, s>>>(a, (int64_t)tiles.x * tiles.y);
+  const int64_t tiles = blocks(a.wy, TW) * blocks(a.wx, TW);
+  const int64_t px = blocks(a.nr, NCC_PR) * blocks(a.nc, NCC_PC), nodes = blocks(a.gny, NODE_R) * blocks(a.gnx, NODE_C);
+  if (tiles > INT32_MAX || (a.grad && (px > INT32_MAX || nodes > INT32_MAX))) return cudaErrorInvalidValue;
+  ncc_tile_kernel<<<(unsigned)tiles, NCC_THREADS, sm, s>>>(a);
+  ncc_loss_kernel<<<1, NCC_THREADS, 0, s>>>(a, tiles);
   if (a.grad) {
-    const dim3 px((unsigned)((a.nr + NCC_PR - 1) / NCC_PR), (unsigned)((a.nc + NCC_PC - 1) / NCC_PC));
-    ncc_pixel_kernel<<<px, NCC_PR, 0, s>>>(a);
-    const dim3 nodes((a.gny + NODE_R - 1) / NODE_R, (a.gnx + NODE_C - 1) / NODE_C);
-    ncc_node_kernel<<<nodes, NODE_THREADS, 0, s>>>(a);
+    ncc_pixel_kernel<<<(unsigned)px, NCC_PR, 0, s>>>(a);
+    ncc_node_kernel<<<(unsigned)nodes, NODE_THREADS, 0, s>>>(a);
   }
   return cudaGetLastError();
 }

@@ -25,3 +25,15 @@ def test_few_rows(hb, orc, ws, rows, window, overlap):
     P = rng.normal(0.0, 0.2, (2, 9, 2)).astype(np.float32)
     grid = (1.5, rows - 2.0 if rows > 2 else 1.0, 2.0, 7.0)
     _agrees(hb, orc, ws, A, B, P, grid, window, overlap)
+
+
+def test_wide_image_and_long_node_axis(hb, orc, ws):
+    """More column blocks than a grid's second dimension holds (65535): 8 image
+    columns and 2 node columns to a block. Displacements are multiples of 1/2 px
+    on nodes 4 px apart, so that FP32 holds every sample's coordinate exactly at
+    this width."""
+    rng = np.random.default_rng(3)
+    A = rng.random((8, 524301)).astype(np.float32)
+    B = (A + 0.2 * rng.random(A.shape)).astype(np.float32)
+    P = (rng.integers(-2, 3, (1, 131075, 2)) / 2).astype(np.float32)
+    _agrees(hb, orc, ws, A, B, P, (4.0, 1.0, 2.0, 4.0), 8, 0)

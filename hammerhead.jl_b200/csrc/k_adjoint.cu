@@ -56,10 +56,9 @@ __device__ __forceinline__ float bs_sample(const float* __restrict__ C, int64_t 
                                            float& gy, float& gx) {
   gy = gx = 0.f;
   if (yy < 1.f || yy > (float)nr || xx < 1.f || xx > (float)nc) return 0.f;
-  int64_t iy = (int64_t)floorf(yy);
-  if (iy > nr - 1) iy = nr - 1;
-  int64_t ix = (int64_t)floorf(xx);
-  if (ix > nc - 1) ix = nc - 1;
+  // a NaN coordinate (from the predictor) takes the first cell; its weights make the sample NaN
+  const int64_t iy = min((int64_t)fmaxf(floorf(yy), 1.f), nr - 1);
+  const int64_t ix = min((int64_t)fmaxf(floorf(xx), 1.f), nc - 1);
   float wy[4], wx[4], dy[4], dx[4];
   cubw_f(yy - (float)iy, wy);
   cubw_f(xx - (float)ix, wx);

@@ -37,3 +37,29 @@ def test_wide_image_and_long_node_axis(hb, orc, ws):
     B = (A + 0.2 * rng.random(A.shape)).astype(np.float32)
     P = (rng.integers(-2, 3, (1, 131075, 2)) / 2).astype(np.float32)
     _agrees(hb, orc, ws, A, B, P, (4.0, 1.0, 2.0, 4.0), 8, 0)
+
+
+def test_nan_node(hb, orc, ws):
+    """A node without a displacement (NaN): the windows it reaches drop out of
+    the loss like flat ones, and only its neighbours' gradients are NaN."""
+    shape, window, overlap, (i, j) = (90, 101), 16, 8, (3, 4)
+    A, B = hb.synthetic.particle_pair(shape, hb.synthetic.uniform_flow(0.7, -0.4), seed=5)
+    grid = (8.5, 10.0, 8.5, 11.0)
+    P = (np.array([0.7, -0.4]) + np.random.default_rng(5).normal(0.0, 0.3, (8, 9, 2))).astype(np.float32)
+    Pn = P.copy()
+    Pn[i, j] = np.nan
+    L, g = hb.NCCLoss(A, B, window=window, overlap=overlap, workspace=ws).value_and_grad(Pn, grid)
+    # pixel rows and columns whose predictor cell has the node as a corner
+    cells = [np.clip(np.floor((np.arange(n) + 1.0 - q0) / sp), 0, m - 2)
+             for n, q0, sp, m in ((shape[0], 8.5, 10.0, 8), (shape[1], 8.5, 11.0, 9))]
+    rows, cols = ((c == k) | (c == k - 1) for c, k in zip(cells, (i, j)))
+    wins = orc.ncc_windows(shape, window, overlap)
+    hit = np.array([rows[r:r + window].any() and cols[c:c + window].any() for r, c in wins])
+    assert 0 < hit.sum() < len(wins)
+    cA, cB = orc.prefilter(A, dtype=np.float64), orc.prefilter(B, dtype=np.float64)
+    L64, g64 = orc.ncc_loss_grad(cA, cB, shape, P.astype(np.float64), grid, windows=wins[~hit], window=window)
+    assert abs(L - L64) <= 1e-5 * abs(L64)
+    far = np.ones(P.shape[:2], bool)
+    far[i - 1:i + 2, j - 1:j + 2] = False
+    assert np.isnan(g[i, j]).all()
+    assert np.linalg.norm((g - g64)[far]) <= 1e-3 * np.linalg.norm(g64[far])

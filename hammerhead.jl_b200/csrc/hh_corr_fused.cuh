@@ -24,6 +24,7 @@
 // is formed from pairs (k, -k) there and the inverse takes that order back
 // to natural order, so no bit-reversal pass exists anywhere.
 #pragma once
+#include "hh_attr.h"
 #include "hh_corr_peaks.cuh"
 #include "hh_corr_seg.cuh"
 
@@ -872,21 +873,13 @@ static cudaError_t launch_nw(const CorrArgs& a, cudaStream_t s, int num_sms) {
   const size_t sm = C::smem();
   if (C::BOXED && !(a.gain && a.box_hi > 0 && a.box_lo >= N / 2 - C::Q && a.box_hi <= N / 2 + C::Q))
     return cudaErrorInvalidValue;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(correlate_kernel<N, W, SRCH, VAR, ANY>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (e != cudaSuccess) return e;
-    // the planes live in shared memory: ask for the largest carveout so the
-    // register budget, not the L1 split, sets the CTAs per SM
-    e = cudaFuncSetAttribute(correlate_kernel<N, W, SRCH, VAR, ANY>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                             (int)cudaSharedmemCarveoutMaxShared);
-    if (e != cudaSuccess) return e;
-    attr_set = true;
-  }
-  int per_sm = 0;
-  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, correlate_kernel<N, W, SRCH, VAR, ANY>, C::NT, sm);
+  static DeviceOnce attr;
+  cudaError_t e = raise_smem_carveout(attr, correlate_kernel<N, W, SRCH, VAR, ANY>, sm);
   if (e != cudaSuccess) return e;
-  if (per_sm < 1) per_sm = 1;
+  int per_sm = 0;
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, correlate_kernel<N, W, SRCH, VAR, ANY>, C::NT, sm);
+  if (e != cudaSuccess) return e;
+  if (per_sm < 1) return cudaErrorLaunchOutOfResources;
   const int64_t units = (a.njobs + C::WPC - 1) / C::WPC;
   int64_t grid = (int64_t)per_sm * num_sms;
   if (grid > units) grid = units;

@@ -442,13 +442,10 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS) correlate_general_kern
 }
 
 template <int THREADS, bool BOXED> static cudaError_t launch_general(const CorrArgs& a, cudaStream_t s) {
-  static bool attr = false;  // raised to the device's limit once: launches of different shapes may share a graph
-  if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(correlate_general_kernel<THREADS, BOXED>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-    if (e != cudaSuccess) return e;
-    attr = true;
-  }
+  // raised to the device's limit at once: launches of different shapes may share a graph
+  static DeviceOnce attr;
+  const cudaError_t e = raise_smem(attr, correlate_general_kernel<THREADS, BOXED>, 227 * 1024);
+  if (e != cudaSuccess) return e;
   const int64_t grid = a.njobs < a.gscr_slices ? a.njobs : a.gscr_slices;
   correlate_general_kernel<THREADS, BOXED><<<(unsigned)grid, THREADS, a.gc_smem_bytes, s>>>(a);
   return cudaGetLastError();

@@ -27,6 +27,7 @@
 // (half the issue slots used at 16 to 20 warps per SM; complex sums are packed
 // instructions, cadd2); times beside the dispatch in launch_corr_nw.
 #pragma once
+#include "hh_attr.h"
 #include "hh_corr_peaks.cuh"
 
 namespace hh {
@@ -470,19 +471,13 @@ template <int N, int W, int KC, bool PHASE> static cudaError_t launch_seg_k(cons
   const size_t sm = C::smem();
   if (C::BOXED && !(a.gain && a.box_hi > 0 && a.box_lo >= C::H - C::Q && a.box_hi <= C::H + C::Q))
     return cudaErrorInvalidValue;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(correlate_seg_kernel<N, W, KC, PHASE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(correlate_seg_kernel<N, W, KC, PHASE>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                             (int)cudaSharedmemCarveoutMaxShared);
-    if (e != cudaSuccess) return e;
-    attr_set = true;
-  }
-  int per_sm = 0;
-  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, correlate_seg_kernel<N, W, KC, PHASE>, C::NT, sm);
+  static DeviceOnce attr;
+  cudaError_t e = raise_smem_carveout(attr, correlate_seg_kernel<N, W, KC, PHASE>, sm);
   if (e != cudaSuccess) return e;
-  if (per_sm < 1) per_sm = 1;
+  int per_sm = 0;
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, correlate_seg_kernel<N, W, KC, PHASE>, C::NT, sm);
+  if (e != cudaSuccess) return e;
+  if (per_sm < 1) return cudaErrorLaunchOutOfResources;
   const int64_t units = (a.njobs + C::WIN - 1) / C::WIN;
   int64_t grid = (int64_t)per_sm * num_sms;
   if (grid > units) grid = units;

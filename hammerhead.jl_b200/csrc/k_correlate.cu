@@ -1,6 +1,7 @@
 // Launches of the window correlation: the dispatch to the fused kernels (one
 // translation unit per FFT size, k_corr_<N>.cu), the general-shape kernel,
 // the analysis of caller-supplied planes and the peak epilogue.
+#include "hh_attr.h"
 #include "hh_corr_peaks.cuh"
 
 namespace hh {

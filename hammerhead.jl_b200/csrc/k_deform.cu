@@ -19,6 +19,7 @@
 #include <math.h>
 #include <stdint.h>
 
+#include "hh_attr.h"
 #include "hh_batch.h"
 #include "hh_internal.h"
 #include "hh_pred.cuh"
@@ -613,27 +614,20 @@ __global__ void __launch_bounds__(32 * BSC_WARPS) bspline_row_tiles_kernel(PrefF
 }
 
 static cudaError_t set_tile_smem() {
-  static bool done = false;
-  if (done) return cudaSuccess;
-  for (cudaError_t e : {cudaFuncSetAttribute(b_bspline_col_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)BSC_SMEM),
-                        cudaFuncSetAttribute(b_bspline_col_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)BSC_SMEM),
-                        cudaFuncSetAttribute(b_bspline_row_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)BSC_SMEM),
-                        cudaFuncSetAttribute(b_bspline_row_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)BSC_SMEM),
-                        cudaFuncSetAttribute(bspline_col_tiles_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)BSC_SMEM),
-                        cudaFuncSetAttribute(bspline_col_tiles_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)BSC_SMEM),
-                        cudaFuncSetAttribute(bspline_row_tiles_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)BSC_SMEM),
-                        cudaFuncSetAttribute(bspline_row_tiles_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)BSC_SMEM)})
-    if (e != cudaSuccess) return e;
-  done = true;
-  return cudaSuccess;
+  static DeviceOnce done;
+  return done([] {
+    const auto limit = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    for (cudaError_t e : {cudaFuncSetAttribute(b_bspline_col_kernel<0>, limit, (int)BSC_SMEM),
+                          cudaFuncSetAttribute(b_bspline_col_kernel<1>, limit, (int)BSC_SMEM),
+                          cudaFuncSetAttribute(b_bspline_row_kernel<0>, limit, (int)BSC_SMEM),
+                          cudaFuncSetAttribute(b_bspline_row_kernel<1>, limit, (int)BSC_SMEM),
+                          cudaFuncSetAttribute(bspline_col_tiles_kernel<0>, limit, (int)BSC_SMEM),
+                          cudaFuncSetAttribute(bspline_col_tiles_kernel<1>, limit, (int)BSC_SMEM),
+                          cudaFuncSetAttribute(bspline_row_tiles_kernel<0>, limit, (int)BSC_SMEM),
+                          cudaFuncSetAttribute(bspline_row_tiles_kernel<1>, limit, (int)BSC_SMEM)})
+      if (e != cudaSuccess) return e;
+    return cudaSuccess;
+  });
 }
 
 static unsigned tile_blocks(int64_t witems) {

@@ -911,7 +911,7 @@ template <int W> static cudaError_t launch_uq_warp(const UQArgs& a, cudaStream_t
   int per_sm = 0;
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, uq_warp_kernel<W>, UQW_THREADS, sm);
   if (e != cudaSuccess) return e;
-  if (per_sm < 1) per_sm = 1;
+  if (per_sm < 1) return cudaErrorLaunchOutOfResources;
   int64_t grid = (int64_t)per_sm * num_sms;
   const int64_t units = (a.njobs + C::NWIN - 1) / C::NWIN;
   if (grid > units) grid = units;
@@ -932,7 +932,8 @@ cudaError_t launch_uq(const UQArgs& a, cudaStream_t s, int num_sms) {
       int per_sm = 0;
       e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, uq_general_kernel<true>, UQ_THREADS, sm);
       if (e != cudaSuccess) return e;
-      int64_t grid = (int64_t)(per_sm < 1 ? 1 : per_sm) * num_sms;
+      if (per_sm < 1) return cudaErrorLaunchOutOfResources;
+      int64_t grid = (int64_t)per_sm * num_sms;
       if (grid > a.njobs) grid = a.njobs;
       uq_general_kernel<true><<<(unsigned)grid, UQ_THREADS, sm, s>>>(a, offs);
       return cudaGetLastError();
@@ -964,7 +965,7 @@ cudaError_t launch_uq(const UQArgs& a, cudaStream_t s, int num_sms) {
   int per_sm = 0;
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, uq_kernel, UQ_THREADS, sm);
   if (e != cudaSuccess) return e;
-  if (per_sm < 1) per_sm = 1;
+  if (per_sm < 1) return cudaErrorLaunchOutOfResources;
   int64_t grid = (int64_t)per_sm * num_sms;
   if (grid > a.njobs) grid = a.njobs;
   uq_kernel<<<(unsigned)grid, UQ_THREADS, sm, s>>>(a, offs);

@@ -618,6 +618,7 @@ __device__ __forceinline__ void scan_rows(TK& tk, const float* R, int ldr, int K
           const uint16_t q = list[LANES + lane];
           __syncwarp(gm);
           list[lane] = q;
+          __syncwarp(gm);  // past the entries left, the next rows write these words again, by other lanes
           cnt -= LANES;
         }
       }

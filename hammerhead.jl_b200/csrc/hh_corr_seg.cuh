@@ -152,6 +152,7 @@ __device__ __forceinline__ void seg_scan_rows(TK& tk, const float* R, int K, con
           list[l] = q;
           cnt -= SEG;
         }
+        __syncwarp();  // past the entries left, the next rows write these words again, by other lanes
       }
     }
   }

@@ -133,9 +133,9 @@ template <int S, class T> __device__ __forceinline__ double median_net_d(T (&a)[
 
 // The slots of cell (r, c): bit s of near_present is set where neighbour s is
 // on the grid and neither flagged nor masked (either may be null). Slots off
-// the grid read the nearest cell on it, so that no load waits behind a branch:
-// a test per neighbour serialises the S loads of each array (1.5 ms for
-// the substitutions of the series below, against 1.2).
+// the grid read the flags of the nearest cell on it, so that no load waits
+// behind a branch: a test per neighbour serialises the S loads of each array
+// (1.5 ms for the substitutions of the series below, against 1.2).
 template <int NB> __device__ __forceinline__ bool near_on(int ny, int nx, int r, int c, int s, int64_t& q) {
   constexpr int D = 2 * NB + 1, S = D * D - 1;
   const int d = s < S / 2 ? s : s + 1;  // skip the centre of the D x D block
@@ -168,6 +168,17 @@ __device__ __forceinline__ uint32_t near_present(int ny, int nx, int r, int c, c
   }
   return on & ~off;
 }
+// *p where `on`, else +inf, as one predicated load: no branch between the loads
+// of a neighbourhood, and no read of a neighbour that does not count, which
+// another thread of the launch may be writing (a cell that counts keeps its
+// value throughout the launch, so the compiler may place the load freely)
+__device__ __forceinline__ float ld_present(const float* p, bool on) {
+  float v;
+  asm("{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %2, 0;\n\tmov.f32 %0, 0f7F800000;\n\t@p ld.global.f32 %0, [%1];\n\t}"
+      : "=f"(v)
+      : "l"(p), "r"((int)on));
+  return v;
+}
 template <int NB, int S>
 __device__ __forceinline__ void near_values(const float* f, int ny, int nx, int r, int c, uint32_t present,
                                             float (&x)[S]) {
@@ -176,10 +187,8 @@ __device__ __forceinline__ void near_values(const float* f, int ny, int nx, int 
   for (int s = 0; s < S; ++s) {
     int64_t q;
     near_on<NB>(ny, nx, r, c, s, q);
-    x[s] = f[q];
+    x[s] = ld_present(f + q, (present >> s) & 1u);
   }
-#pragma unroll
-  for (int s = 0; s < S; ++s) x[s] = (present >> s) & 1u ? x[s] : __int_as_float(0x7f800000);
 }
 
 template <int NB>

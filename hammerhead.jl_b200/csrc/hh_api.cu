@@ -97,7 +97,7 @@ hh_status run_schedule(hh_ctx* ctx, const float* dA, const float* dB, int64_t nr
     HH_TRY(get_tables(ctx, p, tb));
     // the predictor from the validated field of grid gf (build_predictor)
     auto build_pred = [&](const Grid& gf, bool keep) -> hh_status {
-      HH_K(HH_K_VECTOR, 1, 0, 24 * gf.G(), gf.G(),
+      HH_K(HH_K_VECTOR, hh::predictor_launches(gf.any_mask, smoothing, keep), 0, 24 * gf.G(), gf.G(),
            hh::launch_predictor(u, v, gf.any_mask ? gm : nullptr, gf.ny, gf.nx, smoothing, predw_u, predw_v, predu, predv,
                                 keep ? prevu : nullptr, keep ? prevv : nullptr, s));
       pred_src_u = smoothing ? predu : predw_u;

@@ -116,7 +116,7 @@ extern "C" hh_status hh_run_ensemble(hh_ctx* ctx, const hh_batch_pair* pairs, in
     HH_TRY(get_tables(ctx, p, tb));
     if (k > 0) {  // build_predictor from the previous pass's result (src/pipeline.jl:454-464)
       const Grid& pgd = grids[k - 1];
-      HH_K(HH_K_VECTOR, 1, 0, 24 * pgd.G(), pgd.G(),
+      HH_K(HH_K_VECTOR, hh::predictor_launches(pgd.any_mask, smoothing, false), 0, 24 * pgd.G(), pgd.G(),
            hh::launch_predictor(u, v, pgd.any_mask ? gm : nullptr, pgd.ny, pgd.nx, smoothing, predw_u, predw_v, predu, predv,
                                 nullptr, nullptr, s));
       pred_src_u = smoothing ? predu : predw_u;

@@ -173,6 +173,10 @@ cudaError_t launch_combine(float* u, float* v, const float* resu, const float* r
                            const NodePred& pr, float* meas_u, float* meas_v, cudaStream_t s);
 cudaError_t launch_flags(const float* u, const float* v, const float* ratio, const float* moment, int32_t ny, int32_t nx,
                          const FlagRules& r, const uint8_t* gmask, uint8_t* flags, uint8_t* flags2, cudaStream_t s);
+// kernels that launch_predictor launches: the fill, and the smoothing or the copy of the field
+constexpr int predictor_launches(bool masked, bool smoothing, bool keep) {
+  return (masked || !smoothing) + (smoothing || keep);
+}
 cudaError_t launch_predictor(const float* u, const float* v, const uint8_t* gmask, int32_t ny, int32_t nx, bool smoothing,
                              float* wu, float* wv, float* ou, float* ov, float* prev_u, float* prev_v, cudaStream_t s);
 cudaError_t launch_make_jobs(int32_t* jobs, int32_t ny, int32_t nx, const WinGrid& w, cudaStream_t s);

@@ -784,7 +784,7 @@ __global__ void __launch_bounds__(UQ_THREADS) uq_general_kernel(const UQArgs a, 
       const int64_t off = w0 + w.r + w.c * src.ld;
       const float va = src.A[off], vb = src.B[off];
       const bool mk = src.M ? src.M[off] != 0 : false;
-      wa[w.t] = mk ? __int_as_float(0x7fc00000) : va;  // NaN marks a masked pixel until the means are known
+      wa[w.t] = va;
       wb[w.t] = vb;
       if (!mk) {
         sa += (double)va;
@@ -809,11 +809,9 @@ __global__ void __launch_bounds__(UQ_THREADS) uq_general_kernel(const UQArgs a, 
     }
     const float ma = tn > 0 ? (float)(ta / tn) : 0.f, mb = tn > 0 ? (float)(tb / tn) : 0.f;
     for (Walk w(tid, UQ_THREADS, wr); w.t < n; w.next()) {
-      const int64_t off = w0 + w.r + w.c * src.ld;
-      const bool mk = src.M ? src.M[off] != 0 : false;
+      const bool mk = src.M ? src.M[w0 + w.r + w.c * src.ld] != 0 : false;
       const float ap = a.apod[w.t];
-      const float va = src.A[off];
-      wa[w.t] = mk ? 0.f : __fmul_rn(ap, __fsub_rn(va, ma));
+      wa[w.t] = mk ? 0.f : __fmul_rn(ap, __fsub_rn(wa[w.t], ma));
       wb[w.t] = mk ? 0.f : __fmul_rn(ap, __fsub_rn(wb[w.t], mb));
     }
     __syncthreads();

@@ -916,7 +916,6 @@ template <int N, int W> static cudaError_t launch_corr_nw(const CorrArgs& a, cud
 #define HH_CORR_SIZE(N)                                                                                       \
   cudaError_t launch_corr_##N(const CorrArgs& a, int W, cudaStream_t s, int num_sms) {                       \
     return W == N ? launch_corr_nw<N, N>(a, s, num_sms) : launch_corr_nw<N, N / 2>(a, s, num_sms);            \
-  }                                                                                                           \
-  size_t corr_smem_##N(int W) { return W == N ? CorrCfg<N, N>::smem() : CorrCfg<N, N / 2>::smem(); }
+  }
 
 }  // namespace hh

@@ -111,7 +111,6 @@ size_t gcorr_plane_smem(int nr, int nc, int box_rows, int box_cols, int threads)
 // than 24 stages.
 int gcorr_radix_plan(int n, int8_t* radix);
 size_t correlate_record_words(int npeaks);  // per job
-size_t correlate_smem_bytes(int N, int W);
 
 // Device peak analysis of caller-supplied planes.
 struct AnalyzeArgs {

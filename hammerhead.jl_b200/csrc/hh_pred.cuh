@@ -23,16 +23,6 @@ __device__ __forceinline__ void lin_axis(float q, float q0, float step, int n, i
   d = FD(FS(q, k0), FS(k1, k0));
 }
 
-// the bilinear combination at cell (iy, ix) with fractions (dy, dx)
-__device__ __forceinline__ float bilinear_at(const float* f, const PredGrid& g, int iy, float dy, int ix, float dx) {
-  const int iy2 = g.gny == 1 ? iy : iy + 1, ix2 = g.gnx == 1 ? ix : ix + 1;
-  const float f00 = f[iy + ix * g.gny], f01 = f[iy + ix2 * g.gny], f10 = f[iy2 + ix * g.gny],
-              f11 = f[iy2 + ix2 * g.gny];
-  const float a = FA(FM(FS(1.f, dx), f00), FM(dx, f01));
-  const float b = FA(FM(FS(1.f, dx), f10), FM(dx, f11));
-  return FA(FM(FS(1.f, dy), a), FM(dy, b));
-}
-
 __device__ __forceinline__ float bilinear(const float* f, const PredGrid& g, float qy, float qx) {
   int iy, ix;
   float dy, dx;

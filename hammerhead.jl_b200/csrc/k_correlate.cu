@@ -104,9 +104,7 @@ size_t gcorr_plane_smem(int nr, int nc, int box_rows, int box_cols, int threads)
 size_t correlate_record_words(int npeaks) { return (size_t)rec_words(npeaks > 2 ? npeaks : 2); }
 
 #define HH_CORR_SIZES(X) X(16) X(24) X(32) X(48) X(64) X(96) X(128)
-#define X(n)                                                                         \
-  cudaError_t launch_corr_##n(const CorrArgs& a, int W, cudaStream_t s, int num_sms); \
-  size_t corr_smem_##n(int W);
+#define X(n) cudaError_t launch_corr_##n(const CorrArgs& a, int W, cudaStream_t s, int num_sms);
 HH_CORR_SIZES(X)
 #undef X
 
@@ -115,13 +113,6 @@ bool correlate_supported(int N, int W) {
   HH_CORR_SIZES(X)
 #undef X
   return false;
-}
-
-size_t correlate_smem_bytes(int N, int W) {
-#define X(n) if (N == n && (W == n || 2 * W == n)) return corr_smem_##n(W);
-  HH_CORR_SIZES(X)
-#undef X
-  return 0;
 }
 
 cudaError_t launch_correlate(const CorrArgs& a, int N, int W, cudaStream_t s, int num_sms) {

@@ -162,24 +162,37 @@ __device__ __forceinline__ double warp_sum_d(double v) {
   return v;
 }
 
-// Windows of a tile along one axis: as many as fit the side. 64 px (a tile's
-// deformed pixels, float2, take 33 KB) leave 6 CTAs per SM and, at 1024^2 with
-// 16 px windows, more CTAs than SMs, while a pixel is deformed 1.3 times on
-// average; sides of 96 px deform 1.2 times but leave one CTA per SM there
-// (53 us against 40 us). Windows above 32 px need the larger side to share.
-__host__ __device__ __forceinline__ int tile_windows(int W, int step) { return 1 + ((W <= 32 ? 64 : 96) - W) / step; }
-__host__ __device__ __forceinline__ int tile_side(int W, int step) { return W + (tile_windows(W, step) - 1) * step; }
-constexpr int NCC_SIDE = 96;  // the largest
-static size_t tile_smem(int W, int step) {
-  const size_t n = tile_side(W, step);
+// Windows of a tile along one axis: as many as fit the side, but at least
+// NCC_TILES tiles where the image has them. 64 px (a tile's deformed pixels,
+// float2, take 33 KB) leave 6 CTAs per SM and, at 1024^2 with 16 px windows,
+// more CTAs than SMs, while a pixel is deformed 1.3 times on average; sides of
+// 96 px deform 1.2 times but leave one CTA per SM there (53 us against 40 us).
+// Windows above 32 px need the larger side to share. On small images the
+// longest tiles leave a few CTAs with all the windows: loss alone with 13 px
+// windows at every pixel of 92 x 61, 2 tiles 465 us, 260 tiles 32, 3920 (a
+// window each) 59; 16 px at 50 % of 256^2, 25 tiles 45 us, 256 tiles 33; 512^2,
+// 81 tiles 44, 256 tiles 34. Above some 250 tiles the sides decide.
+constexpr int NCC_SIDE = 96;  // the longest
+constexpr int64_t NCC_TILES = 256;
+static int64_t tiles_of(const NccArgs& a, int TW) {
+  return (int64_t)((a.wy + TW - 1) / TW) * ((a.wx + TW - 1) / TW);
+}
+static int tile_windows(const NccArgs& a) {
+  int TW = 1 + ((a.W <= 32 ? 64 : NCC_SIDE) - a.W) / a.step;
+  while (TW > 1 && tiles_of(a, TW) < NCC_TILES) --TW;
+  return TW;
+}
+__host__ __device__ __forceinline__ int tile_side(int W, int step, int TW) { return W + (TW - 1) * step; }
+static size_t tile_smem(int W, int step, int TW) {
+  const size_t n = tile_side(W, step, TW);
   return n * (n + 1) * sizeof(float2) + 2 * n * sizeof(Cell) + NCC_THREADS / 32 * sizeof(double);
 }
 
 // 1. window constants: ncc, abar, bbar, inv = 1/sqrt(Saa Sbb), ca = ncc/Saa, cb = ncc/Sbb;
 //    and per CTA the sum of its ncc (after the constants of all windows)
-__global__ void __launch_bounds__(NCC_THREADS) ncc_tile_kernel(const NccArgs a) {
+__global__ void __launch_bounds__(NCC_THREADS) ncc_tile_kernel(const NccArgs a, int TW) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int W = a.W, n = W * W, TW = tile_windows(W, a.step), side = tile_side(W, a.step), ld = side + 1;
+  const int W = a.W, n = W * W, side = tile_side(W, a.step, TW), ld = side + 1;
   float2* T = reinterpret_cast<float2*>(smem_raw);  // column c of the tile at c * ld
   Cell* ry = reinterpret_cast<Cell*>(T + side * ld);
   Cell* cx = ry + side;
@@ -398,16 +411,15 @@ int64_t ncc_wstat_words(int32_t wy, int32_t wx) { return 7 * (int64_t)wy * wx; }
 
 cudaError_t launch_ncc_loss_grad(const NccArgs& a, cudaStream_t s) {
   if (a.wy < 1 || a.wx < 1 || a.W < 2 || a.W > 64 || a.step < 1) return cudaErrorInvalidValue;
-  const size_t sm = tile_smem(a.W, a.step);
   cudaError_t e = cudaFuncSetAttribute(ncc_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)(NCC_SIDE * (NCC_SIDE + 1) * sizeof(float2) + 4096));
   if (e != cudaSuccess) return e;
   auto blocks = [](int64_t n, int per) { return (n + per - 1) / per; };
-  const int TW = tile_windows(a.W, a.step);
-  const int64_t tiles = blocks(a.wy, TW) * blocks(a.wx, TW);
+  const int TW = tile_windows(a);
+  const int64_t tiles = tiles_of(a, TW);
   const int64_t px = blocks(a.nr, NCC_PR) * blocks(a.nc, NCC_PC), nodes = blocks(a.gny, NODE_R) * blocks(a.gnx, NODE_C);
   if (tiles > INT32_MAX || (a.grad && (px > INT32_MAX || nodes > INT32_MAX))) return cudaErrorInvalidValue;
-  ncc_tile_kernel<<<(unsigned)tiles, NCC_THREADS, sm, s>>>(a);
+  ncc_tile_kernel<<<(unsigned)tiles, NCC_THREADS, tile_smem(a.W, a.step, TW), s>>>(a, TW);
   ncc_loss_kernel<<<1, NCC_THREADS, 0, s>>>(a, tiles);
   if (a.grad) {
     ncc_pixel_kernel<<<(unsigned)px, NCC_PR, 0, s>>>(a);

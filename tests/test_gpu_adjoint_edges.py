@@ -63,3 +63,24 @@ def test_nan_node(hb, orc, ws):
     far[i - 1:i + 2, j - 1:j + 2] = False
     assert np.isnan(g[i, j]).all()
     assert np.linalg.norm((g - g64)[far]) <= 1e-3 * np.linalg.norm(g64[far])
+
+
+def test_small_image_with_many_windows(hb, ws):
+    """Some 3900 windows on 92 x 61 pixels share their tiles among as many CTAs
+    as on 256 x 256: no more than three times its time (two CTAs took ten)."""
+    import time
+
+    def loss_time(shape, overlap):
+        rng = np.random.default_rng(0)
+        A = rng.random(shape).astype(np.float32)
+        loss = hb.NCCLoss(A, A[::-1], window=13, overlap=overlap, workspace=ws)
+        P, grid = np.zeros((4, 4, 2), np.float32), (7.0, shape[0] / 5, 7.0, shape[1] / 5)
+        loss.value(P, grid)
+        times = []
+        for _ in range(20):
+            t = time.perf_counter()
+            loss.value(P, grid)
+            times.append(time.perf_counter() - t)
+        return min(times)
+
+    assert loss_time((92, 61), 12) <= 3 * loss_time((256, 256), 9)

@@ -394,7 +394,6 @@ static hh_status build_plan(hh_ctx* ctx, BPlan& P, const hh_batch_pair* pairs, i
         c.padding = pd.padding;
         c.pd = pd;
         c.special = corr_special(pd);
-        if (!c.special) HH_TRY(gcorr_setup(ctx, pd, c.gen));
         HH_TRY(get_tables(ctx, pd, c.tb));
         S.classes.push_back(std::move(c));
       }
@@ -413,7 +412,8 @@ static hh_status build_plan(hh_ctx* ctx, BPlan& P, const hh_batch_pair* pairs, i
     S.gtot = coff;
     S.dtot = dcoff;
     for (auto& c : S.classes) {
-      c.njobs = (int64_t)c.hjobs.size() / 4;
+      c.gen.njobs = c.njobs = (int64_t)c.hjobs.size() / 4;
+      if (!c.special) HH_TRY(gcorr_setup(ctx, c.pd, c.gen));
       void* d = nullptr;
       HH_CK(ctx_malloc(ctx, &d, std::max<size_t>(c.hjobs.size(), 1) * sizeof(int32_t)));
       c.jobs = static_cast<int32_t*>(d);

@@ -434,7 +434,7 @@ inline bool gcorr_shape_ok(const hh_pass_desc& p) {
 
 // Fill the general-shape fields of a correlation launch: shapes, radix
 // plans, twiddles, chunking and the scratch slice geometry (one slice per
-// CTA, as many as SMs); gcorr_prepare also points it at the context's
+// CTA) for ca.njobs windows; gcorr_prepare also points it at the context's
 // scratch buffer (grown on demand), a batched plan at its own.
 inline hh_status gcorr_setup(hh_ctx* ctx, const hh_pass_desc& p, CorrArgs& ca) {
   ca.wr = p.window[0];
@@ -485,10 +485,16 @@ inline hh_status gcorr_setup(hh_ctx* ctx, const hh_pass_desc& p, CorrArgs& ca) {
     break;
   }
   if (!per_sm) {
-    // Planes that fit no CTA's shared memory go to L2: 256 threads and two
-    // CTAs per SM while their line buffers fit twice, and the slices together
-    // stay within L2 (2.84 -> 2.30 ms for two sweeps of 256 x 256 planes at
-    // 2048^2); else one CTA of 512.
+    // Planes that fit no CTA's shared memory go to L2, one CTA of 512 threads
+    // per SM. Two CTAs of 256 cover each other's waits where both lengths are
+    // transformed in registers, the line buffers fit twice and the slices
+    // together stay within L2: with 4000 windows of 256 x 256 points 4.28
+    // against 4.64 ms, of 128 x 256 2.39 and 2.69; other lengths gain nothing
+    // (280 x 216, 880 windows: 4.24 and 4.28 ms; 122 x 122: 60.5 and 58.4). But
+    // a window takes 1.3 times as long on 256 threads even where it has the SM
+    // for itself, so a round of one window per SM is left to 512: at 256 x 256
+    // 148 windows 226 us on 256 threads and 176 on 512, 290: 324 and 342, 440:
+    // 627 and 508, 740: 932 and 842, 961: 1108 and 1171, 1036: 1237 and 1175.
     auto shape = [&](int threads) {
       const int warps = threads / 32;
       ca.gc_threads = threads;
@@ -500,8 +506,10 @@ inline hh_status gcorr_setup(hh_ctx* ctx, const hh_pass_desc& p, CorrArgs& ca) {
       ca.gc_smem_bytes = ca.gc_smem_lines + hh::gcorr_smem_extra(warps);
       return (size_t)ca.gc_smem_bytes;
     };
+    const int64_t sms = ctx->num_sms, last = ca.njobs % (2 * sms);  // windows of the last round of two per SM
+    const bool single = ca.njobs <= sms || (ca.njobs <= 7 * sms && last > sms / 2 && last <= sms);
     per_sm = 2;
-    if (shape(256) > SM / 2 - CTA || 2 * ctx->num_sms * planes > (size_t)110 << 20) {
+    if (single || lpw == 1 || !gc_reg_length(ca.nfc) || shape(256) > SM / 2 - CTA || 2 * sms * planes > (size_t)110 << 20) {
       per_sm = 1;
       shape(512);
     }

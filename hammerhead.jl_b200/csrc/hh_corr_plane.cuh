@@ -96,28 +96,28 @@ __device__ __forceinline__ void pl_stage(const LineSet& L, int p, int nr, int ts
     }
   }
 }
-// the same for a run-time radix (11 and above): inputs read again per output
+// The same for a run-time radix (11 and above): an item per output, its inputs
+// read again. (An item per butterfly left 14 threads of a CTA with all of a 14 x
+// 41 plane's 41-point rows: 396 us for up to 440 windows, 76 to 85 now.)
 template <bool INV, class Get, class Put>
 __device__ __forceinline__ void pl_stage_any(const LineSet& L, int r, int p, int nr, int tstep, const float2* tw, int tid,
                                              int nt, const Get& get, const Put& put) {
-  for (int it = tid; it < L.n * nr; it += nt) {
-    int l, i;
-    L.item(it, l, i);
-    const int k = i % p, j0 = (i - k) * r + k;
-    for (int q = 0; q < r; ++q) {
-      float2 acc = make_float2(0.f, 0.f);
-      int e = 0;
-      for (int m = 0; m < r; ++m) {
-        float2 x = rounded(get(l, i + m * nr));
-        if (k && m) x = cmul_fixed<INV>(x, tw[m * k * tstep]);
-        if (e) x = cmul_fixed<INV>(x, tw[e * nr]);
-        acc.x += x.x;
-        acc.y += x.y;
-        e += q;
-        if (e >= r) e -= r;
-      }
-      put(l, j0 + q * p, acc);
+  for (int it = tid; it < L.n * nr * r; it += nt) {
+    int l, iq;
+    L.item(it, l, iq);
+    const int q = iq / nr, i = iq - q * nr, k = i % p, j0 = (i - k) * r + k;
+    float2 acc = make_float2(0.f, 0.f);
+    int e = 0;
+    for (int m = 0; m < r; ++m) {
+      float2 x = rounded(get(l, i + m * nr));
+      if (k && m) x = cmul_fixed<INV>(x, tw[m * k * tstep]);
+      if (e) x = cmul_fixed<INV>(x, tw[e * nr]);
+      acc.x += x.x;
+      acc.y += x.y;
+      e += q;
+      if (e >= r) e -= r;
     }
+    put(l, j0 + q * p, acc);
   }
 }
 

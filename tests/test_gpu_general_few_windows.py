@@ -53,3 +53,30 @@ def test_same_results_in_any_number(hb, ws, window, padding):
     many = d.process_windows(p, np.concatenate([jobs] * (300 // len(jobs) + 1)), want_locs=True)[:2]
     for a, b in zip(few, many):
         np.testing.assert_array_equal(a, b[: len(jobs)])
+
+
+def test_time_of_a_prime_length(hb, ws):
+    """Rows of 41 points against rows of 40: the 41 outputs of each are dealt over
+    the CTA's threads, so the direct sums cost a few times the transform of 40
+    points, not sixteen times."""
+    from hammerhead_b200 import _lib, hooks
+
+    A, B = np.random.default_rng(4).random((2, 300, 300)).astype(np.float32)
+    L, prof = _lib.lib(), (_lib.hh_kernel_profile * 5)()
+    d = hooks.DeviceSession(ws)
+    d.stage_pair(A, B)
+    L.hh_set_profiling(ws.ctx, 1)
+    ms = []
+    try:
+        for cols in (40, 41):
+            p = hb.PIVParameters(window_size=(14, cols), overlap=(7, 20))
+            jobs, best = hb.pass_grid(A.shape, p)[3][:100], 1e9
+            for _ in range(6):
+                _lib.check(L.hh_profile_read(ws.ctx, prof, 1), ws.ctx)
+                d.process_windows(p, jobs)
+                _lib.check(L.hh_profile_read(ws.ctx, prof, 1), ws.ctx)
+                best = min(best, prof[0].ms)
+            ms.append(best)
+    finally:
+        L.hh_set_profiling(ws.ctx, 0)
+    assert ms[1] <= 6 * ms[0], ms

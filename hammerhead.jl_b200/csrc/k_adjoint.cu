@@ -268,21 +268,26 @@ __global__ void __launch_bounds__(NCC_THREADS) ncc_tile_kernel(const NccArgs a, 
 }
 
 // 2. pixel displacement gradient (gu, gv) = dL/d(u, v) at every pixel: a
-//    thread keeps its row and walks NCC_PC columns, so what belongs to a row
-//    (predictor cell, windows that hold it) or to a column is formed once
-constexpr int NCC_PR = 128, NCC_PC = 8;
+//    thread keeps its row and walks PC columns, so what belongs to a row
+//    (predictor cell, windows that hold it) or to a column is formed once.
+//    PC = 8 columns where that leaves NCC_PBLOCKS CTAs, fewer on small images,
+//    whose threads would be too few: loss and gradient with 49 px windows at
+//    every pixel of 86 x 76, 8 columns (10 CTAs) 393 us, one 110; 16 px windows
+//    at every pixel of 76 x 71 181 and 65 us; 16 px at 50 % of 256^2 52 and 51.
+constexpr int NCC_PR = 128, NCC_PC = 8;  // NCC_PC: the most columns of a thread
+constexpr int64_t NCC_PBLOCKS = 296;
 struct Span {
   int j0, j1;  // windows j0..j1 hold the row or column
 };
 __device__ __forceinline__ Span span_at(int64_t p, int W, int step, int nw) {
   return Span{p < W ? 0 : (int)((p - W) / step + 1), min(nw - 1, (int)(p / step))};
 }
-__global__ void __launch_bounds__(NCC_PR) ncc_pixel_kernel(const NccArgs a) {
+__global__ void __launch_bounds__(NCC_PR) ncc_pixel_kernel(const NccArgs a, int PC) {
   __shared__ Cell cx[NCC_PC];
   __shared__ Span cw[NCC_PC];
   const Block b = block_of((a.nr + NCC_PR - 1) / NCC_PR);
-  const int64_t P = a.nr * a.nc, r = (int64_t)b.x * NCC_PR + threadIdx.x, c0 = (int64_t)b.y * NCC_PC;
-  const int nc = (int)min((int64_t)NCC_PC, a.nc - c0);
+  const int64_t P = a.nr * a.nc, r = (int64_t)b.x * NCC_PR + threadIdx.x, c0 = (int64_t)b.y * PC;
+  const int nc = (int)min((int64_t)PC, a.nc - c0);
   if (threadIdx.x < nc) {
     cx[threadIdx.x] = cell_at((float)(c0 + threadIdx.x + 1), a.x0, a.xsp, a.gnx);
     cw[threadIdx.x] = span_at(c0 + threadIdx.x, a.W, a.step, a.wx);
@@ -417,12 +422,14 @@ cudaError_t launch_ncc_loss_grad(const NccArgs& a, cudaStream_t s) {
   auto blocks = [](int64_t n, int per) { return (n + per - 1) / per; };
   const int TW = tile_windows(a);
   const int64_t tiles = tiles_of(a, TW);
-  const int64_t px = blocks(a.nr, NCC_PR) * blocks(a.nc, NCC_PC), nodes = blocks(a.gny, NODE_R) * blocks(a.gnx, NODE_C);
+  int PC = NCC_PC;
+  while (PC > 1 && blocks(a.nr, NCC_PR) * blocks(a.nc, PC) < NCC_PBLOCKS) PC /= 2;
+  const int64_t px = blocks(a.nr, NCC_PR) * blocks(a.nc, PC), nodes = blocks(a.gny, NODE_R) * blocks(a.gnx, NODE_C);
   if (tiles > INT32_MAX || (a.grad && (px > INT32_MAX || nodes > INT32_MAX))) return cudaErrorInvalidValue;
   ncc_tile_kernel<<<(unsigned)tiles, NCC_THREADS, tile_smem(a.W, a.step, TW), s>>>(a, TW);
   ncc_loss_kernel<<<1, NCC_THREADS, 0, s>>>(a, tiles);
   if (a.grad) {
-    ncc_pixel_kernel<<<(unsigned)px, NCC_PR, 0, s>>>(a);
+    ncc_pixel_kernel<<<(unsigned)px, NCC_PR, 0, s>>>(a, PC);
     ncc_node_kernel<<<(unsigned)nodes, NODE_THREADS, 0, s>>>(a);
   }
   return cudaGetLastError();

@@ -65,22 +65,37 @@ def test_nan_node(hb, orc, ws):
     assert np.linalg.norm((g - g64)[far]) <= 1e-3 * np.linalg.norm(g64[far])
 
 
+def _least_time(call):
+    import time
+
+    call()
+    times = []
+    for _ in range(20):
+        t = time.perf_counter()
+        call()
+        times.append(time.perf_counter() - t)
+    return min(times)
+
+
 def test_small_image_with_many_windows(hb, ws):
     """Some 3900 windows on 92 x 61 pixels share their tiles among as many CTAs
     as on 256 x 256: no more than three times its time (two CTAs took ten)."""
-    import time
-
     def loss_time(shape, overlap):
         rng = np.random.default_rng(0)
         A = rng.random(shape).astype(np.float32)
         loss = hb.NCCLoss(A, A[::-1], window=13, overlap=overlap, workspace=ws)
         P, grid = np.zeros((4, 4, 2), np.float32), (7.0, shape[0] / 5, 7.0, shape[1] / 5)
-        loss.value(P, grid)
-        times = []
-        for _ in range(20):
-            t = time.perf_counter()
-            loss.value(P, grid)
-            times.append(time.perf_counter() - t)
-        return min(times)
+        return _least_time(lambda: loss.value(P, grid))
 
     assert loss_time((92, 61), 12) <= 3 * loss_time((256, 256), 9)
+
+
+def test_small_image_gradient(hb, ws):
+    """A small image's pixels are dealt over enough threads: with 49 px windows at
+    every pixel, loss and gradient take no more than five times the loss (8 columns
+    a thread took nine)."""
+    rng = np.random.default_rng(0)
+    A = rng.random((86, 76)).astype(np.float32)
+    loss = hb.NCCLoss(A, A[::-1], window=49, overlap=48, workspace=ws)
+    P, grid = np.zeros((20, 20, 2), np.float32), (4.0, 4.0, 4.0, 3.5)
+    assert _least_time(lambda: loss.value_and_grad(P, grid)) <= 5 * _least_time(lambda: loss.value(P, grid))

@@ -114,7 +114,10 @@ template <int N, int W, bool SRCH = false, int VAR = 0> struct CorrCfg {
   static constexpr int NZ1 = PADDED ? (W / N2) : N1;  // nonzero inputs of a forward pass-A line
 
   static constexpr int EPT = (W * W + G - 1) / G;             // window pixels per thread
-  static constexpr bool VIA = !SRCH && EPT > 16;  // pixels wait in the plane for their mean, not in registers
+  // pixels wait in the plane for their mean, not in registers, where they would
+  // spill: search areas of 96 px 558 -> 446 us for 2500 windows, 64 px 166 -> 132,
+  // 48 px (phase) 228 -> 168; the 18 pixels of a 24 px area do better in registers
+  static constexpr bool VIA = EPT > (SRCH ? 18 : 16);
   static constexpr int NPART = SRCH ? 4 : 3;  // FP64 partial sums per warp: A, B, count (and count of B)
   // plane stride in float2; the two windows of a half-warp pair start 16
   // banks apart, so their 32-bit plane accesses (peak scan, real-plane
@@ -258,26 +261,34 @@ __global__ void __launch_bounds__(CorrCfg<N, W, SRCH, VAR>::NT, CorrCfg<N, W, SR
       // apodization; a masked pixel is zero in both and leaves both means
       const int wa = a.win, oa = (W - wa) / 2;
       const int64_t r0 = rs - oa, c0 = cs - oa;
-      float2 z[EPT];
-      bool mk[EPT];
-#pragma unroll
-      for (int i = 0; i < EPT; ++i) {
-        const int e = gt + i * G, p = e % W, q = e / W;
-        const bool in = W * W % G == 0 || e < W * W;
-        const bool ina = (unsigned)(p - oa) < (unsigned)wa && (unsigned)(q - oa) < (unsigned)wa;
-        const int64_t off = (r0 + p) + (c0 + q) * ld;
-        z[i] = make_float2(ld_stream_if(A + off, in && ina), ld_stream_if(B + off, in));
-        mk[i] = !in || ld_stream_if(M + off, in && M) != 0;
-      }
+      // VIA: pixels in batches of LB, stored raw until the means are known
+      constexpr int LB = C::VIA ? 8 : EPT;
+      float2 z[LB];
+      bool mk[EPT];  // masked, or past the area
       double sa = 0.0, sb = 0.0, na = 0.0, nb = 0.0;
 #pragma unroll
-      for (int i = 0; i < EPT; ++i) {
-        const int e = gt + i * G, p = e % W, q = e / W;
-        const bool ina = (unsigned)(p - oa) < (unsigned)wa && (unsigned)(q - oa) < (unsigned)wa;
-        sb += (double)(mk[i] ? 0.f : z[i].y);
-        sa += (double)(mk[i] ? 0.f : z[i].x);  // 0 outside the window
-        nb += mk[i] ? 0.0 : 1.0;
-        na += mk[i] || !ina ? 0.0 : 1.0;
+      for (int i0 = 0; i0 < EPT; i0 += LB) {
+#pragma unroll
+        for (int i = 0; i < LB; ++i) {
+          const int e = gt + (i0 + i) * G, p = e % W, q = e / W;
+          const bool in = W * W % (G * LB) == 0 || e < W * W;
+          const bool ina = (unsigned)(p - oa) < (unsigned)wa && (unsigned)(q - oa) < (unsigned)wa;
+          const int64_t off = (r0 + p) + (c0 + q) * ld;
+          z[i] = make_float2(ld_stream_if(A + off, in && ina), ld_stream_if(B + off, in));
+          const bool m = !in || ld_stream_if(M + off, in && M) != 0;
+          if (i0 + i < EPT) mk[i0 + i] = m;
+        }
+#pragma unroll
+        for (int i = 0; i < LB && i0 + i < EPT; ++i) {
+          const int e = gt + (i0 + i) * G, p = e % W, q = e / W;
+          const bool ina = (unsigned)(p - oa) < (unsigned)wa && (unsigned)(q - oa) < (unsigned)wa;
+          const bool m = mk[i0 + i];
+          sb += (double)(m ? 0.f : z[i].y);
+          sa += (double)(m ? 0.f : z[i].x);  // 0 outside the window
+          nb += m ? 0.0 : 1.0;
+          na += m || !ina ? 0.0 : 1.0;
+          if (C::VIA && (W * W % (G * LB) == 0 || e < W * W)) P[q * LD + p] = z[i];
+        }
       }
       const unsigned gm = grp_mask(G);
 #pragma unroll
@@ -312,10 +323,11 @@ __global__ void __launch_bounds__(CorrCfg<N, W, SRCH, VAR>::NT, CorrCfg<N, W, SR
         if (e < W * W) {
           const int p = e % W, q = e / W;
           const bool ina = (unsigned)(p - oa) < (unsigned)wa && (unsigned)(q - oa) < (unsigned)wa;
+          const float2 x = C::VIA ? P[q * LD + p] : z[i % LB];
           float2 v = make_float2(0.f, 0.f);
           if (!(mk[i] || bad)) {
-            v.y = z[i].y - mb;
-            if (ina) v.x = ld_keep(a.apod + (p - oa) + (q - oa) * wa) * (z[i].x - ma);
+            v.y = x.y - mb;
+            if (ina) v.x = ld_keep(a.apod + (p - oa) + (q - oa) * wa) * (x.x - ma);
           }
           P[q * LD + p] = v;
         }

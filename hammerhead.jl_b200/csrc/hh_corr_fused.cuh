@@ -908,10 +908,18 @@ template <int N, int W> static cudaError_t launch_corr_nw(const CorrArgs& a, cud
   // 16 and 32 points: several windows per warp (hh_corr_seg.cuh) for the
   // regional-maximum finder and the ensemble sums; the exclusion finder, which
   // ranks its peaks in place, keeps this file's kernel. ns per window on one
-  // 2048^2 pair, this kernel / that one: 8 px padded 2.8 / 1.0, 16 px padded
-  // 5.0 / 3.5, 16 px 4.0 / 2.3, 32 px 11.7 / 7.3.
-  if constexpr (N == 16 || N == 32)
-    if (a.variant == 0 && seg_serves(a)) return launch_seg<N, W>(a, s, num_sms);
+  // 2048^2 pair, this kernel / that one: 8 px padded 2.8 / 0.96, 16 px padded
+  // 4.5 / 3.3, 16 px 3.8 / 2.0, 32 px 8.6 / 6.6. While an SM holds all its
+  // windows at once, a warp each, this kernel is the faster one where the peaks
+  // are searched in the whole plane: us, this / that, 16 px 100 windows 24 / 34,
+  // 3000 33 / 34, 5000 42 / 36; 32 px, up to 4 peaks, 100 windows 25 / 28, 2368
+  // 35 / 36, 3000 42 / 38; with more peaks, whose lists take the registers, 100
+  // windows 41 / 62, 6000 79 / 82, 20000 226 / 214. (Padded windows, whose box
+  // is small, and planes without a search stay within 2 us of each other there.)
+  if constexpr (N == 16 || N == 32) {
+    const int from = W < N || a.accumulate ? 0 : (N == 16 ? 24 : (a.npeaks <= 4 ? 16 : 64));  // windows per SM
+    if (a.variant == 0 && seg_serves(a) && a.njobs > (int64_t)from * num_sms) return launch_seg<N, W>(a, s, num_sms);
+  }
   switch (a.variant) {
     case 1: return launch_nw<N, W, false, 1>(a, s, num_sms);
     case 2: return launch_nw<N, W, false, 2>(a, s, num_sms);

@@ -32,6 +32,8 @@ struct BClass {
 
 struct BSlot {
   int64_t gtot = 0, ptot = 0, dtot = 0;  // cells, and pixels and strips that deform
+  bool dwrap = false;                    // the strips' form and columns
+  int dcols = 1;
   int max_maxit = 0;
   bool any_nalt = false, any_replace = false, any_tol = false, any_keep = false, any_next = false;
   bool any_deform = false, any_pred0 = false;
@@ -290,6 +292,14 @@ static hh_status build_plan(hh_ctx* ctx, BPlan& P, const hh_batch_pair* pairs, i
     BSlot& S = P.slots[k];
     std::map<std::tuple<int, int, int, int, int, int, int, int, int, int, int, int>, int> cls;
     int64_t coff = 0, dcoff = 0;
+    // one form for the launch: a lane per row slot if an image asks for it
+    for (int p = 0; p < npairs; ++p) S.dwrap |= deforms[p] && k < P.npass[p] && hh::deform_wraps(pairs[p].nr);
+    S.dcols = hh::deform_cols([&](int n) {
+      int64_t strips = 0;
+      for (int p = 0; p < npairs; ++p)
+        if (deforms[p] && k < P.npass[p]) strips += hh::deform_strips(S.dwrap, pairs[p].nr, pairs[p].nc, n);
+      return strips;
+    });
     for (int p = 0; p < npairs; ++p) {
       const hh_batch_pair& q = pairs[p];
       const hh_pass_desc* ps = passes + so[P.sched[p]];
@@ -364,7 +374,7 @@ static hh_status build_plan(hh_ctx* ctx, BPlan& P, const hh_batch_pair* pairs, i
       const int64_t Gk = (int64_t)gr.ny * gr.nx;
       coff += Gk;
       if (deforms[p]) {
-        dcoff += hh::deform_strips(q.nr, q.nc);
+        dcoff += hh::deform_strips(S.dwrap, q.nr, q.nc, S.dcols);
         S.ptot += q.nr * q.nc;
       }
       S.max_maxit = std::max(S.max_maxit, (int)pd.max_iterations);
@@ -471,7 +481,7 @@ static hh_status issue(hh_ctx* ctx, BPlan& P) {
                                     P.d_slot_sweeps + (size_t)k * np, s));
       charge(HH_K_VECTOR, k, it, -1, 0);
       if (S.any_deform && (it > 1 || S.any_pred0)) {
-        HH_K(HH_K_DEFORM, 1, 120 * Ps, 16 * Ps, S.ptot, hh::launch_b_deform(T, np, P.d_done, it, S.dtot, pu, pv, s));
+        HH_K(HH_K_DEFORM, 1, 120 * Ps, 16 * Ps, S.ptot, hh::launch_b_deform(T, np, P.d_done, it, S.dtot, S.dwrap, S.dcols, pu, pv, s));
         charge(HH_K_DEFORM, k, it, -1, 0);
       }
       for (size_t ci = 0; ci < S.classes.size(); ++ci) {

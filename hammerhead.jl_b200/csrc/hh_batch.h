@@ -105,8 +105,8 @@ cudaError_t launch_b_prefilter(const BPair* bp, int npairs, int64_t qtot, int64_
 cudaError_t launch_b_sweep_begin(const BPair* bp, int npairs, const int32_t* done, int it, int64_t gtot,
                                  const float* pu, const float* pv, float* u, float* v, float* uncu, float* uncv,
                                  int32_t* sweeps, int32_t* slot_sweeps, cudaStream_t s);
-cudaError_t launch_b_deform(const BPair* bp, int npairs, const int32_t* done, int it, int64_t stot, const float* pu,
-                            const float* pv, cudaStream_t s);
+cudaError_t launch_b_deform(const BPair* bp, int npairs, const int32_t* done, int it, int64_t stot, bool wrap, int cols,
+                            const float* pu, const float* pv, cudaStream_t s);
 struct BGrid {  // concatenated grid arrays, indexed by goff + cell
   float *u, *v, *resu, *resv, *ratio, *moment, *alt_u, *alt_v, *meas_u, *meas_v;
   float *prev_u, *prev_v, *predw_u, *predw_v, *pred_u, *pred_v, *unc_u, *unc_v;

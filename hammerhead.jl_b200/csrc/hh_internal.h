@@ -3,6 +3,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <functional>
+
 #include "hammerhead_b200.h"
 
 namespace hh {
@@ -140,7 +142,11 @@ struct PredGrid {
   int32_t gny, gnx;
   float y0, ysp, x0, xsp;
 };
-int64_t deform_strips(int64_t nr, int64_t nc);  // warps' work items of a deformation
+// a deformation's form for images of nr rows, its warps' work items in strips of
+// `cols` columns, and how many columns a launch takes whose strips they give
+bool deform_wraps(int64_t nr);
+int64_t deform_strips(bool wrap, int64_t nr, int64_t nc, int cols);
+int deform_cols(const std::function<int64_t(int)>& strips);
 cudaError_t launch_deform(const float* CA, const float* CB, int64_t nr, int64_t nc, const float* pu,
                           const float* pv, PredGrid g, float* wA, float* wB, cudaStream_t s);
 cudaError_t launch_node_values(const float* pu, const float* pv, PredGrid g, const float* y, int32_t ny,

@@ -129,11 +129,15 @@ __device__ __forceinline__ int spline_cell(float q, int n, bool& in) {
   return min(__float2int_rd(fminf(fmaxf(q, 1.f), (float)n)), n - 1);
 }
 
-// One warp deforms both frames on DEF_ROWS rows from row r0 and the columns
-// [c0, c1): a lane per row, stepping along the columns, so that every load and
-// store of the warp runs down one column. The predictor's cell and fraction are
-// formed once per row and, a lane each, once per column; its corner values are
-// loaded where the columns enter a new cell.
+// One warp deforms both frames on a strip of 32 rows and `cols` columns: a lane
+// per row, stepping along the columns, so that every load and store of the warp
+// runs down one column. The predictor's cell and fraction are formed once per row
+// and, a lane each, once per column; its corner values are loaded where the
+// columns enter a new cell.
+// WRAP, for images whose last strip of rows would leave more than a fifth of the
+// lanes idle: a lane takes a row slot, the rows of one block of `cols` columns
+// followed by those of the next. A warp then has two blocks where it passes from
+// one to the next, or several if the image has fewer than 32 rows.
 //
 // What bounds it: the latency of a column's chain (coordinates, 32 loads, the
 // sums) at 24 warps per SM, then instructions issued (61 % of the slots): a
@@ -142,31 +146,64 @@ __device__ __forceinline__ int spline_cell(float q, int n, bool& in) {
 // instructions in packed form. 2048 x 2048: a thread per pixel with its own
 // divisions and 64-bit indices took 79 us; four rows per thread, whose loads
 // touch four lines each, 70; this takes 52. Strips of 8 columns: 16 and 32 are
-// as fast there (51, 59 us) but leave too few warps at 512 x 512 (8, 13, 24
-// us); 64 registers for 32 warps per SM spill and gain nothing (51 us).
-constexpr int DEF_ROWS = 32, DEF_COLS = 8;  // DEF_COLS <= 32: a lane per column
+// as fast there (51, 59 us); 64 registers for 32 warps per SM spill and gain
+// nothing (51 us). Images with fewer than DEF_STRIPS strips take fewer columns,
+// since a strip's columns are one chain: 100 x 100 12.5 us with 8 columns, 6.9
+// with one; 512 x 512 10.8, 9.7 with 4; 768 x 1024 16.6, 19.0 with 4 (a pixel's
+// share of the cells grows). WRAP: 12 x 36000 20.6 -> 17.0 us, 33 x 33000 30.8 ->
+// 26.9; 2048 x 2048 would take 54.3 instead of 52.2.
+constexpr int DEF_COLS = 8;  // the most columns of a strip
+constexpr int64_t DEF_STRIPS = 148 * 10;
+__host__ __device__ static inline int64_t def_row_strips(int64_t nr) { return (nr + 31) / 32; }
+// columns per strip of an image of nr rows where the launch asks for cols: with
+// WRAP a strip's columns fit the lanes that form their cells (at most 31 / nr + 2
+// blocks)
+__host__ __device__ static inline int def_cols(bool wrap, int64_t nr, int cols) {
+  while (wrap && cols > 1 && (31 / nr + 2) * cols > 32) cols /= 2;
+  return cols;
+}
+__host__ __device__ static inline int64_t def_strips(bool wrap, int64_t nr, int64_t nc, int cols) {
+  const int n = def_cols(wrap, nr, cols);
+  const int64_t blocks = (nc + n - 1) / n;
+  return wrap ? (nr * blocks + 31) / 32 : def_row_strips(nr) * blocks;
+}
+template <bool WRAP>
 __device__ __forceinline__ void deform_strip(const float* __restrict__ CA, const float* __restrict__ CB, int nr, int nc,
                                              const float* __restrict__ pu, const float* __restrict__ pv,
-                                             const PredGrid& g, float* __restrict__ wA, float* __restrict__ wB, int r0,
-                                             int c0, int c1, float minus_zero) {
+                                             const PredGrid& g, float* __restrict__ wA, float* __restrict__ wB,
+                                             int64_t strip, int cols, float minus_zero) {
   const Mul2 mul2{both(minus_zero)};
   const int lane = threadIdx.x & 31;
-  const int r = min(r0 + lane, nr - 1);
-  const bool store = r0 + lane < nr;
   const int64_t ld = (int64_t)nr + 2;
+  int r, c00, c0, c1;  // row; the strip's first column, and this lane's columns [c0, c1)
+  bool store = true;
+  if (WRAP) {
+    const int b0 = (int)(strip * 32 / nr), v = (int)(strip * 32 - (int64_t)b0 * nr) + lane;
+    r = v % nr;
+    c00 = b0 * cols;
+    c0 = c00 + v / nr * cols;
+    c1 = c0 + cols;
+  } else {
+    const int64_t rs = def_row_strips(nr);
+    const int rl = (int)(strip % rs) * 32 + lane;
+    r = min(rl, nr - 1);
+    store = rl < nr;
+    c00 = c0 = (int)(strip / rs) * cols;
+    c1 = min(c0 + cols, nc);
+  }
   const float R = (float)(r + 1);
   int iy, ixl;
   float dy, dxl;
   lin_axis(R, g.y0, g.ysp, g.gny, iy, dy);
-  lin_axis((float)(min(c0 + lane, nc - 1) + 1), g.x0, g.xsp, g.gnx, ixl, dxl);
+  lin_axis((float)(min(c00 + lane, nc - 1) + 1), g.x0, g.xsp, g.gnx, ixl, dxl);
   const int iy2 = g.gny == 1 ? iy : iy + 1;
   const F2 dy2 = both(dy), ey2 = both(FS(1.f, dy)), half = both(0.5f);
   F2 f00 = both(0.f), f01 = f00, f10 = f00, f11 = f00;
   int held = -1;
-  for (int c = c0; c < c1; ++c) {
-    const int ix = __shfl_sync(0xffffffffu, ixl, c - c0);
-    const float dx = __shfl_sync(0xffffffffu, dxl, c - c0);
-    if (ix != held) {  // uniform
+  for (int c = c0; c < c1; ++c) {  // as many for every lane
+    const int ix = __shfl_sync(0xffffffffu, ixl, c - c00);
+    const float dx = __shfl_sync(0xffffffffu, dxl, c - c00);
+    if (ix != held) {  // uniform, with WRAP within a block
       held = ix;
       const int64_t q0 = (int64_t)ix * g.gny, q1 = (int64_t)(g.gnx == 1 ? ix : ix + 1) * g.gny;
       f00 = pk(pu[iy + q0], pv[iy + q0]);
@@ -201,7 +238,7 @@ __device__ __forceinline__ void deform_strip(const float* __restrict__ CA, const
     for (int i = 1; i < 4; ++i) s = add2(s, mul2(wy[i], t[i]));
     float sa, sb;
     unpk(s, sa, sb);
-    if (store) {
+    if (WRAP ? c < nc : store) {
       const int64_t k = r + (int64_t)c * nr;
       wA[k] = inya && inxa ? sa : 0.f;
       wB[k] = inyb && inxb ? sb : 0.f;
@@ -209,30 +246,32 @@ __device__ __forceinline__ void deform_strip(const float* __restrict__ CA, const
   }
 }
 
-// strips of an image: DEF_ROWS rows (fastest) by DEF_COLS columns
-__host__ __device__ static inline int64_t def_row_strips(int64_t nr) { return (nr + DEF_ROWS - 1) / DEF_ROWS; }
-
+template <bool WRAP>
 __global__ void __launch_bounds__(256, 3) deform_kernel(const float* __restrict__ CA, const float* __restrict__ CB, int nr,
                                                      int nc, const float* __restrict__ pu,
                                                      const float* __restrict__ pv, PredGrid g, float* wA, float* wB,
-                                                        float minus_zero) {
-  const int64_t rs = def_row_strips(nr), total = rs * ((nc + DEF_COLS - 1) / DEF_COLS);
-  for (int64_t k = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; k < total; k += ((int64_t)gridDim.x * blockDim.x) >> 5) {
-    const int c0 = (int)(k / rs) * DEF_COLS;
-    deform_strip(CA, CB, nr, nc, pu, pv, g, wA, wB, (int)(k % rs) * DEF_ROWS, c0, min(c0 + DEF_COLS, nc), minus_zero);
-  }
+                                                        int cols, float minus_zero) {
+  const int64_t total = def_strips(WRAP, nr, nc, cols);
+  for (int64_t k = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; k < total; k += ((int64_t)gridDim.x * blockDim.x) >> 5)
+    deform_strip<WRAP>(CA, CB, nr, nc, pu, pv, g, wA, wB, k, def_cols(WRAP, nr, cols), minus_zero);
 }
 
-int64_t deform_strips(int64_t nr, int64_t nc) { return def_row_strips(nr) * ((nc + DEF_COLS - 1) / DEF_COLS); }
+bool deform_wraps(int64_t nr) { return 4 * 32 * def_row_strips(nr) > 5 * nr; }
+int64_t deform_strips(bool wrap, int64_t nr, int64_t nc, int cols) { return def_strips(wrap, nr, nc, cols); }
+int deform_cols(const std::function<int64_t(int)>& strips) {
+  int cols = DEF_COLS;
+  while (cols > 1 && strips(cols) < DEF_STRIPS) cols /= 2;
+  return cols;
+}
 
 cudaError_t launch_deform(const float* CA, const float* CB, int64_t nr, int64_t nc, const float* pu,
                           const float* pv, PredGrid g, float* wA, float* wB, cudaStream_t s) {
-  // a strip forms the predictor's axis cells once, so longer strips are
-  // cheaper; DEF_COLS columns leave a 1024 x 1024 image as many warps as the
-  // chip holds
-  int64_t blocks = (deform_strips(nr, nc) + 7) / 8;
+  const bool wrap = deform_wraps(nr);
+  const int cols = deform_cols([&](int n) { return def_strips(wrap, nr, nc, n); });
+  int64_t blocks = (def_strips(wrap, nr, nc, cols) + 7) / 8;
   if (blocks > 148 * 32) blocks = 148 * 32;
-  deform_kernel<<<(unsigned)blocks, 256, 0, s>>>(CA, CB, (int)nr, (int)nc, pu, pv, g, wA, wB, -0.0f);
+  if (wrap) deform_kernel<true><<<(unsigned)blocks, 256, 0, s>>>(CA, CB, (int)nr, (int)nc, pu, pv, g, wA, wB, cols, -0.0f);
+  else deform_kernel<false><<<(unsigned)blocks, 256, 0, s>>>(CA, CB, (int)nr, (int)nc, pu, pv, g, wA, wB, cols, -0.0f);
   return cudaGetLastError();
 }
 
@@ -734,24 +773,25 @@ cudaError_t launch_b_sweep_begin(const BPair* bp, int npairs, const int32_t* don
 
 // Strips (deform_strip) of every pair that deforms, a warp each; the pair of a
 // strip is looked up once.
+template <bool WRAP>
 __global__ void __launch_bounds__(256, 3) b_deform_kernel(const BPair* __restrict__ bp, int npairs,
-                                                       const int32_t* __restrict__ done, int it, int64_t stot,
+                                                       const int32_t* __restrict__ done, int it, int64_t stot, int cols,
                                                        const float* __restrict__ pu, const float* __restrict__ pv, float minus_zero) {
   for (int64_t k = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; k < stot; k += ((int64_t)gridDim.x * blockDim.x) >> 5) {
     const int p = bp_find<&BPair::dcoff>(bp, npairs, k);
     const BPair& b = bp[p];
     if (!bp_live(b, it, done, p) || !(it > 1 || b.has_pred0) || !b.deforms) continue;  // uniform across the warp
-    const int64_t l = k - b.dcoff, rs = def_row_strips(b.nr);
-    const int c0 = (int)(l / rs) * DEF_COLS;
-    deform_strip(b.coefA, b.coefB, (int)b.nr, (int)b.nc, pu + b.goff, pv + b.goff, b_pred_grid(b, it), b.warpA, b.warpB,
-                 (int)(l % rs) * DEF_ROWS, c0, min(c0 + DEF_COLS, (int)b.nc), minus_zero);
+    deform_strip<WRAP>(b.coefA, b.coefB, (int)b.nr, (int)b.nc, pu + b.goff, pv + b.goff, b_pred_grid(b, it), b.warpA, b.warpB,
+                       k - b.dcoff, def_cols(WRAP, b.nr, cols), minus_zero);
   }
 }
 
-cudaError_t launch_b_deform(const BPair* bp, int npairs, const int32_t* done, int it, int64_t stot, const float* pu,
-                            const float* pv, cudaStream_t s) {
+cudaError_t launch_b_deform(const BPair* bp, int npairs, const int32_t* done, int it, int64_t stot, bool wrap, int cols,
+                            const float* pu, const float* pv, cudaStream_t s) {
   if (stot <= 0) return cudaSuccess;
-  b_deform_kernel<<<b_blocks(stot * 32, 32), 256, 0, s>>>(bp, npairs, done, it, stot, pu, pv, -0.0f);
+  const unsigned blocks = b_blocks(stot * 32, 32);
+  if (wrap) b_deform_kernel<true><<<blocks, 256, 0, s>>>(bp, npairs, done, it, stot, cols, pu, pv, -0.0f);
+  else b_deform_kernel<false><<<blocks, 256, 0, s>>>(bp, npairs, done, it, stot, cols, pu, pv, -0.0f);
   return cudaGetLastError();
 }
 

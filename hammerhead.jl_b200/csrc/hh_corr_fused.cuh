@@ -914,10 +914,11 @@ template <int N, int W> static cudaError_t launch_corr_nw(const CorrArgs& a, cud
   // are searched in the whole plane: us, this / that, 16 px 100 windows 24 / 34,
   // 3000 33 / 34, 5000 42 / 36; 32 px, up to 4 peaks, 100 windows 25 / 28, 2368
   // 35 / 36, 3000 42 / 38; with more peaks, whose lists take the registers, 100
-  // windows 41 / 62, 6000 79 / 82, 20000 226 / 214. (Padded windows, whose box
-  // is small, and planes without a search stay within 2 us of each other there.)
+  // windows 41 / 62, 6000 79 / 82, 20000 226 / 214. Padded windows, whose box is
+  // small, stay within 2 us of each other there, and planes that are only summed
+  // too, but for 16 px (289 windows, 8 pairs 103 / 117 us, 1296 windows 128 / 120).
   if constexpr (N == 16 || N == 32) {
-    const int from = W < N || a.accumulate ? 0 : (N == 16 ? 24 : (a.npeaks <= 4 ? 16 : 64));  // windows per SM
+    const int from = W < N ? 0 : a.accumulate ? (N == 16 ? 6 : 0) : N == 16 ? 24 : a.npeaks <= 4 ? 16 : 64;  // windows per SM
     if (a.variant == 0 && seg_serves(a) && a.njobs > (int64_t)from * num_sms) return launch_seg<N, W>(a, s, num_sms);
   }
   switch (a.variant) {

@@ -42,7 +42,9 @@ namespace hh {
 // alternative shape with one CTA more. Variants 0-3 compute the same
 // arithmetic on another thread mapping or register allocation, so their
 // results are identical. Variant 4 splits each axis's DFT differently
-// (AxisSplitAlt), so its planes differ from variant 0's by rounding.
+// (AxisSplitAlt), so its planes differ from variant 0's by rounding. (At 16
+// and 32 points a launch of variant 0 with enough windows takes another kernel
+// with the same arithmetic: launch_corr_nw.)
 template <int N, int W, bool SRCH = false, int VAR = 0> struct CorrCfg {
   // variant 4: the alternative FFT split (AxisSplitAlt) in the default shape and budget
   static constexpr bool ALT = VAR == 4;
@@ -190,9 +192,9 @@ __global__ void __launch_bounds__(CorrCfg<N, W, SRCH, VAR>::NT, CorrCfg<N, W, SR
   // with the Gaussian apodization, where walking the column strips costs no
   // more (16.5 / 16.9 ns at 48 points, 28.0 / 27.6 at 64, 124 / 126 at 128)
   // and half-warp groups lose (5.6 / 10.1 ns at 32 points: the halves' loops
-  // run one after the other). Unpadded, strips / row maxima: 16.2 / 12.4 ns
-  // at 32 points, 38.2 / 31.2 at 48, 57.8 / 51.9 at 64, 168 / 121 at 96,
-  // 264 / 220 at 128.
+  // run one after the other). Unpadded, strips / row maxima: 8.8 / 7.0
+  // ns at 24 points, 11.4 / 8.8 at 32, 33.6 / 26.5 at 48, 42.9 / 33.9 at 64, 154 /
+  // 104 at 96, 223 / 176 at 128.
   constexpr bool ROWSCAN = W == N;
   constexpr int FN = ROWSCAN ? N : 0;
   // the peak scan's list, in the half of the plane that the real plane leaves
@@ -549,8 +551,9 @@ __global__ void __launch_bounds__(CorrCfg<N, W, SRCH, VAR>::NT, CorrCfg<N, W, SR
       // ga = 1 .. N1/2-1, and for ga = 0 and N1/2 (their own negations) a row
       // of each pair, the self-negated rows 0 and N/2 together. Rows -ra of
       // consecutive ra are consecutive too. A separate spectrum step read and
-      // wrote the whole plane once more: 12.8 ns per window at 48 points
-      // (padded) against 12.3; 64: 22.3 and 21.3; 96: 53.2 and 51.0; 128: 102 and 97.
+      // wrote the whole plane once more, 4 to 5 % of a padded window's time: 12.8
+      // ns at 48 points against 12.3; 64: 22.3 and 21.3; 96: 53.2 and 51.0; 128:
+      // 102 and 97 (11.7, 19.1, 49 and 93 with the later steps).
       constexpr int h2 = N2 / 2, HN = N1 / 2;
 #pragma unroll 1
       for (int it = gt; it < N * HN; it += G) {

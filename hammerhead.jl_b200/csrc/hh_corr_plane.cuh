@@ -12,7 +12,7 @@
 // stages of the same radices, and the 16 x B split for lengths 32, 64, 128 and
 // 256, ping-pong between two planes. The first inverse stage forms the
 // spectrum as it reads. CTAs have 128, 256 or 512 threads by the plane's size
-// (gcorr_setup), so 4 or 2 windows share an SM.
+// (gcorr_setup), up to 6, 2 or 1 of them to an SM.
 // Bound by issue: a warp per line left 12 of 32 lanes busy in a 48-point
 // radix-4 stage and 2 of 16 in the 16-point transforms of a 32-point line
 // (63 k warp instructions per 48 x 32 plane, 21 k now). 8001 windows of

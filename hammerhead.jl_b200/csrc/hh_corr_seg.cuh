@@ -23,9 +23,9 @@
 // the same bit for bit. The pixel loads of a batch carry no branch (the image
 // mask's bytes are gathered apart): with one per pixel the loads went out one
 // by one, and a third of a warp's time was the wait for them (32-point padded
-// windows 4.6 -> 3.5 ns, unpadded 12.1 -> 7.3). Bound by issue and latency
-// (half the issue slots used at 16 to 20 warps per SM; complex sums are packed
-// instructions, cadd2); times beside the dispatch in launch_corr_nw.
+// windows 4.6 -> 3.5 ns, unpadded 12.1 -> 7.3; 3.3 and 6.6 with packed complex
+// sums, cadd2). Bound by issue and latency (half the issue slots used at 16 to
+// 20 warps per SM); which launches take it, and their times, in launch_corr_nw.
 #pragma once
 #include "hh_attr.h"
 #include "hh_corr_peaks.cuh"

@@ -481,7 +481,8 @@ static hh_status issue(hh_ctx* ctx, BPlan& P) {
                                     P.d_slot_sweeps + (size_t)k * np, s));
       charge(HH_K_VECTOR, k, it, -1, 0);
       if (S.any_deform && (it > 1 || S.any_pred0)) {
-        HH_K(HH_K_DEFORM, 1, 120 * Ps, 16 * Ps, S.ptot, hh::launch_b_deform(T, np, P.d_done, it, S.dtot, S.dwrap, S.dcols, pu, pv, s));
+        HH_K(HH_K_DEFORM, 1, 120 * Ps, 16 * Ps, S.ptot,
+             hh::launch_b_deform(T, np, P.d_done, it, S.dtot, S.dwrap, S.dcols, pu, pv, s));
         charge(HH_K_DEFORM, k, it, -1, 0);
       }
       for (size_t ci = 0; ci < S.classes.size(); ++ci) {

@@ -35,7 +35,7 @@ struct BSlot {
   bool dwrap = false;                    // the strips' form and columns
   int dcols = 1;
   int max_maxit = 0;
-  bool any_nalt = false, any_replace = false, any_tol = false, any_keep = false, any_next = false;
+  bool any_near = false, any_wide = false, any_replace = false, any_tol = false, any_keep = false, any_next = false;
   bool any_deform = false, any_pred0 = false;
   std::vector<BClass> classes;
 };
@@ -378,7 +378,7 @@ static hh_status build_plan(hh_ctx* ctx, BPlan& P, const hh_batch_pair* pairs, i
         S.ptot += q.nr * q.nc;
       }
       S.max_maxit = std::max(S.max_maxit, (int)pd.max_iterations);
-      S.any_nalt |= b.nalt > 0;
+      (pd.uod_neighborhood > 2 ? S.any_wide : S.any_near) |= b.nalt > 0;  // substitutions by their neighbourhood
       S.any_replace |= b.replace != 0;
       S.any_tol |= pd.convergence_tol > 0 && pd.max_iterations > 2;
       S.any_keep |= b.keep_measured != 0;
@@ -542,10 +542,10 @@ static hh_status issue(hh_ctx* ctx, BPlan& P) {
           }
         }
       const bool fc = S.any_tol && it >= 2 && it < S.max_maxit;
-      const int nv = 2 + S.any_nalt + S.any_replace + fc;
+      const int nv = 2 + S.any_near + S.any_wide + S.any_replace + fc;
       HH_K(HH_K_VECTOR, nv, 0, 120 * Gs, S.gtot,
-           hh::launch_b_vector(T, np, P.d_done, it, S.gtot, g, S.any_nalt, S.any_replace, S.any_tol, S.max_maxit, s,
-                               nullptr));
+           hh::launch_b_vector(T, np, P.d_done, it, S.gtot, g, S.any_near, S.any_wide, S.any_replace, S.any_tol,
+                               S.max_maxit, s, nullptr));
       charge(HH_K_VECTOR, k, it, -1, 1);
       if (it < S.max_maxit) {
         HH_K(HH_K_VECTOR, P.smoothing ? 2 : 1, 0, 24 * Gs, S.gtot,

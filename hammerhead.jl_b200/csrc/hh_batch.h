@@ -114,7 +114,8 @@ struct BGrid {  // concatenated grid arrays, indexed by goff + cell
   uint32_t* keys;
 };
 cudaError_t launch_b_vector(const BPair* bp, int npairs, int32_t* done, int it, int64_t gtot, const BGrid& g,
-                            bool any_nalt, bool any_replace, bool any_tol, int max_maxit, cudaStream_t s, int* nlaunch);
+                            bool any_near, bool any_wide, bool any_replace, bool any_tol, int max_maxit, cudaStream_t s,
+                            int* nlaunch);
 cudaError_t launch_b_predictor(const BPair* bp, int npairs, const int32_t* done, int it, int mode, int64_t gtot,
                                const BGrid& g, bool smoothing, cudaStream_t s, int* nlaunch);
 cudaError_t launch_b_restore(const BPair* bp, int npairs, int64_t gtot, const BGrid& g, cudaStream_t s);

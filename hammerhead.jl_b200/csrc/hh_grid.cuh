@@ -300,6 +300,10 @@ __device__ __forceinline__ bool near_spread(const float* u, const float* v, int 
 // layers come from the register networks above, as in uod_cell: with indexed
 // arrays in local memory a flagged cell's insertion sorts hold its warp: 3.0
 // ms for the six sweeps of a sparsely seeded 4096 x 4096 series against 1.2.
+// WIDE: 3 and 4 layers (er), whose arrays stay in local memory. Kernels take one
+// form or the other: beside the networks' registers the wide one has a quarter of
+// its warps (500 x 400 cells, 3 layers: 926 us in one kernel, 683 by itself).
+template <bool WIDE>
 __device__ __forceinline__ uint8_t substitute_cell(float* u, float* v, const uint8_t* outl_in, const uint8_t* gmask,
                                                    const float* alt_u, const float* alt_v, int nalt, int ny, int nx,
                                                    int r, int c, int er, double thr) {
@@ -307,10 +311,12 @@ __device__ __forceinline__ uint8_t substitute_cell(float* u, float* v, const uin
   uint8_t o = outl_in[k];
   if (!o || (gmask && gmask[k])) return o;
   double mu, mv, madu, madv;
-  if (er == 1) {
-    if (!near_spread<1>(u, v, ny, nx, r, c, outl_in, gmask, mu, mv, madu, madv)) return o;
-  } else if (er == 2) {
-    if (!near_spread<2>(u, v, ny, nx, r, c, outl_in, gmask, mu, mv, madu, madv)) return o;
+  if constexpr (!WIDE) {
+    if (er == 1) {
+      if (!near_spread<1>(u, v, ny, nx, r, c, outl_in, gmask, mu, mv, madu, madv)) return o;
+    } else {
+      if (!near_spread<2>(u, v, ny, nx, r, c, outl_in, gmask, mu, mv, madu, madv)) return o;
+    }
   } else {
     double bu[UOD_MAXN], bv[UOD_MAXN], tu[UOD_MAXN], tv[UOD_MAXN];
     int n = 0;

@@ -97,15 +97,18 @@ __global__ void b_flags_kernel(const BPair* __restrict__ bp, int npairs, const i
   }
 }
 
-// secondary-peak substitution (src/quality.jl:307-351): outl -> outl2
-__global__ void __launch_bounds__(128, 3) b_substitute_kernel(const BPair* __restrict__ bp, int npairs, const int32_t* __restrict__ done, int it,
-                                    int64_t gtot, BGrid g) {
+// secondary-peak substitution (src/quality.jl:307-351): outl -> outl2, for the
+// pairs whose neighbourhoods have up to 2 layers, or more (WIDE)
+template <bool WIDE>
+__global__ void __launch_bounds__(128, WIDE ? 12 : 3)
+    b_substitute_kernel(const BPair* __restrict__ bp, int npairs, const int32_t* __restrict__ done, int it,
+                        int64_t gtot, BGrid g) {
   B_STRIDE(k, gtot) {
     B_CELL(k, p, b, l)
-    if (!bp_live(b, it, done, p) || b.nalt < 1) continue;
+    if (!bp_live(b, it, done, p) || b.nalt < 1 || (b.uod_nb > 2) != WIDE) continue;
     const int64_t o = b.goff;
     const int r = (int)(l % b.ny), c = (int)(l / b.ny);
-    g.outl2[o + l] = substitute_cell(g.u + o, g.v + o, g.outl + o, b.gmask, g.alt_u + b.aoff, g.alt_v + b.aoff,
+    g.outl2[o + l] = substitute_cell<WIDE>(g.u + o, g.v + o, g.outl + o, b.gmask, g.alt_u + b.aoff, g.alt_v + b.aoff,
                                      b.nalt, b.ny, b.nx, r, c, b.uod_nb, b.uod_thr);
   }
 }
@@ -145,14 +148,19 @@ __global__ void __cluster_dims__(FC_CLUSTER, 1, 1) __launch_bounds__(FC_THREADS)
 }
 
 cudaError_t launch_b_vector(const BPair* bp, int npairs, int32_t* done, int it, int64_t gtot, const BGrid& g,
-                            bool any_nalt, bool any_replace, bool any_tol, int max_maxit, cudaStream_t s, int* nlaunch) {
+                            bool any_near, bool any_wide, bool any_replace, bool any_tol, int max_maxit, cudaStream_t s,
+                            int* nlaunch) {
   if (gtot <= 0) return cudaSuccess;
   int n = 0;
   b_combine_kernel<<<bb_blocks(gtot, 256), 256, 0, s>>>(bp, npairs, done, it, gtot, g);
   b_flags_kernel<<<bb_blocks(gtot, 128), 128, 0, s>>>(bp, npairs, done, it, gtot, g);
   n += 2;
-  if (any_nalt) {
-    b_substitute_kernel<<<bb_blocks(gtot, 128), 128, 0, s>>>(bp, npairs, done, it, gtot, g);
+  if (any_near) {
+    b_substitute_kernel<false><<<bb_blocks(gtot, 128), 128, 0, s>>>(bp, npairs, done, it, gtot, g);
+    ++n;
+  }
+  if (any_wide) {
+    b_substitute_kernel<true><<<bb_blocks(gtot, 128), 128, 0, s>>>(bp, npairs, done, it, gtot, g);
     ++n;
   }
   if (any_replace) {

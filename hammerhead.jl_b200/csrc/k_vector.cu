@@ -81,16 +81,20 @@ cudaError_t launch_uod(const float* u, const float* v, int32_t ny, int32_t nx, d
 // apply_validator! src/quality.jl:466-486): the outlier detection, the peak
 // ratio and the extra validators; masked cells cleared. Written twice: the
 // snapshot that the substitution judges by, and the flags it updates.
-__global__ void flags_kernel(const float* u, const float* v, const float* ratio, const float* moment, int32_t ny,
+__global__ void __launch_bounds__(128, 4) flags_kernel(const float* u, const float* v, const float* ratio, const float* moment, int32_t ny,
                              int32_t nx, FlagRules r, const uint8_t* gmask, uint8_t* flags, uint8_t* flags2) {
   GRID_STRIDE(k, (int64_t)ny * nx) {
     uint8_t f = 0;
     if (!(gmask && gmask[k])) {
       const int gi = (int)(k % ny), gj = (int)(k / ny);
-      if (r.uod) f |= uod_cell(u, v, ny, nx, gi, gj, r.uod_thr, r.uod_nb, 0.1, gmask);
       if (r.min_ratio > 1 && !((double)ratio[k] >= r.min_ratio)) f = 1;
-      for (int q = 0; q < r.nval; ++q) {
-        const hh_validator& vd = r.val[q];
+      // the detection as rule -1 among the extra validators, so that its code is
+      // there once, and 128 registers: twice took 203, too many for the local
+      // arrays of 3 and 4 layers (500 x 400 cells: 1806 and 5588 us instead of
+      // 1098 and 3754; 2 layers 35 and 37)
+#pragma unroll 1
+      for (int q = r.uod ? -1 : 0; q < r.nval; ++q) {
+        const hh_validator vd = q < 0 ? hh_validator{HH_VAL_UOD, r.uod_nb, r.uod_thr, 0, 0, 0.1} : r.val[q];
         if (vd.kind == HH_VAL_PEAK_RATIO) {
           if (!((double)ratio[k] >= vd.threshold)) f = 1;
         } else if (vd.kind == HH_VAL_MOMENT) {
@@ -117,19 +121,22 @@ cudaError_t launch_flags(const float* u, const float* v, const float* ratio, con
   return cudaGetLastError();
 }
 
-__global__ void __launch_bounds__(128, 3) substitute_kernel(float* u, float* v, const uint8_t* outl_in, uint8_t* outl_out, const uint8_t* gmask,
-                                  const float* alt_u, const float* alt_v, int32_t nalt, int32_t ny, int32_t nx,
-                                  int32_t er, double thr) {
+template <bool WIDE>
+__global__ void __launch_bounds__(128, WIDE ? 12 : 3)
+    substitute_kernel(float* u, float* v, const uint8_t* outl_in, uint8_t* outl_out, const uint8_t* gmask,
+                      const float* alt_u, const float* alt_v, int32_t nalt, int32_t ny, int32_t nx, int32_t er,
+                      double thr) {
   GRID_STRIDE(k, (int64_t)ny * nx)
-  outl_out[k] = substitute_cell(u, v, outl_in, gmask, alt_u, alt_v, nalt, ny, nx, (int)(k % ny), (int)(k / ny), er, thr);
+  outl_out[k] = substitute_cell<WIDE>(u, v, outl_in, gmask, alt_u, alt_v, nalt, ny, nx, (int)(k % ny), (int)(k / ny), er, thr);
 }
 
 cudaError_t launch_substitute(float* u, float* v, const uint8_t* outl_in, uint8_t* outl_out, const uint8_t* gmask,
                               const float* alt_u, const float* alt_v, int32_t nalt, int32_t ny, int32_t nx, int32_t er,
                               double thr, cudaStream_t s) {
   if (er < 1 || (2 * er + 1) * (2 * er + 1) - 1 > UOD_MAXN) return cudaErrorInvalidValue;
-  substitute_kernel<<<grid_blocks((int64_t)ny * nx, 128), 128, 0, s>>>(u, v, outl_in, outl_out, gmask, alt_u, alt_v,
-                                                                       nalt, ny, nx, er, thr);
+  const int blocks = grid_blocks((int64_t)ny * nx, 128);
+  if (er > 2) substitute_kernel<true><<<blocks, 128, 0, s>>>(u, v, outl_in, outl_out, gmask, alt_u, alt_v, nalt, ny, nx, er, thr);
+  else substitute_kernel<false><<<blocks, 128, 0, s>>>(u, v, outl_in, outl_out, gmask, alt_u, alt_v, nalt, ny, nx, er, thr);
   return cudaGetLastError();
 }
 

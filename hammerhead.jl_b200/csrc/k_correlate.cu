@@ -18,8 +18,11 @@ namespace hh {
 // 200 KB, 256 x 256 and larger). The scan's threads walk neighbouring columns,
 // so the stride is odd: with one of 32, 64 or 128 floats a warp's 32 columns
 // meet in one bank (0.29 ms for 961 planes of 128 x 128 against 0.09, 0.32
-// ms for 16129 of 32 x 32 against 0.17).
-__global__ void __launch_bounds__(128) analyze_planes_kernel(const AnalyzeArgs a, int lds) {
+// ms for 16129 of 32 x 32 against 0.17). The copy runs through the plane in
+// order, all threads at work whatever its rows, and 64 registers leave 8 CTAs
+// per SM: 10000 planes of 16 x 16 103 -> 83 us, of 32 x 32 122 -> 106 against a
+// lane per row and 72 registers.
+__global__ void __launch_bounds__(128, 8) analyze_planes_kernel(const AnalyzeArgs a, int lds) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int64_t P = (int64_t)a.nr * a.nc;
   float* R = reinterpret_cast<float*>(smem_raw);
@@ -29,12 +32,22 @@ __global__ void __launch_bounds__(128) analyze_planes_kernel(const AnalyzeArgs a
   const int K = a.npeaks > 2 ? a.npeaks : 2;
   PeakOut po{a.du, a.dv, a.ratio, a.moment, a.alt_u, a.alt_v, a.nalt, a.G, a.packed, a.locs};
   const ScanPlan sp = scan_plan(threadIdx.x, 128, 0, a.nr - 1, 0, a.nc - 1);
+  const int er = threadIdx.x % a.nr, ec = threadIdx.x / a.nr, sr = 128 % a.nr, sc = 128 / a.nr;
   for (int64_t pl = blockIdx.x; pl < a.nplanes; pl += gridDim.x) {
     const float* Rp = a.planes + pl * P;
     if (lds) {
-      for (int r = threadIdx.x & 31; r < a.nr; r += 32)
+      // element e of the plane at (e % nr, e / nr), by running indices
+      int r = er, c = ec;
 #pragma unroll 8
-        for (int c = threadIdx.x >> 5; c < a.nc; c += 4) R[c * lds + r] = __ldg(Rp + c * a.nr + r);
+      for (int e = threadIdx.x; e < P; e += 128) {
+        R[c * lds + r] = __ldg(Rp + e);
+        r += sr;
+        c += sc;
+        if (r >= a.nr) {
+          r -= a.nr;
+          ++c;
+        }
+      }
       Rp = R;
     }
     __syncthreads();

@@ -47,7 +47,7 @@ static unsigned rnd = 7;
 static float noise() { rnd = rnd * 1664525u + 1013904223u; return (float)(rnd >> 8) / 16777216.f; }
 int main() {
   int bad = 0;
-  for (int er = 1; er <= 2; ++er)
+  for (int er = 1; er <= 4; ++er)
     for (int masked = 0; masked < 2; ++masked) {
       const int ny = 37, nx = 41, G = ny * nx, nt = 8;
       std::vector<float> u(G), v(G), au(G), av(G);
@@ -70,7 +70,8 @@ int main() {
           for (auto& x : t) x.join();
         };
         cells([&](int k) {
-          o[k] = hh::substitute_cell(uu.data(), vv.data(), flags.data(), m, au.data(), av.data(), 1, ny, nx, k % ny, k / ny, er, 2.0);
+          auto cell = er > 2 ? hh::substitute_cell<true> : hh::substitute_cell<false>;
+          o[k] = cell(uu.data(), vv.data(), flags.data(), m, au.data(), av.data(), 1, ny, nx, k % ny, k / ny, er, 2.0);
         });
         cells([&](int k) {
           if (!hh::repl_invalid(o.data(), m, k)) return;
